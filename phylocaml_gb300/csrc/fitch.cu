@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(160) fitch_tree_kernel(const FitchTreeArgs p) 
 // multiplies the warps per SM by FS_W, which a single postorder walk cannot,
 // and dealing more segments than warps keeps the warps' loads even.
 // ---------------------------------------------------------------------------
-constexpr int FS_W = 4;   // warps per CTA
-constexpr int FS_S = 8;   // segments at most
-constexpr int FS_P = 4;   // tip slices in flight per thread (a power of two)
+constexpr int FS_W = PGPU_SPLIT_WARPS;   // warps per CTA
+constexpr int FS_S = 8;                  // segments at most
+constexpr int FS_P = PGPU_SPLIT_RING;    // tip slices in flight per thread (a power of two)
 static_assert((FS_P & (FS_P - 1)) == 0, "the copy ring is indexed by a mask");
 
 // Shared-memory accesses through 32-bit shared-window addresses.
@@ -1269,9 +1269,12 @@ pgpu_status build_split(pgpu_ctx *ctx, const pgpu_tree *tree, SplitSchedule *out
   return PGPU_OK;
 }
 
+}  // namespace
+
 // the split schedule of `tree`, resident in BUF_SPLIT ({ops, seg, top, tips})
-pgpu_status split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const int4 **ops, const int4 **seg,
-                         const int4 **top, const int4 **wseg, const int32_t **tips) {
+pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitSchedule **out,
+                              const int4 **ops, const int4 **seg, const int4 **top, const int4 **wseg,
+                              const int32_t **tips) {
   const int32_t n_int = tree->n_tips - 1;
   const bool hit = ctx->split_valid && (int32_t)ctx->split_left.size() == n_int &&
                    std::memcmp(ctx->split_left.data(), tree->left, n_int * 4) == 0 &&
@@ -1307,8 +1310,11 @@ pgpu_status split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const int4 **ops,
   *top = *seg + sp.seg.size();
   *wseg = *top + sp.top.size();
   *tips = reinterpret_cast<const int32_t *>(*wseg + sp.wseg.size());
+  *out = &sp;
   return PGPU_OK;
 }
+
+namespace {
 
 template <class Op>
 cudaError_t launch_split(cudaStream_t stream, const FitchSplitArgs &a, size_t tiles) {
@@ -1422,11 +1428,12 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
   if (!tree || tree->n_tips < 2) return pgpu_set_err(ctx, PGPU_ERR_ARG, "fitch_tree: need at least 2 tips");
   if (lb == 64) return tree64_dev(ctx, tree, tips, ld, weights, n_sites, node_sets, site_cost, total);
   FitchSplitArgs a;
-  PGPU_TRY(split_device(ctx, tree, &a.ops, &a.seg, &a.top, &a.wseg, &a.tip_seq));
+  const SplitSchedule *spp;
+  PGPU_TRY(pgpu_split_device(ctx, tree, &spp, &a.ops, &a.seg, &a.top, &a.wseg, &a.tip_seq));
   cudaStream_t s = ctx->stream;
   PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(uint64_t), s));
   if (n_words == 0) return PGPU_OK;
-  const SplitSchedule &sp = ctx->split;
+  const SplitSchedule &sp = *spp;
   a.tips = tips;
   a.weights = weights;
   a.node_sets = node_sets;
@@ -1491,8 +1498,9 @@ pgpu_status pgpu_tcm_tree_split(pgpu_ctx *ctx, const pgpu_tree *tree, const uint
   if (ld % 4 != 0 || ld > 0xffffffffull) return PGPU_OK;
   const size_t n_words = (n_sites + 7) / 8;
   FitchSplitArgs a;
-  PGPU_TRY(split_device(ctx, tree, &a.ops, &a.seg, &a.top, &a.wseg, &a.tip_seq));
-  const SplitSchedule &sp = ctx->split;
+  const SplitSchedule *spp;
+  PGPU_TRY(pgpu_split_device(ctx, tree, &spp, &a.ops, &a.seg, &a.top, &a.wseg, &a.tip_seq));
+  const SplitSchedule &sp = *spp;
   if (split_smem<TcmOp<false>>(sp.rows, false) > ctx->smem_optin) return PGPU_OK;
   a.tips = tips;
   a.weights = weights;

@@ -173,6 +173,15 @@ pgpu_status pgpu_build_schedule(pgpu_ctx *ctx, const pgpu_tree *tree, TreeSchedu
 pgpu_status pgpu_schedule_device(pgpu_ctx *ctx, const pgpu_tree *tree, const TreeSchedule **sch,
                                  const int4 **d_ops, const int32_t **d_tip_seq);
 
+// Shape of the segmented schedule: warps per CTA, rows of the tip-copy ring
+// counted in SplitSchedule::rows, and joining nodes at most.
+constexpr int PGPU_SPLIT_WARPS = 4, PGPU_SPLIT_RING = 4, PGPU_SPLIT_JOINS = PGPU_SPLIT_WARPS * PGPU_SPLIT_RING;
+// Builds (or reuses) the segment schedule of `tree` and makes it resident on
+// the device (fitch.cu).
+pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitSchedule **out,
+                              const int4 **ops, const int4 **seg, const int4 **top, const int4 **wseg,
+                              const int32_t **tips);
+
 // The cost-matrix postorder on the Fitch kernel's segmented schedule
 // (fitch.cu); *launched is false when the tree does not fit its shared
 // memory.

@@ -136,167 +136,258 @@ __global__ void __launch_bounds__(TC_THREADS) tcm_tree_kernel(const TcmArgs a) {
 // ---- wide alphabets: medians formed on the fly ----------------------------
 // For alphabets of up to 32 atomic states (codes of 8, 16 or 32 bits, one
 // site per lane) a table over every pair of codes no longer fits, so each
-// node forms its medians from the TCM itself, held transposed in shared
-// memory (tT[k][x] = tcm[x][k]).  find_median_general / _metric
-// (lib/costMatrix.ml:68-86, 104-122) take, over every atomic pair (a, b) of
-// the two codes, the candidates k minimising tcm[a][k] + tcm[b][k], and keep
-// the pairs reaching the overall minimum.  That is the same as
+// node forms its medians from the TCM itself, one row per atomic state in
+// shared memory.  find_median_general / _metric (lib/costMatrix.ml:68-86,
+// 104-122) take, over every atomic pair (a, b) of the two codes, the
+// candidates k minimising tcm[a][k] + tcm[b][k], and keep the pairs reaching
+// the overall minimum.  That is the same as
 //   best = min_k (C_i[k] + C_j[k]),  C_i[k] = min_{a in i} tcm[a][k],
 //   code = OR of the k reaching it,
 // over all k (general) or the states of i | j (metric): a pair's minimum is
 // never below best, and reaches it exactly where some k does.
 // find_median_equal (:89-101) intersects at tcm[0][0] or unites at
-// tcm[0][1].  A TCM declared symmetric has its table filled for i <= j and
-// mirrored (:150-156), so the codes are ordered first.
+// tcm[0][1].  All three are symmetric in i and j, so a TCM declared
+// symmetric (its table filled for i <= j and mirrored, :150-156) needs no
+// ordering of the codes.
+//
+// tcm_wide_kernel walks the segmented schedule of the Fitch kernel (four
+// warps per CTA, each its own subtrees of the same 32 sites, a site per
+// lane), so a warp's chain is a quarter of the postorder and 20,000 sites
+// give 2,500 warps instead of 625.  C_i is built a whole row at a time: one
+// 16-byte shared load and packed minima per 4 words for every state of the
+// code, instead of a scalar search per candidate k.  With every cost at most
+// 16,383 a word holds two states as 16-bit halves (j and j + W), so a sum of
+// two costs stays below the padding's 2 x 0x7fff; larger costs take a word
+// per state.  A row for the code "every state" (missing data) makes that
+// code as short as a single state.  The row stride is an odd multiple of 16
+// bytes, so the rows of 8 lanes' 16-byte loads fall in distinct banks.
+// Bound by instruction issue (the per-state minima and sums), not by memory.
+// 128 taxa x 20,003 sites of 20 states, metric rule: 65 us a call against
+// 1,252 us with one thread per word searching the candidates one by one.
 struct TcmWideArgs {
   const uint32_t *tips;      // [n_tips][ld] lanes of LB bits
   const uint32_t *weights;   // [n_sites] or null
-  const uint32_t *tcmT;      // [S][S] transposed costs
-  const int4 *ops;
+  const uint32_t *rows;      // [S + 1][row stride] packed costs, the last row "every state"
+  const int4 *ops, *seg, *top, *wseg;
   uint32_t *node_sets;
   uint32_t *site_cost;
   unsigned long long *total;
   int *flag;
   size_t ld, n_words, n_sites;
-  int n_tips, n_ops, depth, S, mode, symmetric;
+  int n_tips, n_top, depth, S, mode;
+  uint32_t equal, unequal;   // the equal rule's costs tcm[0][0], tcm[0][1]
 };
 
-template <int LB>
-__device__ __forceinline__ uint32_t wide_median(const uint32_t *tT, int S, int mode, int sym,
-                                                uint32_t a, uint32_t b, uint32_t &cost,
-                                                bool &none) {
-  const uint32_t all = S == 32 ? 0xffffffffu : (1u << S) - 1u;
-  if (a == 0u || b == 0u || (a & ~all) || (b & ~all)) {
-    none = true;
-    cost = 0;
-    return 0u;
-  }
-  if (sym && a > b) {
-    const uint32_t t = a;
-    a = b;
-    b = t;
-  }
-  if (mode == PGPU_TCM_EQUAL) {
-    const uint32_t inter = a & b;
-    cost = inter ? tT[0] : tT[1 * S + 0];   // tcm[0][0] or tcm[0][1]
-    return inter ? inter : (a | b);
-  }
-  const uint32_t cand = mode == PGPU_TCM_METRIC ? (a | b) : all;
-  uint32_t best = 0xffffffffu, code = 0u;
-  for (int k = 0; k < S; ++k) {
-    if (!((cand >> k) & 1u)) continue;
-    const uint32_t *row = tT + k * S;
-    uint32_t ca = 0xffffffffu, cb = 0xffffffffu;
-    for (uint32_t m = a; m; m &= m - 1) ca = min(ca, row[__ffs(m) - 1]);
-    for (uint32_t m = b; m; m &= m - 1) cb = min(cb, row[__ffs(m) - 1]);
-    const uint32_t c = ca + cb;
-    if (c < best) {
-      best = c;
-      code = 1u << k;
-    } else if (c == best) {
-      code |= 1u << k;
+// words from one packed row to the next: an odd number of 16-byte units
+__host__ __device__ constexpr int wide_stride(int W) { return W % 8 == 0 ? W + 4 : W; }
+
+constexpr uint32_t TW_PAD16 = 0x7fffu;       // a state that does not exist, 16-bit costs
+constexpr uint32_t TW_PAD32 = 0x3fffffffu;   // ... and 32-bit costs
+constexpr int32_t TW_MAX16 = 0x3fff;         // largest cost of the 16-bit form
+
+// C[k] = min over the states s of `code` of row s, in W packed words
+template <int W, bool U16>
+__device__ __forceinline__ void wide_min_rows(const uint32_t *rows, int S, uint32_t all, uint32_t code,
+                                              uint32_t (&c)[W]) {
+  auto load = [&](int s, uint32_t (&r)[W]) {
+    const uint4 *q = reinterpret_cast<const uint4 *>(rows + s * wide_stride(W));
+#pragma unroll
+    for (int j = 0; j < W / 4; ++j) {
+      const uint4 v = q[j];
+      r[4 * j] = v.x, r[4 * j + 1] = v.y, r[4 * j + 2] = v.z, r[4 * j + 3] = v.w;
     }
+  };
+  const bool every = code == all;
+  load(every ? S : __ffs(code) - 1, c);
+  for (uint32_t m = every ? 0u : code & (code - 1u); m; m &= m - 1u) {
+    uint32_t r[W];
+    load(__ffs(m) - 1, r);
+#pragma unroll
+    for (int j = 0; j < W; ++j) c[j] = U16 ? __vminu2(c[j], r[j]) : min(c[j], r[j]);
   }
-  cost = best;
-  return code;
 }
 
-template <int LB>
-__global__ void __launch_bounds__(TC_THREADS) tcm_wide_kernel(const TcmWideArgs a) {
+// the median of codes a and b; none is set (and the code is 0) where the
+// pair has no median
+template <int W, bool U16>
+__device__ __forceinline__ uint32_t wide_median(const TcmWideArgs &p, const uint32_t *rows, uint32_t all,
+                                                uint32_t a, uint32_t b, uint32_t &cost, bool &none) {
+  const bool bad = a == 0u || b == 0u || ((a | b) & ~all);
+  none |= bad;
+  if (p.mode == PGPU_TCM_EQUAL) {
+    const uint32_t inter = a & b;
+    cost = bad ? 0u : inter ? p.equal : p.unequal;
+    return bad ? 0u : inter ? inter : (a | b);
+  }
+  if (bad) a = b = 1u;
+  const uint32_t cand = p.mode == PGPU_TCM_METRIC ? (a | b) : all;
+  uint32_t s[W], t[W];
+  wide_min_rows<W, U16>(rows, p.S, all, a, s);
+  wide_min_rows<W, U16>(rows, p.S, all, b, t);
+  uint32_t best, code;
+  if (U16) {
+    // sums of states outside the candidates become 0xffff in their half
+    const uint32_t out = ~cand;
+    const uint32_t out2 = (out & ((1u << W) - 1u)) | ((out >> W) << 16);
+    best = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      s[j] = (s[j] + t[j]) | (((out2 >> j) & 0x00010001u) * 0xffffu);
+      best = __vminu2(best, s[j]);
+    }
+    best = min(best & 0xffffu, best >> 16);
+    const uint32_t best2 = best * 0x00010001u;
+    // 0 in a half that reaches best, else 1 (no half is below best)
+    uint32_t off = 0u;
+#pragma unroll
+    for (int j = 0; j < W; ++j) off |= __vminu2(s[j] - best2, 0x00010001u) << j;
+    code = (~off & ((1u << W) - 1u)) | ((~off >> 16) << W);
+  } else {
+    best = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      s[j] += t[j];
+      if (!((cand >> j) & 1u)) s[j] = 0xffffffffu;
+      best = min(best, s[j]);
+    }
+    code = 0u;
+#pragma unroll
+    for (int j = 0; j < W; ++j) code |= s[j] == best ? 1u << j : 0u;
+  }
+  cost = bad ? 0u : best;
+  return bad ? 0u : code & cand;
+}
+
+template <int LB> struct WideLane;
+template <> struct WideLane<8> { using T = uint8_t; };
+template <> struct WideLane<16> { using T = uint16_t; };
+template <> struct WideLane<32> { using T = uint32_t; };
+
+template <int LB, int W, bool U16>
+__global__ void __launch_bounds__(PGPU_SPLIT_WARPS * 32) tcm_wide_kernel(const TcmWideArgs p) {
+  using T = typename WideLane<LB>::T;
   constexpr int PER = 32 / LB;
-  constexpr uint32_t LMASK = LB == 32 ? 0xffffffffu : (1u << LB) - 1u;
-  __shared__ uint32_t tT[32 * 32];
-  __shared__ unsigned long long red[TC_THREADS / 32];
-  extern __shared__ uint32_t stk[];   // [depth][TC_THREADS]
-  const int t = threadIdx.x, lane = t & 31;
-  for (int i = t; i < a.S * a.S; i += TC_THREADS) tT[i] = __ldg(a.tcmT + i);
+  extern __shared__ __align__(16) uint32_t wsm[];
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int n_row = (p.S + 1) * wide_stride(W);
+  uint32_t *rows = wsm;
+  uint32_t *stk0 = wsm + n_row + (size_t)w * p.depth * 32 + lane;   // this lane's column
+  uint32_t *join = wsm + n_row + (size_t)PGPU_SPLIT_WARPS * p.depth * 32 + lane;
+  uint32_t *sitecnt = wsm + n_row + (size_t)(PGPU_SPLIT_WARPS * p.depth + PGPU_SPLIT_JOINS) * 32;
+  for (int i = tid; i < n_row; i += PGPU_SPLIT_WARPS * 32) rows[i] = __ldg(p.rows + i);
+  if (tid < 32) sitecnt[tid] = 0u;
   __syncthreads();
-  const size_t w = (size_t)blockIdx.x * TC_THREADS + t;
-  const bool on = w < a.n_words;
+  const uint32_t all = p.S == 32 ? 0xffffffffu : (1u << p.S) - 1u;
+  const size_t site = (size_t)blockIdx.x * 32 + lane;
+  const bool in = site < p.n_words * PER;   // the lane's place exists in the rows
+  const bool valid = site < p.n_sites;
   // lanes past the last site read as atomic state 0, which always has a
   // median, and are written as zero
-  uint32_t valid = 0u;
-  if (on) {
-#pragma unroll
-    for (int l = 0; l < PER; ++l)
-      if (w * PER + l < a.n_sites) valid |= LMASK << (l * LB);
-  }
-  uint32_t fill = 0u;
-#pragma unroll
-  for (int l = 0; l < PER; ++l) fill |= 1u << (l * LB);
-  fill &= ~valid;
-  auto tip = [&](int ch) -> uint32_t {
-    const uint32_t x = on ? __ldg(a.tips + (size_t)ch * a.ld + w) : 0u;
-    return (x & valid) | fill;
+  const T *col = reinterpret_cast<const T *>(p.tips) + site;
+  T *out = reinterpret_cast<T *>(p.node_sets) + site;
+  const size_t ldt = p.ld * PER;
+  auto tip = [&](int ch) -> uint32_t { return valid ? (uint32_t)__ldg(col + (size_t)ch * ldt) : 1u; };
+  auto put = [&](int k, uint32_t m) {
+    if (in) out[(size_t)k * ldt] = (T)(valid ? m : 0u);
   };
-  uint32_t cnt[PER];
-#pragma unroll
-  for (int l = 0; l < PER; ++l) cnt[l] = 0;
-  uint32_t top = 0;
-  int sp = 0;
-  bool ok = true, none = false;
-  for (int i = 0; i < a.n_ops && ok; ++i) {
-    const int4 op = __ldg(a.ops + i);
-    const int kind = (op.y >= a.n_tips ? 1 : 0) | (op.z >= a.n_tips ? 2 : 0);
-    uint32_t xa, xb;
-    if (kind == 0) {
-      if (i > 0) {
-        if (sp < a.depth) stk[sp++ * TC_THREADS + t] = top;
-        else ok = false;
-      }
-      xa = tip(op.y);
-      xb = tip(op.z);
-    } else if (kind == 1) {
-      xa = top;
-      xb = tip(op.z);
-    } else if (kind == 2) {
-      xa = tip(op.y);
-      xb = top;
-    } else {
-      if (sp > 0) {
-        xa = stk[--sp * TC_THREADS + t];
+  uint32_t acc = 0;
+  bool none = false;
+
+  // ---- each warp walks its segments ----
+  const int4 ws = p.wseg[w];
+  for (int q = 0; q < ws.y; ++q) {
+    const int4 sg = p.seg[ws.x + q];   // {op_off, n_ops, tip_off, n_tips}
+    uint32_t *stk = stk0 + (q + 1) * 32;   // rows below hold earlier results
+    const int4 *ops = p.ops + sg.x;
+    int4 op = __ldg(ops);
+    // a step's tips are loaded one step ahead, so their latency passes
+    // while the step before is computed
+    uint32_t ta = op.y < p.n_tips ? tip(op.y) : 0u, tb = op.z < p.n_tips ? tip(op.z) : 0u;
+    uint32_t top = 0;
+    int sp = 0;
+    for (int i = 0; i < sg.y; ++i) {
+      const int4 next = i + 1 < sg.y ? __ldg(ops + i + 1) : op;
+      uint32_t na = 0u, nb = 0u;
+      if (next.y < p.n_tips) na = tip(next.y);
+      if (next.z < p.n_tips) nb = tip(next.z);
+      const bool a_tip = op.y < p.n_tips, b_tip = op.z < p.n_tips;
+      uint32_t x = ta, y = tb;
+      if (a_tip && b_tip) {   // the previous result waits on the stack
+        if (i > 0) stk[32 * sp++] = top;
+      } else if (a_tip) {
+        y = top;
       } else {
-        ok = false;
-        xa = fill;
+        x = b_tip ? top : stk[32 * --sp];
+        if (!b_tip) y = top;
       }
-      xb = top;
-    }
-    uint32_t out = 0;
-#pragma unroll
-    for (int l = 0; l < PER; ++l) {
       uint32_t c;
-      bool nm = false;
-      const uint32_t m = wide_median<LB>(tT, a.S, a.mode, a.symmetric, (xa >> (l * LB)) & LMASK,
-                                         (xb >> (l * LB)) & LMASK, c, nm);
-      out |= m << (l * LB);
-      cnt[l] += c;
-      none |= nm;
+      top = wide_median<W, U16>(p, rows, all, x, y, c, none);
+      acc += c;
+      put(op.x, top);
+      op = next, ta = na, tb = nb;
     }
-    out = (out & valid) | fill;
-    if (on) a.node_sets[(size_t)op.x * a.ld + w] = out & valid;
-    top = out;
+    stk0[q * 32] = top;
   }
-  unsigned long long tot = 0;
-  if (on && ok) {
-#pragma unroll
-    for (int l = 0; l < PER; ++l) {
-      const size_t s = w * PER + l;
-      if (s < a.n_sites) {
-        if (a.site_cost) a.site_cost[s] = cnt[l];
-        tot += (unsigned long long)(a.weights ? __ldg(a.weights + s) : 1u) * cnt[l];
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if (lane == 0) red[t >> 5] = tot;
-  if (__any_sync(0xffffffffu, none) && lane == 0) atomicOr(a.flag, PGPU_FLAG_BADCODE);
-  if (!ok) atomicOr(a.flag, PGPU_FLAG_BADCODE);
   __syncthreads();
-  if (t == 0) {
-    unsigned long long s2 = 0;
-    for (int k = 0; k < TC_THREADS / 32; ++k) s2 += red[k];
-    if (s2) atomicAdd(a.total, s2);
+  // ---- warp 0 joins the segments ----
+  if (w == 0)
+    for (int i = 0; i < p.n_top; ++i) {
+      const int4 op = __ldg(p.top + i);
+      uint32_t ch[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int ref = h == 0 ? op.y : op.z;
+        if (ref >= 0) ch[h] = tip(ref);
+        else if (ref > -1000)
+          ch[h] = wsm[n_row + ((size_t)((-1 - ref) >> 5) * p.depth + ((-1 - ref) & 31)) * 32 + lane];
+        else ch[h] = join[32 * (-1000 - ref)];
+      }
+      uint32_t c;
+      const uint32_t m = wide_median<W, U16>(p, rows, all, ch[0], ch[1], c, none);
+      acc += c;
+      put(op.x, m);
+      join[32 * i] = m;
+    }
+  atomicAdd(sitecnt + lane, acc);
+  if (__any_sync(0xffffffffu, none) && lane == 0) atomicOr(p.flag, PGPU_FLAG_BADCODE);
+  __syncthreads();
+  if (w == 0) {
+    const uint32_t v = sitecnt[lane];
+    unsigned long long tot = 0;
+    if (valid) {
+      if (p.site_cost) p.site_cost[site] = v;
+      tot = (unsigned long long)(p.weights ? __ldg(p.weights + site) : 1u) * v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    if (lane == 0 && tot) atomicAdd(p.total, tot);
+  }
+}
+
+template <int LB, int W, bool U16>
+cudaError_t launch_wide(const TcmWideArgs &a, size_t smem, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(tcm_wide_kernel<LB, W, U16>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)std::max<size_t>(smem, 48 * 1024));
+  if (e != cudaSuccess) return e;
+  const size_t grid = (a.n_words * (32 / LB) + 31) / 32;
+  tcm_wide_kernel<LB, W, U16><<<(unsigned)grid, PGPU_SPLIT_WARPS * 32, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+// W: packed words per row, the smallest multiple of 4 (16-bit halves) or of
+// 8 (32-bit) that holds the states
+template <bool U16>
+cudaError_t launch_wide_lb(int lb, int W, const TcmWideArgs &a, size_t smem, cudaStream_t s) {
+  constexpr int U = U16 ? 4 : 8;
+  if (lb == 8) return launch_wide<8, U, U16>(a, smem, s);
+  if (lb == 16)
+    return W == U ? launch_wide<16, U, U16>(a, smem, s) : launch_wide<16, 2 * U, U16>(a, smem, s);
+  switch (W / U) {
+    case 1: return launch_wide<32, U, U16>(a, smem, s);
+    case 2: return launch_wide<32, 2 * U, U16>(a, smem, s);
+    case 3: return launch_wide<32, 3 * U, U16>(a, smem, s);
+    default: return launch_wide<32, 4 * U, U16>(a, smem, s);
   }
 }
 
@@ -456,23 +547,35 @@ pgpu_status tree_wide_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *
   const size_t n_words = (n_sites + per - 1) / per;
   if (ld < n_words)
     return pgpu_set_err(ctx, PGPU_ERR_ARG, "tcm_tree_wide: ld_words (%zu) < %zu", ld, n_words);
-  const TreeSchedule *sch;
-  const int4 *d_ops;
+  TcmWideArgs a{};
   const int32_t *d_seq;
-  PGPU_TRY(pgpu_schedule_device(ctx, tree, &sch, &d_ops, &d_seq));
+  const SplitSchedule *sp;
+  PGPU_TRY(pgpu_split_device(ctx, tree, &sp, &a.ops, &a.seg, &a.top, &a.wseg, &d_seq));
+  // the packed rows: row x holds tcm[x][k] for every k, row S their minima
+  const bool u16 = emax <= TW_MAX16;
+  const int unit = u16 ? 4 : 8;
+  const int W = ((u16 ? (S + 1) / 2 : S) + unit - 1) / unit * unit, stride = wide_stride(W);
+  const size_t n_row = (size_t)(S + 1) * stride;
   void *h, *d;
-  PGPU_TRY(pgpu_stage(ctx, (size_t)S * S * sizeof(uint32_t), &h, &d));
-  uint32_t *tT = static_cast<uint32_t *>(h);
-  for (int x = 0; x < S; ++x)
-    for (int k = 0; k < S; ++k) tT[k * S + x] = (uint32_t)tcm[x * S + k];
-  PGPU_TRY(pgpu_stage_commit(ctx, (size_t)S * S * sizeof(uint32_t)));
+  PGPU_TRY(pgpu_stage(ctx, n_row * sizeof(uint32_t), &h, &d));
+  uint32_t *rows = static_cast<uint32_t *>(h);
+  for (int x = 0; x <= S; ++x)
+    for (int j = 0; j < stride; ++j) {
+      auto cost = [&](int k) -> uint32_t {
+        if (j >= W || k >= S) return u16 ? TW_PAD16 : TW_PAD32;
+        if (x < S) return (uint32_t)tcm[x * S + k];
+        int32_t c = tcm[k];
+        for (int y = 1; y < S; ++y) c = std::min(c, tcm[y * S + k]);
+        return (uint32_t)c;
+      };
+      rows[(size_t)x * stride + j] = u16 ? cost(j) | cost(j + W) << 16 : cost(j);
+    }
+  PGPU_TRY(pgpu_stage_commit(ctx, n_row * sizeof(uint32_t)));
   PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
   if (n_words == 0) return PGPU_OK;
-  TcmWideArgs a;
   a.tips = tips;
   a.weights = weights;
-  a.tcmT = static_cast<const uint32_t *>(d);
-  a.ops = d_ops;
+  a.rows = static_cast<const uint32_t *>(d);
   a.node_sets = node_sets;
   a.site_cost = site_cost;
   a.total = total;
@@ -481,31 +584,21 @@ pgpu_status tree_wide_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *
   a.n_words = n_words;
   a.n_sites = n_sites;
   a.n_tips = tree->n_tips;
-  a.n_ops = (int)sch->ops.size();
-  a.depth = std::max(sch->max_depth, 1);
+  a.n_top = (int)sp->top.size();
+  a.depth = sp->rows - PGPU_SPLIT_RING;   // the kernel keeps no copy ring
   a.S = S;
   a.mode = mode;
-  a.symmetric = symmetric ? 1 : 0;
-  const size_t smem = (size_t)a.depth * TC_THREADS * sizeof(uint32_t);
-  if (smem + sizeof(uint32_t) * 32 * 32 > (size_t)ctx->smem_optin)
+  a.equal = (uint32_t)tcm[0];
+  a.unequal = S > 1 ? (uint32_t)tcm[1] : 0u;
+  const size_t smem =
+      (n_row + ((size_t)PGPU_SPLIT_WARPS * a.depth + PGPU_SPLIT_JOINS + 1) * 32) * sizeof(uint32_t);
+  if (smem > (size_t)ctx->smem_optin)
     return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "tcm_tree_wide: tree too deep (%d stack entries)",
                         a.depth);
-  const unsigned grid = (unsigned)((n_words + TC_THREADS - 1) / TC_THREADS);
-  cudaError_t e = cudaSuccess;
-  switch (lb) {
-    case 8:
-      e = cudaFuncSetAttribute(tcm_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) tcm_wide_kernel<8><<<grid, TC_THREADS, smem, ctx->stream>>>(a);
-      break;
-    case 16:
-      e = cudaFuncSetAttribute(tcm_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) tcm_wide_kernel<16><<<grid, TC_THREADS, smem, ctx->stream>>>(a);
-      break;
-    default:
-      e = cudaFuncSetAttribute(tcm_wide_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) tcm_wide_kernel<32><<<grid, TC_THREADS, smem, ctx->stream>>>(a);
-      break;
-  }
+  if ((n_words * per + 31) / 32 > 0x7fffffffu)
+    return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "tcm_tree_wide: too many sites");
+  const cudaError_t e = u16 ? launch_wide_lb<true>(lb, W, a, smem, ctx->stream)
+                            : launch_wide_lb<false>(lb, W, a, smem, ctx->stream);
   PGPU_CUDA(ctx, e);
   return pgpu_after_launch(ctx, "tcm_wide_kernel");
 }

@@ -1,4 +1,5 @@
 // Context management, error reporting and the grow-only device buffers.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -99,6 +100,42 @@ pgpu_status pgpu_copy_stream(pgpu_ctx *ctx) {
   return PGPU_OK;
 }
 
+// Pinned staging for small per-call parameters, so that no call waits for the
+// stream: PGPU_STAGES blocks take turns, and a block is refilled once the
+// copy issued from it that many uses earlier is done.
+pgpu_status pgpu_stage(pgpu_ctx *ctx, size_t bytes, void **host, void **dev) {
+  const int k = ctx->stage_next;
+  ctx->stage_next = (k + 1) % PGPU_STAGES;
+  if (ctx->stage_ev[k]) PGPU_CUDA(ctx, cudaEventSynchronize(ctx->stage_ev[k]));
+  if (ctx->stage_cap[k] < bytes) {
+    if (ctx->stage_h[k]) cudaFreeHost(ctx->stage_h[k]);
+    if (ctx->stage_d[k]) cudaFree(ctx->stage_d[k]);
+    ctx->stage_h[k] = nullptr;
+    ctx->stage_d[k] = nullptr;
+    ctx->stage_cap[k] = 0;
+    const size_t want = std::max<size_t>(bytes, 64 * 1024);
+    PGPU_CUDA(ctx, cudaMallocHost(&ctx->stage_h[k], want));
+    PGPU_CUDA(ctx, cudaMalloc(&ctx->stage_d[k], want));
+    ctx->stage_cap[k] = want;
+  }
+  if (!ctx->stage_ev[k]) PGPU_CUDA(ctx, cudaEventCreateWithFlags(&ctx->stage_ev[k], cudaEventDisableTiming));
+  *host = ctx->stage_h[k];
+  if (dev) *dev = ctx->stage_d[k];
+  ctx->stage_cur = k;
+  return PGPU_OK;
+}
+
+pgpu_status pgpu_stage_copy(pgpu_ctx *ctx, void *dst, size_t bytes) {
+  const int k = ctx->stage_cur;
+  PGPU_CUDA(ctx, cudaMemcpyAsync(dst, ctx->stage_h[k], bytes, cudaMemcpyHostToDevice, ctx->stream));
+  PGPU_CUDA(ctx, cudaEventRecord(ctx->stage_ev[k], ctx->stream));
+  return PGPU_OK;
+}
+
+pgpu_status pgpu_stage_commit(pgpu_ctx *ctx, size_t bytes) {
+  return pgpu_stage_copy(ctx, ctx->stage_d[ctx->stage_cur], bytes);
+}
+
 extern "C" {
 
 int pgpu_version(void) { return 100; }
@@ -149,7 +186,7 @@ void pgpu_destroy(pgpu_ctx *ctx) {
   for (int i = 0; i < BUF_COUNT; ++i)
     if (ctx->buf[i]) cudaFree(ctx->buf[i]);
   if (ctx->d_flag) cudaFree(ctx->d_flag);
-  for (int k = 0; k < 2; ++k) {
+  for (int k = 0; k < PGPU_STAGES; ++k) {
     if (ctx->stage_h[k]) cudaFreeHost(ctx->stage_h[k]);
     if (ctx->stage_d[k]) cudaFree(ctx->stage_d[k]);
     if (ctx->stage_ev[k]) cudaEventDestroy(ctx->stage_ev[k]);

@@ -226,11 +226,19 @@ struct Fp32 {
     y[2] = v.z;
     y[3] = v.w;
   }
-  // y[i] = x[i] + sum_j D[i][j] x[j]
-  __device__ static void rows(const Coef *D, const V *x, V *y) {
+  // a row of load_tip's layout whose 16-byte halves lie at the shared-window
+  // addresses a and b (one here)
+  __device__ static void load_row_s(uint32_t a, uint32_t, V *y) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(y[0]), "=f"(y[1]), "=f"(y[2]), "=f"(y[3]) : "r"(a) : "memory");
+  }
+  // y[i] = x[i] + sum_j D[i][j] x[j]; the 16-byte units of D lie `us` units
+  // apart (the rate classes of a branch interleaved), here and in the other
+  // forms
+  __device__ static void rows(const Coef *D, const V *x, V *y, int us = 1) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float4 d = reinterpret_cast<const float4 *>(D)[i];
+      const float4 d = reinterpret_cast<const float4 *>(D)[i * us];
       float s = d.x * x[0];
       s = fmaf(d.y, x[1], s);
       s = fmaf(d.z, x[2], s);
@@ -272,11 +280,15 @@ struct Fp64 {
     y[2] = b.x;
     y[3] = b.y;
   }
-  __device__ static void rows(const Coef *P, const V *x, V *y) {
+  __device__ static void load_row_s(uint32_t a, uint32_t b, V *y) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y[0]), "=d"(y[1]) : "r"(a) : "memory");
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y[2]), "=d"(y[3]) : "r"(b) : "memory");
+  }
+  __device__ static void rows(const Coef *P, const V *x, V *y, int us = 1) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const double2 a = reinterpret_cast<const double2 *>(P)[2 * i];
-      const double2 b = reinterpret_cast<const double2 *>(P)[2 * i + 1];
+      const double2 a = reinterpret_cast<const double2 *>(P)[2 * i * us];
+      const double2 b = reinterpret_cast<const double2 *>(P)[(2 * i + 1) * us];
       double s = a.x * x[0];
       s = fma(a.y, x[1], s);
       s = fma(b.x, x[2], s);
@@ -325,6 +337,12 @@ struct Ff32 {
     y[2] = {b.x, b.z};
     y[3] = {b.y, b.w};
   }
+  __device__ static void load_row_s(uint32_t a, uint32_t b, V *y) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(y[0].h), "=f"(y[1].h), "=f"(y[0].l), "=f"(y[1].l) : "r"(a) : "memory");
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(y[2].h), "=f"(y[3].h), "=f"(y[2].l), "=f"(y[3].l) : "r"(b) : "memory");
+  }
   // y[e] = a[e] b[e] for four elements, two per packed float2 instruction:
   // each product exact and left unnormalised, as mul
   __device__ static void mul4(const V *a, const V *b, V *y) {
@@ -349,7 +367,7 @@ struct Ff32 {
   // two rows per instruction, each lane rounded as the scalar instruction
   // would be), reading P in the P32_PAIRS_ROWS4 layout: float4 4 (i / 2) + j
   // = {hi P[i][j], hi P[i+1][j], lo P[i][j], lo P[i+1][j]}.
-  __device__ static void rows(const Coef *P, const V *x, V *y) {
+  __device__ static void rows(const Coef *P, const V *x, V *y, int us = 1) {
     const float4 *Q = reinterpret_cast<const float4 *>(P);
     const float2 m1 = make_float2(-1.0f, -1.0f);
 #pragma unroll
@@ -357,7 +375,7 @@ struct Ff32 {
       float2 sh = make_float2(0.0f, 0.0f), lo = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float4 q = Q[ip * 4 + j];
+        const float4 q = Q[(ip * 4 + j) * us];
         const float2 ph = make_float2(q.x, q.y), pl = make_float2(q.z, q.w);
         const float2 xh = make_float2(x[j].h, x[j].h), xl = make_float2(x[j].l, x[j].l);
         const float2 p = __fmul2_rn(ph, xh);

@@ -31,6 +31,7 @@ enum {
   BUF_I,
   BUF_J,
   BUF_SPLIT,
+  BUF_OPS2,
   BUF_COUNT
 };
 
@@ -64,6 +65,23 @@ struct SplitSchedule {
   std::vector<int4> top;       // {k, ref_a, ref_b, 0} in postorder
 };
 
+// A tree as the pruning kernel walks it: subtrees of up to `level` tips are
+// leaves of a reduced tree (prune.cu).
+struct PrunePlan {
+  bool valid = false;
+  int asked = 0, level = 0, R = 0, n_codes = 0, depth = 1;
+  std::vector<int32_t> left, right;   // the tree this was made from
+  std::vector<int4> ops;              // {branch of the internal first child or -1, ... second}
+  std::vector<int4> leaves;           // {tip, tip or -1, tip or -1, first row}, in reading order
+  std::vector<int4> made;             // collapsed leaves {leaf, branch, cherry's branch or -1}
+  size_t made_rows = 0;               // their rows over all rate classes
+  size_t row_bytes = 0;
+  const int4 *d_ops = nullptr, *d_leaves = nullptr, *d_made = nullptr;
+  const uint32_t *d_unit = nullptr;   // 16-byte unit of each leaf's first row
+};
+
+constexpr int PGPU_STAGES = 4;
+
 // column chunks (at most) of the host-buffer calls' copies: 2-D copies of
 // narrower columns overlap each other worse
 constexpr int PGPU_COPY_CHUNKS = 4;
@@ -90,11 +108,13 @@ struct pgpu_ctx {
   bool split_valid = false;
   std::vector<int32_t> split_left, split_right;
   SplitSchedule split;
-  // double-buffered pinned staging of small per-call parameters
-  void *stage_h[2] = {};
-  void *stage_d[2] = {};
-  size_t stage_cap[2] = {};
-  cudaEvent_t stage_ev[2] = {};
+  // the last tree pruned, as the kernel walks it (resident in BUF_OPS2)
+  PrunePlan prune_plan;
+  // pinned staging of small per-call parameters, blocks taking turns
+  void *stage_h[PGPU_STAGES] = {};
+  void *stage_d[PGPU_STAGES] = {};
+  size_t stage_cap[PGPU_STAGES] = {};
+  cudaEvent_t stage_ev[PGPU_STAGES] = {};
   int stage_next = 0, stage_cur = 0;
   // words of a state-set row per CTA of the Fitch tree kernel (0: picked
   // per launch)
@@ -158,10 +178,12 @@ pgpu_status pgpu_after_launch(pgpu_ctx *ctx, const char *what);
 pgpu_status pgpu_check_flag(pgpu_ctx *ctx, const char *what);
 // Pinned host block and its device twin for `bytes` of small parameters;
 // fill *host, then pgpu_stage_commit copies it on the context's stream.
-// Two blocks alternate, so the host only waits for the copy issued two
-// calls earlier.
+// PGPU_STAGES blocks take turns, so the host only waits for the copy issued
+// that many uses earlier.  pgpu_stage_copy copies the block to dst instead
+// of its twin.
 pgpu_status pgpu_stage(pgpu_ctx *ctx, size_t bytes, void **host, void **dev);
 pgpu_status pgpu_stage_commit(pgpu_ctx *ctx, size_t bytes);
+pgpu_status pgpu_stage_copy(pgpu_ctx *ctx, void *dst, size_t bytes);
 
 // ---------------------------------------------------------------------------
 // tree schedule (schedule.cpp)

@@ -449,6 +449,91 @@ __global__ void __launch_bounds__(128) tip_table_kernel(const TipTabArgs p) {
   }
 }
 
+// Everything a pruning call over 4 states needs of its models before the
+// walk, in one launch: every branch's P matrices in the form's layout, and
+// the tips' rows P(t) code_tab[c], one CTA per branch and model (blockIdx.y).
+// A branch's exponentials are formed once (tip_table_kernel forms 16 times as
+// many: FP64 runs at 1/64 of the FP32 rate here): 512 taxa, 4 classes, 8 us
+// against 26 us for the two launches.  P is formed as I + U (exp(D t) - I) U^-1
+// with expm1, so the small off-diagonal entries of a short branch keep their
+// relative precision instead of being what is left of sums of order 1.
+//
+// The rate classes are interleaved in units of 16 bytes: unit k of class r of
+// a branch is at k R + r, the row of code c and class r of a tip at c R + r.
+struct DnaSetupArgs {
+  const double *U, *lam, *Ui;   // model m at 16 m, 4 m, 16 m
+  const double *t;              // [2 n_tips - 2]
+  const double *rates;          // [R]; model m at m R
+  const double *code_tab;       // [n_codes][4]
+  char *P, *rows;
+  size_t P_stride, rows_stride;
+  int R, n_tips, n_codes, precision;
+  const int *status;
+  int *flag;
+  unsigned *done;               // cleared: per model, then n_flags ints per model
+  int *row_flag;
+  int n_flags;
+};
+
+__global__ void __launch_bounds__(128) dna_setup_kernel(const DnaSetupArgs p) {
+  __shared__ double sU[16], sUi[16], e[8][4], sP[8][16];
+  const int b = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, R = p.R;
+  if (b == 0) {
+    if (tid == 0) p.done[m] = 0u;
+    for (int i = tid; i < p.n_flags; i += 128) p.row_flag[(size_t)m * p.n_flags + i] = 0;
+  }
+  if (p.status[m]) {
+    if (b == 0 && tid == 0) atomicOr(p.flag, pgpu_model_flag(p.status[m]));
+    return;
+  }
+  if (tid < 16) {
+    sU[tid] = p.U[16 * m + tid];
+    sUi[tid] = p.Ui[16 * m + tid];
+  }
+  const double *rates = p.rates + (size_t)m * R;
+  const double t = p.t[b];
+  if (tid < 4 * R) e[tid >> 2][tid & 3] = expm1(p.lam[4 * m + (tid & 3)] * rates[tid >> 2] * t);
+  __syncthreads();
+  char *P = p.P + m * p.P_stride + (size_t)b * R * (p.precision == 32 ? 64 : 128);
+  for (int o = tid; o < R * 16; o += 128) {
+    const int r = o >> 4, i = (o >> 2) & 3, j = o & 3;
+    double d = 0.0;   // P - I; the identity below an effective time of 1e-10, as in compose_kernel
+    if (t * rates[r] >= 1e-10)
+      for (int k = 0; k < 4; ++k) d = fma(sU[i * 4 + k] * e[r][k], sUi[k * 4 + j], d);
+    const double v = i == j ? 1.0 + d : d;
+    sP[r][i * 4 + j] = v;
+    if (p.precision == 64) {
+      reinterpret_cast<double *>(P)[((2 * i + (j >> 1)) * R + r) * 2 + (j & 1)] = v;
+    } else if (p.precision == 32) {
+      reinterpret_cast<float *>(P)[(i * R + r) * 4 + j] = (float)d;
+    } else {
+      // two rows at a time, {hi P[i][j], hi P[i+1][j], lo P[i][j], lo P[i+1][j]}
+      float *q = reinterpret_cast<float *>(P) + (((i >> 1) * 4 + j) * R + r) * 4 + (i & 1);
+      const float hi = (float)v;
+      q[0] = hi;
+      q[2] = (float)(v - (double)hi);
+    }
+  }
+  if (b >= p.n_tips) return;
+  __syncthreads();
+  char *rows = p.rows + m * p.rows_stride + (size_t)b * R * p.n_codes * (p.precision == 32 ? 16 : 32);
+  for (int o = tid; o < p.n_codes * R * 4; o += 128) {
+    const int i = o & 3, r = (o >> 2) % R, c = (o >> 2) / R;
+    double v = 0.0;
+    for (int j = 0; j < 4; ++j) v = fma(sP[r][i * 4 + j], p.code_tab[c * 4 + j], v);
+    if (p.precision == 64) {
+      reinterpret_cast<double *>(rows)[o] = v;
+    } else if (p.precision == 32) {
+      reinterpret_cast<float *>(rows)[o] = (float)v;
+    } else {   // element pairs first: {h0, h1, l0, l1}, {h2, h3, l2, l3}
+      float *q = reinterpret_cast<float *>(rows) + (size_t)(o >> 2) * 8 + (i >> 1) * 4 + (i & 1);
+      const float hi = (float)v;
+      q[0] = hi;
+      q[2] = (float)(v - (double)hi);
+    }
+  }
+}
+
 size_t eig_smem(int S) {
   const int N = S + (S & 1);
   return sizeof(double) * (2 * (size_t)N * LDA + N) + sizeof(int) * 2 * (size_t)N;
@@ -509,6 +594,88 @@ pgpu_status pgpu_launch_tip_table(pgpu_ctx *ctx, const double *U_dev, const doub
                                       (int)std::max<size_t>(smem, 1024)));
   tip_table_kernel<<<dim3(n_tips, R, n_models), 128, smem, ctx->stream>>>(a);
   return pgpu_after_launch(ctx, "tip_table_kernel");
+}
+
+pgpu_status pgpu_launch_dna_setup(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
+                                  const double *Ui_dev, int n_models, const double *t_dev, int n_tips,
+                                  const double *rates_dev, int R, const double *code_tab_dev, int n_codes,
+                                  int precision, void *P_dev, size_t P_stride, void *rows_dev,
+                                  size_t rows_stride, const int *status_dev, unsigned *done_dev,
+                                  int *row_flag_dev, int n_flags) {
+  DnaSetupArgs a{U_dev, lam_dev, Ui_dev, t_dev, rates_dev, code_tab_dev, (char *)P_dev, (char *)rows_dev,
+                 P_stride, rows_stride, R, n_tips, n_codes, precision, status_dev, ctx->d_flag, done_dev,
+                 row_flag_dev, n_flags};
+  dna_setup_kernel<<<dim3(2 * n_tips - 2, n_models), 128, 0, ctx->stream>>>(a);
+  return pgpu_after_launch(ctx, "dna_setup_kernel");
+}
+
+// jacobi_eig_kernel's method for one 4 x 4 matrix on the host: cyclic Jacobi
+// on B = Pi^1/2 Q Pi^-1/2, the same checks and the same stopping rule.  Its
+// 20 to 30 dependent FP64 divisions and roots take the GPU 36 us and a CPU
+// core about one.
+int pgpu_host_eig4(const double *Q, const double *pi, double *U, double *lam, double *Ui) {
+  double A[4][4], V[4][4], root[4];
+  int bad = 0;
+  for (int i = 0; i < 4; ++i) {
+    if (!std::isfinite(pi[i]) || !(pi[i] > 0.0)) bad |= 1;
+    root[i] = std::sqrt(pi[i]);
+  }
+  for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j) {
+      if (!std::isfinite(Q[4 * i + j])) bad |= 1;
+      const double v = root[i] * Q[4 * i + j] / root[j], vt = root[j] * Q[4 * j + i] / root[i];
+      if (std::fabs(v - vt) > 1e-10 * (std::fabs(v) + std::fabs(vt)) + 1e-300 && std::fabs(v - vt) > 1e-12)
+        bad |= 2;
+      A[i][j] = 0.5 * (v + vt);
+      V[i][j] = i == j ? 1.0 : 0.0;
+    }
+  if (bad) return (bad & 1) ? PGPU_ERR_NAN : PGPU_ERR_NONREVERSIBLE;
+  int status = PGPU_ERR_EIGEN;
+  for (int sweep = 0; sweep < 40; ++sweep) {
+    double off = 0.0, fro = 0.0;
+    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) {
+        fro += A[i][j] * A[i][j];
+        if (i != j) off += A[i][j] * A[i][j];
+      }
+    if (off <= 1e-34 * fro) {
+      status = 0;
+      break;
+    }
+    for (int a = 0; a < 3; ++a)
+      for (int b = a + 1; b < 4; ++b) {
+        const double apq = A[a][b];
+        if (!(std::fabs(apq) > 1e-300)) continue;
+        const double th = (A[b][b] - A[a][a]) / (2.0 * apq);
+        double t;
+        if (th == 0.0) t = 1.0;
+        else if (std::fabs(th) > 1e150) t = 0.5 / th;
+        else t = std::copysign(1.0, th) / (std::fabs(th) + std::sqrt(th * th + 1.0));
+        const double c = 1.0 / std::sqrt(t * t + 1.0), s = t * c;
+        for (int j = 0; j < 4; ++j) {
+          const double x = A[a][j], y = A[b][j];
+          A[a][j] = c * x - s * y;
+          A[b][j] = s * x + c * y;
+        }
+        for (int i = 0; i < 4; ++i) {
+          const double x = A[i][a], y = A[i][b];
+          A[i][a] = c * x - s * y;
+          A[i][b] = s * x + c * y;
+          const double u = V[i][a], v = V[i][b];
+          V[i][a] = c * u - s * v;
+          V[i][b] = s * u + c * v;
+        }
+        A[a][b] = A[b][a] = 0.0;
+      }
+  }
+  for (int i = 0; i < 4; ++i) {
+    lam[i] = A[i][i];
+    for (int j = 0; j < 4; ++j) {
+      U[4 * i + j] = V[i][j] / root[i];
+      Ui[4 * i + j] = V[j][i] * root[j];
+    }
+  }
+  return status;
 }
 
 // ---------------------------------------------------------------------------

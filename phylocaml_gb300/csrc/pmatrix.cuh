@@ -45,3 +45,19 @@ pgpu_status pgpu_launch_tip_table(pgpu_ctx *ctx, const double *U_dev, const doub
                                   const double *rates_dev, int R, const double *code_tab_dev,
                                   int n_codes, void *out_dev, int form, const int *status_dev,
                                   int n_models = 1, size_t model_bytes = 0);
+
+// The setup of a pruning call over 4 states in one launch (dna_setup_kernel):
+// the P matrices of the 2 n_tips - 2 branches and the tips' rows, rate
+// classes interleaved, for the form `precision` (32: P - I, 48: float pairs,
+// 64: double), model m at P_stride and rows_stride bytes.  Clears done_dev[m]
+// and row_flag_dev[m][n_flags].
+pgpu_status pgpu_launch_dna_setup(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
+                                  const double *Ui_dev, int n_models, const double *t_dev, int n_tips,
+                                  const double *rates_dev, int R, const double *code_tab_dev, int n_codes,
+                                  int precision, void *P_dev, size_t P_stride, void *rows_dev,
+                                  size_t rows_stride, const int *status_dev, unsigned *done_dev,
+                                  int *row_flag_dev, int n_flags);
+
+// Eigen system of one reversible 4 x 4 rate matrix on the host; 0 or a
+// PGPU_ERR_* status as the GPU solver gives.
+int pgpu_host_eig4(const double *Q, const double *pi, double *U, double *lam, double *Ui);

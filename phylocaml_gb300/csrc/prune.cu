@@ -9,27 +9,41 @@
 //   L_s         = sum_r probs[r] sum_i pi[i] CLV_root[r][i]
 //   lnL         = sum_s w_s (log L_s + e_s ln 2)
 //
-// One kernel scores the whole tree (prune_tree_kernel):
-//   warp 0, lane 0   producer: streams each tip's row of pattern codes for the
-//                    CTA's tile, in the order the schedule reads them, into a
-//                    shared ring with 1-D bulk copies on mbarriers;
-//   consumer warps   one pattern per thread; the conditional likelihood
-//                    vectors of internal nodes live on a per-thread stack in
-//                    shared memory (top entry in registers), so no CLV ever
-//                    goes to HBM.  After every node the vector is rescaled by
-//                    an exact power of two when its largest entry drops below
-//                    2^-32 (FP32) or 2^-256 (FP64) and the exponent is added
-//                    to the pattern's integer scaler e_s.
+// A subtree of two or three tips has few distinct columns however many
+// patterns there are: n_codes^2 or n_codes^3 combinations of codes.  Where
+// that is less than half the patterns, every such subtree (the largest ones
+// of at most three tips) becomes one leaf of a reduced tree, and
+// prune_prep_kernel fills its rows P(t) CLV for every combination with the
+// same arithmetic as a node of the walk.  In a Yule tree half the internal
+// nodes lie in such subtrees.
+//
+// One kernel then scores the whole tree (prune_tree_kernel):
+//   warp 0, lane 0   producer: streams the transition matrices of each
+//                    step's internal children into a shared ring with 1-D
+//                    bulk copies on mbarriers;
+//   consumer warps   one (pattern, rate class) per thread; the conditional
+//                    likelihood vectors of internal nodes live on a
+//                    per-thread stack in shared memory (top entry in
+//                    registers), so no CLV ever goes to HBM.  A leaf's row is
+//                    gathered by the thread itself, three leaves ahead, with
+//                    cp.async into its own shared slots, by an index that
+//                    prune_prep_kernel formed from the tips' codes.  After
+//                    every node the vector is rescaled by an exact power of
+//                    two when its largest entry drops below 2^-32 (FP32) or
+//                    2^-256 (FP64) and the exponent is added to the
+//                    pattern's integer scaler e_s.
 // The root log-likelihoods are weighted and summed in FP64 with error-free
 // TwoSum steps (a compensated reduction), one (sum, compensation) pair per
-// CTA; prune_finalize_kernel adds the pairs in contiguous chunks with Neumaier's
-// method, so the result does not depend on scheduling.
+// CTA; the last CTA adds the pairs in contiguous chunks, so the result does
+// not depend on scheduling.
 //
 // T = float is the FP32 form, T = double the FP64 comparison form; both use
 // P matrices built in FP64 on the GPU (pmatrix.cu), the FP32 form rounding
 // them once.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <type_traits>
 
 #include "pgpu_internal.cuh"
 #include "forms.cuh"
@@ -39,111 +53,240 @@ namespace {
 using namespace pgpu_forms;
 
 struct PruneArgs {
-  const uint8_t *tip_codes;   // [n_tips][ld_pat]
-  const void *P;              // [2n-2][R][S][S] coefficients of the form (see below)
-  const void *tiptab;         // [n_tips][R][n_codes][S] tip rows P(t,r) code_tab[c] (form's values)
-  const double *code_tab;     // [n_codes][S]
+  const uint16_t *index;      // [n_leaf][ld_index]: each pattern's row of the leaf
+  const void *P;              // per branch: 16-byte unit k of rate class r at k R + r
+  const void *rows;           // leaf rows, [n_codes^k][R] per leaf (form's values)
+  const int *row_exp;         // power of two taken out of each collapsed leaf's row
+  const int *row_flag;        // per model: some exponent is not zero
   const double *pi;           // [S]
   const double *probs;        // [R]
   const double *weights;      // [n_pat] or null
   double *site_lnl;           // [n_pat] or null
   double2 *partials;          // [n_models][n_tiles_total], by tile
-  const int4 *ops;            // schedule
-  const int32_t *tip_seq;
+  unsigned *done;             // [n_models] CTAs finished, zeroed by the setup kernel
+  double *lnl;                // [n_models]
+  const int4 *ops;            // {branch of the internal first child or -1, ... second, -, -}
+  const uint32_t *leaf_unit;  // 16-byte unit of each leaf's first row, in the order the steps read them
   int *flag;
   // several models over the same tree and patterns: CTA row blockIdx.y
-  // scores model blockIdx.y, whose P blocks and tip rows lie P_stride and
-  // tab_stride bytes after the previous model's, pi and probs 4 and R
-  // doubles after, and whose partial sums follow the previous model's
-  size_t P_stride, tab_stride;
+  // scores model blockIdx.y, whose P blocks and leaf rows lie P_stride and
+  // rows_stride bytes after the previous model's, pi and probs 4 and R
+  // doubles after, its exponents exp_stride ints after, and whose partial
+  // sums follow the previous model's
+  size_t P_stride, rows_stride, exp_stride;
   // a launch may cover tiles tile_base .. tile_base + gridDim.x - 1 of
   // n_tiles_total (the host-buffer entry point launches one per copied chunk)
   size_t tile_base, n_tiles_total;
-  size_t ld_pat, n_pat;
-  int n_tips, n_ops, n_codes, R, NP, depth;
+  size_t index_col;           // pattern of index's first column
+  size_t ld_index, n_pat;
+  uint32_t exp_unit;          // unit of row_exp's first row
+  int n_ops, n_leaf, n_codes, R, NP, depth;
 };
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 constexpr int PR_THREADS = 256;   // consumer threads per CTA
+constexpr int PR_LEAVES = 3;      // leaf rows in flight per thread
 
-// Ring depth in postorder steps (a power of two) and the CTAs each SM should
-// hold.  The pair form's slots and stack are twice the FP32 form's, so its
-// ring is shorter to fit three CTAs (27 warps) per SM.  growth: how much
-// larger each column chunk of host tip codes is than the one before; a
-// chunk's copy must end while the previous chunk is scored, and a wave of
-// scoring takes about 2.5 (FP32), 6 (pair) or 30 (FP64) times as long as
-// copying its tip codes.
+// CTAs each SM should hold, and growth: how much larger each column chunk of
+// host tip codes is than the one before; a chunk's copy must end while the
+// previous chunk is scored.
 template <typename Pol> struct PruneTune {
-  static constexpr int stages = 8, min_ctas = 1, growth = 8;
+  static constexpr int min_ctas = 1, growth = 8;
 };
 template <> struct PruneTune<pgpu_forms::Ff32> {
-  static constexpr int stages = 4, min_ctas = 3, growth = 4;
+  static constexpr int min_ctas = 3, growth = 2;
 };
 template <> struct PruneTune<pgpu_forms::Fp32> {
-  static constexpr int stages = 8, min_ctas = 4, growth = 2;
+  static constexpr int min_ctas = 4, growth = 2;
 };
-// Steps per ring barrier: the producer stages PR_GROUP consecutive steps
-// under one mbarrier phase, so the consumers wait and release once per group.
-constexpr int PR_GROUP = 2;
+// Ring of the coefficient blocks, in postorder steps (a power of two).  The
+// producer stages PR_GROUP consecutive steps under one mbarrier phase, so
+// the consumers wait and release once per group.
+constexpr int PR_STAGES = 8, PR_GROUP = 2;
 
-// Shared memory of one CTA: the ring of per-op slots, then the CLV stack.
-// A slot holds everything one postorder step reads, staged by the producer:
-//   [0, NP)            tip codes of child a (if a is a tip)
-//   [NP, 2 NP)         tip codes of child b
-//   coef block a       R x 16 coefficients of the branch above a (internal a)
-//   coef block b
-//   tip block a        R x n_codes x 4 tip rows of the branch above a (tip a)
-//   tip block b
+// Shared memory of one CTA: the ring of step slots (the coefficient blocks
+// R x 16 of the first and the second child, where internal), the threads'
+// leaf slots, then the CLV stack (the results set aside: one less than the
+// schedule's depth, the top being in registers).
 template <typename Pol>
 struct PruneLayout {
   using V = typename Pol::V;
   using Coef = typename Pol::Coef;
   __host__ __device__ static size_t coef_bytes(int R) { return (size_t)R * 16 * sizeof(Coef); }
-  __host__ __device__ static size_t tip_bytes(int R, int n_codes) {
-    return (size_t)R * n_codes * 4 * sizeof(V);
-  }
-  __host__ __device__ static size_t coef_off(int NP) { return 2 * (size_t)NP; }
-  __host__ __device__ static size_t tip_off(int NP, int R) { return coef_off(NP) + 2 * coef_bytes(R); }
-  __host__ __device__ static size_t slot_bytes(int NP, int R, int n_codes) {
-    return (tip_off(NP, R) + 2 * tip_bytes(R, n_codes) + 127) & ~size_t(127);
-  }
+  __host__ __device__ static size_t slot_bytes(int R) { return (2 * coef_bytes(R) + 127) & ~size_t(127); }
   __host__ __device__ static size_t ring_off() { return 128; }
-  __host__ __device__ static size_t stk_off(int NP, int R, int n_codes) {
-    return ring_off() + (size_t)PruneTune<Pol>::stages * slot_bytes(NP, R, n_codes);
+  __host__ __device__ static size_t leaf_off(int R) { return ring_off() + PR_STAGES * slot_bytes(R); }
+  __host__ __device__ static size_t stk_off(int R) {
+    return leaf_off(R) + (size_t)PR_LEAVES * 4 * PR_THREADS * sizeof(V);
   }
-  __host__ __device__ static size_t bytes(int NP, int R, int n_codes, int depth) {
-    return stk_off(NP, R, n_codes) + (size_t)depth * 4 * PR_THREADS * sizeof(V);
+  __host__ __device__ static size_t bytes(int R, int depth) {
+    return stk_off(R) + (size_t)(depth > 1 ? depth - 1 : 0) * 4 * PR_THREADS * sizeof(V);
   }
 };
 
-// One CTA: 32 producer threads + PR_THREADS consumers.  Consumer warp w
-// works on rate class w % RT (R <= RT of them active) for 32 patterns of the
-// tile; each thread holds the 4 state values of one (pattern, rate class)
-// and its own power-of-two scaler.  All lanes of a warp read the same
-// coefficient block (a shared-memory broadcast).
+// Exact power-of-two rescaling of one rate class's vector (each rate class
+// keeps its own scaler; the root aligns them).  An all-zero vector (a site
+// the tree cannot produce) rescales to zeros again and ends as log 0 = -inf.
+template <typename Pol, typename M>
+__device__ __forceinline__ void rescale_vec(typename Pol::V *acc, M mx, int &escale) {
+  const int ex = frexp_exp(mx);
+  escale += ex;
+  // two steps when the largest entry is subnormal, so each factor stays a
+  // normal power of two
+  const int k1 = min(-ex, 120), k2 = -ex - k1;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k1);
+  if (k2 > 0) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k2);
+  }
+}
+template <typename Pol>
+__device__ __forceinline__ auto largest(const typename Pol::V *acc) {
+  return fmax(fmax(Pol::mag(acc[0]), Pol::mag(acc[1])), fmax(Pol::mag(acc[2]), Pol::mag(acc[3])));
+}
+
+// Rows of the collapsed leaves: P(t_v) CLV_v for every combination of the
+// leaf's codes, (c0 n + c1) for tips 0 and 1, ((c0 n + c1) n + c2) with tip 2
+// beside the cherry of tips 0 and 1.  A thread per combination.
+struct TableArgs {
+  void *rows;            // tips' rows first: [n_tips][n_codes][R]
+  const void *P;
+  const int4 *leaves;
+  const int4 *made;      // {leaf, branch of the leaf, branch of its cherry or -1, -}
+  int *row_exp, *row_flag;
+  size_t P_stride, rows_stride, exp_stride;
+  size_t exp_base;       // row of row_exp's first entry
+  int R, n_codes, n_made, blocks;   // blocks: CTAs per (leaf, rate class)
+  const int *status;     // model m at m
+};
+
+// Row of every leaf for every pattern, in the leaves' reading order, so that
+// the walk reads one 16-bit index where it would read up to three codes in
+// each of a pattern's rate classes.  A code outside the table raises the
+// error word and reads as the last.
+struct IndexArgs {
+  const uint8_t *tip_codes;   // [n_tips][ld_pat]
+  const int4 *leaves;         // {tip, tip or -1, tip or -1, first row}
+  uint16_t *index;            // [n_leaf][ld_index], column 0 = pattern col0
+  size_t ld_pat, ld_index, col0, cols, n_pat;
+  int n_codes, blocks;        // blocks: CTAs per leaf, 1,024 patterns each
+  int *flag;
+};
+
+__device__ __forceinline__ void leaf_index(const IndexArgs &p, int block) {
+  const int4 lf = __ldg(p.leaves + block / p.blocks);
+  const size_t col = ((size_t)(block % p.blocks) * 256 + threadIdx.x) * 4;
+  if (col >= p.cols) return;
+  const size_t pat = p.col0 + col;   // a multiple of 4, and rows are multiples of 16 long
+  uint32_t row[4] = {0, 0, 0, 0};
+  const uint32_t top = (uint32_t)p.n_codes - 1u;
+  bool bad = false;
+#pragma unroll
+  for (int h = 0; h < 3; ++h) {
+    const int t = h == 0 ? lf.x : h == 1 ? lf.y : lf.z;
+    if (t < 0) break;
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(p.tip_codes + (size_t)t * p.ld_pat + pat));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t c = (w >> (8 * q)) & 255u;
+      bad |= c > top && pat + q < p.n_pat;
+      row[q] = row[q] * (uint32_t)p.n_codes + min(c, top);
+    }
+  }
+  if (bad) atomicOr(p.flag, PGPU_FLAG_BADCODE);
+  *reinterpret_cast<uint2 *>(p.index + (size_t)(block / p.blocks) * p.ld_index + col) =
+      make_uint2(row[0] | row[1] << 16, row[2] | row[3] << 16);
+}
+
+// CTAs 0 .. n_table - 1: the collapsed leaves' rows (model by model); the
+// rest: leaf indexes.
+template <typename Pol>
+__global__ void __launch_bounds__(256) prune_prep_kernel(const TableArgs p, const IndexArgs ix, int n_table) {
+  using V = typename Pol::V;
+  using Coef = typename Pol::Coef;
+  if ((int)blockIdx.x >= n_table) {
+    leaf_index(ix, (int)blockIdx.x - n_table);
+    return;
+  }
+  const int per_model = p.n_made * p.R * p.blocks;
+  const int m = blockIdx.x / per_model, at_block = blockIdx.x % per_model, lr = at_block / p.blocks;
+  const int4 mk = __ldg(p.made + lr / p.R);
+  const int r = lr % p.R, NC = p.n_codes;
+  const int4 lf = __ldg(p.leaves + mk.x);
+  const bool three = lf.z >= 0;
+  const int n = three ? NC * NC * NC : NC * NC;
+  const int q = (at_block % p.blocks) * 256 + threadIdx.x;
+  if (q >= n || p.status[m]) return;
+  char *rows = static_cast<char *>(p.rows) + m * p.rows_stride;
+  const char *P = static_cast<const char *>(p.P) + m * p.P_stride;
+  auto coef = [&](int branch) {
+    return reinterpret_cast<const Coef *>(P + (size_t)branch * p.R * 16 * sizeof(Coef) + 16 * r);
+  };
+  auto tip = [&](int t, int c, V *y) { Pol::load_tip(rows, ((size_t)t * NC + c) * p.R + r, y); };
+  const int c01 = three ? q / NC : q;
+  V x[4], y[4], acc[4];
+  int ex = 0;
+  tip(lf.x, c01 / NC, x);
+  tip(lf.y, c01 % NC, y);
+  Pol::mul4(x, y, acc);
+  auto mx = largest<Pol>(acc);
+  if (mx < Pol::thresh) rescale_vec<Pol>(acc, mx, ex);
+  if (three) {
+    Pol::rows(coef(mk.z), acc, x, p.R);
+    tip(lf.z, q % NC, y);
+    Pol::mul4(x, y, acc);
+    mx = largest<Pol>(acc);
+    if (mx < Pol::thresh) rescale_vec<Pol>(acc, mx, ex);
+  }
+  Pol::rows(coef(mk.y), acc, x, p.R);
+  const size_t at = (size_t)(uint32_t)lf.w + (size_t)q * p.R + r;
+  Pol::store4(rows, at, x);
+  p.row_exp[m * p.exp_stride + (at - p.exp_base)] = ex;
+  if (ex) p.row_flag[m] = 1;   // every writer writes 1
+}
+
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// One CTA: 32 producer threads + PR_THREADS consumers.  Consumer c works on
+// rate class c % RT (R <= RT of them active) of pattern c / RT of the tile;
+// it holds the 4 state values and its own power-of-two scaler.  The classes
+// of a pattern sit in neighbouring lanes and interleaved in memory, so a
+// pattern's leaf row is one 128-byte line for all of them (four classes of
+// the pair form): a warp's gather touches 8 lines.  With a warp per class it
+// touched up to 32, and the line lookups bounded the kernel.
+//
+// Bound by the float-pair arithmetic of the rows and products (FMA pipe).
+// 512 taxa x 446,427 patterns, 4 rate classes, pair form: TIME_NEW with the
+// collapsed subtrees (about half the steps), 7.12 ms walking every node with
+// the tip rows staged per step by the producer.
 template <typename Pol, int RT>
 __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
     prune_tree_kernel(const PruneArgs p) {
   using V = typename Pol::V;
   using Coef = typename Pol::Coef;
   using L = PruneLayout<Pol>;
-  constexpr int ST = PruneTune<Pol>::stages, NT = PR_THREADS, G = PR_GROUP, NB = ST / G;
+  constexpr int ST = PR_STAGES, NT = PR_THREADS, G = PR_GROUP, NB = ST / G;
+  constexpr int VU = 4 * sizeof(V) / 16;   // 16-byte units of a row
   static_assert(ST % G == 0 && (NB & (NB - 1)) == 0, "ring depth must be a power-of-two number of groups");
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ double2 red[NT / 32];
   __shared__ double2 xch[RT][NT / RT];   // per pattern and rate class: (part, scaler)
   __shared__ int step_kind[ST];          // per step slot: which of the consumer's step cases
-  const int NP = p.NP, R = p.R, NC = p.n_codes;
+  __shared__ int last_cta;
+  const int NP = p.NP, R = p.R;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);     // [NB]
   uint64_t *empty = full + NB;                              // [NB]
-  const size_t SB = L::slot_bytes(NP, R, NC);
+  const size_t SB = L::slot_bytes(R);
   unsigned char *ring = smem + L::ring_off();               // [ST][SB]
-  V *stk = reinterpret_cast<V *>(smem + L::stk_off(NP, R, NC));   // [depth][4][NT]
+  V *stk = reinterpret_cast<V *>(smem + L::stk_off(R));     // [depth - 1][4][NT]
   const size_t tile = p.tile_base + blockIdx.x;
   const size_t tile0 = tile * NP;
   const int tid = threadIdx.x;
-  const size_t CB = L::coef_bytes(R), TB = L::tip_bytes(R, NC);
+  const size_t CB = L::coef_bytes(R);
 
   if (tid == 0) {
     for (int s = 0; s < NB; ++s) {
@@ -155,13 +298,11 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   __syncthreads();
 
   if (tid < 32) {
-    // producer: everything step i reads goes into slot i % ST
+    // producer: the coefficient blocks step i reads go into slot i % ST
     if (tid == 0) {
-      const uint32_t code_bytes = (uint32_t)min((size_t)NP, p.ld_pat - tile0);
       const unsigned char *Pg = static_cast<const unsigned char *>(p.P) + blockIdx.y * p.P_stride;
-      const unsigned char *Tg = static_cast<const unsigned char *>(p.tiptab) + blockIdx.y * p.tab_stride;
-      // step i goes into step slot i % ST; group q (steps qG .. qG + G - 1)
-      // completes barrier q % NB once per pass over the ring
+      // group q (steps qG .. qG + G - 1) completes barrier q % NB once per
+      // pass over the ring
       int groups = 0;
       for (int g0 = 0; g0 < p.n_ops; g0 += G) {
         const int q = g0 / G, b = q & (NB - 1), round = q / NB;
@@ -172,29 +313,18 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
         for (int k = 0; k < gn; ++k) {
           const int4 op = __ldg(p.ops + g0 + k);
           ops[k] = op;
-          for (int h = 0; h < 2; ++h) {
-            const int ch = h == 0 ? op.y : op.z;
-            tx += ch < p.n_tips ? code_bytes + (uint32_t)TB : (uint32_t)CB;
-          }
+          tx += (op.x >= 0 ? (uint32_t)CB : 0u) + (op.y >= 0 ? (uint32_t)CB : 0u);
           // bit 0: first child internal, bit 1: second child internal; 4
           // marks the first step, which has no earlier result to set aside.
           // The arrive below releases these stores to the consumers' wait.
-          const int kind = (op.y >= p.n_tips ? 1 : 0) | (op.z >= p.n_tips ? 2 : 0);
+          const int kind = (op.x >= 0 ? 1 : 0) | (op.y >= 0 ? 2 : 0);
           step_kind[(g0 + k) & (ST - 1)] = g0 + k == 0 ? 4 : kind;
         }
         mbar_arrive_expect_tx(&full[b], tx);
         for (int k = 0; k < gn; ++k) {
           unsigned char *sl = ring + (size_t)((g0 + k) & (ST - 1)) * SB;
-          for (int h = 0; h < 2; ++h) {
-            const int ch = h == 0 ? ops[k].y : ops[k].z;
-            if (ch < p.n_tips) {
-              bulk_g2s(sl + (size_t)h * NP, p.tip_codes + (size_t)ch * p.ld_pat + tile0, code_bytes,
-                       &full[b]);
-              bulk_g2s(sl + L::tip_off(NP, R) + h * TB, Tg + (size_t)ch * TB, (uint32_t)TB, &full[b]);
-            } else {
-              bulk_g2s(sl + L::coef_off(NP) + h * CB, Pg + (size_t)ch * CB, (uint32_t)CB, &full[b]);
-            }
-          }
+          if (ops[k].x >= 0) bulk_g2s(sl, Pg + (size_t)ops[k].x * CB, (uint32_t)CB, &full[b]);
+          if (ops[k].y >= 0) bulk_g2s(sl + CB, Pg + (size_t)ops[k].y * CB, (uint32_t)CB, &full[b]);
         }
         groups = q + 1;
       }
@@ -205,31 +335,75 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
     return;
   }
 
-  // consumer warp w works on rate class w % RT for 32 patterns, so every
-  // coefficient read of a warp is a broadcast of one rate's P block
-  const int c = tid - 32, lane = tid & 31, cwarp = c >> 5;
-  const int r = cwarp % RT, pl = (cwarp / RT) * 32 + lane;
+  const int c = tid - 32, lane = tid & 31;
+  const int r = c % RT, pl = c / RT;
   const size_t pat = tile0 + pl;
   const bool active = pat < p.n_pat;
   const bool rate_on = r < R;
-  // warps of a rate class beyond R (R < RT) repeat class R - 1 and are
+  // lanes of a rate class beyond R (R < RT) repeat class R - 1 and are
   // dropped at the root, so the step loop has no branch on the rate
   const int rr = min(r, R - 1);
+
+  // leaf pipeline: this thread's slots take turns; the next leaf's index is
+  // read a leaf before its row is gathered
+  const uint16_t *index = p.index + ((active ? pat : p.n_pat - 1) - p.index_col);   // idle lanes repeat the last pattern
+  const uint32_t *unit = p.leaf_unit;
+  const char *rows = static_cast<const char *>(p.rows) + blockIdx.y * p.rows_stride + (size_t)rr * (4 * sizeof(V));
+  const uint32_t RU = (uint32_t)R * VU;
+  constexpr uint32_t SLOT = VU * NT * 16u;
+  const uint32_t slot0 = smem_u32(smem + L::leaf_off(R)) + 16u * c;   // [slot][VU][NT] of 16 bytes
+  uint32_t put = slot0, get = slot0;
+  const bool scaled_rows = p.row_flag[blockIdx.y] != 0;
+  int to_read = p.n_leaf, to_gather = p.n_leaf, pending = 0, escale = 0;
+  uint32_t next_row = 0, next_unit = 0;
+  auto read_index = [&]() {
+    if (to_read > 0) {
+      next_row = __ldg(index);
+      next_unit = __ldg(unit);
+      index += p.ld_index;
+      ++unit;
+      --to_read;
+    }
+  };
+  auto gather = [&]() {
+    if (to_gather > 0) {
+      const uint32_t u = next_unit + next_row * RU;
+      const char *src = rows + (size_t)u * 16;
+#pragma unroll
+      for (int k = 0; k < VU; ++k) cp_async_16(put + k * NT * 16u, src + 16 * k);
+      if (scaled_rows && u >= p.exp_unit)
+        escale += __ldg(p.row_exp + blockIdx.y * p.exp_stride + (u - p.exp_unit) / VU + rr);
+      put = put + SLOT == slot0 + PR_LEAVES * SLOT ? slot0 : put + SLOT;
+      --to_gather;
+      read_index();
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // empty groups keep the count in step
+  };
+  // the next leaf's row into y; PEND of the younger groups may be in flight
+  auto leaf_row = [&](V *y, auto pend) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(decltype(pend)::value) : "memory");
+    Pol::load_row_s(get, get + NT * 16u, y);
+    get = get + SLOT == slot0 + PR_LEAVES * SLOT ? slot0 : get + SLOT;
+    ++pending;
+  };
+  using Pend0 = std::integral_constant<int, PR_LEAVES - 1>;   // the next leaf
+  using Pend1 = std::integral_constant<int, PR_LEAVES - 2>;   // the one after it
+  read_index();
+#pragma unroll
+  for (int j = 0; j < PR_LEAVES; ++j) gather();
 
   // The stack discipline is fixed by the schedule: in postorder the result
   // of step i - 1 is always the second child of step i when that child is
   // internal, else its first child when that one is internal; a step with
-  // two tip children leaves it pending (push), and a step with two internal
+  // two leaves leaves it pending (push), and a step with two internal
   // children takes its first child from the stack (pop).  So the top of the
   // stack lives in registers and each step is one of four straight-line
   // cases, chosen by a warp-uniform branch.
   V top[4];
   V *my = stk + c;   // this thread's column of the stack: entry (k, e) at my[(4 k + e) NT]
-  int sp = 0, escale = 0;
-  uint32_t code_max = 0;
+  int sp = 0;
   bool ok = true;
-  const size_t tipb = L::tip_off(NP, R) + (size_t)rr * NC * 4 * sizeof(V);
-  const size_t coefb = L::coef_off(NP) + (size_t)rr * 16 * sizeof(Coef);
+  const size_t coefb = (size_t)rr * 16;
 
   for (int g0 = 0; g0 < p.n_ops && ok; g0 += G) {
     const int q = g0 / G, b = q & (NB - 1);
@@ -240,89 +414,69 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
     }
 #pragma unroll
     for (int k = 0; k < G; ++k) {
-    const int i = g0 + k;
-    if (i >= p.n_ops) break;
-    const int slot = i & (ST - 1);
-    const int kind = step_kind[slot];
-    const unsigned char *sl = ring + (size_t)slot * SB;
-    V acc[4];
-    {
-      auto tip = [&](int h, V *y) {
-        const uint32_t code = sl[h * NP + pl];
-        code_max = max(code_max, code);
-        Pol::load_tip(sl + tipb + h * TB, min(code, (uint32_t)NC - 1u), y);
-      };
-      auto coef = [&](int h) { return reinterpret_cast<const Coef *>(sl + coefb + h * CB); };
-      V y0[4], y1[4];
-      switch (kind) {
-        case 0:   // two tips; the previous result waits on the stack
-          if (sp < p.depth) {
+      const int i = g0 + k;
+      if (i >= p.n_ops) break;
+      const int slot = i & (ST - 1);
+      const int kind = step_kind[slot];
+      const unsigned char *sl = ring + (size_t)slot * SB + coefb;
+      V acc[4];
+      {
+        auto coef = [&](int h) { return reinterpret_cast<const Coef *>(sl + h * CB); };
+        V y0[4], y1[4];
+        switch (kind) {
+          case 0:   // two leaves; the previous result waits on the stack
+            if (sp + 1 < p.depth) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) my[(4 * sp + e) * NT] = top[e];
-            ++sp;
-          } else {
-            ok = false;   // schedule and stack size disagree
+              for (int e = 0; e < 4; ++e) my[(4 * sp + e) * NT] = top[e];
+              ++sp;
+            } else {
+              ok = false;   // schedule and stack size disagree
+            }
+            [[fallthrough]];
+          case 4:   // the first step: two leaves, nothing to set aside
+            leaf_row(y0, Pend0{});
+            leaf_row(y1, Pend1{});
+            break;
+          case 1:   // internal first child (the previous result), leaf second
+            Pol::rows(coef(0), top, y0, R);
+            leaf_row(y1, Pend0{});
+            break;
+          case 2:   // leaf first, internal second child (the previous result)
+            Pol::rows(coef(1), top, y1, R);
+            leaf_row(y0, Pend0{});
+            break;
+          default: {   // 3, both internal: the first from the stack
+            V xa[4];
+            if (sp > 0) {
+              --sp;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) xa[e] = my[(4 * sp + e) * NT];
+            } else {
+              ok = false;   // schedule and stack disagree
+#pragma unroll
+              for (int e = 0; e < 4; ++e) xa[e] = Pol::zero();
+            }
+            Pol::rows(coef(0), xa, y0, R);
+            Pol::rows(coef(1), top, y1, R);
           }
-          tip(0, y0);
-          tip(1, y1);
-          break;
-        case 4:   // the first step: two tips, nothing to set aside
-          tip(0, y0);
-          tip(1, y1);
-          break;
-        case 1:   // internal first child (the previous result), tip second
-          Pol::rows(coef(0), top, y0);
-          tip(1, y1);
-          break;
-        case 2:   // tip first, internal second child (the previous result)
-          tip(0, y0);
-          Pol::rows(coef(1), top, y1);
-          break;
-        default: {   // 3, both internal: the first from the stack
-          V xa[4];
-          if (sp > 0) {
-            --sp;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) xa[e] = my[(4 * sp + e) * NT];
-          } else {
-            ok = false;   // schedule and stack disagree
-#pragma unroll
-            for (int e = 0; e < 4; ++e) xa[e] = Pol::zero();
-          }
-          Pol::rows(coef(0), xa, y0);
-          Pol::rows(coef(1), top, y1);
         }
+        Pol::mul4(y0, y1, acc);
       }
-      Pol::mul4(y0, y1, acc);
-    }
-    // exact power-of-two rescaling of this rate class's vector (each rate
-    // class keeps its own scaler; the root aligns them); rare, so the warp
-    // only enters when some lane needs it.  An all-zero vector (a site the
-    // tree cannot produce) rescales to zeros again and ends as log 0 = -inf.
-    auto mx = fmax(fmax(Pol::mag(acc[0]), Pol::mag(acc[1])), fmax(Pol::mag(acc[2]), Pol::mag(acc[3])));
-    if (__any_sync(0xffffffffu, mx < Pol::thresh)) {
-      if (mx < Pol::thresh) {
-        const int ex = frexp_exp(mx);
-        escale += ex;
-        // two steps when the largest entry is subnormal, so each factor
-        // stays a normal power of two
-        const int k1 = min(-ex, 120), k2 = -ex - k1;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k1);
-        if (k2 > 0) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k2);
-        }
+      // the slots read above are refilled once their values are in use
+      for (; pending > 0; --pending) gather();
+      // rare, so the warp only enters when some lane needs it
+      const auto mx = largest<Pol>(acc);
+      if (__any_sync(0xffffffffu, mx < Pol::thresh)) {
+        if (mx < Pol::thresh) rescale_vec<Pol>(acc, mx, escale);
       }
-    }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) top[e] = acc[e];
+      for (int e = 0; e < 4; ++e) top[e] = acc[e];
     }
     // this warp is done with the group's step slots
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[b]);
   }
-  if (active && r == 0 && rate_on && code_max >= (uint32_t)NC) atomicOr(p.flag, PGPU_FLAG_BADCODE);
+  asm volatile("cp.async.wait_all;" ::: "memory");
 
   // root: sum over rate classes of probs[r] 2^e_r sum_i pi_i x_i, in FP64;
   // the rate classes of a pattern meet in shared memory
@@ -355,20 +509,41 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   const int cw = c >> 5;
   if (lane == 0) red[cw] = make_double2(s, comp);
   asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
+  const double2 *parts = p.partials + (size_t)blockIdx.y * p.n_tiles_total;
   if (cw == 0) {
     double2 v = lane < NT / 32 ? red[lane] : make_double2(0.0, 0.0);
     double ss = v.x, cc = v.y;
     warp_csum(ss, cc);
-    if (lane == 0) p.partials[(size_t)blockIdx.y * p.n_tiles_total + tile] = make_double2(ss, cc);
+    if (lane == 0) {
+      p.partials[(size_t)blockIdx.y * p.n_tiles_total + tile] = make_double2(ss, cc);
+      __threadfence();
+      last_cta = atomicAdd(p.done + blockIdx.y, 1u) == (unsigned)p.n_tiles_total - 1u;
+    }
   }
-}
-
-// Neumaier sum of the per-CTA (sum, compensation) pairs in CTA order, one
-// CTA per model.
-__global__ void __launch_bounds__(1024) prune_finalize_kernel(const double2 *partials, int n,
-                                                             double *out) {
-  const double v = csum_block<1024>(partials + (size_t)blockIdx.x * n, n);
-  if (threadIdx.x == 0) out[blockIdx.x] = v;
+  asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
+  if (!last_cta) return;
+  // the model's last CTA: every partial, in contiguous chunks of the tiles
+  // and a fixed butterfly, so the total does not depend on which CTA it is
+  __threadfence();
+  const size_t per = (p.n_tiles_total + NT - 1) / NT;
+  const size_t lo = min((size_t)c * per, p.n_tiles_total), hi = min(lo + per, p.n_tiles_total);
+  s = comp = 0.0;
+  for (size_t i = lo; i < hi; ++i) {
+    const double2 v = __ldcg(parts + i);
+    double u, e;
+    two_sum(s, v.x, u, e);
+    s = u;
+    comp += e + v.y;
+  }
+  warp_csum(s, comp);
+  if (lane == 0) red[cw] = make_double2(s, comp);
+  asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
+  if (cw == 0) {
+    double2 v = lane < NT / 32 ? red[lane] : make_double2(0.0, 0.0);
+    double ss = v.x, cc = v.y;
+    warp_csum(ss, cc);
+    if (lane == 0) p.lnl[blockIdx.y] = ss + cc;
+  }
 }
 
 template <typename Pol, int RT>
@@ -388,7 +563,7 @@ pgpu_status launch_prune_rt(pgpu_ctx *ctx, PruneArgs &a, size_t n_tiles, size_t 
 struct HostTips {
   const uint8_t *host;   // [n_tips][n_pat]
   uint8_t *dev;          // [n_tips][ld_pat]
-  size_t n_tips;
+  size_t n_tips, ld_pat;
 };
 
 // The launches of one scoring: tile ranges [bounds[k], bounds[k + 1]).
@@ -438,7 +613,7 @@ pgpu_status plan_prune(pgpu_ctx *ctx, PruneArgs &a, int RT, int n_models, const 
   const size_t n_tiles = (a.n_pat + a.NP - 1) / a.NP;
   a.n_tiles_total = n_tiles;
   a.tile_base = 0;
-  pl.smem = PruneLayout<Pol>::bytes(a.NP, a.R, a.n_codes, a.depth);
+  pl.smem = PruneLayout<Pol>::bytes(a.R, a.depth);
   if (pl.smem > ctx->smem_optin)
     return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: %zu bytes of shared memory needed (tree too deep)",
                         pl.smem);
@@ -453,29 +628,63 @@ pgpu_status plan_prune(pgpu_ctx *ctx, PruneArgs &a, int RT, int n_models, const 
     for (int k = 0; k < pl.K; ++k) {
       const size_t c0 = pl.bounds[k] * a.NP, c1 = std::min(pl.bounds[k + 1] * a.NP, a.n_pat);
       if (c1 > c0)
-        PGPU_CUDA(ctx, cudaMemcpy2DAsync(ht->dev + c0, a.ld_pat, ht->host + c0, a.n_pat, c1 - c0, ht->n_tips,
+        PGPU_CUDA(ctx, cudaMemcpy2DAsync(ht->dev + c0, ht->ld_pat, ht->host + c0, a.n_pat, c1 - c0, ht->n_tips,
                                          cudaMemcpyHostToDevice, ctx->copy_stream));
       PGPU_CUDA(ctx, cudaEventRecord(ctx->copy_ev[k], ctx->copy_stream));
     }
   return PGPU_OK;
 }
 
-// With several chunks, consecutive launches alternate between the context
-// stream and the auxiliary one, so a chunk's CTAs take the SMs the previous
-// chunk's CTAs leave instead of waiting for the whole launch to drain (the
-// tiles are disjoint; each launch waits only for its own columns).
+// Tables and leaf indexes of the patterns of tiles [t0, t1), or either alone.
+template <typename Pol>
+pgpu_status launch_prep(pgpu_ctx *ctx, const TableArgs &t, int n_models, IndexArgs &x, int n_leaf, size_t pat0,
+                        size_t pat1, bool tables, cudaStream_t stream) {
+  const size_t n_table = tables ? (size_t)t.n_made * t.R * t.blocks * n_models : 0;
+  x.col0 = pat0;
+  x.cols = pat1 - pat0;
+  x.blocks = (int)((x.cols + 1023) / 1024);
+  const size_t grid = n_table + (size_t)n_leaf * x.blocks;
+  if (grid == 0) return PGPU_OK;
+  if (grid > 0x7fffffff) return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: too many patterns and leaves");
+  prune_prep_kernel<Pol><<<(unsigned)grid, 256, 0, stream>>>(t, x, (int)n_table);
+  return pgpu_after_launch(ctx, "prune_prep_kernel");
+}
+
+// Launches every tile.  With the codes in host memory in several chunks,
+// consecutive launches alternate between the context stream and the
+// auxiliary one, so a chunk's CTAs take the SMs the previous chunk's CTAs
+// leave instead of waiting for the whole launch to drain (the tiles are
+// disjoint; each launch waits only for its own columns).  Where the leaf
+// indexes of all patterns would take more than index_cols columns, pieces of
+// that many take turns in one buffer, on the context stream alone.
 template <typename Pol, int RT>
-pgpu_status launch_prune_chunks(pgpu_ctx *ctx, PruneArgs &a, const ChunkPlan &pl, int n_models, bool host) {
-  const bool fork = host && pl.K > 1;
+pgpu_status launch_prune_chunks(pgpu_ctx *ctx, PruneArgs &a, const ChunkPlan &pl, int n_models, bool host,
+                                const TableArgs &t, IndexArgs &x, size_t index_cols) {
+  const bool whole = index_cols >= a.n_tiles_total * a.NP;
+  const bool fork = host && pl.K > 1 && whole;
+  const size_t piece = whole ? a.n_tiles_total : index_cols / a.NP;
+  bool tables = t.n_made > 0;
   if (fork) {
+    if (tables) PGPU_TRY(launch_prep<Pol>(ctx, t, n_models, x, 0, 0, 0, true, ctx->stream));
+    tables = false;
     PGPU_CUDA(ctx, cudaEventRecord(ctx->aux_ev[0], ctx->stream));
     PGPU_CUDA(ctx, cudaStreamWaitEvent(ctx->aux_stream, ctx->aux_ev[0], 0));
   }
+  uint16_t *index = x.index;
   for (int k = 0; k < pl.K; ++k) {
     const cudaStream_t ks = fork && (k & 1) ? ctx->aux_stream : ctx->stream;
     if (host) PGPU_CUDA(ctx, cudaStreamWaitEvent(ks, ctx->copy_ev[k], 0));
-    a.tile_base = pl.bounds[k];
-    PGPU_TRY((launch_prune_rt<Pol, RT>(ctx, a, pl.bounds[k + 1] - pl.bounds[k], pl.smem, n_models, ks)));
+    for (size_t t0 = pl.bounds[k]; t0 < pl.bounds[k + 1]; t0 += piece) {
+      const size_t t1 = std::min(t0 + piece, pl.bounds[k + 1]);
+      const size_t p0 = t0 * a.NP, p1 = std::min(t1 * a.NP, a.n_pat);
+      x.index = whole ? index + p0 : index;
+      PGPU_TRY(launch_prep<Pol>(ctx, t, n_models, x, a.n_leaf, p0, p1, tables, ks));
+      tables = false;
+      a.index = x.index;
+      a.index_col = p0;
+      a.tile_base = t0;
+      PGPU_TRY((launch_prune_rt<Pol, RT>(ctx, a, t1 - t0, pl.smem, n_models, ks)));
+    }
   }
   if (fork) {
     PGPU_CUDA(ctx, cudaEventRecord(ctx->aux_ev[1], ctx->aux_stream));
@@ -486,48 +695,17 @@ pgpu_status launch_prune_chunks(pgpu_ctx *ctx, PruneArgs &a, const ChunkPlan &pl
 }
 
 template <typename Pol>
-pgpu_status launch_prune(pgpu_ctx *ctx, PruneArgs &a, int RT, int n_models, const ChunkPlan &pl, bool host) {
+pgpu_status launch_prune(pgpu_ctx *ctx, PruneArgs &a, int RT, int n_models, const ChunkPlan &pl, bool host,
+                         const TableArgs &t, IndexArgs &x, size_t index_cols) {
   switch (RT) {
-    case 1: return launch_prune_chunks<Pol, 1>(ctx, a, pl, n_models, host);
-    case 2: return launch_prune_chunks<Pol, 2>(ctx, a, pl, n_models, host);
-    case 4: return launch_prune_chunks<Pol, 4>(ctx, a, pl, n_models, host);
-    default: return launch_prune_chunks<Pol, 8>(ctx, a, pl, n_models, host);
+    case 1: return launch_prune_chunks<Pol, 1>(ctx, a, pl, n_models, host, t, x, index_cols);
+    case 2: return launch_prune_chunks<Pol, 2>(ctx, a, pl, n_models, host, t, x, index_cols);
+    case 4: return launch_prune_chunks<Pol, 4>(ctx, a, pl, n_models, host, t, x, index_cols);
+    default: return launch_prune_chunks<Pol, 8>(ctx, a, pl, n_models, host, t, x, index_cols);
   }
 }
 
 }  // namespace
-
-// Double-buffered pinned staging for the small per-call parameters, so the
-// device-pointer entry points never synchronise the stream.
-pgpu_status pgpu_stage(pgpu_ctx *ctx, size_t bytes, void **host, void **dev) {
-  const int k = ctx->stage_next;
-  ctx->stage_next ^= 1;
-  if (ctx->stage_ev[k]) PGPU_CUDA(ctx, cudaEventSynchronize(ctx->stage_ev[k]));
-  if (ctx->stage_cap[k] < bytes) {
-    if (ctx->stage_h[k]) cudaFreeHost(ctx->stage_h[k]);
-    if (ctx->stage_d[k]) cudaFree(ctx->stage_d[k]);
-    ctx->stage_h[k] = nullptr;
-    ctx->stage_d[k] = nullptr;
-    ctx->stage_cap[k] = 0;
-    const size_t want = std::max<size_t>(bytes, 64 * 1024);
-    PGPU_CUDA(ctx, cudaMallocHost(&ctx->stage_h[k], want));
-    PGPU_CUDA(ctx, cudaMalloc(&ctx->stage_d[k], want));
-    ctx->stage_cap[k] = want;
-  }
-  if (!ctx->stage_ev[k]) PGPU_CUDA(ctx, cudaEventCreateWithFlags(&ctx->stage_ev[k], cudaEventDisableTiming));
-  *host = ctx->stage_h[k];
-  *dev = ctx->stage_d[k];
-  ctx->stage_cur = k;
-  return PGPU_OK;
-}
-
-pgpu_status pgpu_stage_commit(pgpu_ctx *ctx, size_t bytes) {
-  const int k = ctx->stage_cur;
-  PGPU_CUDA(ctx, cudaMemcpyAsync(ctx->stage_d[k], ctx->stage_h[k], bytes, cudaMemcpyHostToDevice,
-                                 ctx->stream));
-  PGPU_CUDA(ctx, cudaEventRecord(ctx->stage_ev[k], ctx->stream));
-  return PGPU_OK;
-}
 
 namespace {
 using namespace pgpu_forms;
@@ -548,7 +726,8 @@ pgpu_status check_model(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_codes
 
 // all small per-call parameters in one staged block
 struct Staged {
-  double *Q, *pi, *rates, *probs, *tab, *brlen;
+  double *Q, *pi, *rates, *probs, *tab, *brlen, *U, *lam, *Ui;
+  int *status;
   size_t bytes;
 };
 
@@ -566,6 +745,11 @@ Staged stage_layout(int S, int R, int n_codes, int n_br, int V) {
   s.probs = (double *)take((size_t)V * R);
   s.tab = (double *)take((size_t)n_codes * S);
   s.brlen = (double *)take(n_br);
+  // the eigen systems, where the host solves them
+  s.U = (double *)take((size_t)V * S * S);
+  s.lam = (double *)take((size_t)V * S);
+  s.Ui = (double *)take((size_t)V * S * S);
+  s.status = (int *)take(V);
   s.bytes = off;
   return s;
 }
@@ -575,9 +759,130 @@ Ptr *rebase(void *base, Ptr *off) {
   return reinterpret_cast<Ptr *>(static_cast<char *>(base) + reinterpret_cast<size_t>(off));
 }
 
+// The reduced tree a call walks, kept on the context (with its device copy)
+// for further calls on the same tree.
+//
+// level: tips of the largest subtree that becomes a leaf (1: none).  A
+// collapsed leaf costs n_codes^k table rows where the walk would compute its
+// k - 1 nodes for every pattern, so it is worth it while the table is the
+// smaller side: at most half the patterns (16 codes: from 8,192 patterns on
+// three tips, from 512 on two).  call_bytes is what one row takes over all
+// models; the tables of a call stay below 1 GB.
+pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes, size_t n_pat,
+                       size_t row_bytes, size_t call_bytes, const PrunePlan **out) {
+  const int32_t n = tree->n_tips, n_int = n - 1;
+  const size_t NC = (size_t)n_codes;
+  int level = 2 * NC * NC * NC <= n_pat && NC * NC * NC <= 65536 ? 3 : 2 * NC * NC <= n_pat ? 2 : 1;
+  PrunePlan &pl = ctx->prune_plan;
+  const bool same_tree = pl.valid && (int32_t)pl.left.size() == n_int &&
+                         std::memcmp(pl.left.data(), tree->left, n_int * 4) == 0 &&
+                         std::memcmp(pl.right.data(), tree->right, n_int * 4) == 0;
+  if (same_tree && pl.R == R && pl.n_codes == n_codes && pl.row_bytes == row_bytes && pl.asked == level &&
+      pl.made_rows * call_bytes <= (size_t)1 << 30) {
+    *out = &pl;
+    return PGPU_OK;
+  }
+  TreeSchedule sch;
+  PGPU_TRY(pgpu_build_schedule(ctx, tree, &sch));   // validates the tree
+  pl.valid = false;
+  pl.asked = level;
+  pl.R = R;
+  pl.n_codes = n_codes;
+  pl.row_bytes = row_bytes;
+  std::vector<int32_t> tips(n_int), id(2 * n - 1), branch, left, right;
+  for (int32_t k = 0; k < n_int; ++k) {
+    const int32_t a = tree->left[k], b = tree->right[k];
+    tips[k] = (a < n ? 1 : tips[a - n]) + (b < n ? 1 : tips[b - n]);
+  }
+  for (;; --level) {
+    // leaves: tips and maximal subtrees of at most `level` tips below the
+    // root; {leaf, branch, cherry's branch} of the latter
+    std::vector<int4> leaf;
+    pl.made.clear();
+    pl.made_rows = 0;
+    std::vector<uint8_t> inside(2 * n - 1, 0);   // below a collapsed node, or one
+    auto small = [&](int32_t v) { return v < n || (v != 2 * n - 2 && tips[v - n] <= level); };
+    for (int32_t v = 2 * n - 2; v >= n; --v)
+      for (const int32_t c : {tree->left[v - n], tree->right[v - n]})
+        if (inside[v] || small(v)) inside[c] = 1;
+    branch.clear();
+    left.clear();
+    right.clear();
+    for (int32_t v = 0; v < 2 * n - 2; ++v) {
+      if (inside[v] || !small(v)) continue;
+      id[v] = (int32_t)leaf.size();
+      branch.push_back(v);
+      if (v < n) {
+        leaf.push_back(make_int4(v, -1, -1, (int)(uint32_t)((size_t)v * R * NC)));
+        continue;
+      }
+      int32_t a = tree->left[v - n], b = tree->right[v - n], cherry = -1;
+      if (a < n && b >= n) std::swap(a, b);
+      int4 lf = make_int4(a, b, -1, (int)(uint32_t)((size_t)n * R * NC + pl.made_rows));
+      if (a >= n) {
+        cherry = a;
+        lf = make_int4(tree->left[a - n], tree->right[a - n], b, lf.w);
+      }
+      pl.made.push_back(make_int4((int)leaf.size(), v, cherry, 0));
+      pl.made_rows += (size_t)R * NC * NC * (cherry >= 0 ? NC : 1);
+      leaf.push_back(lf);
+    }
+    const size_t n_rows = (size_t)n * R * NC + pl.made_rows, most = NC * NC * (level == 3 ? NC : 1);
+    if (level > 1 && (n_rows > 0x7fffffffull || pl.made_rows * call_bytes > (size_t)1 << 30 ||
+                      pl.made.size() * R * ((most + 255) / 256) > 0x7fffffff))
+      continue;
+    if (n_rows > 0x7fffffffull) return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: 2^31 leaf rows or more");
+    pl.level = level;
+    const int32_t nl = (int32_t)leaf.size();
+    int32_t next = nl;
+    for (int32_t v = n; v <= 2 * n - 2; ++v) {
+      if (inside[v] || small(v)) continue;
+      id[v] = next++;
+      if (v < 2 * n - 2) branch.push_back(v);
+      left.push_back(id[tree->left[v - n]]);
+      right.push_back(id[tree->right[v - n]]);
+    }
+    pgpu_tree red{nl, left.data(), right.data(), nullptr};
+    PGPU_TRY(pgpu_build_schedule(ctx, &red, &sch));
+    // steps, and the leaves in the order the steps read them
+    std::vector<int32_t> place(nl);
+    for (int32_t j = 0; j < nl; ++j) place[sch.tip_seq[j]] = j;
+    pl.ops.clear();
+    for (const SchedOp &op : sch.ops)
+      pl.ops.push_back(make_int4(op.a >= nl ? branch[op.a] : -1, op.b >= nl ? branch[op.b] : -1, 0, 0));
+    pl.leaves.assign(nl, int4());
+    for (int32_t j = 0; j < nl; ++j) pl.leaves[j] = leaf[sch.tip_seq[j]];
+    for (int4 &m : pl.made) m.x = place[m.x];
+    pl.depth = std::max(sch.max_depth, 1);
+    break;
+  }
+  // resident on the device: {ops, leaves, made, units}
+  const size_t n_all = pl.ops.size() + pl.leaves.size() + pl.made.size();
+  const size_t bytes = 16 * n_all + 4 * pl.leaves.size();
+  void *h, *dst;
+  PGPU_TRY(pgpu_buf(ctx, BUF_OPS2, bytes, &dst));
+  PGPU_TRY(pgpu_stage(ctx, bytes, &h, nullptr));
+  int4 *q = static_cast<int4 *>(h);
+  q = std::copy(pl.ops.begin(), pl.ops.end(), q);
+  q = std::copy(pl.leaves.begin(), pl.leaves.end(), q);
+  q = std::copy(pl.made.begin(), pl.made.end(), q);
+  uint32_t *unit = reinterpret_cast<uint32_t *>(q);
+  for (const int4 &lf : pl.leaves) *unit++ = (uint32_t)lf.w * (uint32_t)(row_bytes / 16);
+  PGPU_TRY(pgpu_stage_copy(ctx, dst, bytes));
+  pl.d_ops = static_cast<const int4 *>(dst);
+  pl.d_leaves = pl.d_ops + pl.ops.size();
+  pl.d_made = pl.d_leaves + pl.leaves.size();
+  pl.d_unit = reinterpret_cast<const uint32_t *>(pl.d_made + pl.made.size());
+  pl.left.assign(tree->left, tree->left + n_int);
+  pl.right.assign(tree->right, tree->right + n_int);
+  pl.valid = true;
+  *out = &pl;
+  return PGPU_OK;
+}
+
 // Scores n_models models (same state and rate-class counts) over one tree
-// and one set of patterns: lnl_dev[v] for model v.  One eigendecomposition
-// launch for all models, a P and a tip-table build per model, then one
+// and one set of patterns: lnl_dev[v] for model v.  One launch each for all
+// models' eigen systems, P matrices, tip rows and collapsed leaves, then one
 // pruning launch whose CTA rows are the models.
 // host_tips: the codes are still in host memory (n_pat bytes per row) and
 // tips is the device buffer they go to; they are copied in chunks that
@@ -603,15 +908,16 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
     return pgpu_set_err(ctx, PGPU_ERR_ARG,
                         "prune: ld_pat (%zu) must be a multiple of 16 and >= n_pat, rows 16-byte aligned",
                         ld_pat);
-  const TreeSchedule *sch;
-  const int4 *dops;
-  const int32_t *dseq;
-  PGPU_TRY(pgpu_schedule_device(ctx, tree, &sch, &dops, &dseq));
   const int V = n_models;
   const int S = models[0].n_states, R = models[0].n_rates, n = tree->n_tips, n_br = 2 * n - 2;
+  if (!tree->left || !tree->right || n < 2)
+    return pgpu_set_err(ctx, PGPU_ERR_ARG, "tree: null tree or fewer than 2 tips");
   for (int i = 0; i < n_br; ++i)
     if (!(tree->brlen[i] >= 0.0) || !std::isfinite(tree->brlen[i]))
       return pgpu_set_err(ctx, PGPU_ERR_ARG, "prune: branch length %d is negative or not finite", i);
+  const size_t row_bytes = precision == 32 ? 16 : 32;
+  const PrunePlan *pp;
+  PGPU_TRY(prune_plan(ctx, tree, R, codes->n_codes, n_pat, row_bytes, row_bytes * V, &pp));
 
   // stage every model's Q, pi, rates, probs, then the code table and the
   // branch lengths
@@ -627,47 +933,72 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   }
   std::copy(codes->table, codes->table + (size_t)codes->n_codes * S, rebase(h, lay.tab));
   std::copy(tree->brlen, tree->brlen + n_br, rebase(h, lay.brlen));
+  // A handful of 4 x 4 eigen systems is quicker on the host (about 1 us
+  // each) than in a launch of its own (36 us, however many).
+  const bool host_eig = V <= 24;
+  if (host_eig)
+    for (int v = 0; v < V; ++v)
+      rebase(h, lay.status)[v] =
+          pgpu_host_eig4(models[v].Q, models[v].pi, rebase(h, lay.U) + (size_t)v * 16,
+                         rebase(h, lay.lam) + (size_t)v * 4, rebase(h, lay.Ui) + (size_t)v * 16);
   PGPU_TRY(pgpu_stage_commit(ctx, lay.bytes));
 
-  // device scratch: eigen systems, P matrices, tip rows, per-CTA partial sums
+  // device scratch: eigen systems, P matrices, leaf rows (every tip's, then
+  // the collapsed leaves'), their exponents, and per-CTA partial sums
   const int RT = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : 8;
   const size_t n_tiles = (n_pat + (PR_THREADS / RT) - 1) / (PR_THREADS / RT);
   const size_t SS = (size_t)S * S;
   const size_t coef = precision == 32 ? 4 : 8;   // float, double, or float pair
   const size_t p_bytes = align16((size_t)n_br * R * SS * coef);
-  const size_t tt_bytes =
-      align16((size_t)n * R * codes->n_codes * S * (precision == 32 ? 4 : 8));
-  void *deig, *dP, *dpart, *dtt;
-  PGPU_TRY(pgpu_buf(ctx, BUF_H, (size_t)V * (2 * SS + S) * 8 + (size_t)V * sizeof(int) + 64, &deig));
+  const size_t tip_rows = (size_t)n * R * codes->n_codes, made_rows = pp->made_rows;
+  const size_t rows_bytes = align16((tip_rows + made_rows) * row_bytes);
+  const int n_leaf = (int)pp->leaves.size();
+  void *dP, *dpart, *drows, *dexp;
   PGPU_TRY(pgpu_buf(ctx, BUF_I, (size_t)V * p_bytes, &dP));
   PGPU_TRY(pgpu_buf(ctx, BUF_G, std::max<size_t>(n_tiles, 1) * V * sizeof(double2), &dpart));
-  PGPU_TRY(pgpu_buf(ctx, BUF_J, (size_t)V * tt_bytes, &dtt));
-  double *dU = (double *)deig, *dUi = dU + V * SS, *dlam = dUi + V * SS;
-  int *dst = reinterpret_cast<int *>(dlam + (size_t)V * S);
+  PGPU_TRY(pgpu_buf(ctx, BUF_J, (size_t)V * rows_bytes, &drows));
+  // CTA counters and exponent flags (cleared by the setup kernel), then exponents
+  const size_t clear = align16((size_t)V * 2 * sizeof(int));
+  PGPU_TRY(pgpu_buf(ctx, BUF_E, clear + (size_t)V * made_rows * sizeof(int), &dexp));
+  const double *dU = rebase(d, lay.U), *dUi = rebase(d, lay.Ui), *dlam = rebase(d, lay.lam);
+  const int *dst = rebase(d, lay.status);
+  if (!host_eig) {
+    void *deig;
+    PGPU_TRY(pgpu_buf(ctx, BUF_H, (size_t)V * ((2 * SS + S) * 8 + sizeof(int)) + 64, &deig));
+    double *u = static_cast<double *>(deig);
+    int *st = reinterpret_cast<int *>(u + V * (2 * SS + S));
+    PGPU_TRY(pgpu_launch_eig(ctx, rebase(d, lay.Q), rebase(d, lay.pi), S, V, u, u + 2 * V * SS, u + V * SS, st));
+    dU = u;
+    dUi = u + V * SS;
+    dlam = u + 2 * V * SS;
+    dst = st;
+  }
   PruneArgs a;
-  a.tiptab = dtt;
-  a.tip_codes = tips;
   a.P = dP;
-  a.code_tab = rebase(d, lay.tab);
+  a.rows = drows;
+  a.done = static_cast<unsigned *>(dexp);
+  a.row_flag = static_cast<const int *>(dexp) + V;
+  a.row_exp = reinterpret_cast<const int *>(static_cast<const char *>(dexp) + clear);
   a.pi = rebase(d, lay.pi);
   a.probs = rebase(d, lay.probs);
   a.weights = weights;
   a.site_lnl = site_lnl_dev;
   a.partials = (double2 *)dpart;
-  a.ops = dops;
-  a.tip_seq = dseq;
+  a.lnl = lnl_dev;
+  a.ops = pp->d_ops;
+  a.leaf_unit = pp->d_unit;
   a.flag = ctx->d_flag;
   a.P_stride = p_bytes;
-  a.tab_stride = tt_bytes;
-  a.ld_pat = ld_pat;
+  a.rows_stride = rows_bytes;
+  a.exp_stride = made_rows;
+  a.exp_unit = (uint32_t)(tip_rows * (row_bytes / 16));
   a.n_pat = n_pat;
-  a.n_tips = n;
-  a.n_ops = (int)sch->ops.size();
-  a.n_codes = codes->n_codes;
+  a.n_ops = (int)pp->ops.size();
+  a.n_leaf = n_leaf;
   a.R = R;
   a.NP = 0;
-  a.depth = std::max(sch->max_depth, 1);
-  HostTips ht{host_tips, const_cast<uint8_t *>(tips), (size_t)n};
+  a.depth = pp->depth;
+  HostTips ht{host_tips, const_cast<uint8_t *>(tips), (size_t)n, ld_pat};
   const HostTips *htp = host_tips ? &ht : nullptr;
   ChunkPlan pl;
   if (n_pat > 0) {
@@ -675,27 +1006,49 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
     else if (precision == 48) PGPU_TRY(plan_prune<Ff32>(ctx, a, RT, V, htp, pl));
     else PGPU_TRY(plan_prune<Fp64>(ctx, a, RT, V, htp, pl));
   }
-  PGPU_TRY(pgpu_launch_eig(ctx, rebase(d, lay.Q), rebase(d, lay.pi), S, V, dU, dlam, dUi, dst));
-  // every model's P matrices, then every model's tip rows in FP64, stored in
-  // the form's value type: one launch each for all V models
-  PGPU_TRY(pgpu_launch_compose(ctx, dU, dlam, dUi, S, rebase(d, lay.brlen), n_br,
-                               rebase(d, lay.rates), R, precision == 64 ? (double *)dP : nullptr,
-                               precision == 64 ? nullptr : (float *)dP, false, dst,
-                               precision == 32 ? P32_MINUS_I : precision == 48 ? P32_PAIRS_ROWS4
-                                                                               : P32_PLAIN,
-                               V, p_bytes));
-  PGPU_TRY(pgpu_launch_tip_table(ctx, dU, dlam, dUi, S, rebase(d, lay.brlen), n,
-                                 rebase(d, lay.rates), R, rebase(d, lay.tab), codes->n_codes, dtt,
-                                 precision == 32 ? 0 : precision == 48 ? 3 : 2, dst, V, tt_bytes));
+  // every model's P matrices and tip rows, formed in FP64 and stored in the
+  // form's value type
+  PGPU_TRY(pgpu_launch_dna_setup(ctx, dU, dlam, dUi, V, rebase(d, lay.brlen), n, rebase(d, lay.rates), R,
+                                 rebase(d, lay.tab), codes->n_codes, precision, dP, p_bytes, drows,
+                                 rows_bytes, dst, a.done, const_cast<int *>(a.row_flag), 1));
   if (n_pat == 0) {
     PGPU_CUDA(ctx, cudaMemsetAsync(lnl_dev, 0, (size_t)V * sizeof(double), ctx->stream));
     return PGPU_OK;
   }
-  if (precision == 32) PGPU_TRY(launch_prune<Fp32>(ctx, a, RT, V, pl, htp != nullptr));
-  else if (precision == 48) PGPU_TRY(launch_prune<Ff32>(ctx, a, RT, V, pl, htp != nullptr));
-  else PGPU_TRY(launch_prune<Fp64>(ctx, a, RT, V, pl, htp != nullptr));
-  prune_finalize_kernel<<<V, 1024, 0, ctx->stream>>>((const double2 *)dpart, (int)n_tiles, lnl_dev);
-  return pgpu_after_launch(ctx, "prune_finalize_kernel");
+  TableArgs t{};
+  t.rows = drows;
+  t.P = dP;
+  t.leaves = pp->d_leaves;
+  t.made = pp->d_made;
+  t.row_exp = const_cast<int *>(a.row_exp);
+  t.row_flag = const_cast<int *>(a.row_flag);
+  t.P_stride = p_bytes;
+  t.rows_stride = rows_bytes;
+  t.exp_stride = made_rows;
+  t.exp_base = tip_rows;
+  t.R = R;
+  t.n_codes = codes->n_codes;
+  t.n_made = (int)pp->made.size();
+  t.status = dst;
+  const size_t most = (size_t)codes->n_codes * codes->n_codes * (pp->level == 3 ? codes->n_codes : 1);
+  t.blocks = (int)((most + 255) / 256);
+  // leaf indexes: of all patterns, or in pieces of at most 1 GB
+  const size_t tile = PR_THREADS / RT;
+  const size_t cols = std::min(n_tiles, std::max<size_t>(((size_t)1 << 29) / n_leaf / tile, 1)) * tile;
+  IndexArgs x{};
+  x.tip_codes = tips;
+  x.leaves = pp->d_leaves;
+  x.ld_pat = ld_pat;
+  x.ld_index = a.ld_index = cols;
+  x.n_pat = n_pat;
+  x.n_codes = codes->n_codes;
+  x.flag = ctx->d_flag;
+  void *dix;
+  PGPU_TRY(pgpu_buf(ctx, BUF_D, (size_t)n_leaf * cols * sizeof(uint16_t), &dix));
+  x.index = static_cast<uint16_t *>(dix);
+  if (precision == 32) return launch_prune<Fp32>(ctx, a, RT, V, pl, htp != nullptr, t, x, cols);
+  if (precision == 48) return launch_prune<Ff32>(ctx, a, RT, V, pl, htp != nullptr, t, x, cols);
+  return launch_prune<Fp64>(ctx, a, RT, V, pl, htp != nullptr, t, x, cols);
 }
 
 }  // namespace

@@ -459,7 +459,8 @@ __global__ void __launch_bounds__(128) tip_table_kernel(const TipTabArgs p) {
 // relative precision instead of being what is left of sums of order 1.
 //
 // The rate classes are interleaved in units of 16 bytes: unit k of class r of
-// a branch is at k R + r, the row of code c and class r of a tip at c R + r.
+// a branch is at k RT + r (RT >= R), the row of code c and class r of a tip at
+// c R + r.
 struct DnaSetupArgs {
   const double *U, *lam, *Ui;   // model m at 16 m, 4 m, 16 m
   const double *t;              // [2 n_tips - 2]
@@ -467,7 +468,7 @@ struct DnaSetupArgs {
   const double *code_tab;       // [n_codes][4]
   char *P, *rows;
   size_t P_stride, rows_stride;
-  int R, n_tips, n_codes, precision;
+  int R, RT, n_tips, n_codes, precision;
   const int *status;
   int *flag;
   unsigned *done;               // cleared: per model, then n_flags ints per model
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(128) dna_setup_kernel(const DnaSetupArgs p) {
   const double t = p.t[b];
   if (tid < 4 * R) e[tid >> 2][tid & 3] = expm1(p.lam[4 * m + (tid & 3)] * rates[tid >> 2] * t);
   __syncthreads();
-  char *P = p.P + m * p.P_stride + (size_t)b * R * (p.precision == 32 ? 64 : 128);
+  char *P = p.P + m * p.P_stride + (size_t)b * p.RT * (p.precision == 32 ? 64 : 128);
   for (int o = tid; o < R * 16; o += 128) {
     const int r = o >> 4, i = (o >> 2) & 3, j = o & 3;
     double d = 0.0;   // P - I; the identity below an effective time of 1e-10, as in compose_kernel
@@ -503,12 +504,12 @@ __global__ void __launch_bounds__(128) dna_setup_kernel(const DnaSetupArgs p) {
     const double v = i == j ? 1.0 + d : d;
     sP[r][i * 4 + j] = v;
     if (p.precision == 64) {
-      reinterpret_cast<double *>(P)[((2 * i + (j >> 1)) * R + r) * 2 + (j & 1)] = v;
+      reinterpret_cast<double *>(P)[((2 * i + (j >> 1)) * p.RT + r) * 2 + (j & 1)] = v;
     } else if (p.precision == 32) {
-      reinterpret_cast<float *>(P)[(i * R + r) * 4 + j] = (float)d;
+      reinterpret_cast<float *>(P)[(i * p.RT + r) * 4 + j] = (float)d;
     } else {
       // two rows at a time, {hi P[i][j], hi P[i+1][j], lo P[i][j], lo P[i+1][j]}
-      float *q = reinterpret_cast<float *>(P) + (((i >> 1) * 4 + j) * R + r) * 4 + (i & 1);
+      float *q = reinterpret_cast<float *>(P) + (((i >> 1) * 4 + j) * p.RT + r) * 4 + (i & 1);
       const float hi = (float)v;
       q[0] = hi;
       q[2] = (float)(v - (double)hi);
@@ -598,12 +599,12 @@ pgpu_status pgpu_launch_tip_table(pgpu_ctx *ctx, const double *U_dev, const doub
 
 pgpu_status pgpu_launch_dna_setup(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
                                   const double *Ui_dev, int n_models, const double *t_dev, int n_tips,
-                                  const double *rates_dev, int R, const double *code_tab_dev, int n_codes,
-                                  int precision, void *P_dev, size_t P_stride, void *rows_dev,
+                                  const double *rates_dev, int R, int RT, const double *code_tab_dev,
+                                  int n_codes, int precision, void *P_dev, size_t P_stride, void *rows_dev,
                                   size_t rows_stride, const int *status_dev, unsigned *done_dev,
                                   int *row_flag_dev, int n_flags) {
   DnaSetupArgs a{U_dev, lam_dev, Ui_dev, t_dev, rates_dev, code_tab_dev, (char *)P_dev, (char *)rows_dev,
-                 P_stride, rows_stride, R, n_tips, n_codes, precision, status_dev, ctx->d_flag, done_dev,
+                 P_stride, rows_stride, R, RT, n_tips, n_codes, precision, status_dev, ctx->d_flag, done_dev,
                  row_flag_dev, n_flags};
   dna_setup_kernel<<<dim3(2 * n_tips - 2, n_models), 128, 0, ctx->stream>>>(a);
   return pgpu_after_launch(ctx, "dna_setup_kernel");

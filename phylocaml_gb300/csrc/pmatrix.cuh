@@ -53,8 +53,8 @@ pgpu_status pgpu_launch_tip_table(pgpu_ctx *ctx, const double *U_dev, const doub
 // and row_flag_dev[m][n_flags].
 pgpu_status pgpu_launch_dna_setup(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
                                   const double *Ui_dev, int n_models, const double *t_dev, int n_tips,
-                                  const double *rates_dev, int R, const double *code_tab_dev, int n_codes,
-                                  int precision, void *P_dev, size_t P_stride, void *rows_dev,
+                                  const double *rates_dev, int R, int RT, const double *code_tab_dev,
+                                  int n_codes, int precision, void *P_dev, size_t P_stride, void *rows_dev,
                                   size_t rows_stride, const int *status_dev, unsigned *done_dev,
                                   int *row_flag_dev, int n_flags);
 

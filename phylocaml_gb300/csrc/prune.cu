@@ -53,8 +53,8 @@ namespace {
 using namespace pgpu_forms;
 
 struct PruneArgs {
-  const uint16_t *index;      // [n_leaf][ld_index]: each pattern's row of the leaf
-  const void *P;              // per branch: 16-byte unit k of rate class r at k R + r
+  const uint16_t *index;      // [n_leaf + PR_PAD][ld_index]: each pattern's row of the leaf
+  const void *P;              // per branch: 16-byte unit k of rate class r at k RT + r
   const void *rows;           // leaf rows, [n_codes^k][R] per leaf (form's values)
   const int *row_exp;         // power of two taken out of each collapsed leaf's row
   const int *row_flag;        // per model: some exponent is not zero
@@ -65,7 +65,7 @@ struct PruneArgs {
   double2 *partials;          // [n_models][n_tiles_total], by tile
   unsigned *done;             // [n_models] CTAs finished, zeroed by the setup kernel
   double *lnl;                // [n_models]
-  const int4 *ops;            // {branch of the internal first child or -1, ... second, -, -}
+  const int4 *ops;            // {internal children, branch of the first, of the second, -}
   const uint32_t *leaf_unit;  // 16-byte unit of each leaf's first row, in the order the steps read them
   int *flag;
   // several models over the same tree and patterns: CTA row blockIdx.y
@@ -80,13 +80,14 @@ struct PruneArgs {
   size_t index_col;           // pattern of index's first column
   size_t ld_index, n_pat;
   uint32_t exp_unit;          // unit of row_exp's first row
-  int n_ops, n_leaf, n_codes, R, NP, depth;
+  int n_ops, n_leaf, R, NP, depth;
 };
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 constexpr int PR_THREADS = 256;   // consumer threads per CTA
 constexpr int PR_LEAVES = 3;      // leaf rows in flight per thread
+constexpr int PR_PAD = PR_LEAVES + 1;   // row-0 leaves after the last, so that the pipeline runs on unchecked
 
 // CTAs each SM should hold, and growth: how much larger each column chunk of
 // host tip codes is than the one before; a chunk's copy must end while the
@@ -103,25 +104,26 @@ template <> struct PruneTune<pgpu_forms::Fp32> {
 // Ring of the coefficient blocks, in postorder steps (a power of two).  The
 // producer stages PR_GROUP consecutive steps under one mbarrier phase, so
 // the consumers wait and release once per group.
-constexpr int PR_STAGES = 8, PR_GROUP = 2;
+constexpr int PR_STAGES = 8, PR_GROUP = 4;
 
 // Shared memory of one CTA: the ring of step slots (the coefficient blocks
-// R x 16 of the first and the second child, where internal), the threads'
+// RT x 16 of the internal children), the threads'
 // leaf slots, then the CLV stack (the results set aside: one less than the
 // schedule's depth, the top being in registers).
 template <typename Pol>
 struct PruneLayout {
   using V = typename Pol::V;
   using Coef = typename Pol::Coef;
-  __host__ __device__ static size_t coef_bytes(int R) { return (size_t)R * 16 * sizeof(Coef); }
-  __host__ __device__ static size_t slot_bytes(int R) { return (2 * coef_bytes(R) + 127) & ~size_t(127); }
-  __host__ __device__ static size_t ring_off() { return 128; }
-  __host__ __device__ static size_t leaf_off(int R) { return ring_off() + PR_STAGES * slot_bytes(R); }
-  __host__ __device__ static size_t stk_off(int R) {
-    return leaf_off(R) + (size_t)PR_LEAVES * 4 * PR_THREADS * sizeof(V);
+  __host__ __device__ static constexpr uint32_t coef_bytes(int RT) { return (uint32_t)(RT * 16 * sizeof(Coef)); }
+  __host__ __device__ static constexpr uint32_t ring_off() { return 128; }
+  __host__ __device__ static constexpr uint32_t leaf_off(int RT) {
+    return ring_off() + PR_STAGES * 2 * coef_bytes(RT);
   }
-  __host__ __device__ static size_t bytes(int R, int depth) {
-    return stk_off(R) + (size_t)(depth > 1 ? depth - 1 : 0) * 4 * PR_THREADS * sizeof(V);
+  __host__ __device__ static constexpr uint32_t stk_off(int RT) {
+    return leaf_off(RT) + (uint32_t)(PR_LEAVES * 4 * PR_THREADS * sizeof(V));
+  }
+  __host__ __device__ static size_t bytes(int RT, int depth) {
+    return stk_off(RT) + (size_t)(depth > 1 ? depth - 1 : 0) * 4 * PR_THREADS * sizeof(V);
   }
 };
 
@@ -149,7 +151,8 @@ __device__ __forceinline__ auto largest(const typename Pol::V *acc) {
 
 // Rows of the collapsed leaves: P(t_v) CLV_v for every combination of the
 // leaf's codes, (c0 n + c1) for tips 0 and 1, ((c0 n + c1) n + c2) with tip 2
-// beside the cherry of tips 0 and 1.  A thread per combination.
+// beside the cherry of tips 0 and 1.  A thread per (c0, c1), which forms the
+// cherry once for every c2.
 struct TableArgs {
   void *rows;            // tips' rows first: [n_tips][n_codes][R]
   const void *P;
@@ -158,7 +161,7 @@ struct TableArgs {
   int *row_exp, *row_flag;
   size_t P_stride, rows_stride, exp_stride;
   size_t exp_base;       // row of row_exp's first entry
-  int R, n_codes, n_made, blocks;   // blocks: CTAs per (leaf, rate class)
+  int R, RT, n_codes, n_made, blocks;   // blocks: CTAs per (leaf, rate class)
   const int *status;     // model m at m
 };
 
@@ -171,33 +174,46 @@ struct IndexArgs {
   const int4 *leaves;         // {tip, tip or -1, tip or -1, first row}
   uint16_t *index;            // [n_leaf][ld_index], column 0 = pattern col0
   size_t ld_pat, ld_index, col0, cols, n_pat;
-  int n_codes, blocks;        // blocks: CTAs per leaf, 1,024 patterns each
+  int n_codes, blocks;        // blocks: CTAs per leaf, 256 x IX_PATTERNS patterns each
   int *flag;
 };
 
+// 16 patterns per thread: one 16-byte load per tip and two 16-byte stores
+// (128 against 220 us for 256 leaves of 446,427 patterns with 4).
+constexpr int IX_PATTERNS = 16;
+
 __device__ __forceinline__ void leaf_index(const IndexArgs &p, int block) {
   const int4 lf = __ldg(p.leaves + block / p.blocks);
-  const size_t col = ((size_t)(block % p.blocks) * 256 + threadIdx.x) * 4;
+  const size_t col = ((size_t)(block % p.blocks) * 256 + threadIdx.x) * IX_PATTERNS;
   if (col >= p.cols) return;
-  const size_t pat = p.col0 + col;   // a multiple of 4, and rows are multiples of 16 long
-  uint32_t row[4] = {0, 0, 0, 0};
+  const size_t pat = p.col0 + col;   // a multiple of 16, as are the rows' lengths
   const uint32_t top = (uint32_t)p.n_codes - 1u;
+  const int tips[3] = {lf.x, lf.y, lf.z};
+  uint4 w[3];
+#pragma unroll
+  for (int h = 0; h < 3; ++h)
+    if (tips[h] >= 0) w[h] = __ldg(reinterpret_cast<const uint4 *>(p.tip_codes + (size_t)tips[h] * p.ld_pat + pat));
+  uint32_t row[IX_PATTERNS];
+#pragma unroll
+  for (int q = 0; q < IX_PATTERNS; ++q) row[q] = 0u;
   bool bad = false;
 #pragma unroll
   for (int h = 0; h < 3; ++h) {
-    const int t = h == 0 ? lf.x : h == 1 ? lf.y : lf.z;
-    if (t < 0) break;
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(p.tip_codes + (size_t)t * p.ld_pat + pat));
+    if (tips[h] < 0) break;
+    const uint32_t v[4] = {w[h].x, w[h].y, w[h].z, w[h].w};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t c = (w >> (8 * q)) & 255u;
+    for (int q = 0; q < IX_PATTERNS; ++q) {
+      const uint32_t c = (v[q / 4] >> (8 * (q % 4))) & 255u;
       bad |= c > top && pat + q < p.n_pat;
       row[q] = row[q] * (uint32_t)p.n_codes + min(c, top);
     }
   }
   if (bad) atomicOr(p.flag, PGPU_FLAG_BADCODE);
-  *reinterpret_cast<uint2 *>(p.index + (size_t)(block / p.blocks) * p.ld_index + col) =
-      make_uint2(row[0] | row[1] << 16, row[2] | row[3] << 16);
+  uint4 *out = reinterpret_cast<uint4 *>(p.index + (size_t)(block / p.blocks) * p.ld_index + col);
+#pragma unroll
+  for (int q = 0; q < IX_PATTERNS; q += 8)
+    out[q / 8] = make_uint4(row[q] | row[q + 1] << 16, row[q + 2] | row[q + 3] << 16,
+                            row[q + 4] | row[q + 5] << 16, row[q + 6] | row[q + 7] << 16);
 }
 
 // CTAs 0 .. n_table - 1: the collapsed leaves' rows (model by model); the
@@ -215,36 +231,43 @@ __global__ void __launch_bounds__(256) prune_prep_kernel(const TableArgs p, cons
   const int4 mk = __ldg(p.made + lr / p.R);
   const int r = lr % p.R, NC = p.n_codes;
   const int4 lf = __ldg(p.leaves + mk.x);
-  const bool three = lf.z >= 0;
-  const int n = three ? NC * NC * NC : NC * NC;
-  const int q = (at_block % p.blocks) * 256 + threadIdx.x;
-  if (q >= n || p.status[m]) return;
+  const int q = (at_block % p.blocks) * 256 + threadIdx.x;   // codes of tips 0 and 1
+  if (q >= NC * NC || p.status[m]) return;
   char *rows = static_cast<char *>(p.rows) + m * p.rows_stride;
   const char *P = static_cast<const char *>(p.P) + m * p.P_stride;
   auto coef = [&](int branch) {
-    return reinterpret_cast<const Coef *>(P + (size_t)branch * p.R * 16 * sizeof(Coef) + 16 * r);
+    return reinterpret_cast<const Coef *>(P + (size_t)branch * p.RT * 16 * sizeof(Coef) + 16 * r);
   };
   auto tip = [&](int t, int c, V *y) { Pol::load_tip(rows, ((size_t)t * NC + c) * p.R + r, y); };
-  const int c01 = three ? q / NC : q;
-  V x[4], y[4], acc[4];
-  int ex = 0;
-  tip(lf.x, c01 / NC, x);
-  tip(lf.y, c01 % NC, y);
-  Pol::mul4(x, y, acc);
-  auto mx = largest<Pol>(acc);
-  if (mx < Pol::thresh) rescale_vec<Pol>(acc, mx, ex);
-  if (three) {
-    Pol::rows(coef(mk.z), acc, x, p.R);
-    tip(lf.z, q % NC, y);
+  auto node = [&](const V *x, const V *y, V *acc, int ex) {
     Pol::mul4(x, y, acc);
-    mx = largest<Pol>(acc);
+    const auto mx = largest<Pol>(acc);
     if (mx < Pol::thresh) rescale_vec<Pol>(acc, mx, ex);
+    return ex;
+  };
+  auto put = [&](const V *x, int combination, int ex) {
+    const size_t at = (size_t)(uint32_t)lf.w + (size_t)combination * p.R + r;
+    Pol::store4(rows, at, x);
+    p.row_exp[m * p.exp_stride + (at - p.exp_base)] = ex;
+    if (ex) p.row_flag[m] = 1;   // every writer writes 1
+  };
+  V x[4], y[4], acc[4];
+  tip(lf.x, q / NC, x);
+  tip(lf.y, q % NC, y);
+  const int ex = node(x, y, acc, 0);
+  if (lf.z < 0) {
+    Pol::rows(coef(mk.y), acc, x, p.RT);
+    put(x, q, ex);
+    return;
   }
-  Pol::rows(coef(mk.y), acc, x, p.R);
-  const size_t at = (size_t)(uint32_t)lf.w + (size_t)q * p.R + r;
-  Pol::store4(rows, at, x);
-  p.row_exp[m * p.exp_stride + (at - p.exp_base)] = ex;
-  if (ex) p.row_flag[m] = 1;   // every writer writes 1
+  V cherry[4];
+  Pol::rows(coef(mk.z), acc, cherry, p.RT);
+  for (int c = 0; c < NC; ++c) {
+    tip(lf.z, c, y);
+    const int e2 = node(cherry, y, acc, ex);
+    Pol::rows(coef(mk.y), acc, x, p.RT);
+    put(x, q * NC + c, e2);
+  }
 }
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
@@ -260,9 +283,10 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
 // touched up to 32, and the line lookups bounded the kernel.
 //
 // Bound by the float-pair arithmetic of the rows and products (FMA pipe).
-// 512 taxa x 446,427 patterns, 4 rate classes, pair form: TIME_NEW with the
-// collapsed subtrees (about half the steps), 7.12 ms walking every node with
-// the tip rows staged per step by the producer.
+// 512 taxa x 446,427 patterns, 4 rate classes, pair form: 4.02 ms with
+// the collapsed subtrees (about half the steps), 7.12 ms walking every node
+// with the tip rows staged per step by the producer; issue slots 58 %, FMA
+// pipe 53 %.
 template <typename Pol, int RT>
 __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
     prune_tree_kernel(const PruneArgs p) {
@@ -275,18 +299,18 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ double2 red[NT / 32];
   __shared__ double2 xch[RT][NT / RT];   // per pattern and rate class: (part, scaler)
-  __shared__ int step_kind[ST];          // per step slot: which of the consumer's step cases
+  __shared__ int step_kind[ST];          // per step slot: internal children
   __shared__ int last_cta;
-  const int NP = p.NP, R = p.R;
+  constexpr int NP = NT / RT;
+  const int R = p.R;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);     // [NB]
   uint64_t *empty = full + NB;                              // [NB]
-  const size_t SB = L::slot_bytes(R);
+  constexpr uint32_t CB = L::coef_bytes(RT), SB = 2 * CB;
   unsigned char *ring = smem + L::ring_off();               // [ST][SB]
-  V *stk = reinterpret_cast<V *>(smem + L::stk_off(R));     // [depth - 1][4][NT]
+  V *stk = reinterpret_cast<V *>(smem + L::stk_off(RT));    // [depth - 1][4][NT]
   const size_t tile = p.tile_base + blockIdx.x;
   const size_t tile0 = tile * NP;
   const int tid = threadIdx.x;
-  const size_t CB = L::coef_bytes(R);
 
   if (tid == 0) {
     for (int s = 0; s < NB; ++s) {
@@ -311,20 +335,16 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
         int4 ops[G];
         uint32_t tx = 0;
         for (int k = 0; k < gn; ++k) {
-          const int4 op = __ldg(p.ops + g0 + k);
-          ops[k] = op;
-          tx += (op.x >= 0 ? (uint32_t)CB : 0u) + (op.y >= 0 ? (uint32_t)CB : 0u);
-          // bit 0: first child internal, bit 1: second child internal; 4
-          // marks the first step, which has no earlier result to set aside.
-          // The arrive below releases these stores to the consumers' wait.
-          const int kind = (op.x >= 0 ? 1 : 0) | (op.y >= 0 ? 2 : 0);
-          step_kind[(g0 + k) & (ST - 1)] = g0 + k == 0 ? 4 : kind;
+          ops[k] = __ldg(p.ops + g0 + k);
+          tx += (uint32_t)ops[k].x * CB;
+          // the arrive below releases this store to the consumers' wait
+          step_kind[(g0 + k) & (ST - 1)] = ops[k].x;
         }
         mbar_arrive_expect_tx(&full[b], tx);
         for (int k = 0; k < gn; ++k) {
           unsigned char *sl = ring + (size_t)((g0 + k) & (ST - 1)) * SB;
-          if (ops[k].x >= 0) bulk_g2s(sl, Pg + (size_t)ops[k].x * CB, (uint32_t)CB, &full[b]);
-          if (ops[k].y >= 0) bulk_g2s(sl + CB, Pg + (size_t)ops[k].y * CB, (uint32_t)CB, &full[b]);
+          if (ops[k].x > 0) bulk_g2s(sl, Pg + (size_t)ops[k].y * CB, CB, &full[b]);
+          if (ops[k].x > 1) bulk_g2s(sl + CB, Pg + (size_t)ops[k].z * CB, CB, &full[b]);
         }
         groups = q + 1;
       }
@@ -338,132 +358,94 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   const int c = tid - 32, lane = tid & 31;
   const int r = c % RT, pl = c / RT;
   const size_t pat = tile0 + pl;
-  const bool active = pat < p.n_pat;
-  const bool rate_on = r < R;
   // lanes of a rate class beyond R (R < RT) repeat class R - 1 and are
   // dropped at the root, so the step loop has no branch on the rate
   const int rr = min(r, R - 1);
 
-  // leaf pipeline: this thread's slots take turns; the next leaf's index is
-  // read a leaf before its row is gathered
-  const uint16_t *index = p.index + ((active ? pat : p.n_pat - 1) - p.index_col);   // idle lanes repeat the last pattern
-  const uint32_t *unit = p.leaf_unit;
+  // leaf pipeline: the slots hold the rows of the next PR_LEAVES leaves, get
+  // the first of them; a slot is refilled with the row PR_LEAVES on as soon
+  // as its values are in use, by an index read a leaf before that
+  const uint16_t *index = p.index + (min(pat, p.n_pat - 1) - p.index_col);   // idle lanes repeat the last pattern
   const char *rows = static_cast<const char *>(p.rows) + blockIdx.y * p.rows_stride + (size_t)rr * (4 * sizeof(V));
+  const uint32_t *unit = p.leaf_unit;
   const uint32_t RU = (uint32_t)R * VU;
   constexpr uint32_t SLOT = VU * NT * 16u;
-  const uint32_t slot0 = smem_u32(smem + L::leaf_off(R)) + 16u * c;   // [slot][VU][NT] of 16 bytes
-  uint32_t put = slot0, get = slot0;
+  const uint32_t slot0 = smem_u32(smem + L::leaf_off(RT)) + 16u * c;   // [slot][VU][NT] of 16 bytes
   const bool scaled_rows = p.row_flag[blockIdx.y] != 0;
-  int to_read = p.n_leaf, to_gather = p.n_leaf, pending = 0, escale = 0;
-  uint32_t next_row = 0, next_unit = 0;
-  auto read_index = [&]() {
-    if (to_read > 0) {
-      next_row = __ldg(index);
-      next_unit = __ldg(unit);
-      index += p.ld_index;
-      ++unit;
-      --to_read;
-    }
-  };
-  auto gather = [&]() {
-    if (to_gather > 0) {
-      const uint32_t u = next_unit + next_row * RU;
-      const char *src = rows + (size_t)u * 16;
+  int escale = 0;
+  uint32_t next_row = __ldg(index), next_unit = __ldg(unit);
+  auto after = [&](uint32_t slot) { return slot == slot0 + (PR_LEAVES - 1) * SLOT ? slot0 : slot + SLOT; };
+  auto refill = [&](uint32_t slot) {
+    const uint32_t u = next_unit + next_row * RU;
+    const char *src = rows + (size_t)u * 16;
 #pragma unroll
-      for (int k = 0; k < VU; ++k) cp_async_16(put + k * NT * 16u, src + 16 * k);
-      if (scaled_rows && u >= p.exp_unit)
-        escale += __ldg(p.row_exp + blockIdx.y * p.exp_stride + (u - p.exp_unit) / VU + rr);
-      put = put + SLOT == slot0 + PR_LEAVES * SLOT ? slot0 : put + SLOT;
-      --to_gather;
-      read_index();
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");   // empty groups keep the count in step
+    for (int k = 0; k < VU; ++k) cp_async_16(slot + k * NT * 16u, src + 16 * k);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (scaled_rows && u >= p.exp_unit)
+      escale += __ldg(p.row_exp + blockIdx.y * p.exp_stride + (u - p.exp_unit) / VU + rr);
+    index += p.ld_index;
+    next_row = __ldg(index);
+    next_unit = __ldg(++unit);
   };
-  // the next leaf's row into y; PEND of the younger groups may be in flight
-  auto leaf_row = [&](V *y, auto pend) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(decltype(pend)::value) : "memory");
-    Pol::load_row_s(get, get + NT * 16u, y);
-    get = get + SLOT == slot0 + PR_LEAVES * SLOT ? slot0 : get + SLOT;
-    ++pending;
-  };
-  using Pend0 = std::integral_constant<int, PR_LEAVES - 1>;   // the next leaf
-  using Pend1 = std::integral_constant<int, PR_LEAVES - 2>;   // the one after it
-  read_index();
+  uint32_t get = slot0;
 #pragma unroll
-  for (int j = 0; j < PR_LEAVES; ++j) gather();
+  for (int j = 0; j < PR_LEAVES; ++j) refill(slot0 + j * SLOT);
 
   // The stack discipline is fixed by the schedule: in postorder the result
-  // of step i - 1 is always the second child of step i when that child is
-  // internal, else its first child when that one is internal; a step with
-  // two leaves leaves it pending (push), and a step with two internal
-  // children takes its first child from the stack (pop).  So the top of the
-  // stack lives in registers and each step is one of four straight-line
-  // cases, chosen by a warp-uniform branch.
+  // of step i - 1 is always a child of step i when any child of it is
+  // internal; a step with two leaves sets the previous result aside (push),
+  // and a step with two internal children takes its first child from the
+  // stack (pop).  So the top of the stack lives in registers and each step is
+  // one of three straight-line cases, chosen by a warp-uniform branch.
   V top[4];
   V *my = stk + c;   // this thread's column of the stack: entry (k, e) at my[(4 k + e) NT]
-  int sp = 0;
+  int sp = -1;       // entries set aside, -1 before the first step
   bool ok = true;
-  const size_t coefb = (size_t)rr * 16;
+  const unsigned char *coefs = ring + rr * 16;
 
-  for (int g0 = 0; g0 < p.n_ops && ok; g0 += G) {
+#pragma unroll 1
+  for (int g0 = 0; g0 < p.n_ops; g0 += G) {
     const int q = g0 / G, b = q & (NB - 1);
-    const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[b], (q / NB) & 1, p.flag));
-    if (!got) {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[b], (q / NB) & 1, p.flag))) {
       ok = false;
       break;
     }
+    const int g1 = min(g0 + G, p.n_ops);
+#pragma unroll 1
+    for (int i = g0; i < g1; ++i) {
+      const int slot = i & (ST - 1), kind = step_kind[slot];
+      const Coef *coef = reinterpret_cast<const Coef *>(coefs + slot * SB);
+      V acc[4], y0[4], y1[4];
+      if (kind == 1) {          // the previous result and a leaf
+        asm volatile("cp.async.wait_group %0;" ::"n"(PR_LEAVES - 1) : "memory");
+        Pol::load_row_s(get, get + NT * 16u, y1);
+        Pol::rows(coef, top, y0, RT);
+        Pol::mul4(y0, y1, acc);
+        refill(get);
+        get = after(get);
+      } else if (kind == 0) {   // two leaves; the previous result waits on the stack
+        if (sp >= 0) {
 #pragma unroll
-    for (int k = 0; k < G; ++k) {
-      const int i = g0 + k;
-      if (i >= p.n_ops) break;
-      const int slot = i & (ST - 1);
-      const int kind = step_kind[slot];
-      const unsigned char *sl = ring + (size_t)slot * SB + coefb;
-      V acc[4];
-      {
-        auto coef = [&](int h) { return reinterpret_cast<const Coef *>(sl + h * CB); };
-        V y0[4], y1[4];
-        switch (kind) {
-          case 0:   // two leaves; the previous result waits on the stack
-            if (sp + 1 < p.depth) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) my[(4 * sp + e) * NT] = top[e];
-              ++sp;
-            } else {
-              ok = false;   // schedule and stack size disagree
-            }
-            [[fallthrough]];
-          case 4:   // the first step: two leaves, nothing to set aside
-            leaf_row(y0, Pend0{});
-            leaf_row(y1, Pend1{});
-            break;
-          case 1:   // internal first child (the previous result), leaf second
-            Pol::rows(coef(0), top, y0, R);
-            leaf_row(y1, Pend0{});
-            break;
-          case 2:   // leaf first, internal second child (the previous result)
-            Pol::rows(coef(1), top, y1, R);
-            leaf_row(y0, Pend0{});
-            break;
-          default: {   // 3, both internal: the first from the stack
-            V xa[4];
-            if (sp > 0) {
-              --sp;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) xa[e] = my[(4 * sp + e) * NT];
-            } else {
-              ok = false;   // schedule and stack disagree
-#pragma unroll
-              for (int e = 0; e < 4; ++e) xa[e] = Pol::zero();
-            }
-            Pol::rows(coef(0), xa, y0, R);
-            Pol::rows(coef(1), top, y1, R);
-          }
+          for (int e = 0; e < 4; ++e) my[(4 * sp + e) * NT] = top[e];
         }
+        ++sp;
+        asm volatile("cp.async.wait_group %0;" ::"n"(PR_LEAVES - 2) : "memory");
+        const uint32_t second = after(get);
+        Pol::load_row_s(get, get + NT * 16u, y0);
+        Pol::load_row_s(second, second + NT * 16u, y1);
+        Pol::mul4(y0, y1, acc);
+        refill(get);
+        refill(second);
+        get = after(second);
+      } else {                  // both internal: the first from the stack
+        --sp;
+        V xa[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) xa[e] = my[(4 * sp + e) * NT];
+        Pol::rows(coef, xa, y0, RT);
+        Pol::rows(reinterpret_cast<const Coef *>(coefs + slot * SB + CB), top, y1, RT);
         Pol::mul4(y0, y1, acc);
       }
-      // the slots read above are refilled once their values are in use
-      for (; pending > 0; --pending) gather();
       // rare, so the warp only enters when some lane needs it
       const auto mx = largest<Pol>(acc);
       if (__any_sync(0xffffffffu, mx < Pol::thresh)) {
@@ -481,7 +463,7 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   // root: sum over rate classes of probs[r] 2^e_r sum_i pi_i x_i, in FP64;
   // the rate classes of a pattern meet in shared memory
   double part = 0.0;
-  if (ok && rate_on) {
+  if (ok && r < R) {
     const double *pi = p.pi + (size_t)blockIdx.y * 4, *probs = p.probs + (size_t)blockIdx.y * R;
     double lr = 0.0;
 #pragma unroll
@@ -491,18 +473,21 @@ __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
   xch[r][pl] = make_double2(part, (double)escale);
   asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
   double s = 0.0, comp = 0.0;
-  if (r == 0) {
+  // the first NP threads take a pattern each: FP64 costs a warp the same
+  // however few of its lanes work
+  if (c < NP) {
     int emax = -0x7fffffff;
-    for (int q = 0; q < R; ++q) emax = max(emax, (int)xch[q][pl].y);
+    for (int q = 0; q < R; ++q) emax = max(emax, (int)xch[q][c].y);
     double site = 0.0;
     for (int q = 0; q < R; ++q) {
-      const double2 v = xch[q][pl];
+      const double2 v = xch[q][c];
       site += ldexp(v.x, (int)v.y - emax);
     }
-    if (ok && active) {
+    const size_t mine = tile0 + c;
+    if (ok && mine < p.n_pat) {
       const double lnl = log(site) + (double)emax * 0.69314718055994530942;
-      if (p.site_lnl) p.site_lnl[pat] = lnl;
-      s = p.weights ? p.weights[pat] * lnl : lnl;
+      if (p.site_lnl) p.site_lnl[mine] = lnl;
+      s = p.weights ? p.weights[mine] * lnl : lnl;
     }
   }
   warp_csum(s, comp);
@@ -613,7 +598,7 @@ pgpu_status plan_prune(pgpu_ctx *ctx, PruneArgs &a, int RT, int n_models, const 
   const size_t n_tiles = (a.n_pat + a.NP - 1) / a.NP;
   a.n_tiles_total = n_tiles;
   a.tile_base = 0;
-  pl.smem = PruneLayout<Pol>::bytes(a.R, a.depth);
+  pl.smem = PruneLayout<Pol>::bytes(RT, a.depth);
   if (pl.smem > ctx->smem_optin)
     return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: %zu bytes of shared memory needed (tree too deep)",
                         pl.smem);
@@ -642,7 +627,7 @@ pgpu_status launch_prep(pgpu_ctx *ctx, const TableArgs &t, int n_models, IndexAr
   const size_t n_table = tables ? (size_t)t.n_made * t.R * t.blocks * n_models : 0;
   x.col0 = pat0;
   x.cols = pat1 - pat0;
-  x.blocks = (int)((x.cols + 1023) / 1024);
+  x.blocks = (int)((x.cols + 256 * IX_PATTERNS - 1) / (256 * IX_PATTERNS));
   const size_t grid = n_table + (size_t)n_leaf * x.blocks;
   if (grid == 0) return PGPU_OK;
   if (grid > 0x7fffffff) return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: too many patterns and leaves");
@@ -827,9 +812,9 @@ pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes,
       pl.made_rows += (size_t)R * NC * NC * (cherry >= 0 ? NC : 1);
       leaf.push_back(lf);
     }
-    const size_t n_rows = (size_t)n * R * NC + pl.made_rows, most = NC * NC * (level == 3 ? NC : 1);
+    const size_t n_rows = (size_t)n * R * NC + pl.made_rows;
     if (level > 1 && (n_rows > 0x7fffffffull || pl.made_rows * call_bytes > (size_t)1 << 30 ||
-                      pl.made.size() * R * ((most + 255) / 256) > 0x7fffffff))
+                      pl.made.size() * R * ((NC * NC + 255) / 256) > 0x7fffffff))
       continue;
     if (n_rows > 0x7fffffffull) return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "prune: 2^31 leaf rows or more");
     pl.level = level;
@@ -844,13 +829,17 @@ pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes,
     }
     pgpu_tree red{nl, left.data(), right.data(), nullptr};
     PGPU_TRY(pgpu_build_schedule(ctx, &red, &sch));
-    // steps, and the leaves in the order the steps read them
+    // steps, and the leaves in the order the steps read them, then row 0
+    // of the first tip PR_PAD times
     std::vector<int32_t> place(nl);
     for (int32_t j = 0; j < nl; ++j) place[sch.tip_seq[j]] = j;
     pl.ops.clear();
-    for (const SchedOp &op : sch.ops)
-      pl.ops.push_back(make_int4(op.a >= nl ? branch[op.a] : -1, op.b >= nl ? branch[op.b] : -1, 0, 0));
-    pl.leaves.assign(nl, int4());
+    for (const SchedOp &op : sch.ops) {
+      const int br[2] = {op.a >= nl ? branch[op.a] : -1, op.b >= nl ? branch[op.b] : -1};
+      const int k = (br[0] >= 0) + (br[1] >= 0);
+      pl.ops.push_back(make_int4(k, br[0] >= 0 ? br[0] : br[1], br[1], 0));
+    }
+    pl.leaves.assign(nl + PR_PAD, make_int4(-1, -1, -1, 0));
     for (int32_t j = 0; j < nl; ++j) pl.leaves[j] = leaf[sch.tip_seq[j]];
     for (int4 &m : pl.made) m.x = place[m.x];
     pl.depth = std::max(sch.max_depth, 1);
@@ -949,10 +938,10 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   const size_t n_tiles = (n_pat + (PR_THREADS / RT) - 1) / (PR_THREADS / RT);
   const size_t SS = (size_t)S * S;
   const size_t coef = precision == 32 ? 4 : 8;   // float, double, or float pair
-  const size_t p_bytes = align16((size_t)n_br * R * SS * coef);
+  const size_t p_bytes = align16((size_t)n_br * RT * SS * coef);
   const size_t tip_rows = (size_t)n * R * codes->n_codes, made_rows = pp->made_rows;
   const size_t rows_bytes = align16((tip_rows + made_rows) * row_bytes);
-  const int n_leaf = (int)pp->leaves.size();
+  const int n_leaf = (int)pp->leaves.size();   // the padding included
   void *dP, *dpart, *drows, *dexp;
   PGPU_TRY(pgpu_buf(ctx, BUF_I, (size_t)V * p_bytes, &dP));
   PGPU_TRY(pgpu_buf(ctx, BUF_G, std::max<size_t>(n_tiles, 1) * V * sizeof(double2), &dpart));
@@ -1008,7 +997,7 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   }
   // every model's P matrices and tip rows, formed in FP64 and stored in the
   // form's value type
-  PGPU_TRY(pgpu_launch_dna_setup(ctx, dU, dlam, dUi, V, rebase(d, lay.brlen), n, rebase(d, lay.rates), R,
+  PGPU_TRY(pgpu_launch_dna_setup(ctx, dU, dlam, dUi, V, rebase(d, lay.brlen), n, rebase(d, lay.rates), R, RT,
                                  rebase(d, lay.tab), codes->n_codes, precision, dP, p_bytes, drows,
                                  rows_bytes, dst, a.done, const_cast<int *>(a.row_flag), 1));
   if (n_pat == 0) {
@@ -1027,11 +1016,11 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   t.exp_stride = made_rows;
   t.exp_base = tip_rows;
   t.R = R;
+  t.RT = RT;
   t.n_codes = codes->n_codes;
   t.n_made = (int)pp->made.size();
   t.status = dst;
-  const size_t most = (size_t)codes->n_codes * codes->n_codes * (pp->level == 3 ? codes->n_codes : 1);
-  t.blocks = (int)((most + 255) / 256);
+  t.blocks = (codes->n_codes * codes->n_codes + 255) / 256;
   // leaf indexes: of all patterns, or in pieces of at most 1 GB
   const size_t tile = PR_THREADS / RT;
   const size_t cols = std::min(n_tiles, std::max<size_t>(((size_t)1 << 29) / n_leaf / tile, 1)) * tile;

@@ -23,16 +23,24 @@
 // One thread per (pattern, rate class): RL = the power of two >= R lanes
 // per pattern, so a pattern's maximum is a shuffle over its lanes.  Loads
 // of a child's vector are contiguous per thread and contiguous across the
-// warp, so the kernel streams at HBM speed; P blocks are read through the
-// read-only cache.  Each CTA writes a compensated partial of its cost, and
-// the last CTA to finish adds the partials in CTA order, so costs are
-// deterministic.
+// warp.  Integer weights make a node's cost an exact integer sum, one atomic
+// add per CTA; with fractional weights each CTA writes a compensated partial
+// and the last CTA adds them in CTA order, so costs are deterministic.
+//
+// Four states (clv_median4_kernel): a branch's P matrices are 16 numbers per
+// rate class, formed on the host when its length is set and passed with the
+// launch, and a leaf is its codes -- a CTA forms P x for every code in shared
+// memory -- so a leaf is one copy, a branch length no device work, and a
+// median one launch that reads n_pat bytes for a leaf instead of n_pat R S
+// values.  Other state counts build P in a launch per branch and store
+// leaves as vectors.
 //
 // Handles are allocated stream-ordered (cudaMallocAsync) on the context's
 // stream; passing the node's previous value (the reference's `t option`)
 // reuses its memory instead.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "pgpu_internal.cuh"
@@ -54,22 +62,38 @@ struct pgpu_lk {
   // sum_p w_p e_p in int64 on the integer units, the FP64 units being slow
   bool int_w = false;
   int32_t *wint = nullptr;   // [n_pat] or null (all 1)
-  long long *ipart = nullptr;   // per-CTA integer partial sums
   unsigned *counter = nullptr;
   size_t n_cta = 0;
   long long live = 0;        // handles not yet destroyed
+  double *zero = nullptr;    // a leaf's cost
+  // four states: the eigen system on the host, the code table in the storage
+  // type, and whether leaves stay codes (their rows fit shared memory)
+  double hU[16] = {}, hUi[16] = {}, hlam[4] = {}, hrates[8] = {};
+  void *tabv = nullptr;
+  bool leaf_codes = false;
+  int resident[3] = {};      // CTAs of clv_median4_kernel per SM, by neighbour count (0: not asked yet)
+  std::vector<pgpu_clv *> unchecked;   // leaves whose codes no kernel has read yet
 };
 
 struct pgpu_clv {
   pgpu_lk *lk = nullptr;
-  char *mem = nullptr;       // one stream-ordered allocation
+  char *mem = nullptr;       // stream-ordered: scalars, P, codes
+  char *vec = nullptr;       // stream-ordered: x, ex (allocated when first needed)
   void *x = nullptr;         // [n_pat][R][S]
   int32_t *ex = nullptr;     // [n_pat]
-  void *P = nullptr;         // [R][S][S] of the branch above
-  double *scal = nullptr;    // [0] cost, [1] branch length, [2] root cost
+  void *P = nullptr;         // [R][S][S] of the branch above (not for 4 states)
+  uint8_t *codes = nullptr;  // a leaf's codes (4 states)
+  // [0], [1] the cost: a double in [0], or with integer weights an int64 in
+  // [slot] (a median adds to the other slot, which the median before it
+  // cleared); [2] root cost, [3] branch length
+  double *scal = nullptr;
+  int slot = 0;
+  double P4[8][16];          // P of the branch above, 4 states
   double brlen = 0.0;
   bool has_P = false;
   bool leaf = false;
+  bool expanded = false;     // a leaf whose vector is in x
+  int unchecked = -1;        // index in the model's list
 };
 
 namespace {
@@ -128,13 +152,10 @@ __device__ __forceinline__ void cta_partial_and_finish(double s, double c, doubl
   }
 }
 
-// The same for an exact integer sum v: the last CTA adds the per-CTA
-// partials in int64 and writes scale * total.
+// An exact integer sum v over the CTA, added to *acc.
 template <int NT>
-__device__ __forceinline__ void cta_i64_and_finish(long long v, long long *part, unsigned *counter,
-                                                   double *out, double scale) {
+__device__ __forceinline__ void cta_add_i64(long long v, long long *acc) {
   __shared__ long long red[NT / 32];
-  __shared__ bool last;
   const int t = threadIdx.x, lane = t & 31;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -143,28 +164,8 @@ __device__ __forceinline__ void cta_i64_and_finish(long long v, long long *part,
   if (t < 32) {
     long long x = lane < NT / 32 ? red[lane] : 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) {
-      part[blockIdx.x] = x;
-      __threadfence();
-      last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  long long sum = 0;
-  for (unsigned i = t; i < gridDim.x; i += NT) sum += __ldcg(part + i);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  __syncthreads();
-  if (lane == 0) red[t >> 5] = sum;
-  __syncthreads();
-  if (t == 0) {
-    long long tot = 0;
-    for (int k = 0; k < NT / 32; ++k) tot += red[k];
-    *out = scale * (double)tot;
-    *counter = 0u;
+    for (int o = NT / 64; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0 && x) atomicAdd(reinterpret_cast<unsigned long long *>(acc), (unsigned long long)x);
   }
 }
 
@@ -202,14 +203,24 @@ struct MedArgs {
   int n_ch, S, R, RL;
   int int_w;                 // integer weights: exact int64 cost sums
   const int32_t *wint;
-  long long *ipart;
+  long long *acc, *acc_next;   // this median's sum (zero), and the one to clear
 };
+
+constexpr double NEG_LN2 = -0.69314718055994530942;
 
 // 16-byte vector access to one (pattern, rate class) row of 4 states
 template <typename V> struct Row4;
 template <> struct Row4<float> {
   __device__ __forceinline__ static void load(const float *p, float *v) {
     const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+  }
+  __device__ __forceinline__ static void load_l2(const float *p, float *v) {
+    const float4 q = __ldcg(reinterpret_cast<const float4 *>(p));
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+  }
+  __device__ __forceinline__ static void load_shared(const float *p, float *v) {
+    const float4 q = *reinterpret_cast<const float4 *>(p);
     v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
   }
   __device__ __forceinline__ static void store(float *p, const float *v) {
@@ -222,27 +233,36 @@ template <> struct Row4<double> {
     const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
     v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
   }
+  __device__ __forceinline__ static void load_l2(const double *p, double *v) {
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
+    const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  }
+  __device__ __forceinline__ static void load_shared(const double *p, double *v) {
+    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  }
   __device__ __forceinline__ static void store(double *p, const double *v) {
     reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
     reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
   }
 };
 
-// y = prod_k P_k x_k, normalised per pattern.  SC: the state count at
-// compile time (4), or 0 for any S up to 64 read at run time.  A grid of a
-// few CTAs per SM strides over the (pattern, rate class) items, a warp at a
+// y = prod_k P_k x_k, normalised per pattern, for any S up to 64.  A grid of
+// a few CTAs per SM strides over the (pattern, rate class) items, a warp at a
 // time (the stride is a multiple of 32, so a pattern's RL lanes stay in one
-// warp and one iteration); each thread keeps one compensated cost sum and
-// the CTA reduces it once at the end.
-template <typename V, int SC>
+// warp and one iteration); each thread keeps one cost sum and the CTA reduces
+// it once at the end.
+template <typename V>
 __global__ void __launch_bounds__(CLV_THREADS) clv_median_kernel(const MedArgs a) {
-  const int S = SC ? SC : a.S, R = a.R, RL = a.RL;
+  const int S = a.S, R = a.R, RL = a.RL;
   const int lane = threadIdx.x & 31;
   const size_t n_items = a.n_pat * (size_t)RL;
   const size_t stride = (size_t)gridDim.x * CLV_THREADS;
   V *y = static_cast<V *>(a.y);
   double s = 0.0, c = 0.0;
   long long iacc = 0;
+  if (a.int_w && blockIdx.x == 0 && threadIdx.x == 0) *a.acc_next = 0;
   for (size_t base = (size_t)blockIdx.x * CLV_THREADS + (threadIdx.x & ~31); base < n_items;
        base += stride) {
     const size_t g = base + lane;
@@ -264,62 +284,28 @@ __global__ void __launch_bounds__(CLV_THREADS) clv_median_kernel(const MedArgs a
     }
     V m = (V)0;
     int e;
-    if (SC == 4) {
-      V acc[4] = {(V)1, (V)1, (V)1, (V)1};
-      if (act) {
+    if (act) {
+      for (int i = 0; i < S; ++i) {
+        V v = (V)1;
         for (int k = 0; k < a.n_ch; ++k) {
-          V xv[4], Pr[16];
-          Row4<V>::load(static_cast<const V *>(a.x[k]) + off, xv);
-          const V *P = static_cast<const V *>(a.P[k]) + (size_t)r * 16;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) Row4<V>::load(P + 4 * i, Pr + 4 * i);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            V t = (V)0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) t = fma(Pr[4 * i + j], xv[j], t);
-            acc[i] *= t;
-          }
+          const V *xs = static_cast<const V *>(a.x[k]) + off;
+          const V *P = static_cast<const V *>(a.P[k]) + ((size_t)r * S + i) * S;
+          V t = (V)0;
+          for (int j = 0; j < S; ++j) t = fma(__ldg(P + j), xs[j], t);
+          v *= t;
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) m = acc[i] > m ? acc[i] : m;
+        y[off + i] = v;
+        m = v > m ? v : m;
       }
-      V mm = m;
-      for (int o = 1; o < RL; o <<= 1) {
-        const V q = __shfl_xor_sync(0xffffffffu, mm, o);
-        mm = q > mm ? q : mm;
-      }
-      e = frexp_exp(mm);
-      if (act) {
-        V out[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) out[i] = scale2<V>(acc[i], -e);
-        Row4<V>::store(y + off, out);
-      }
-    } else {
-      if (act) {
-        for (int i = 0; i < S; ++i) {
-          V v = (V)1;
-          for (int k = 0; k < a.n_ch; ++k) {
-            const V *xs = static_cast<const V *>(a.x[k]) + off;
-            const V *P = static_cast<const V *>(a.P[k]) + ((size_t)r * S + i) * S;
-            V t = (V)0;
-            for (int j = 0; j < S; ++j) t = fma(__ldg(P + j), xs[j], t);
-            v *= t;
-          }
-          y[off + i] = v;
-          m = v > m ? v : m;
-        }
-      }
-      V mm = m;
-      for (int o = 1; o < RL; o <<= 1) {
-        const V q = __shfl_xor_sync(0xffffffffu, mm, o);
-        mm = q > mm ? q : mm;
-      }
-      e = frexp_exp(mm);
-      if (act)
-        for (int i = 0; i < S; ++i) y[off + i] = scale2<V>(y[off + i], -e);
     }
+    V mm = m;
+    for (int o = 1; o < RL; o <<= 1) {
+      const V q = __shfl_xor_sync(0xffffffffu, mm, o);
+      mm = q > mm ? q : mm;
+    }
+    e = frexp_exp(mm);
+    if (act)
+      for (int i = 0; i < S; ++i) y[off + i] = scale2<V>(y[off + i], -e);
     // exponent bookkeeping and this node's cost, by the pattern's first lane
     if (lead) {
       a.ey[p] = e + ex_sum;
@@ -334,10 +320,173 @@ __global__ void __launch_bounds__(CLV_THREADS) clv_median_kernel(const MedArgs a
     }
   }
   // cost = -ln 2 * sum_p w_p e_p
-  if (a.int_w)
-    cta_i64_and_finish<CLV_THREADS>(iacc, a.ipart, a.counter, a.cost, -0.69314718055994530942);
-  else
-    cta_partial_and_finish<CLV_THREADS>(s, c, a.part, a.counter, a.cost, -0.69314718055994530942);
+  if (a.int_w) cta_add_i64<CLV_THREADS>(iacc, a.acc);
+  else cta_partial_and_finish<CLV_THREADS>(s, c, a.part, a.counter, a.cost, NEG_LN2);
+}
+
+// The same for four states.  The next item's reads in flight while one is
+// computed, P and the leaves' rows by code in shared memory.
+// 100,003 patterns, 4 classes, float: 6.3 us a median over a 128-taxon tree (18
+// at 446,427) against 14.4 us with vectors for leaves, P read per item and one
+// item in flight; P in registers spills at 4 CTAs per SM (8.0 us), and at 2
+// or 3 CTAs too few reads are in flight (8.3, 7.4).
+template <typename V, int NCH>
+struct Med4Args {
+  const V *x[NCH];           // internal neighbours; null: a leaf
+  const int32_t *ex[NCH];
+  const uint8_t *codes[NCH];
+  V P[NCH][8 * 16];
+  V *y;
+  int32_t *ey;
+  const V *tab;              // [n_codes][4]
+  const double *weights;
+  double2 *part;
+  unsigned *counter;
+  double *cost;
+  size_t n_pat;
+  int R, RL, rl_shift, n_codes, int_w;   // RL = 1 << rl_shift
+  const int32_t *wint;
+  long long *acc, *acc_next;
+  int *flag;
+};
+
+template <typename V, int NCH>
+__global__ void __launch_bounds__(CLV_THREADS, sizeof(V) == 4 ? 4 : 2) clv_median4_kernel(const __grid_constant__ Med4Args<V, NCH> a) {
+  extern __shared__ __align__(16) unsigned char clv_sm[];
+  V *sP = reinterpret_cast<V *>(clv_sm);            // [NCH][4 rows][R][4]: a warp's classes side by side
+  V *rows = sP + NCH * a.R * 16;                    // per leaf neighbour [n_codes][R][4]
+  const int R = a.R, RL = a.RL, tid = threadIdx.x, lane = tid & 31;
+  const int n_rows = a.n_codes * R * 4;
+#pragma unroll
+  for (int k = 0; k < NCH; ++k)
+    for (int i = tid; i < R * 16; i += CLV_THREADS) sP[k * R * 16 + (((i >> 2) & 3) * R + (i >> 4)) * 4 + (i & 3)] = a.P[k][i];
+  __syncthreads();
+  int n_leaf = 0;
+#pragma unroll
+  for (int k = 0; k < NCH; ++k)
+    if (!a.x[k]) {
+      for (int o = tid; o < n_rows; o += CLV_THREADS) {
+        const int i = o & 3, r = (o >> 2) % R, c = (o >> 2) / R;
+        V t = (V)0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t = fma(sP[k * R * 16 + (i * R + r) * 4 + j], __ldg(a.tab + 4 * c + j), t);
+        rows[n_leaf * n_rows + o] = t;
+      }
+      ++n_leaf;
+    }
+  __syncthreads();
+  const size_t n_items = a.n_pat * (size_t)RL, stride = (size_t)gridDim.x * CLV_THREADS;
+  // the stride is a multiple of RL, so a thread keeps its rate class
+  const size_t first = (size_t)blockIdx.x * CLV_THREADS + tid;
+  const int r = (int)(first & (RL - 1));
+  const bool rate_on = r < R;
+  // Launched while the kernel before drains (programmatic stream
+  // serialisation): nothing above depends on it.  From here on its vectors
+  // are read, past the read-only path, which may keep lines from before.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (a.int_w && blockIdx.x == 0 && tid == 0) *a.acc_next = 0;
+  double s = 0.0, c = 0.0;
+  long long iacc = 0;
+  uint32_t bad = 0;
+  // what one item reads; the next item's is on its way while one is computed
+  struct Item {
+    V x[NCH][4];
+    uint32_t code[NCH];
+    int ex;
+    int32_t wi;
+    double wd;
+  };
+  const bool lead = r == 0;   // the pattern's first lane keeps its exponents and cost
+  auto fetch = [&](size_t g, Item &it) {
+    it.ex = 0;
+    it.wi = 1;
+    it.wd = 1.0;
+    if (g >= n_items || !rate_on) return;
+    const size_t p = g >> a.rl_shift;
+#pragma unroll
+    for (int k = 0; k < NCH; ++k) {
+      if (a.x[k]) Row4<V>::load_l2(a.x[k] + (p * R + r) * 4, it.x[k]);
+      else it.code[k] = __ldcg(a.codes[k] + p);
+      if (lead && a.x[k]) it.ex += __ldcg(a.ex[k] + p);
+    }
+    if (lead) {
+      if (a.wint) it.wi = __ldg(a.wint + p);
+      else if (!a.int_w && a.weights) it.wd = __ldg(a.weights + p);
+    }
+  };
+  Item cur, next;
+  size_t g = first;
+  fetch(g, cur);
+  // whole warps stay in the loop: RL lanes of a pattern share a warp
+  for (size_t base = first - lane; base < n_items; base += stride) {
+    const bool act = g < n_items && rate_on;
+    fetch(g + stride, next);
+    V acc[4] = {(V)1, (V)1, (V)1, (V)1}, m = (V)0;
+    if (act) {
+      int leaf = 0;
+#pragma unroll
+      for (int k = 0; k < NCH; ++k) {
+        V t[4];
+        if (a.x[k]) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            V Pr[4];
+            Row4<V>::load_shared(sP + k * R * 16 + (i * R + r) * 4, Pr);
+            t[i] = (V)0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[i] = fma(Pr[j], cur.x[k][j], t[i]);
+          }
+        } else {
+          bad |= cur.code[k] >= (uint32_t)a.n_codes;
+          Row4<V>::load_shared(
+              rows + leaf * n_rows + (min(cur.code[k], (uint32_t)a.n_codes - 1u) * R + r) * 4, t);
+          ++leaf;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] *= t[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m = acc[i] > m ? acc[i] : m;
+    }
+    for (int o = 1; o < RL; o <<= 1) {
+      const V q = __shfl_xor_sync(0xffffffffu, m, o);
+      m = q > m ? q : m;
+    }
+    const int e = frexp_exp(m);
+    if (act) {
+      const size_t p = g >> a.rl_shift;
+      V out[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[i] = scale2<V>(acc[i], -e);
+      Row4<V>::store(a.y + (p * R + r) * 4, out);
+      if (lead) {
+        a.ey[p] = e + cur.ex;
+        if (a.int_w) {
+          iacc += (long long)cur.wi * e;
+        } else {
+          double t, err;
+          two_sum(s, cur.wd * (double)e, t, err);
+          s = t;
+          c += err;
+        }
+      }
+    }
+    cur = next;
+    g += stride;
+  }
+  if (bad) atomicOr(a.flag, PGPU_FLAG_BADCODE);
+  if (a.int_w) cta_add_i64<CLV_THREADS>(iacc, a.acc);
+  else cta_partial_and_finish<CLV_THREADS>(s, c, a.part, a.counter, a.cost, NEG_LN2);
+}
+
+// codes at or above n_codes raise the error word
+__global__ void __launch_bounds__(CLV_THREADS) clv_codes_kernel(const uint8_t *codes, size_t n, int n_codes,
+                                                                int *flag) {
+  bool bad = false;
+  for (size_t i = (size_t)blockIdx.x * CLV_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * CLV_THREADS)
+    bad |= codes[i] >= n_codes;
+  if (bad) atomicOr(flag, PGPU_FLAG_BADCODE);
 }
 
 // root_cost: -sum_p w_p log(sum_r probs_r sum_i pi_i x[p][r][i]); the
@@ -377,19 +526,85 @@ __global__ void __launch_bounds__(CLV_THREADS) clv_root_kernel(
   cta_partial_and_finish<CLV_THREADS>(s, c, part, counter, out, -1.0);
 }
 
-// costs of many nodes: out[i] = *src[i]
+// The same for four states, a thread per pattern: FP64 costs a warp the same
+// however few of its lanes work (100,003 patterns, 4 classes: 38 us, 80
+// with a lane per rate class).
+template <typename V>
+__global__ void __launch_bounds__(CLV_THREADS) clv_root4_kernel(
+    const V *x, const int32_t *ex, const double *pi, const double *probs, const double *weights,
+    size_t n_pat, int R, double *site_lnl, double2 *part, unsigned *counter, double *out) {
+  double s = 0.0, c = 0.0;
+  const double pi4[4] = {pi[0], pi[1], pi[2], pi[3]};
+  for (size_t p = (size_t)blockIdx.x * CLV_THREADS + threadIdx.x; p < n_pat;
+       p += (size_t)gridDim.x * CLV_THREADS) {
+    double v = 0.0;
+    for (int r = 0; r < R; ++r) {
+      V xs[4];
+      Row4<V>::load(x + (p * R + r) * 4, xs);
+      double q = 0.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q = fma(pi4[i], (double)xs[i], q);
+      v = fma(q, probs[r], v);
+    }
+    const double site = log(v);
+    if (site_lnl) site_lnl[p] = site + (double)ex[p] * 0.69314718055994530942;
+    double t, err;
+    two_sum(s, weights ? weights[p] * site : site, t, err);
+    s = t;
+    c += err;
+  }
+  cta_partial_and_finish<CLV_THREADS>(s, c, part, counter, out, -1.0);
+}
+
+// costs of many nodes: out[i] = *src[i], or of the int64 there
 __global__ void __launch_bounds__(256) clv_gather_kernel(const double *const *src, size_t n,
-                                                        double *out) {
+                                                        double *out, int int_w) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
-    out[i] = *src[i];
+    out[i] = int_w ? NEG_LN2 * (double)*reinterpret_cast<const long long *>(src[i]) : *src[i];
 }
 
 pgpu_status lk_err(pgpu_lk *lk, pgpu_status st, const char *msg) {
   return pgpu_set_err(lk->ctx, st, "%s", msg);
 }
 
-// allocation of a handle for lk (or reuse of `reuse`'s memory)
+pgpu_status clv_malloc(pgpu_ctx *ctx, size_t bytes, char **out) {
+  void *mem = nullptr;
+  const cudaError_t e = cudaMallocAsync(&mem, bytes, ctx->stream);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return pgpu_set_err(ctx, e == cudaErrorMemoryAllocation ? PGPU_ERR_OOM : PGPU_ERR_CUDA,
+                        "likelihood: node allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  }
+  *out = static_cast<char *>(mem);
+  return PGPU_OK;
+}
+
+// no kernel needs to read t's codes to find a bad one any more
+void clv_checked(pgpu_clv *t) {
+  if (t->unchecked < 0) return;
+  auto &u = t->lk->unchecked;
+  u[t->unchecked] = u.back();
+  u[t->unchecked]->unchecked = t->unchecked;
+  u.pop_back();
+  t->unchecked = -1;
+}
+
+// reads the codes of every leaf that nothing has read yet, so that a bad
+// code is reported by the calls that synchronise
+pgpu_status check_leaves(pgpu_lk *lk) {
+  pgpu_ctx *ctx = lk->ctx;
+  while (!lk->unchecked.empty()) {
+    pgpu_clv *t = lk->unchecked.back();
+    const unsigned grid = (unsigned)std::min<size_t>((lk->n_pat + CLV_THREADS - 1) / CLV_THREADS, 1024);
+    clv_codes_kernel<<<grid, CLV_THREADS, 0, ctx->stream>>>(t->codes, lk->n_pat, lk->n_codes, ctx->d_flag);
+    PGPU_TRY(pgpu_after_launch(ctx, "clv_codes_kernel"));
+    clv_checked(t);
+  }
+  return PGPU_OK;
+}
+
+// a handle for lk (or `reuse`, its memory taken over), without its vector
 pgpu_status clv_alloc(pgpu_lk *lk, pgpu_clv *reuse, pgpu_clv **out) {
   pgpu_ctx *ctx = lk->ctx;
   if (reuse) {
@@ -398,32 +613,135 @@ pgpu_status clv_alloc(pgpu_lk *lk, pgpu_clv *reuse, pgpu_clv **out) {
     *out = reuse;
     reuse->has_P = false;
     reuse->leaf = false;
+    reuse->expanded = false;
     reuse->brlen = 0.0;
+    clv_checked(reuse);
     return PGPU_OK;
   }
-  const size_t vb = vbytes(lk);
-  const size_t xb = al256(lk->n_pat * lk->R * lk->S * vb), eb = al256(lk->n_pat * 4),
-               pb = al256((size_t)lk->R * lk->S * lk->S * vb), sb = 256;
+  const size_t pb = lk->S == 4 ? 0 : al256((size_t)lk->R * lk->S * lk->S * vbytes(lk));
+  const size_t cb = lk->leaf_codes ? al256(lk->n_pat) : 0;
   pgpu_clv *t = new (std::nothrow) pgpu_clv();
   if (!t) return lk_err(lk, PGPU_ERR_OOM, "likelihood: host allocation failed");
-  void *mem = nullptr;
-  cudaError_t e = cudaMallocAsync(&mem, xb + eb + pb + sb, ctx->stream);
-  if (e != cudaSuccess) {
+  pgpu_status st = clv_malloc(ctx, 256 + pb + cb, &t->mem);
+  if (st == PGPU_OK && cudaMemsetAsync(t->mem, 0, 32, ctx->stream) != cudaSuccess) {
     (void)cudaGetLastError();
+    st = lk_err(lk, PGPU_ERR_CUDA, "likelihood: clearing a node failed");
+  }
+  if (st != PGPU_OK) {
+    if (t->mem) cudaFreeAsync(t->mem, ctx->stream);
     delete t;
-    return pgpu_set_err(ctx, e == cudaErrorMemoryAllocation ? PGPU_ERR_OOM : PGPU_ERR_CUDA,
-                        "likelihood: node allocation of %zu bytes failed: %s", xb + eb + pb + sb,
-                        cudaGetErrorString(e));
+    return st;
   }
   t->lk = lk;
-  t->mem = static_cast<char *>(mem);
-  t->x = t->mem;
-  t->ex = reinterpret_cast<int32_t *>(t->mem + xb);
-  t->P = t->mem + xb + eb;
-  t->scal = reinterpret_cast<double *>(t->mem + xb + eb + pb);
+  t->scal = reinterpret_cast<double *>(t->mem);
+  t->P = t->mem + 256;
+  t->codes = reinterpret_cast<uint8_t *>(t->mem + 256 + pb);
   lk->live++;
   *out = t;
   return PGPU_OK;
+}
+
+// the node's vector memory
+pgpu_status clv_vector(pgpu_clv *t) {
+  if (t->vec) return PGPU_OK;
+  pgpu_lk *lk = t->lk;
+  const size_t xb = al256(lk->n_pat * lk->R * lk->S * vbytes(lk));
+  PGPU_TRY(clv_malloc(lk->ctx, xb + al256(lk->n_pat * 4), &t->vec));
+  t->x = t->vec;
+  t->ex = reinterpret_cast<int32_t *>(t->vec + xb);
+  return PGPU_OK;
+}
+
+void clv_free(pgpu_clv *t) {
+  pgpu_ctx *ctx = t->lk->ctx;
+  clv_checked(t);
+  if (t->vec) cudaFreeAsync(t->vec, ctx->stream);
+  cudaFreeAsync(t->mem, ctx->stream);
+  t->lk->live--;
+  delete t;
+}
+
+// a leaf's vector from its codes
+pgpu_status clv_expand(pgpu_clv *t, const uint8_t *codes) {
+  pgpu_lk *lk = t->lk;
+  pgpu_ctx *ctx = lk->ctx;
+  PGPU_TRY(clv_vector(t));
+  const size_t n = lk->n_pat * lk->R * lk->S;
+  const unsigned grid = (unsigned)((n + CLV_THREADS - 1) / CLV_THREADS);
+  if (lk->precision == 32)
+    clv_leaf_kernel<float><<<grid, CLV_THREADS, 0, ctx->stream>>>(codes, lk->tab, lk->n_codes, lk->n_pat, lk->S,
+                                                                  lk->R, (float *)t->x, t->ex, ctx->d_flag);
+  else
+    clv_leaf_kernel<double><<<grid, CLV_THREADS, 0, ctx->stream>>>(codes, lk->tab, lk->n_codes, lk->n_pat,
+                                                                   lk->S, lk->R, (double *)t->x, t->ex,
+                                                                   ctx->d_flag);
+  PGPU_TRY(pgpu_after_launch(ctx, "clv_leaf_kernel"));
+  t->expanded = true;
+  clv_checked(t);
+  return PGPU_OK;
+}
+
+const double *cost_at(const pgpu_clv *t) {
+  return t->leaf ? t->lk->zero : t->scal + (t->lk->int_w ? t->slot : 0);
+}
+
+template <typename V, int NCH>
+pgpu_status launch_median4(pgpu_lk *lk, pgpu_clv *t, pgpu_clv *const *ch) {
+  pgpu_ctx *ctx = lk->ctx;
+  Med4Args<V, NCH> a;
+  int n_leaf = 0;
+  for (int k = 0; k < NCH; ++k) {
+    const bool vec = !ch[k]->leaf || ch[k]->expanded;
+    a.x[k] = vec ? static_cast<const V *>(ch[k]->x) : nullptr;
+    a.ex[k] = vec ? ch[k]->ex : nullptr;
+    a.codes[k] = vec ? nullptr : ch[k]->codes;
+    n_leaf += !vec;
+    for (int i = 0; i < lk->R * 16; ++i) a.P[k][i] = (V)ch[k]->P4[i / 16][i % 16];
+  }
+  a.y = static_cast<V *>(t->x);
+  a.ey = t->ex;
+  a.tab = static_cast<const V *>(lk->tabv);
+  a.weights = lk->weights;
+  a.part = lk->part;
+  a.counter = lk->counter;
+  a.cost = t->scal;
+  a.n_pat = lk->n_pat;
+  a.R = lk->R;
+  a.RL = lk->RL;
+  a.rl_shift = lk->RL == 1 ? 0 : lk->RL == 2 ? 1 : lk->RL == 4 ? 2 : 3;
+  a.n_codes = lk->n_codes;
+  a.int_w = lk->int_w ? 1 : 0;
+  a.wint = lk->wint;
+  a.acc = reinterpret_cast<long long *>(t->scal + t->slot);
+  a.acc_next = reinterpret_cast<long long *>(t->scal + (t->slot ^ 1));
+  a.flag = ctx->d_flag;
+  const size_t smem = sizeof(V) * (size_t)lk->R * (NCH * 16 + (size_t)n_leaf * lk->n_codes * 4);
+  if (lk->resident[NCH - 1] == 0 || smem > 48 * 1024)
+    PGPU_CUDA(ctx, cudaFuncSetAttribute(clv_median4_kernel<V, NCH>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+  // one wave of CTAs at most: each pays its prologue (P and the leaves' rows
+  // to shared memory) once
+  int &res = lk->resident[NCH - 1];
+  if (res == 0) {
+    const size_t most = sizeof(V) * (size_t)lk->R * NCH * (16 + (size_t)lk->n_codes * 4);
+    PGPU_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                       &res, clv_median4_kernel<V, NCH>, CLV_THREADS, lk->leaf_codes ? most : smem));
+    res = std::max(res, 1);
+  }
+  const size_t want = (lk->n_pat * lk->RL + CLV_THREADS - 1) / CLV_THREADS;
+  const size_t most_cta = std::min<size_t>(lk->n_cta, (size_t)res * std::max(ctx->num_sms, 1));
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)std::max<size_t>(std::min(want, most_cta), 1));
+  c.blockDim = dim3(CLV_THREADS);
+  c.dynamicSmemBytes = smem;
+  c.stream = ctx->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  PGPU_CUDA(ctx, cudaLaunchKernelEx(&c, clv_median4_kernel<V, NCH>, a));
+  return pgpu_after_launch(ctx, "clv_median4_kernel");
 }
 
 pgpu_status check_cta(pgpu_lk *lk) {
@@ -433,22 +751,42 @@ pgpu_status check_cta(pgpu_lk *lk) {
   return PGPU_OK;
 }
 
-pgpu_status median(pgpu_lk *lk, pgpu_clv *reuse, const pgpu_clv *const *ch, int n_ch,
+pgpu_status median(pgpu_lk *lk, pgpu_clv *reuse, const pgpu_clv *const *nbr, int n_ch,
                    pgpu_clv **out) {
   if (!lk || !out) return PGPU_ERR_ARG;
   pgpu_ctx *ctx = lk->ctx;
   for (int k = 0; k < n_ch; ++k) {
-    if (!ch[k]) return lk_err(lk, PGPU_ERR_ARG, "likelihood: null neighbour");
-    if (ch[k]->lk != lk) return lk_err(lk, PGPU_ERR_ARG, "likelihood: neighbour of another model");
-    if (!ch[k]->has_P)
+    if (!nbr[k]) return lk_err(lk, PGPU_ERR_ARG, "likelihood: null neighbour");
+    if (nbr[k]->lk != lk) return lk_err(lk, PGPU_ERR_ARG, "likelihood: neighbour of another model");
+    if (!nbr[k]->has_P)
       return lk_err(lk, PGPU_ERR_ARG,
                     "likelihood: a neighbour has no branch length (pgpu_clv_set_brlen)");
-    if (ch[k] == reuse)
+    if (nbr[k] == reuse)
       return lk_err(lk, PGPU_ERR_ARG, "likelihood: the reused node is also a neighbour");
   }
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+  pgpu_clv *const *ch = const_cast<pgpu_clv *const *>(nbr);
   pgpu_clv *t = nullptr;
   PGPU_TRY(clv_alloc(lk, reuse, &t));
+  pgpu_status st = clv_vector(t);
+  if (st != PGPU_OK) {
+    if (!reuse) clv_free(t);
+    return st;
+  }
+  if (lk->int_w) t->slot ^= 1;
+  if (lk->S == 4) {
+    for (int k = 0; k < n_ch; ++k)
+      if (ch[k]->leaf) clv_checked(ch[k]);   // the kernel checks the codes it reads
+    if (lk->precision == 32)
+      st = n_ch == 1 ? launch_median4<float, 1>(lk, t, ch)
+                     : n_ch == 2 ? launch_median4<float, 2>(lk, t, ch) : launch_median4<float, 3>(lk, t, ch);
+    else
+      st = n_ch == 1 ? launch_median4<double, 1>(lk, t, ch)
+                     : n_ch == 2 ? launch_median4<double, 2>(lk, t, ch) : launch_median4<double, 3>(lk, t, ch);
+    PGPU_TRY(st);
+    *out = t;
+    return PGPU_OK;
+  }
   MedArgs a{};
   for (int k = 0; k < n_ch; ++k) {
     a.x[k] = ch[k]->x;
@@ -460,7 +798,8 @@ pgpu_status median(pgpu_lk *lk, pgpu_clv *reuse, const pgpu_clv *const *ch, int 
   a.weights = lk->weights;
   a.int_w = lk->int_w ? 1 : 0;
   a.wint = lk->wint;
-  a.ipart = lk->ipart;
+  a.acc = reinterpret_cast<long long *>(t->scal + t->slot);
+  a.acc_next = reinterpret_cast<long long *>(t->scal + (t->slot ^ 1));
   a.part = lk->part;
   a.counter = lk->counter;
   a.cost = t->scal;
@@ -470,13 +809,8 @@ pgpu_status median(pgpu_lk *lk, pgpu_clv *reuse, const pgpu_clv *const *ch, int 
   a.R = lk->R;
   a.RL = lk->RL;
   const unsigned grid = (unsigned)lk->n_cta;
-  if (lk->precision == 32) {
-    if (lk->S == 4) clv_median_kernel<float, 4><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
-    else clv_median_kernel<float, 0><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
-  } else {
-    if (lk->S == 4) clv_median_kernel<double, 4><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
-    else clv_median_kernel<double, 0><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
-  }
+  if (lk->precision == 32) clv_median_kernel<float><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
+  else clv_median_kernel<double><<<grid, CLV_THREADS, 0, ctx->stream>>>(a);
   PGPU_TRY(pgpu_after_launch(ctx, "clv_median_kernel"));
   *out = t;
   return PGPU_OK;
@@ -532,7 +866,7 @@ pgpu_status pgpu_lk_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_co
                orates = take(R * 8), oprobs = take(R * 8),
                otab = take((size_t)codes->n_codes * S * 8), ow = take(n_pat * 8), oq = take(SS * 8),
                ost = take(64), opart = take(lk->n_cta * sizeof(double2)),
-               owi = take(n_pat * 4), oipart = take(lk->n_cta * sizeof(long long));
+               owi = take(n_pat * 4), otabv = take((size_t)codes->n_codes * S * vbytes(lk)), ozero = take(8);
   const size_t bytes = off;
   void *blk = nullptr;
   cudaError_t e = cudaMalloc(&blk, bytes);
@@ -556,7 +890,10 @@ pgpu_status pgpu_lk_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_co
   lk->status = reinterpret_cast<int *>(base + ost);
   lk->counter = reinterpret_cast<unsigned *>(lk->status + 4);
   lk->part = reinterpret_cast<double2 *>(base + opart);
-  lk->ipart = reinterpret_cast<long long *>(base + oipart);
+  lk->tabv = base + otabv;
+  lk->zero = reinterpret_cast<double *>(base + ozero);
+  // a leaf neighbour's rows stay within a third of 96 KB
+  lk->leaf_codes = S == 4 && (size_t)codes->n_codes * R * 4 * vbytes(lk) <= 32 * 1024;
   // integer weights, small enough that sum_p w_p e_p fits int64 (|e_p| <= 1074)
   std::vector<int32_t> wi;
   lk->int_w = true;
@@ -595,10 +932,24 @@ pgpu_status pgpu_lk_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_co
   if (weights) LK_CUDA(cudaMemcpyAsync(w, weights, n_pat * 8, cudaMemcpyHostToDevice, s));
   if (lk->wint) LK_CUDA(cudaMemcpyAsync(lk->wint, wi.data(), n_pat * 4, cudaMemcpyHostToDevice, s));
   LK_CUDA(cudaMemsetAsync(lk->status, 0, 64, s));
+  LK_CUDA(cudaMemsetAsync(lk->zero, 0, 8, s));
+  std::vector<float> tabf;
+  if (S == 4) {
+    const size_t n = (size_t)codes->n_codes * 4;
+    for (size_t i = 0; i < n && precision == 32; ++i) tabf.push_back((float)codes->table[i]);
+    LK_CUDA(cudaMemcpyAsync(lk->tabv, precision == 32 ? (const void *)tabf.data() : codes->table,
+                            n * vbytes(lk), cudaMemcpyHostToDevice, s));
+  }
   pgpu_status st = pgpu_launch_eig(ctx, q, lk->pi, S, 1, lk->U, lk->lam, lk->Ui, lk->status);
   if (st != PGPU_OK) return fail(st);
   int *hst = reinterpret_cast<int *>(ctx->h_pinned);
   LK_CUDA(cudaMemcpyAsync(hst, lk->status, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (S == 4) {
+    LK_CUDA(cudaMemcpyAsync(lk->hU, lk->U, sizeof lk->hU, cudaMemcpyDeviceToHost, s));
+    LK_CUDA(cudaMemcpyAsync(lk->hUi, lk->Ui, sizeof lk->hUi, cudaMemcpyDeviceToHost, s));
+    LK_CUDA(cudaMemcpyAsync(lk->hlam, lk->lam, sizeof lk->hlam, cudaMemcpyDeviceToHost, s));
+    std::copy(m->rates, m->rates + R, lk->hrates);
+  }
   LK_CUDA(cudaStreamSynchronize(s));
 #undef LK_CUDA
   if (*hst) {
@@ -628,23 +979,29 @@ pgpu_status pgpu_clv_leaf(pgpu_lk *lk, pgpu_clv *reuse, const uint8_t *codes, pg
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
   pgpu_clv *t = nullptr;
   PGPU_TRY(clv_alloc(lk, reuse, &t));
-  // the codes are copied into the context's tip buffer; later calls on the
-  // stream are ordered after this leaf's kernel
-  void *dc;
-  PGPU_TRY(pgpu_buf(ctx, BUF_TIPS, std::max<size_t>(lk->n_pat, 16), &dc));
-  PGPU_CUDA(ctx, cudaMemcpyAsync(dc, codes, lk->n_pat, cudaMemcpyHostToDevice, ctx->stream));
-  const size_t n = lk->n_pat * lk->R * lk->S;
-  const unsigned grid = (unsigned)((n + CLV_THREADS - 1) / CLV_THREADS);
-  if (lk->precision == 32)
-    clv_leaf_kernel<float><<<grid, CLV_THREADS, 0, ctx->stream>>>(
-        (const uint8_t *)dc, lk->tab, lk->n_codes, lk->n_pat, lk->S, lk->R, (float *)t->x, t->ex,
-        ctx->d_flag);
-  else
-    clv_leaf_kernel<double><<<grid, CLV_THREADS, 0, ctx->stream>>>(
-        (const uint8_t *)dc, lk->tab, lk->n_codes, lk->n_pat, lk->S, lk->R, (double *)t->x, t->ex,
-        ctx->d_flag);
-  PGPU_TRY(pgpu_after_launch(ctx, "clv_leaf_kernel"));
-  PGPU_CUDA(ctx, cudaMemsetAsync(t->scal, 0, sizeof(double), ctx->stream));
+  const cudaStream_t s = ctx->stream;
+  if (lk->leaf_codes) {
+    // the codes themselves are the leaf; its first reader checks them
+    // Up to 1 MB they go through the pinned staging blocks: a copy straight
+    // from pageable memory holds the caller up (20 us against 9 at 100 KB).
+    if (lk->n_pat <= (size_t)1 << 20) {
+      void *h;
+      PGPU_TRY(pgpu_stage(ctx, lk->n_pat, &h, nullptr));
+      std::memcpy(h, codes, lk->n_pat);
+      PGPU_TRY(pgpu_stage_copy(ctx, t->codes, lk->n_pat));
+    } else {
+      PGPU_CUDA(ctx, cudaMemcpyAsync(t->codes, codes, lk->n_pat, cudaMemcpyHostToDevice, s));
+    }
+    t->unchecked = (int)lk->unchecked.size();
+    lk->unchecked.push_back(t);
+  } else {
+    // the codes are copied into the context's tip buffer; later calls on the
+    // stream are ordered after this leaf's kernel
+    void *dc;
+    PGPU_TRY(pgpu_buf(ctx, BUF_TIPS, std::max<size_t>(lk->n_pat, 16), &dc));
+    PGPU_CUDA(ctx, cudaMemcpyAsync(dc, codes, lk->n_pat, cudaMemcpyHostToDevice, s));
+    PGPU_TRY(clv_expand(t, (const uint8_t *)dc));
+  }
   t->leaf = true;
   *out = t;
   return PGPU_OK;
@@ -656,14 +1013,29 @@ pgpu_status pgpu_clv_set_brlen(pgpu_clv *t, double brlen) {
   pgpu_ctx *ctx = lk->ctx;
   if (!(brlen >= 0.0) || !std::isfinite(brlen))
     return lk_err(lk, PGPU_ERR_ARG, "likelihood: branch length must be finite and >= 0");
+  if (lk->S == 4) {
+    // compose_kernel's arithmetic, 16 numbers per rate class
+    for (int r = 0; r < lk->R; ++r) {
+      const bool ident = !(brlen * lk->hrates[r] >= 1e-10);
+      double e[4];
+      for (int k = 0; k < 4; ++k) e[k] = ident ? 1.0 : std::exp(lk->hlam[k] * lk->hrates[r] * brlen);
+      for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j) {
+          double v = 0.0;
+          for (int k = 0; k < 4; ++k) v = std::fma(lk->hU[4 * i + k] * e[k], lk->hUi[4 * k + j], v);
+          t->P4[r][4 * i + j] = ident ? (i == j ? 1.0 : 0.0) : v;
+        }
+    }
+    t->brlen = brlen;
+    t->has_P = true;
+    return PGPU_OK;
+  }
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
-  void *h, *d;
-  PGPU_TRY(pgpu_stage(ctx, sizeof(double), &h, &d));
+  void *h;
+  PGPU_TRY(pgpu_stage(ctx, sizeof(double), &h, nullptr));
   *static_cast<double *>(h) = brlen;
-  PGPU_TRY(pgpu_stage_commit(ctx, sizeof(double)));
-  PGPU_CUDA(ctx, cudaMemcpyAsync(t->scal + 1, d, sizeof(double), cudaMemcpyDeviceToDevice,
-                                 ctx->stream));
-  PGPU_TRY(pgpu_launch_compose(ctx, lk->U, lk->lam, lk->Ui, lk->S, t->scal + 1, 1, lk->rates, lk->R,
+  PGPU_TRY(pgpu_stage_copy(ctx, t->scal + 3, sizeof(double)));
+  PGPU_TRY(pgpu_launch_compose(ctx, lk->U, lk->lam, lk->Ui, lk->S, t->scal + 3, 1, lk->rates, lk->R,
                                lk->precision == 64 ? (double *)t->P : nullptr,
                                lk->precision == 64 ? nullptr : (float *)t->P, false, lk->status,
                                P32_PLAIN));
@@ -699,11 +1071,12 @@ pgpu_status pgpu_clv_cost(pgpu_clv *t, double *cost) {
   if (!t || !cost) return PGPU_ERR_ARG;
   pgpu_ctx *ctx = t->lk->ctx;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+  PGPU_TRY(check_leaves(t->lk));
   double *h = reinterpret_cast<double *>(ctx->h_pinned);
-  PGPU_CUDA(ctx, cudaMemcpyAsync(h, t->scal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  PGPU_CUDA(ctx, cudaMemcpyAsync(h, cost_at(t), sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   PGPU_TRY(pgpu_check_flag(ctx, "likelihood"));
-  *cost = *h;
+  *cost = t->lk->int_w ? NEG_LN2 * (double)*reinterpret_cast<const long long *>(h) : *h;
   return PGPU_OK;
 }
 
@@ -715,15 +1088,16 @@ pgpu_status pgpu_clv_costs(pgpu_lk *lk, const pgpu_clv *const *nodes, size_t n, 
     if (!nodes[i] || nodes[i]->lk != lk)
       return lk_err(lk, PGPU_ERR_ARG, "likelihood: a node is null or belongs to another model");
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+  PGPU_TRY(check_leaves(lk));
   void *h, *d, *dout;
   PGPU_TRY(pgpu_stage(ctx, n * sizeof(double *), &h, &d));
   const double **src = static_cast<const double **>(h);
-  for (size_t i = 0; i < n; ++i) src[i] = nodes[i]->scal;
+  for (size_t i = 0; i < n; ++i) src[i] = cost_at(nodes[i]);
   PGPU_TRY(pgpu_stage_commit(ctx, n * sizeof(double *)));
   PGPU_TRY(pgpu_buf(ctx, BUF_F, n * sizeof(double), &dout));
   const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 1024);
   clv_gather_kernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const double *const *>(d), n,
-                                                   static_cast<double *>(dout));
+                                                   static_cast<double *>(dout), lk->int_w ? 1 : 0);
   PGPU_TRY(pgpu_after_launch(ctx, "clv_gather_kernel"));
   PGPU_CUDA(ctx, cudaMemcpyAsync(costs, dout, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -735,10 +1109,22 @@ pgpu_status pgpu_clv_root_cost(pgpu_clv *t, double *cost, double *site_lnl) {
   pgpu_lk *lk = t->lk;
   pgpu_ctx *ctx = lk->ctx;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+  if (t->leaf && !t->expanded) PGPU_TRY(clv_expand(t, t->codes));
+  PGPU_TRY(check_leaves(lk));
   void *dsl = nullptr;
   if (site_lnl) PGPU_TRY(pgpu_buf(ctx, BUF_SITECOST, lk->n_pat * 8, &dsl));
   const unsigned grid = (unsigned)lk->n_cta;
-  if (lk->precision == 32)
+  if (lk->S == 4) {
+    const unsigned g4 = (unsigned)std::min<size_t>((lk->n_pat + CLV_THREADS - 1) / CLV_THREADS, lk->n_cta);
+    if (lk->precision == 32)
+      clv_root4_kernel<float><<<g4, CLV_THREADS, 0, ctx->stream>>>(
+          (const float *)t->x, t->ex, lk->pi, lk->probs, lk->weights, lk->n_pat, lk->R, (double *)dsl,
+          lk->part, lk->counter, t->scal + 2);
+    else
+      clv_root4_kernel<double><<<g4, CLV_THREADS, 0, ctx->stream>>>(
+          (const double *)t->x, t->ex, lk->pi, lk->probs, lk->weights, lk->n_pat, lk->R, (double *)dsl,
+          lk->part, lk->counter, t->scal + 2);
+  } else if (lk->precision == 32)
     clv_root_kernel<float><<<grid, CLV_THREADS, 0, ctx->stream>>>(
         (const float *)t->x, t->ex, lk->pi, lk->probs, lk->weights, lk->n_pat, lk->S, lk->R,
         lk->RL, (double *)dsl, lk->part, lk->counter, t->scal + 2);
@@ -761,9 +1147,7 @@ void pgpu_clv_destroy(pgpu_clv *t) {
   if (!t) return;
   pgpu_ctx *ctx = t->lk->ctx;
   cudaSetDevice(ctx->device);
-  cudaFreeAsync(t->mem, ctx->stream);
-  t->lk->live--;
-  delete t;
+  clv_free(t);
 }
 
 }  // extern "C"

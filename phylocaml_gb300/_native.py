@@ -38,9 +38,9 @@ class NativeError(RuntimeError):
 class PgpuTree(C.Structure):
     _fields_ = [
         ("n_tips", C.c_int32),
-        ("left", C.POINTER(C.c_int32)),
-        ("right", C.POINTER(C.c_int32)),
-        ("brlen", C.POINTER(C.c_double)),
+        ("left", C.c_void_p),    # int32 [n_tips - 1]
+        ("right", C.c_void_p),
+        ("brlen", C.c_void_p),   # double [2 n_tips - 2] or null
     ]
 
 
@@ -228,12 +228,12 @@ def make_tree(left: np.ndarray, right: np.ndarray, brlen: np.ndarray | None = No
     keep = [left, right]
     t = PgpuTree()
     t.n_tips = len(left) + 1
-    t.left = left.ctypes.data_as(C.POINTER(C.c_int32))
-    t.right = right.ctypes.data_as(C.POINTER(C.c_int32))
+    t.left = left.__array_interface__["data"][0]
+    t.right = right.__array_interface__["data"][0]
     if brlen is not None:
         brlen = np.ascontiguousarray(brlen, dtype=np.float64)
         keep.append(brlen)
-        t.brlen = brlen.ctypes.data_as(C.POINTER(C.c_double))
+        t.brlen = brlen.__array_interface__["data"][0]
     return t, keep
 
 

@@ -1074,7 +1074,6 @@ pgpu_status pgpu_clv_cost(pgpu_clv *t, double *cost) {
   PGPU_TRY(check_leaves(t->lk));
   double *h = reinterpret_cast<double *>(ctx->h_pinned);
   PGPU_CUDA(ctx, cudaMemcpyAsync(h, cost_at(t), sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   PGPU_TRY(pgpu_check_flag(ctx, "likelihood"));
   *cost = t->lk->int_w ? NEG_LN2 * (double)*reinterpret_cast<const long long *>(h) : *h;
   return PGPU_OK;
@@ -1100,7 +1099,6 @@ pgpu_status pgpu_clv_costs(pgpu_lk *lk, const pgpu_clv *const *nodes, size_t n, 
                                                    static_cast<double *>(dout), lk->int_w ? 1 : 0);
   PGPU_TRY(pgpu_after_launch(ctx, "clv_gather_kernel"));
   PGPU_CUDA(ctx, cudaMemcpyAsync(costs, dout, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return pgpu_check_flag(ctx, "likelihood");
 }
 
@@ -1137,7 +1135,6 @@ pgpu_status pgpu_clv_root_cost(pgpu_clv *t, double *cost, double *site_lnl) {
   PGPU_CUDA(ctx, cudaMemcpyAsync(h, t->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (site_lnl)
     PGPU_CUDA(ctx, cudaMemcpyAsync(site_lnl, dsl, lk->n_pat * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   PGPU_TRY(pgpu_check_flag(ctx, "likelihood"));
   *cost = *h;
   return PGPU_OK;

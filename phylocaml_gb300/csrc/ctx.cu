@@ -46,10 +46,10 @@ pgpu_status pgpu_after_launch(pgpu_ctx *ctx, const char *what) {
 }
 
 pgpu_status pgpu_check_flag(pgpu_ctx *ctx, const char *what) {
-  int flag = 0;
-  PGPU_CUDA(ctx, cudaMemcpyAsync(&flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  int *h = reinterpret_cast<int *>(static_cast<char *>(ctx->h_pinned) + PGPU_PINNED_FLAG);
+  PGPU_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  const int flag = *h;
   if (flag) {
     PGPU_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     if (flag & PGPU_FLAG_TIMEOUT)
@@ -164,7 +164,7 @@ pgpu_status pgpu_create(pgpu_ctx **out, int device) {
   if (e == cudaSuccess) ctx->own_stream = true;
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_flag, 256);
   if (e == cudaSuccess) e = cudaMemset(ctx->d_flag, 0, 256);
-  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_pinned, 4096);
+  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_pinned, PGPU_PINNED);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     pgpu_destroy(ctx);
@@ -230,7 +230,6 @@ pgpu_status pgpu_set_stream(pgpu_ctx *ctx, void *cuda_stream) {
 pgpu_status pgpu_synchronize(pgpu_ctx *ctx) {
   if (!ctx) return PGPU_ERR_ARG;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return pgpu_check_flag(ctx, "synchronize");
 }
 

@@ -1164,8 +1164,7 @@ cudaError_t launch_tree(cudaStream_t stream, int lb, const FitchTreeArgs &args, 
 // child with the larger stack need first).  Segments go to the FS_W warps
 // longest first, each to the least loaded warp.
 pgpu_status build_split(pgpu_ctx *ctx, const pgpu_tree *tree, SplitSchedule *out) {
-  TreeSchedule check;
-  PGPU_TRY(pgpu_build_schedule(ctx, tree, &check));   // validates the tree
+  PGPU_TRY(pgpu_check_tree(ctx, tree));
   const int32_t n = tree->n_tips, n_int = n - 1;
   const int32_t *L = tree->left, *R = tree->right;
   std::vector<int32_t> size(n_int, 1), need(2 * n - 1, 0);
@@ -1287,10 +1286,13 @@ pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitS
         16 * (sp.ops.size() + sp.seg.size() + sp.top.size() + sp.wseg.size()) + 4 * sp.tips.size();
     void *d;
     PGPU_TRY(pgpu_buf(ctx, BUF_SPLIT, std::max<size_t>(bytes, 16), &d));
-    std::vector<unsigned char> h(std::max<size_t>(bytes, 16));
+    // through pinned staging: a search scores another tree with every call
+    void *hv;
+    PGPU_TRY(pgpu_stage(ctx, bytes, &hv, nullptr));
+    unsigned char *h = static_cast<unsigned char *>(hv);
     size_t off = 0;
     auto put = [&](const void *src, size_t b) {
-      if (b) std::memcpy(h.data() + off, src, b);
+      if (b) std::memcpy(h + off, src, b);
       off += b;
     };
     put(sp.ops.data(), 16 * sp.ops.size());
@@ -1298,8 +1300,7 @@ pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitS
     put(sp.top.data(), 16 * sp.top.size());
     put(sp.wseg.data(), 16 * sp.wseg.size());
     put(sp.tips.data(), 4 * sp.tips.size());
-    PGPU_CUDA(ctx, cudaMemcpyAsync(d, h.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
-    PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // h is a temporary
+    PGPU_TRY(pgpu_stage_copy(ctx, d, bytes));
     ctx->split_left.assign(tree->left, tree->left + n_int);
     ctx->split_right.assign(tree->right, tree->right + n_int);
     ctx->split_valid = true;
@@ -1703,7 +1704,6 @@ pgpu_status pgpu_fitch_tree(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t
       PGPU_CUDA(ctx, cudaMemcpyAsync(site_cost, dsc, n_sites * 4, cudaMemcpyDeviceToHost, s));
     uint64_t *ht = reinterpret_cast<uint64_t *>(ctx->h_pinned);
     PGPU_CUDA(ctx, cudaMemcpyAsync(ht, dtot, 8, cudaMemcpyDeviceToHost, s));
-    PGPU_CUDA(ctx, cudaStreamSynchronize(s));
     PGPU_TRY(pgpu_check_flag(ctx, "fitch_tree"));
     *total = *ht;
     return PGPU_OK;
@@ -1738,7 +1738,6 @@ pgpu_status pgpu_fitch_tree(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t
   }
   uint64_t *ht = reinterpret_cast<uint64_t *>(ctx->h_pinned);
   PGPU_CUDA(ctx, cudaMemcpyAsync(ht, dtot, 8, cudaMemcpyDeviceToHost, s));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(s));
   if (chunked) PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->d2h_stream));
   PGPU_TRY(pgpu_check_flag(ctx, "fitch_tree"));
   *total = *ht;

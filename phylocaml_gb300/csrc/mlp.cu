@@ -948,7 +948,6 @@ pgpu_status pgpu_mlp_grads(pgpu_mlp *nn, const float *X_dev, const float *t_dev,
   PGPU_CUDA(nn->ctx, cudaSetDevice(nn->ctx->device));
   PGPU_TRY(mlp_backprop(nn, X_dev, t_dev, sw_dev, n, loss_host, nullptr));
   PGPU_CUDA(nn->ctx, cudaMemcpyAsync(grad_host, nn->g, N_PARAMS * 4, cudaMemcpyDeviceToHost, nn->ctx->stream));
-  PGPU_CUDA(nn->ctx, cudaStreamSynchronize(nn->ctx->stream));
   return pgpu_check_flag(nn->ctx, "mlp_grads");
 }
 
@@ -971,7 +970,6 @@ pgpu_status pgpu_mlp_train_step(pgpu_mlp *nn, const float *X_dev, const float *t
   PGPU_TRY(mlp_backprop(nn, X_dev, t_dev, sw_dev, n, loss_host, &a));
   nn->step += 1;
   if (loss_host) {
-    PGPU_CUDA(nn->ctx, cudaStreamSynchronize(nn->ctx->stream));
     return pgpu_check_flag(nn->ctx, "mlp_train_step");
   }
   return PGPU_OK;

@@ -81,6 +81,10 @@ struct PrunePlan {
 };
 
 constexpr int PGPU_STAGES = 4;
+// bytes of pgpu_ctx::h_pinned, and where the error word's copy lies in it
+constexpr size_t PGPU_PINNED = 4096, PGPU_PINNED_FLAG = PGPU_PINNED - 64;
+// host calls put inputs and results up to this size through the staging blocks
+constexpr size_t PGPU_STAGE_MOST = 128 * 1024;
 
 // column chunks (at most) of the host-buffer calls' copies: 2-D copies of
 // narrower columns overlap each other worse
@@ -174,7 +178,8 @@ pgpu_status pgpu_set_err(pgpu_ctx *ctx, pgpu_status st, const char *fmt, ...);
 pgpu_status pgpu_buf(pgpu_ctx *ctx, int slot, size_t bytes, void **out);
 // Launch bookkeeping: checks the launch error and counts it.
 pgpu_status pgpu_after_launch(pgpu_ctx *ctx, const char *what);
-// Reads and clears the device error word after a synchronize.
+// Waits for the context's stream, then reads and clears the device error
+// word: a host call queues its result copies and ends with this.
 pgpu_status pgpu_check_flag(pgpu_ctx *ctx, const char *what);
 // Pinned host block and its device twin for `bytes` of small parameters;
 // fill *host, then pgpu_stage_commit copies it on the context's stream.
@@ -189,6 +194,8 @@ pgpu_status pgpu_stage_copy(pgpu_ctx *ctx, void *dst, size_t bytes);
 // tree schedule (schedule.cpp)
 // ---------------------------------------------------------------------------
 
+// Validates the tree's child arrays.
+pgpu_status pgpu_check_tree(pgpu_ctx *ctx, const pgpu_tree *tree);
 pgpu_status pgpu_build_schedule(pgpu_ctx *ctx, const pgpu_tree *tree, TreeSchedule *out);
 // Builds (or reuses) the schedule of `tree` and makes its ops and tip
 // sequence resident on the device.

@@ -14,7 +14,7 @@
 
 #include "pgpu_internal.cuh"
 
-pgpu_status pgpu_build_schedule(pgpu_ctx *ctx, const pgpu_tree *tree, TreeSchedule *out) {
+pgpu_status pgpu_check_tree(pgpu_ctx *ctx, const pgpu_tree *tree) {
   if (!tree || !tree->left || !tree->right)
     return pgpu_set_err(ctx, PGPU_ERR_ARG, "tree: null tree or child arrays");
   const int32_t n = tree->n_tips;
@@ -35,6 +35,12 @@ pgpu_status pgpu_build_schedule(pgpu_ctx *ctx, const pgpu_tree *tree, TreeSchedu
     if (uses[id] != 1)
       return pgpu_set_err(ctx, PGPU_ERR_ARG, "tree: node %d is the child of %d nodes (must be 1)",
                           id, uses[id]);
+  return PGPU_OK;
+}
+
+pgpu_status pgpu_build_schedule(pgpu_ctx *ctx, const pgpu_tree *tree, TreeSchedule *out) {
+  PGPU_TRY(pgpu_check_tree(ctx, tree));
+  const int32_t n = tree->n_tips, n_int = n - 1, n_nodes = 2 * n - 1;
 
   // stack need of every internal node and which child to evaluate first
   std::vector<int32_t> need(n_nodes, 0);
@@ -112,12 +118,15 @@ pgpu_status pgpu_schedule_device(pgpu_ctx *ctx, const pgpu_tree *tree, const Tre
     PGPU_TRY(pgpu_build_schedule(ctx, tree, &ctx->sched));
     PGPU_TRY(pgpu_buf(ctx, BUF_OPS, ctx->sched.ops.size() * sizeof(SchedOp), &dops));
     PGPU_TRY(pgpu_buf(ctx, BUF_TIPSEQ, ctx->sched.tip_seq.size() * sizeof(int32_t), &dseq));
-    // synchronous copies: the host vectors may change on the next call
-    PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    PGPU_CUDA(ctx, cudaMemcpy(dops, ctx->sched.ops.data(), ctx->sched.ops.size() * sizeof(SchedOp),
-                              cudaMemcpyHostToDevice));
-    PGPU_CUDA(ctx, cudaMemcpy(dseq, ctx->sched.tip_seq.data(),
-                              ctx->sched.tip_seq.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    const size_t ob = ctx->sched.ops.size() * sizeof(SchedOp);
+    const size_t tb = ctx->sched.tip_seq.size() * sizeof(int32_t);
+    void *h;
+    PGPU_TRY(pgpu_stage(ctx, ob, &h, nullptr));
+    std::memcpy(h, ctx->sched.ops.data(), ob);
+    PGPU_TRY(pgpu_stage_copy(ctx, dops, ob));
+    PGPU_TRY(pgpu_stage(ctx, tb, &h, nullptr));
+    std::memcpy(h, ctx->sched.tip_seq.data(), tb);
+    PGPU_TRY(pgpu_stage_copy(ctx, dseq, tb));
     ctx->sched_left.assign(tree->left, tree->left + n_int);
     ctx->sched_right.assign(tree->right, tree->right + n_int);
     ctx->sched_valid = true;

@@ -1611,7 +1611,6 @@ pgpu_status run_fitch_scan(pgpu_spr *s) {
 }
 
 pgpu_status sync_check(pgpu_spr *s, const char *what) {
-  PGPU_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
   return pgpu_check_flag(s->ctx, what);
 }
 

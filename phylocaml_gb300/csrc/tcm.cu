@@ -460,10 +460,7 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
     return pgpu_set_err(ctx, PGPU_ERR_OVERFLOW,
                         "tcm_tree: a site's cost can reach %llu x %d, above 2^32 - 1",
                         (unsigned long long)emax, tree->n_tips - 1);
-  const TreeSchedule *sch;
-  const int4 *d_ops;
-  const int32_t *d_seq;
-  PGPU_TRY(pgpu_schedule_device(ctx, tree, &sch, &d_ops, &d_seq));
+  if (n_words == 0) PGPU_TRY(pgpu_check_tree(ctx, tree));
   void *h, *d;
   PGPU_TRY(pgpu_stage(ctx, 256 * sizeof(uint32_t), &h, &d));
   std::memcpy(h, table, 256 * sizeof(uint32_t));
@@ -481,6 +478,10 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
                                static_cast<const uint32_t *>(d), period, node_sets, site_cost, total,
                                &launched, io));
   if (launched) return PGPU_OK;
+  const TreeSchedule *sch;
+  const int4 *d_ops;
+  const int32_t *d_seq;
+  PGPU_TRY(pgpu_schedule_device(ctx, tree, &sch, &d_ops, &d_seq));
   const size_t n = (size_t)tree->n_tips;
   if (io)
     PGPU_CUDA(ctx, cudaMemcpy2DAsync(const_cast<uint32_t *>(tips), ld * 4, io->tips, n_words * 4, n_words * 4,
@@ -678,7 +679,6 @@ pgpu_status pgpu_tcm_tree_wide(pgpu_ctx *ctx, const pgpu_tree *tree, const uint3
   }
   uint64_t *ht = reinterpret_cast<uint64_t *>(ctx->h_pinned);
   PGPU_CUDA(ctx, cudaMemcpyAsync(ht, dtot, 8, cudaMemcpyDeviceToHost, s));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(s));
   PGPU_TRY(pgpu_check_flag(ctx, "tcm_tree_wide"));
   *total = *ht;
   return PGPU_OK;
@@ -768,7 +768,6 @@ pgpu_status pgpu_tcm_tree(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *
       PGPU_CUDA(ctx, cudaMemcpyAsync(site_cost, dsc, n_sites * 4, cudaMemcpyDeviceToHost, s));
     uint64_t *ht = reinterpret_cast<uint64_t *>(ctx->h_pinned);
     PGPU_CUDA(ctx, cudaMemcpyAsync(ht, dtot, 8, cudaMemcpyDeviceToHost, s));
-    PGPU_CUDA(ctx, cudaStreamSynchronize(s));
     PGPU_TRY(pgpu_check_flag(ctx, "tcm_tree"));
     *total = *ht;
     return PGPU_OK;
@@ -793,7 +792,6 @@ pgpu_status pgpu_tcm_tree(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *
     PGPU_CUDA(ctx, cudaMemcpyAsync(site_cost, dsc, n_sites * 4, cudaMemcpyDeviceToHost, s));
   uint64_t *ht = reinterpret_cast<uint64_t *>(ctx->h_pinned);
   PGPU_CUDA(ctx, cudaMemcpyAsync(ht, dtot, 8, cudaMemcpyDeviceToHost, s));
-  PGPU_CUDA(ctx, cudaStreamSynchronize(s));
   PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->d2h_stream));
   PGPU_TRY(pgpu_check_flag(ctx, "tcm_tree"));
   *total = *ht;

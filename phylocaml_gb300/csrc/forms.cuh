@@ -213,6 +213,8 @@ struct Fp32 {
   __device__ static V zero() { return 0.0f; }
   __device__ static float mag(V v) { return v; }
   __device__ static double to_d(V v) { return (double)v; }
+  __device__ static float to_f(V v) { return v; }
+  __device__ static ff to_ff(V v) { return {v, 0.0f}; }
   __device__ static V mul(V a, V b) { return a * b; }
   __device__ static void mul4(const V *a, const V *b, V *y) {
 #pragma unroll
@@ -226,6 +228,12 @@ struct Fp32 {
     y[2] = v.z;
     y[3] = v.w;
   }
+  // load_tip and store4 of vectors in global memory, 32-byte aligned in the
+  // 32-byte forms: one request each, so that a warp's store fills whole
+  // sectors (the SPR pool took 4.2 ms with two 16-byte halves a vector and
+  // 3.5 with one request, nothing else changed)
+  __device__ static void load_g(const void *tab, size_t at, V *y) { load_tip(tab, at, y); }
+  __device__ static void store_g(void *tab, size_t at, const V *y) { store4(tab, at, y); }
   // a row of load_tip's layout whose 16-byte halves lie at the shared-window
   // addresses a and b (one here)
   __device__ static void load_row_s(uint32_t a, uint32_t, V *y) {
@@ -266,6 +274,7 @@ struct Fp64 {
   __device__ static V zero() { return 0.0; }
   __device__ static double mag(V v) { return v; }
   __device__ static double to_d(V v) { return v; }
+  __device__ static float to_f(V v) { return (float)v; }
   __device__ static V mul(V a, V b) { return a * b; }
   __device__ static void mul4(const V *a, const V *b, V *y) {
 #pragma unroll
@@ -279,6 +288,16 @@ struct Fp64 {
     y[1] = a.y;
     y[2] = b.x;
     y[3] = b.y;
+  }
+  __device__ static void load_g(const void *tab, size_t at, V *y) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(y[0]), "=d"(y[1]), "=d"(y[2]), "=d"(y[3])
+                 : "l"(static_cast<const char *>(tab) + 32 * at));
+  }
+  __device__ static void store_g(void *tab, size_t at, const V *y) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(static_cast<char *>(tab) + 32 * at), "d"(y[0]),
+                 "d"(y[1]), "d"(y[2]), "d"(y[3])
+                 : "memory");
   }
   __device__ static void load_row_s(uint32_t a, uint32_t b, V *y) {
     asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y[0]), "=d"(y[1]) : "r"(a) : "memory");
@@ -316,6 +335,8 @@ struct Ff32 {
   __device__ static V zero() { return {0.0f, 0.0f}; }
   __device__ static float mag(V v) { return v.h; }
   __device__ static double to_d(V v) { return (double)v.h + (double)v.l; }
+  __device__ static float to_f(V v) { return __fadd_rn(v.h, v.l); }
+  __device__ static ff to_ff(V v) { return v; }
   // exact product left unnormalised: the low word stays within a few ulps
   // of the high word, which every consumer of the pair tolerates
   __device__ static V mul(V a, V b) {
@@ -336,6 +357,18 @@ struct Ff32 {
     y[1] = {a.y, a.w};
     y[2] = {b.x, b.z};
     y[3] = {b.y, b.w};
+  }
+  __device__ static void load_g(const void *tab, size_t at, V *y) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(y[0].h), "=f"(y[1].h), "=f"(y[0].l), "=f"(y[1].l), "=f"(y[2].h), "=f"(y[3].h), "=f"(y[2].l),
+                   "=f"(y[3].l)
+                 : "l"(static_cast<const char *>(tab) + 32 * at));
+  }
+  __device__ static void store_g(void *tab, size_t at, const V *y) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(static_cast<char *>(tab) + 32 * at),
+                 "f"(y[0].h), "f"(y[1].h), "f"(y[0].l), "f"(y[1].l), "f"(y[2].h), "f"(y[3].h), "f"(y[2].l),
+                 "f"(y[3].l)
+                 : "memory");
   }
   __device__ static void load_row_s(uint32_t a, uint32_t b, V *y) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"

@@ -12,7 +12,10 @@
 // its side, M[d] = P(t) L[d] and H[d] = P(t/2) L[d], with per-pattern
 // power-of-two scalers, for all patterns and rate classes, in HBM.  A
 // thread owns one (pattern, rate class) and walks the pass order, so no
-// thread reads a vector another thread wrote.
+// thread reads a vector another thread wrote.  H is only read where moves
+// are scored, so the pass writes it when that is what it was asked for, and
+// spr_half_kernel adds it to a pool made without it (the branch-length
+// rounds make several that nothing scores from).
 //
 // Scan (spr_scan_kernel, one CTA per prune x pattern-block group): removing
 // the subtree on p's side of (p,u) changes only the vectors that look
@@ -78,6 +81,11 @@ __device__ __forceinline__ void rescale(typename Pol::V *acc, int &sc) {
   }
 }
 
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
 struct PoolArgs {
   void *L, *M, *H;
   int32_t *sc;
@@ -91,7 +99,12 @@ struct PoolArgs {
   int n_ops, R, NP;
 };
 
-template <typename Pol, int RT>
+// HBM-bound: two or three vectors written and up to two read per step.  The
+// next step's vectors are read while this step is computed, unless this step
+// makes them (then they pass in registers); depth-first order keeps what a
+// step reads recent.  256 taxa x 45,675 patterns, pair form: 2.88 ms without
+// H; level by level and with nothing read ahead it was 7.2 ms with H.
+template <typename Pol, int RT, bool HALF>
 __global__ void __launch_bounds__(SPR_NT) spr_pool_kernel(const PoolArgs a) {
   using V = typename Pol::V;
   using Coef = typename Pol::Coef;
@@ -101,38 +114,82 @@ __global__ void __launch_bounds__(SPR_NT) spr_pool_kernel(const PoolArgs a) {
   const bool on = r < a.R;
   const int R = a.R;
   auto vi = [&](int d) { return ((size_t)d * a.np + pat) * R + r; };
-  for (int i = 0; i < a.n_ops; ++i) {
-    const int4 op = __ldg(a.ops + i);
-    V acc[4];
-    int s = a.sc[(size_t)op.y * a.np + pat] + a.sc[(size_t)op.z * a.np + pat];
-    if (on) {
-      V x[4], y[4];
-      Pol::load_tip(a.M, vi(op.y), x);
-      Pol::load_tip(a.M, vi(op.z), y);
+  V x[4], y[4], m[4];
+  int sx = 0, sy = 0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] = Pol::mul(x[e], y[e]);
-    } else {
+  for (int e = 0; e < 4; ++e) x[e] = y[e] = m[e] = Pol::zero();
+  auto read = [&](int d, V *v, int &sv) {
+    sv = a.sc[(size_t)d * a.np + pat];
+    if (on) Pol::load_g(a.M, vi(d), v);
+  };
+  // a step's transition blocks come one step ahead into the warp's own shared
+  // buffer, the 16-byte units of its classes interleaved
+  constexpr int U = 16 * sizeof(Coef) / 16, UNITS = U * RT;
+  __shared__ uint4 dsh[SPR_NW][2][HALF ? 2 : 1][UNITS];
+  auto blocks = [&](int buf, int ed) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] = Pol::zero();
+    for (int k = 0; k < (UNITS + 31) / 32; ++k) {
+      const int q = k * 32 + lane, cls = q / U;
+      if (cls < R) {
+        const uint4 *src = static_cast<const uint4 *>(a.Dfull) + (size_t)ed * R * U + q;
+        copy16(&dsh[c >> 5][buf][0][(q % U) * RT + cls], src);
+        if (HALF) copy16(&dsh[c >> 5][buf][HALF ? 1 : 0][(q % U) * RT + cls],
+                         static_cast<const uint4 *>(a.Dhalf) + (size_t)ed * R * U + q);
+      }
     }
+    asm volatile("cp.async.commit_group;");
+  };
+  int4 op = a.n_ops > 0 ? __ldg(a.ops) : make_int4(0, 0, 0, 0);
+  if (a.n_ops > 0) {
+    blocks(0, op.x >> 1);
+    read(op.y, x, sx);
+    read(op.z, y, sy);
+  }
+  for (int i = 0; i < a.n_ops; ++i) {
+    const int4 next = i + 1 < a.n_ops ? __ldg(a.ops + i + 1) : op;
+    const bool more = i + 1 < a.n_ops;
+    V acc[4];
+    int s = sx + sy;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = Pol::mul(x[e], y[e]);
+    const bool from_x = next.y == op.x, from_y = next.z == op.x;
+    if (more && !from_x) read(next.y, x, sx);
+    if (more && !from_y) read(next.z, y, sy);
     rescale<Pol, RT>(acc, s);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();   // this step's blocks are here, and all lanes are done with the step before's
+    if (more) blocks((i + 1) & 1, next.x >> 1);
+    const uint4(*dw)[UNITS] = dsh[c >> 5][i & 1];
     if (on) {
-      const int ed = op.x >> 1;
-      V m[4], h[4];
-      Pol::rows(static_cast<const Coef *>(a.Dfull) + ((size_t)ed * R + r) * 16, acc, m);
-      Pol::rows(static_cast<const Coef *>(a.Dhalf) + ((size_t)ed * R + r) * 16, acc, h);
-      Pol::store4(a.L, vi(op.x), acc);
-      Pol::store4(a.M, vi(op.x), m);
-      Pol::store4(a.H, vi(op.x), h);
+      Pol::rows(reinterpret_cast<const Coef *>(&dw[0][r]), acc, m, RT);
+      Pol::store_g(a.L, vi(op.x), acc);
+      Pol::store_g(a.M, vi(op.x), m);
+      if (HALF) {
+        V h[4];
+        Pol::rows(reinterpret_cast<const Coef *>(&dw[HALF ? 1 : 0][r]), acc, h, RT);
+        Pol::store_g(a.H, vi(op.x), h);
+      }
     }
     if (r == 0) a.sc[(size_t)op.x * a.np + pat] = s;
+    if (from_x) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = m[e];
+      sx = s;
+    }
+    if (from_y) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = m[e];
+      sy = s;
+    }
+    op = next;
+    __syncwarp();   // the scalers of a pattern are written by its first lane
   }
   // log-likelihood across edge 0: L[side a] . P(t) L[side b]
   double part = 0.0;
   if (on) {
     V x[4], y[4];
-    Pol::load_tip(a.L, vi(0), x);
-    Pol::load_tip(a.M, vi(1), y);
+    Pol::load_g(a.L, vi(0), x);
+    Pol::load_g(a.M, vi(1), y);
     double lr = 0.0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) lr += a.pi[e] * Pol::to_d(Pol::mul(x[e], y[e]));
@@ -162,7 +219,7 @@ struct TipArgs {
   void *L, *M, *H;
   int32_t *sc;
   const void *tipfull, *tiphalf;   // [n_tips][R][n_codes][4] values of the form
-  const double *code_tab;          // [n_codes][4]
+  const void *code_rows;           // [n_codes] vectors of the form
   const uint8_t *codes;            // [n_tips][ld]
   const int4 *tips;                // {dedge, tip, edge, 0}
   int *flag;
@@ -170,30 +227,53 @@ struct TipArgs {
   int R, n_codes;
 };
 
-template <typename Pol>
+// A thread per (pattern, rate class), so that a warp's vectors are one run of
+// memory.  LM: L, M and the scalers; HALF: H.  256 taxa x 45,675 patterns, L
+// and M: 0.45 ms (6.7 TB/s) with the codes' vectors ready in the form, 1.32
+// with their FP64 values converted in every thread.
+template <typename Pol, bool LM, bool HALF>
 __global__ void __launch_bounds__(256) spr_tip_kernel(const TipArgs a) {
   using V = typename Pol::V;
-  const size_t pat = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (pat >= a.np) return;
+  const unsigned i = blockIdx.x * 256 + threadIdx.x;   // np R < 2^32: three such arrays per edge fit in memory
+  if (i >= a.np * a.R) return;
+  const unsigned pat = i / (unsigned)a.R;
+  const int r = (int)(i - pat * (unsigned)a.R);
   const int4 t = a.tips[blockIdx.y];
   int code = pat < a.n_pat ? a.codes[(size_t)t.y * a.ld + pat] : 0;
   if (code >= a.n_codes) {
     atomicOr(a.flag, PGPU_FLAG_BADCODE);
     code = 0;
   }
-  V l[4], m[4], h[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) l[e] = Pol::from_d(a.code_tab[code * 4 + e]);
-  for (int r = 0; r < a.R; ++r) {
-    const size_t at = ((size_t)t.x * a.np + pat) * a.R + r;
-    const size_t tt = ((size_t)t.y * a.R + r) * a.n_codes + code;
-    Pol::load_tip(a.tipfull, tt, m);
-    Pol::load_tip(a.tiphalf, tt, h);
-    Pol::store4(a.L, at, l);
-    Pol::store4(a.M, at, m);
-    Pol::store4(a.H, at, h);
+  const size_t at = (size_t)t.x * a.np * a.R + i;
+  const size_t tt = ((size_t)t.y * a.R + r) * a.n_codes + code;
+  V v[4];
+  if (LM) {
+    Pol::load_g(a.code_rows, code, v);
+    Pol::store_g(a.L, at, v);
+    Pol::load_g(a.tipfull, tt, v);
+    Pol::store_g(a.M, at, v);
+    if (r == 0) a.sc[(size_t)t.x * a.np + pat] = 0;
   }
-  a.sc[(size_t)t.x * a.np + pat] = 0;
+  if (HALF) {
+    Pol::load_g(a.tiphalf, tt, v);
+    Pol::store_g(a.H, at, v);
+  }
+}
+
+// H of every internal directed edge of a pool made without it.
+template <typename Pol>
+__global__ void __launch_bounds__(256) spr_half_kernel(const void *L, void *H, const void *Dhalf, const int4 *ops,
+                                                       size_t np, unsigned R) {
+  using V = typename Pol::V;
+  using Coef = typename Pol::Coef;
+  const unsigned i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= np * R) return;
+  const int d = __ldg(ops + blockIdx.y).x;
+  const int r = (int)(i % R);
+  V x[4], h[4];
+  Pol::load_g(L, (size_t)d * np * R + i, x);
+  Pol::rows(static_cast<const Coef *>(Dhalf) + ((size_t)(d >> 1) * R + r) * 16, x, h);
+  Pol::store_g(H, (size_t)d * np * R + i, h);
 }
 
 __global__ void __launch_bounds__(1024) spr_pool_finalize_kernel(const double2 *partials, int n,
@@ -212,7 +292,7 @@ struct ScanArgs {
   const SprStep *steps;
   const SprPrune *prunes;
   const double *pi, *probs;
-  const float *wts;           // [np], zero beyond n_pat
+  const float2 *wts;          // [np] float pairs, zero beyond n_pat
   const float4 *logtab;       // 64 entries
   double *partials;           // [n_groups][n_moves]
   int *flag;
@@ -271,11 +351,12 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
     const size_t pat = (size_t)blk * a.NP + pl;
     auto vi = [&](int d) { return ((size_t)d * a.np + pat) * R + r; };
     auto scv = [&](int d) { return a.sc[(size_t)d * a.np + pat]; };
-    const float w = a.wts[pat];
+    const float2 wp = a.wts[pat];
+    const ff w{wp.x, wp.y};
     V vp[4];
     const int scp = EMIT ? 0 : scv(pr.dp);
     if (on && !EMIT) {
-      Pol::load_tip(a.M, vi(pr.dp), vp);
+      Pol::load_g(a.M, vi(pr.dp), vp);
 #pragma unroll
       for (int e = 0; e < 4; ++e) vp[e] = Pol::mul(vp[e], piv[e]);
     } else {
@@ -301,8 +382,8 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
         V ms[4], mg[4];
         if (on) {
           V ls[4], lg[4];
-          Pol::load_tip(a.L, vi(st.d1), ls);
-          Pol::load_tip(a.L, vi(st.d2), lg);
+          Pol::load_g(a.L, vi(st.d1), ls);
+          Pol::load_g(a.L, vi(st.d2), lg);
           Pol::rows(Dm, lg, ms);   // into s, from g's side across the joined edge
           Pol::rows(Dm, ls, mg);
         } else {
@@ -335,8 +416,8 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
       int sc1 = in_sc + s2, sc2 = in_sc + s1;
       if (on) {
         V m1[4], m2[4];
-        Pol::load_tip(a.M, vi(st.d1), m1);
-        Pol::load_tip(a.M, vi(st.d2), m2);
+        Pol::load_g(a.M, vi(st.d1), m1);
+        Pol::load_g(a.M, vi(st.d2), m2);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           l1[e] = Pol::mul(in[e], m2[e]);
@@ -362,7 +443,7 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
           for (int h = 0; h < 2; ++h) {
             const int out = h == 0 ? st.out1 : st.out2;
             if (out < 0) continue;
-            Pol::load_tip(a.H, vi(h == 0 ? st.d1 : st.d2), hh);
+            Pol::load_g(a.H, vi(h == 0 ? st.d1 : st.d2), hh);
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[e] = Pol::mul(h == 0 ? h1[e] : h2[e], hh[e]);
             if (side_b) {
@@ -372,7 +453,7 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
               for (int e = 0; e < 4; ++e) y[e] = Pol::mul(x[e], Pol::from_d(a.probs[r] * a.pi[e]));
             }
             const size_t slot = (size_t)(out - a.slot_base);
-            Pol::store4(a.xout, (slot * a.np + pat) * R + r, y);
+            Pol::store_g(a.xout, (slot * a.np + pat) * R + r, y);
             if (r == 0) a.xsc[slot * a.np + pat] = h == 0 ? sc1 + s1 : sc2 + s2;
           }
         }
@@ -381,13 +462,13 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
         if (on) {
           V hh[4];
           if (st.out1 >= 0) {
-            Pol::load_tip(a.H, vi(st.d1), hh);
+            Pol::load_g(a.H, vi(st.d1), hh);
 #pragma unroll
             for (int e = 0; e < 4; ++e) p1 = Pol::add(p1, Pol::mul(Pol::mul(h1[e], hh[e]), vp[e]));
             p1 = Pol::mul(p1, prob);
           }
           if (st.out2 >= 0) {
-            Pol::load_tip(a.H, vi(st.d2), hh);
+            Pol::load_g(a.H, vi(st.d2), hh);
 #pragma unroll
             for (int e = 0; e < 4; ++e) p2 = Pol::add(p2, Pol::mul(Pol::mul(h2[e], hh[e]), vp[e]));
             p2 = Pol::mul(p2, prob);
@@ -399,13 +480,13 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
           p2 = Pol::add(p2, Pol::shfl_xor(p2, o));
         }
         ff v1{0.0f, 0.0f}, v2{0.0f, 0.0f};
-        if (w != 0.0f) {
+        if (w.h != 0.0f) {
           if (mine1 && st.out1 >= 0) {
-            if (Pol::positive(p1)) v1 = ff_mul(Pol::site_log(p1, sc1 + s1 + scp, ltab), ff{w, 0.0f});
+            if (Pol::positive(p1)) v1 = ff_mul(Pol::site_log(p1, sc1 + s1 + scp, ltab), w);
             else atomicOr(a.flag, PGPU_FLAG_NAN);
           }
           if (mine2 && st.out2 >= 0) {
-            if (Pol::positive(p2)) v2 = ff_mul(Pol::site_log(p2, sc2 + s2 + scp, ltab), ff{w, 0.0f});
+            if (Pol::positive(p2)) v2 = ff_mul(Pol::site_log(p2, sc2 + s2 + scp, ltab), w);
             else atomicOr(a.flag, PGPU_FLAG_NAN);
           }
         }
@@ -450,16 +531,33 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
   }
 }
 
-// lnl[m] = sum over CTA groups of the partial sums, in group order
-__global__ void spr_reduce_kernel(const double *partials, int n_groups, size_t n_moves, double *lnl) {
-  const size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n_moves) return;
+// lnl[m] = sum over CTA groups of the partial sums: slice y of a move's groups
+// by thread (move, y), the slices in order.  A chain over all the groups kept
+// a few moves of 714 groups waiting 210 us; 56 us in 32 slices.
+constexpr int RED_Y = 32;
+__global__ void __launch_bounds__(32 * RED_Y) spr_reduce_kernel(const double *partials, int n_groups, size_t n_moves,
+                                                                double *lnl) {
+  __shared__ double2 part[RED_Y][33];
+  const int x = threadIdx.x, y = threadIdx.y;
+  const size_t m = (size_t)blockIdx.x * 32 + x;
+  const int per = (n_groups + RED_Y - 1) / RED_Y, g0 = y * per, g1 = min(g0 + per, n_groups);
   double s = 0.0, c = 0.0;
-  for (int g = 0; g < n_groups; ++g) {
+  if (m < n_moves)
+    for (int g = g0; g < g1; ++g) {
+      double t, e;
+      two_sum(s, partials[(size_t)g * n_moves + m], t, e);
+      s = t;
+      c += e;
+    }
+  part[y][x] = make_double2(s, c);
+  __syncthreads();
+  if (y != 0 || m >= n_moves) return;
+  for (int k = 1; k < RED_Y; ++k) {
+    const double2 v = part[k][x];
     double t, e;
-    two_sum(s, partials[(size_t)g * n_moves + m], t, e);
+    two_sum(s, v.x, t, e);
     s = t;
-    c += e;
+    c += e + v.y;
   }
   lnl[m] = s + c;
 }
@@ -488,7 +586,7 @@ struct PairArgs {
   const int32_t *xsc;       // [slot][np]
   const int4 *tiles;        // {cut, j0, k0, 0}
   const TbrCutDev *cuts;
-  const float *wts;         // [np], zero beyond n_pat
+  const float2 *wts;        // [np] float pairs, zero beyond n_pat
   const float4 *logtab;
   double *partials;         // [n_groups][n_moves]
   int *flag;
@@ -567,7 +665,7 @@ __global__ void __launch_bounds__(256) tbr_pair_kernel(const PairArgs a) {
       int sc = 0;
       if (idx < (side == 0 ? cut.nA : cut.nB)) {
         const size_t slot = (size_t)((side == 0 ? cut.slotA : cut.slotB) + idx);
-        Pol::load_tip(a.X, (slot * a.np + pat) * R + r, v);
+        Pol::load_g(a.X, (slot * a.np + pat) * R + r, v);
         sc = a.xsc[slot * a.np + pat];
       } else {
 #pragma unroll
@@ -581,14 +679,14 @@ __global__ void __launch_bounds__(256) tbr_pair_kernel(const PairArgs a) {
     __syncthreads();
     if (!mine) continue;
     for (int p = 0; p < TB_PB; ++p) {
-      const float w = a.wts[pat0 + p];
-      if (w == 0.0f) continue;
+      const float2 w = a.wts[pat0 + p];
+      if (w.x == 0.0f) continue;
       const V *xr = Xs + (size_t)jj * RS + (size_t)p * R * 4;
       const V *zr = Zs + (size_t)kk * RS + (size_t)p * R * 4;
       const V acc = pair_dot<Pol>(xr, zr, R * 4);
       if (Pol::positive(acc))
         sum = ff_add(sum, ff_mul(Pol::site_log(acc, xs[jj * TB_PB + p] + ys[kk * TB_PB + p], ltab),
-                                 ff{w, 0.0f}));
+                                 ff{w.x, w.y}));
       else
         atomicOr(a.flag, PGPU_FLAG_NAN);
     }
@@ -601,37 +699,44 @@ __global__ void __launch_bounds__(256) tbr_pair_kernel(const PairArgs a) {
 // ---------------------------------------------------------------------------
 // Fitch sets on the directed edges and the parsimony length of every move
 // ---------------------------------------------------------------------------
-constexpr uint32_t LANE_MSB = 0x88888888u;
-
-__device__ __forceinline__ uint32_t empty_lanes(uint32_t v) {
-  const uint32_t nz = (((v & ~LANE_MSB) + ~LANE_MSB) | v) & LANE_MSB;
-  return nz ^ LANE_MSB;
+// The state sets of 32 patterns are four words, one per state (bit j: pattern
+// 32 q + j holds the state), so that a Fitch step is eight three-input logic
+// operations on 32 patterns and the empty joins are one word: 28 operations
+// with the four states of a pattern side by side in nibbles.
+//   empty = no state in both; set = (a & b) or, where empty, a | b
+__device__ __forceinline__ uint32_t meet(uint4 a, uint4 b) {
+  return (a.x & b.x) | (a.y & b.y) | (a.z & b.z) | (a.w & b.w);
 }
-__device__ __forceinline__ uint32_t fitch_set(uint32_t a, uint32_t b, uint32_t *empty) {
-  const uint32_t x = a & b;
-  const uint32_t e = empty_lanes(x);
-  const uint32_t fill = e | (e - (e >> 3));
-  *empty = e;
-  return (x & ~fill) | ((a | b) & fill);
+__device__ __forceinline__ uint4 fitch4(uint4 a, uint4 b, uint32_t *empty) {
+  const uint32_t none = ~meet(a, b);
+  *empty = none;
+  return make_uint4((a.x & b.x) | ((a.x | b.x) & none), (a.y & b.y) | ((a.y | b.y) & none),
+                    (a.z & b.z) | ((a.z | b.z) & none), (a.w & b.w) | ((a.w | b.w) & none));
 }
-__device__ __forceinline__ uint4 fitch4(uint4 a, uint4 b, uint4 *e) {
-  uint4 o;
-  o.x = fitch_set(a.x, b.x, &e->x);
-  o.y = fitch_set(a.y, b.y, &e->y);
-  o.z = fitch_set(a.z, b.z, &e->z);
-  o.w = fitch_set(a.w, b.w, &e->w);
-  return o;
-}
-// weighted count of the lanes flagged in e (lane MSBs), weights as bit planes
-__device__ __forceinline__ uint32_t wcount(uint4 e, const uint4 *planes, size_t stride, int n_planes,
-                                           size_t at) {
-  uint32_t s = 0;
-  for (int b = 0; b < n_planes; ++b) {
-    const uint4 p = planes[(size_t)b * stride + at];
-    s += (uint32_t)(__popc(e.x & p.x) + __popc(e.y & p.y) + __popc(e.z & p.z) + __popc(e.w & p.w)) << b;
+// weighted count of the patterns flagged in a word, the weights as bit planes;
+// a thread reads the low planes of its patterns once
+constexpr int WPLANES = 8;
+struct WeightPlanes {
+  const uint32_t *p;
+  size_t stride;
+  int n;
+  uint32_t low[WPLANES];
+  __device__ void load(const uint32_t *planes, size_t w4, int n_planes, size_t at, bool in) {
+    p = planes + at;
+    stride = w4;
+    n = in ? n_planes : 0;
+#pragma unroll
+    for (int b = 0; b < WPLANES; ++b) low[b] = b < n ? p[b * stride] : 0u;
   }
-  return s;
-}
+  __device__ uint32_t count(uint32_t f) const {
+    uint32_t s = 0;
+#pragma unroll
+    for (int b = 0; b < WPLANES; ++b)
+      if (b < n) s += (uint32_t)__popc(f & low[b]) << b;
+    for (int b = WPLANES; b < n; ++b) s += (uint32_t)__popc(f & p[b * stride]) << b;
+    return s;
+  }
+};
 
 struct FitchTipArgs {
   uint4 *F;
@@ -643,84 +748,107 @@ struct FitchTipArgs {
 };
 
 __global__ void __launch_bounds__(256) spr_fitch_tip_kernel(const FitchTipArgs a) {
-  const size_t q = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (q >= a.W4) return;
+  const size_t pat = (size_t)blockIdx.x * 256 + threadIdx.x;
   const int4 t = a.tips[blockIdx.y];
-  uint32_t wv[4];
-  for (int k = 0; k < 4; ++k) {
-    uint32_t word = 0;
-    for (int j = 0; j < 8; ++j) {
-      const size_t pat = (q * 4 + k) * 8 + j;
-      uint32_t m = 0;
-      if (pat < a.n_pat) {
-        const int code = a.codes[(size_t)t.y * a.ld + pat];
-        m = code < a.n_codes ? a.code_mask[code] : 0xFu;
-      }
-      word |= (m & 0xFu) << (4 * j);
-    }
-    wv[k] = word;
+  uint32_t m = 0;
+  if (pat < a.n_pat) {
+    const int code = a.codes[(size_t)t.y * a.ld + pat];
+    m = code < a.n_codes ? a.code_mask[code] : 0xFu;
   }
-  a.F[(size_t)t.x * a.W4 + q] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+  uint4 w;
+  w.x = __ballot_sync(0xffffffffu, m & 1u);
+  w.y = __ballot_sync(0xffffffffu, m & 2u);
+  w.z = __ballot_sync(0xffffffffu, m & 4u);
+  w.w = __ballot_sync(0xffffffffu, m & 8u);
+  if ((threadIdx.x & 31) == 0 && (pat >> 5) < a.W4) a.F[(size_t)t.x * a.W4 + (pat >> 5)] = w;
 }
 
 struct FitchPoolArgs {
   uint4 *F;
   const int4 *ops;
-  const uint4 *planes;
+  const uint32_t *planes;   // [n_planes][W4]
   unsigned long long *cnt;   // [n_ops + 1]: local cost of each op, then edge 0's join
   size_t W4;
   int n_ops, n_planes;
 };
 
-__device__ __forceinline__ void block_add_u64(uint32_t v, unsigned long long *dst) {
-  __shared__ unsigned long long acc;
-  if (threadIdx.x == 0) acc = 0;
-  __syncthreads();
-  v = __reduce_add_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0 && v) atomicAdd(&acc, (unsigned long long)v);
-  __syncthreads();
-  if (threadIdx.x == 0 && acc) atomicAdd(dst, acc);
-}
-
-__global__ void __launch_bounds__(256) spr_fitch_pool_kernel(const FitchPoolArgs a) {
-  const size_t q = (size_t)blockIdx.x * 256 + threadIdx.x;
+// Bound by the chain of steps: a thread owns 32 patterns of every directed
+// edge, so a small alignment has few warps.  The next step's sets are read
+// while this one is computed and each warp adds its own count, with no barrier
+// in the chain; CTAs of two warps spread over the SMs.  762 steps x 45,675
+// patterns: 0.29 ms against 0.85 with 256-thread CTAs adding up each step.
+constexpr int FPOOL_NT = 64;
+__global__ void __launch_bounds__(FPOOL_NT) spr_fitch_pool_kernel(const FitchPoolArgs a) {
+  const size_t q = (size_t)blockIdx.x * FPOOL_NT + threadIdx.x;
   const bool in = q < a.W4;
+  WeightPlanes wp;
+  wp.load(a.planes, a.W4, a.n_planes, in ? q : 0, in);
+  auto get = [&](int d) { return in ? a.F[(size_t)d * a.W4 + q] : make_uint4(0, 0, 0, 0); };
+  auto add = [&](uint32_t e, unsigned long long *dst) {
+    const uint32_t v = __reduce_add_sync(0xffffffffu, wp.count(e));
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, (unsigned long long)v);
+  };
+  uint4 x = make_uint4(0, 0, 0, 0), y = x;
+  int4 op = a.n_ops > 0 ? __ldg(a.ops) : make_int4(0, 0, 0, 0);
+  if (a.n_ops > 0) {
+    x = get(op.y);
+    y = get(op.z);
+  }
   for (int i = 0; i < a.n_ops; ++i) {
-    const int4 op = __ldg(a.ops + i);
-    uint32_t v = 0;
-    if (in) {
-      uint4 e;
-      const uint4 o = fitch4(a.F[(size_t)op.y * a.W4 + q], a.F[(size_t)op.z * a.W4 + q], &e);
-      a.F[(size_t)op.x * a.W4 + q] = o;
-      v = wcount(e, a.planes, a.W4, a.n_planes, q);
+    const bool more = i + 1 < a.n_ops;
+    const int4 next = more ? __ldg(a.ops + i + 1) : op;
+    uint32_t e;
+    const uint4 o = fitch4(x, y, &e);
+    if (in) a.F[(size_t)op.x * a.W4 + q] = o;
+    if (more) {
+      x = next.y == op.x ? o : get(next.y);
+      y = next.z == op.x ? o : get(next.z);
     }
-    block_add_u64(v, a.cnt + i);
+    add(e, a.cnt + i);
+    op = next;
   }
-  uint32_t v = 0;
-  if (in) {
-    uint4 e;
-    (void)fitch4(a.F[q], a.F[a.W4 + q], &e);
-    v = wcount(e, a.planes, a.W4, a.n_planes, q);
-  }
-  block_add_u64(v, a.cnt + a.n_ops);
+  uint32_t e;
+  (void)fitch4(get(0), get(1), &e);
+  add(e, a.cnt + a.n_ops);
 }
 
-// lenF[d]: parsimony length of the subtree on d's side; lenF[nd] = tree length
-__global__ void spr_fitch_len_kernel(const int4 *ops, int n_ops, const unsigned long long *cnt,
-                                     unsigned long long *lenF, int nd) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// lenF[d]: parsimony length of the subtree on d's side; lenF[nd] = tree
+// length.  One thread adds along the steps; the others bring the steps and
+// hold the lengths in shared memory while the tree has room there (a step
+// took 160 ns from global memory).
+constexpr int FLEN_NT = 256;
+__global__ void __launch_bounds__(FLEN_NT) spr_fitch_len_kernel(const int4 *ops, int n_ops,
+                                                                const unsigned long long *cnt,
+                                                                unsigned long long *lenF, int nd, int in_shared) {
+  extern __shared__ unsigned long long len_sh[];
+  __shared__ int4 op_sh[FLEN_NT];
+  __shared__ unsigned long long cnt_sh[FLEN_NT];
+  unsigned long long *len = in_shared ? len_sh : lenF;
   // tips (and everything) start at 0; ops fill in dependency order
-  for (int d = 0; d < nd; ++d) lenF[d] = 0;
-  for (int i = 0; i < n_ops; ++i) {
-    const int4 op = ops[i];
-    lenF[op.x] = lenF[op.y] + lenF[op.z] + cnt[i];
+  for (int d = threadIdx.x; d < nd; d += FLEN_NT) len[d] = 0;
+  for (int i0 = 0; i0 < n_ops; i0 += FLEN_NT) {
+    const int k = min(FLEN_NT, n_ops - i0);
+    __syncthreads();
+    if ((int)threadIdx.x < k) {
+      op_sh[threadIdx.x] = ops[i0 + threadIdx.x];
+      cnt_sh[threadIdx.x] = cnt[i0 + threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int i = 0; i < k; ++i) {
+        const int4 op = op_sh[i];
+        len[op.x] = len[op.y] + len[op.z] + cnt_sh[i];
+      }
   }
-  lenF[nd] = lenF[0] + lenF[1] + cnt[n_ops];
+  __syncthreads();
+  if (in_shared)
+    for (int d = threadIdx.x; d < nd; d += FLEN_NT) lenF[d] = len_sh[d];
+  if (threadIdx.x == 0) lenF[nd] = len[0] + len[1] + cnt[n_ops];
 }
 
 struct FitchScanArgs {
   const uint4 *F;
-  const uint4 *planes;
+  const uint32_t *planes;   // [n_planes][W4]
   const SprStep *steps;
   const SprPrune *prunes;
   unsigned long long *ins;     // [n_moves] weighted empty joins with the pruned set
@@ -747,7 +875,8 @@ __global__ void __launch_bounds__(256) spr_fitch_scan_kernel(const FitchScanArgs
   uint4 cur = make_uint4(0, 0, 0, 0);
   int sp = 0;
   bool have = false, ok = true;
-  auto count = [&](uint4 e) { return in ? wcount(e, a.planes, a.W4, a.n_planes, qq) : 0u; };
+  WeightPlanes wp;
+  wp.load(a.planes, a.W4, a.n_planes, qq, in);
   auto add = [&](unsigned int *dst, uint32_t v) {
     v = __reduce_add_sync(0xffffffffu, v);
     if ((c & 31) == 0 && v) atomicAdd(dst, v);
@@ -756,9 +885,7 @@ __global__ void __launch_bounds__(256) spr_fitch_scan_kernel(const FitchScanArgs
     const SprStep st = a.steps[pr.step_off + si];
     if (st.flags & SPR_START) {
       const uint4 fs = Fd(st.d1), fg = Fd(st.d2);
-      uint4 e;
-      (void)fitch4(fs, fg, &e);
-      add(&join_acc, count(e));
+      add(&join_acc, wp.count(~meet(fs, fg)));
       const bool ds = st.flags & SPR_DOWN1, dg = st.flags & SPR_DOWN2;
       const bool g_first = ds && dg && (st.flags & SPR_FIRST2);
       if (ds && dg) {
@@ -776,20 +903,14 @@ __global__ void __launch_bounds__(256) spr_fitch_scan_kernel(const FitchScanArgs
       cur = stk[(size_t)sp * 256 + c];
     }
     const uint4 f1 = Fd(st.d1), f2 = Fd(st.d2);
-    uint4 e;
+    uint32_t e;
     const uint4 r1 = fitch4(cur, f2, &e);   // y's side seen from c1
     const uint4 r2 = fitch4(cur, f1, &e);
     if (st.out1 >= 0) {
-      const uint4 root = fitch4(r1, f1, &e);
-      const uint4 x = make_uint4(fp.x & root.x, fp.y & root.y, fp.z & root.z, fp.w & root.w);
-      add(&red[st.out1 - pr.move_off],
-          count(make_uint4(empty_lanes(x.x), empty_lanes(x.y), empty_lanes(x.z), empty_lanes(x.w))));
+      add(&red[st.out1 - pr.move_off], wp.count(~meet(fp, fitch4(r1, f1, &e))));
     }
     if (st.out2 >= 0) {
-      const uint4 root = fitch4(r2, f2, &e);
-      const uint4 x = make_uint4(fp.x & root.x, fp.y & root.y, fp.z & root.z, fp.w & root.w);
-      add(&red[st.out2 - pr.move_off],
-          count(make_uint4(empty_lanes(x.x), empty_lanes(x.y), empty_lanes(x.z), empty_lanes(x.w))));
+      add(&red[st.out2 - pr.move_off], wp.count(~meet(fp, fitch4(r2, f2, &e))));
     }
     const bool dn1 = st.flags & SPR_DOWN1, dn2 = st.flags & SPR_DOWN2;
     if (dn1 || dn2) {
@@ -817,40 +938,58 @@ __global__ void __launch_bounds__(256) spr_fitch_scan_kernel(const FitchScanArgs
 // ---------------------------------------------------------------------------
 struct SummaryArgs {
   const void *L;
-  const double *probs, *weights;
+  const double *probs;
+  const float2 *weights;   // [np] float pairs
   float *out;   // [nd][4]
   size_t np, n_pat;
-  int R;
+  int R, RT, rt_shift;
   double inv_w;   // 1 / total weight
 };
 
-// weighted mean over patterns of the state profile L_i / sum_j L_j
+// weighted mean over patterns of the state profile L_i / sum_j L_j.  The FP32
+// values of a vector are summed as float pairs (a reciprocal with its
+// remainder, exact products, exact sums): 48 bits on the FP32 units, where
+// FP64 divisions and sums made the kernel six times as long as reading L.
+// 1,018 directed edges x 45,675 patterns x 4 classes: 0.84 ms against 6.3.
 template <typename Pol>
 __global__ void __launch_bounds__(256) spr_summary_kernel(const SummaryArgs a) {
   using V = typename Pol::V;
   __shared__ double red[4][8];
-  const int d = blockIdx.x;
-  double acc[4] = {0, 0, 0, 0}, wsum = 0.0;
-  for (size_t pat = threadIdx.x; pat < a.n_pat; pat += 256) {
-    const double w = a.weights[pat];
-    for (int r = 0; r < a.R; ++r) {
+  const int d = blockIdx.x, r = threadIdx.x & (a.RT - 1), np_cta = 256 >> a.rt_shift;
+  ff acc[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+  if (r < a.R)
+    for (size_t pat = threadIdx.x >> a.rt_shift; pat < a.n_pat; pat += np_cta) {
       V x[4];
-      Pol::load_tip(a.L, ((size_t)d * a.np + pat) * a.R + r, x);
+      Pol::load_g(a.L, ((size_t)d * a.np + pat) * a.R + r, x);
       float f[4], s = 0.0f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        f[e] = (float)Pol::to_d(x[e]);
+        f[e] = Pol::to_f(x[e]);
         s += f[e];
       }
-      const double k = s > 0.0f ? w * a.probs[r] / s : 0.0;
+      if (!(s > 0.0f)) continue;
+      if (s < 0x1p-100f) {   // a class far below the others: 1 / s has to be finite
+        s *= 0x1p64f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] += k * f[e];
+        for (int e = 0; e < 4; ++e) f[e] *= 0x1p64f;
+      }
+      // q = w / s as a pair
+      const float2 w = a.weights[pat];
+      const float c = __frcp_rn(s);
+      const ff inv{c, __fmul_rn(__fmaf_rn(-c, s, 1.0f), c)};
+      const ff q = ff_mul(inv, ff{w.x, w.y});
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float p = __fmul_rn(q.h, f[e]);
+        float lo = __fmaf_rn(q.h, f[e], -p);
+        lo = __fmaf_rn(q.l, f[e], lo);
+        const ff t = fast_two_sum(fmaxf(acc[e].h, p), fminf(acc[e].h, p));   // no term is negative
+        acc[e] = {t.h, __fadd_rn(acc[e].l, __fadd_rn(t.l, lo))};
+      }
     }
-    wsum += w;
-  }
-  (void)wsum;
+  const double prob = r < a.R ? a.probs[r] : 0.0;
   for (int e = 0; e < 4; ++e) {
-    double v = acc[e];
+    double v = prob * ((double)acc[e].h + (double)acc[e].l);
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) red[e][threadIdx.x >> 5] = v;
   }
@@ -961,24 +1100,130 @@ struct BlArgs {
 // S[e][pat][r][k] = (sum_i pi_i L[a|b]_i U_ik) (sum_j Ui_kj L[b|a]_j), so that
 // the site likelihood across edge e is sum_r probs_r sum_k S_k exp(lam_k rate_r t)
 template <typename Pol>
+__device__ __forceinline__ float eigen_product(const BlArgs &a, const typename Pol::V *x, const typename Pol::V *y,
+                                               int k) {
+  double A = 0.0, B = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    A += a.pi[j] * Pol::to_d(x[j]) * a.U[j * 4 + k];
+    B += a.Ui[k * 4 + j] * Pol::to_d(y[j]);
+  }
+  return (float)(A * B);
+}
+
 __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
-  using V = typename Pol::V;
+  using Pol = Fp64;
+  using V = Pol::V;
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= a.np * a.R) return;
   const int e = blockIdx.y;
   V x[4], y[4];
-  Pol::load_tip(a.L, (size_t)(2 * e) * a.np * a.R + i, x);
-  Pol::load_tip(a.L, (size_t)(2 * e + 1) * a.np * a.R + i, y);
+  Pol::load_g(a.L, (size_t)(2 * e) * a.np * a.R + i, x);
+  Pol::load_g(a.L, (size_t)(2 * e + 1) * a.np * a.R + i, y);
   float s[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    double A = 0.0, B = 0.0;
+  for (int k = 0; k < 4; ++k) s[k] = eigen_product<Pol>(a, x, y, k);
+  reinterpret_cast<float4 *>(a.S)[(size_t)e * a.np * a.R + i] = make_float4(s[0], s[1], s[2], s[3]);
+}
+
+// The same from FP32 values and float pairs, on the FP32 units: each eigen
+// product is a sum of four signed terms, exact products and exact sums
+// (TwoSum) in pairs, two eigenvectors to a packed float2 instruction.  S is
+// the float that FP64 gives: where the pairs' error leaves two candidates
+// (Ziv's rounding test, error at most 2^-45 of the terms' sizes) the value is
+// formed again in FP64.  A value below 2^-28 of the terms it came from is
+// left as it is: the other eigenvectors' float roundings are larger.
+// 509 edges x 45,675 patterns x 4 classes, pair form: 1.66 ms against 11.4
+// in FP64, which this GPU runs at 1/64 of the FP32 rate.
+__device__ __forceinline__ float2 neg2(float2 v) { return __fmul2_rn(v, make_float2(-1.0f, -1.0f)); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &e) {
+  s = __fadd2_rn(a, b);
+  const float2 bb = sub2(s, a);
+  e = __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
+// sum_j c_j x_j for two eigenvectors, normalised, and the sum of the terms'
+// sizes; c as {hi, hi', lo, lo'}
+__device__ __forceinline__ void eigen_pair(const float4 (*c)[2], int kp, const ff *x, float2 &sum, float2 &err,
+                                           float2 &mag) {
+  float2 s = make_float2(0.0f, 0.0f), lo = s;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      A += a.pi[j] * Pol::to_d(x[j]) * a.U[j * 4 + k];
-      B += a.Ui[k * 4 + j] * Pol::to_d(y[j]);
+  for (int j = 0; j < 4; ++j) {
+    const float4 q = c[j][kp];
+    const float2 ch = make_float2(q.x, q.y), cl = make_float2(q.z, q.w);
+    const float2 xh = make_float2(x[j].h, x[j].h), xl = make_float2(x[j].l, x[j].l);
+    const float2 p = __fmul2_rn(ch, xh);
+    float2 e = __ffma2_rn(ch, xh, neg2(p));
+    e = __ffma2_rn(ch, xl, e);
+    e = __ffma2_rn(cl, xh, e);
+    mag = j == 0 ? make_float2(fabsf(p.x), fabsf(p.y)) : make_float2(mag.x + fabsf(p.x), mag.y + fabsf(p.y));
+    if (j == 0) {
+      s = p;
+      lo = e;
+    } else {
+      float2 t, te;
+      two_sum2(s, p, t, te);
+      s = t;
+      lo = __fadd2_rn(lo, __fadd2_rn(te, e));
     }
-    s[k] = (float)(A * B);
+  }
+  two_sum2(s, lo, sum, err);
+}
+
+template <typename Pol>
+__global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
+  using V = typename Pol::V;
+  __shared__ float4 cA[4][2], cB[4][2];   // [j][eigenvector pair]
+  if (threadIdx.x < 32) {
+    const int side = threadIdx.x >> 4, j = (threadIdx.x >> 2) & 3, k = threadIdx.x & 3;
+    const double v = side == 0 ? a.pi[j] * a.U[j * 4 + k] : a.Ui[k * 4 + j];
+    float *dst = reinterpret_cast<float *>(side == 0 ? &cA[j][k >> 1] : &cB[j][k >> 1]) + (k & 1);
+    const float h = (float)v;
+    dst[0] = h;
+    dst[2] = (float)(v - (double)h);
+  }
+  __syncthreads();
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= a.np * a.R) return;
+  const int e = blockIdx.y;
+  V xv[4], yv[4];
+  Pol::load_g(a.L, (size_t)(2 * e) * a.np * a.R + i, xv);
+  Pol::load_g(a.L, (size_t)(2 * e + 1) * a.np * a.R + i, yv);
+  ff x[4], y[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {   // normalised: the stored low words may be a few ulps
+    x[j] = Pol::to_ff(xv[j]);
+    y[j] = Pol::to_ff(yv[j]);
+    x[j] = fast_two_sum(x[j].h, x[j].l);
+    y[j] = fast_two_sum(y[j].h, y[j].l);
+  }
+  float s[4];
+  int unsure = 0;
+#pragma unroll
+  for (int kp = 0; kp < 2; ++kp) {
+    float2 ah, al, am, bh, bl, bm;
+    eigen_pair(cA, kp, x, ah, al, am);
+    eigen_pair(cB, kp, y, bh, bl, bm);
+    const float2 p = __fmul2_rn(ah, bh);
+    float2 er = __ffma2_rn(ah, bh, neg2(p));
+    er = __ffma2_rn(ah, bl, er);
+    er = __ffma2_rn(al, bh, er);
+    const float2 v = __fadd2_rn(p, er), rest = sub2(er, sub2(v, p));
+    const float2 all = __fmul2_rn(am, bm);
+    const float2 d = __fmul2_rn(make_float2(0x1p-45f, 0x1p-45f),
+                                make_float2(fmaf(fabsf(ah.x), bm.x, fabsf(bh.x) * am.x),
+                                            fmaf(fabsf(ah.y), bm.y, fabsf(bh.y) * am.y)));
+    const float2 up = __fadd2_rn(v, __fadd2_rn(rest, d)), down = __fadd2_rn(v, sub2(rest, d));
+    s[2 * kp] = v.x;
+    s[2 * kp + 1] = v.y;
+    if (!(up.x == down.x) && !(fabsf(v.x) < 0x1p-28f * all.x)) unsure |= 1 << (2 * kp);
+    if (!(up.y == down.y) && !(fabsf(v.y) < 0x1p-28f * all.y)) unsure |= 2 << (2 * kp);
+  }
+  if (unsure) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (unsure >> k & 1) s[k] = eigen_product<Pol>(a, xv, yv, k);
   }
   reinterpret_cast<float4 *>(a.S)[(size_t)e * a.np * a.R + i] = make_float4(s[0], s[1], s[2], s[3]);
 }
@@ -1088,21 +1333,23 @@ struct pgpu_spr {
   // model
   double *Q = nullptr, *pi = nullptr, *rates = nullptr, *probs = nullptr, *ctab = nullptr,
          *U = nullptr, *Ui = nullptr, *lam = nullptr;
+  void *crows = nullptr;   // the code table as vectors of the form
   int *status = nullptr;
   uint8_t *cmask = nullptr;
   double *w = nullptr;
-  float *wf = nullptr;
+  float2 *w2 = nullptr;   // weights as float pairs
   float4 *logtab = nullptr;
   // pool
   void *L = nullptr, *M = nullptr, *H = nullptr;
   int32_t *sc = nullptr;
   void *Dfull = nullptr, *tipfull = nullptr, *tiphalf = nullptr;
   double *elen = nullptr, *tiplen = nullptr, *newlen = nullptr;
-  int4 *ops = nullptr, *tips = nullptr;
+  int4 *ops = nullptr, *tips = nullptr, *half_list = nullptr;
   double2 *pool_part = nullptr;
   double *tree_lnl = nullptr, *site_lnl = nullptr;
   // fitch
-  uint4 *F = nullptr, *planes = nullptr;
+  uint4 *F = nullptr;
+  uint32_t *planes = nullptr;
   unsigned long long *cntF = nullptr, *lenF = nullptr, *ins = nullptr, *join = nullptr;
   float *summ = nullptr;
   // scratch
@@ -1114,7 +1361,7 @@ struct pgpu_spr {
   PoolPlan pp;
   SprPlan all, sel;
   SprPlanDev all_d, sel_d;
-  bool pool_valid = false, plan_valid = false, fitch_valid = false, summ_valid = false;
+  bool pp_valid = false, pool_valid = false, half_valid = false, plan_valid = false, fitch_valid = false, summ_valid = false;
   int join_distance = 0;   // 0: every SPR move; d: regraft edges at most d nodes from the break
   // TBR: plan, emit walks on the device, attach vectors of a batch of cuts
   TbrPlan tbr;
@@ -1182,7 +1429,7 @@ pgpu_status compose(pgpu_spr *s, const double *t_dev, int n_br, void *out) {
 }
 
 template <typename Pol, int RT>
-pgpu_status launch_pool_rt(pgpu_spr *s) {
+pgpu_status launch_pool_rt(pgpu_spr *s, bool half) {
   PoolArgs a;
   a.L = s->L;
   a.M = s->M;
@@ -1201,12 +1448,12 @@ pgpu_status launch_pool_rt(pgpu_spr *s) {
   a.n_ops = (int)s->pp.ops.size();
   a.R = s->R;
   a.NP = s->NP;
-  spr_pool_kernel<Pol, RT><<<(unsigned)(s->np / s->NP), SPR_NT, 0, s->ctx->stream>>>(a);
+  if (half) spr_pool_kernel<Pol, RT, true><<<(unsigned)(s->np / s->NP), SPR_NT, 0, s->ctx->stream>>>(a);
+  else spr_pool_kernel<Pol, RT, false><<<(unsigned)(s->np / s->NP), SPR_NT, 0, s->ctx->stream>>>(a);
   return pgpu_after_launch(s->ctx, "spr_pool_kernel");
 }
 
-template <typename Pol>
-pgpu_status launch_pool(pgpu_spr *s) {
+TipArgs tip_args(pgpu_spr *s) {
   TipArgs t;
   t.L = s->L;
   t.M = s->M;
@@ -1214,7 +1461,7 @@ pgpu_status launch_pool(pgpu_spr *s) {
   t.sc = s->sc;
   t.tipfull = s->tipfull;
   t.tiphalf = s->tiphalf;
-  t.code_tab = s->ctab;
+  t.code_rows = s->crows;
   t.codes = s->codes;
   t.tips = s->tips;
   t.flag = s->ctx->d_flag;
@@ -1223,21 +1470,76 @@ pgpu_status launch_pool(pgpu_spr *s) {
   t.ld = s->ld;
   t.R = s->R;
   t.n_codes = s->n_codes;
-  spr_tip_kernel<Pol><<<dim3((unsigned)((s->np + 255) / 256), (unsigned)s->n), 256, 0, s->ctx->stream>>>(t);
+  return t;
+}
+
+unsigned item_ctas(const pgpu_spr *s) { return (unsigned)((s->np * s->R + 255) / 256); }
+
+template <typename Pol>
+pgpu_status launch_pool(pgpu_spr *s, bool half) {
+  const TipArgs t = tip_args(s);
+  const dim3 g(item_ctas(s), (unsigned)s->n);
+  if (half) spr_tip_kernel<Pol, true, true><<<g, 256, 0, s->ctx->stream>>>(t);
+  else spr_tip_kernel<Pol, true, false><<<g, 256, 0, s->ctx->stream>>>(t);
   PGPU_TRY(pgpu_after_launch(s->ctx, "spr_tip_kernel"));
   switch (s->RT) {
-    case 1: return launch_pool_rt<Pol, 1>(s);
-    case 2: return launch_pool_rt<Pol, 2>(s);
-    case 4: return launch_pool_rt<Pol, 4>(s);
-    default: return launch_pool_rt<Pol, 8>(s);
+    case 1: return launch_pool_rt<Pol, 1>(s, half);
+    case 2: return launch_pool_rt<Pol, 2>(s, half);
+    case 4: return launch_pool_rt<Pol, 4>(s, half);
+    default: return launch_pool_rt<Pol, 8>(s, half);
   }
 }
 
-// Rebuilds everything that depends on the topology and branch lengths.
-pgpu_status ensure_pool(pgpu_spr *s) {
-  if (s->pool_valid) return PGPU_OK;
+// H of the listed directed edges of a pool made without it: tips {dedge, tip,
+// edge, 0} and internal ones {dedge, ...}
+template <typename Pol>
+pgpu_status launch_half(pgpu_spr *s, const int4 *tips, size_t n_tips, const int4 *ops, size_t n_ops) {
+  if (n_tips) {
+    TipArgs t = tip_args(s);
+    t.tips = tips;
+    spr_tip_kernel<Pol, false, true><<<dim3(item_ctas(s), (unsigned)n_tips), 256, 0, s->ctx->stream>>>(t);
+    PGPU_TRY(pgpu_after_launch(s->ctx, "spr_tip_kernel"));
+  }
+  const void *Dhalf = static_cast<char *>(s->Dfull) + (size_t)s->T.n_edges() * s->cbytes;
+  for (size_t i = 0; i < n_ops; i += 65535) {
+    const unsigned k = (unsigned)std::min<size_t>(n_ops - i, 65535);
+    spr_half_kernel<Pol><<<dim3(item_ctas(s), k), 256, 0, s->ctx->stream>>>(s->L, s->H, Dhalf, ops + i, s->np,
+                                                                           (unsigned)s->R);
+    PGPU_TRY(pgpu_after_launch(s->ctx, "spr_half_kernel"));
+  }
+  return PGPU_OK;
+}
+
+pgpu_status tip_rows(pgpu_spr *s, bool half) {
+  return pgpu_launch_tip_table(s->ctx, s->U, s->lam, s->Ui, 4, s->elen + 2 * s->T.n_edges() + (half ? s->n : 0),
+                               s->n, s->rates, s->R, s->ctab, s->n_codes, half ? s->tiphalf : s->tipfull,
+                               tip_form(s->precision), s->status);
+}
+
+pgpu_status add_half(pgpu_spr *s, const int4 *tips, size_t n_tips, const int4 *ops, size_t n_ops) {
+  if (n_tips) PGPU_TRY(tip_rows(s, true));
+  if (s->precision == 32) return launch_half<Fp32>(s, tips, n_tips, ops, n_ops);
+  if (s->precision == 48) return launch_half<Ff32>(s, tips, n_tips, ops, n_ops);
+  return launch_half<Fp64>(s, tips, n_tips, ops, n_ops);
+}
+
+void ensure_pool_plan(pgpu_spr *s) {
+  if (s->pp_valid) return;
+  spr_pool_plan(s->T, &s->pp);
+  s->pp_valid = true;
+}
+
+// Rebuilds everything that depends on the topology and branch lengths; half:
+// with the vectors at the edges' middles, which scoring moves reads.
+pgpu_status ensure_pool(pgpu_spr *s, bool half = false) {
+  if (s->pool_valid) {
+    if (!half || s->half_valid) return PGPU_OK;
+    PGPU_TRY(add_half(s, s->tips, (size_t)s->n, s->ops, s->pp.ops.size()));
+    s->half_valid = true;
+    return PGPU_OK;
+  }
   SprTopo &T = s->T;
-  spr_pool_plan(T, &s->pp);
+  ensure_pool_plan(s);
   const int ne = T.n_edges();
   std::vector<double> h(2 * ne + 2 * s->n);
   for (int e = 0; e < ne; ++e) {
@@ -1252,16 +1554,15 @@ pgpu_status ensure_pool(pgpu_spr *s) {
   PGPU_TRY(upload(s, s->ops, s->pp.ops.data(), s->pp.ops.size()));
   PGPU_TRY(upload(s, s->tips, s->pp.tips.data(), s->pp.tips.size()));
   PGPU_TRY(compose(s, s->elen, 2 * ne, s->Dfull));
-  for (int half = 0; half < 2; ++half)
-    PGPU_TRY(pgpu_launch_tip_table(s->ctx, s->U, s->lam, s->Ui, 4, s->elen + 2 * ne + half * s->n, s->n,
-                                   s->rates, s->R, s->ctab, s->n_codes,
-                                   half ? s->tiphalf : s->tipfull, tip_form(s->precision), s->status));
-  if (s->precision == 32) PGPU_TRY(launch_pool<Fp32>(s));
-  else if (s->precision == 48) PGPU_TRY(launch_pool<Ff32>(s));
-  else PGPU_TRY(launch_pool<Fp64>(s));
+  PGPU_TRY(tip_rows(s, false));
+  if (half) PGPU_TRY(tip_rows(s, true));
+  if (s->precision == 32) PGPU_TRY(launch_pool<Fp32>(s, half));
+  else if (s->precision == 48) PGPU_TRY(launch_pool<Ff32>(s, half));
+  else PGPU_TRY(launch_pool<Fp64>(s, half));
   spr_pool_finalize_kernel<<<1, 1024, 0, s->ctx->stream>>>(s->pool_part, (int)(s->np / s->NP), s->tree_lnl);
   PGPU_TRY(pgpu_after_launch(s->ctx, "spr_pool_finalize_kernel"));
   s->pool_valid = true;
+  s->half_valid = half;
   return PGPU_OK;
 }
 
@@ -1288,7 +1589,7 @@ pgpu_status upload_plan(pgpu_spr *s, const SprPlan &p, SprPlanDev *d) {
 
 pgpu_status ensure_plan(pgpu_spr *s) {
   if (s->plan_valid) return PGPU_OK;
-  PGPU_TRY(ensure_pool(s));
+  ensure_pool_plan(s);
   spr_plan_all(s->T, s->pp, &s->all, s->join_distance);
   PGPU_TRY(upload_plan(s, s->all, &s->all_d));
   s->plan_valid = true;
@@ -1309,7 +1610,7 @@ pgpu_status launch_scan_rt(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, i
   a.prunes = d.prunes;
   a.pi = s->pi;
   a.probs = s->probs;
-  a.wts = s->wf;
+  a.wts = s->w2;
   a.logtab = s->logtab;
   a.partials = s->partials;
   a.flag = s->ctx->d_flag;
@@ -1347,10 +1648,34 @@ pgpu_status launch_scan(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, int 
   }
 }
 
+// H of the edges that the moves of plan p regraft onto.  Fewer moves than the
+// tree has directed edges read the H of a few of them only, and a pool made
+// without H gets just those: 32 moves on 256 taxa x 45,675 patterns took
+// 2.52 ms for all 1,018 and 0.06 ms for their own.
+pgpu_status ensure_half(pgpu_spr *s, const SprPlan &p) {
+  const size_t nd = (size_t)s->T.n_dedges();
+  if (p.moves.size() >= nd) return ensure_pool(s, true);
+  PGPU_TRY(ensure_pool(s));
+  if (s->half_valid) return PGPU_OK;
+  std::vector<int4> list[2];   // tips, internal
+  std::vector<uint8_t> seen(nd, 0);
+  for (const SprMove &m : p.moves) {
+    if (seen[m.dc]) continue;
+    seen[m.dc] = 1;
+    const int src = s->T.dsrc(m.dc);
+    list[src < s->n ? 0 : 1].push_back(make_int4(m.dc, src, m.dc >> 1, 0));
+  }
+  int4 *at = s->half_list;
+  PGPU_TRY(upload(s, at, list[0].data(), list[0].size()));
+  PGPU_TRY(upload(s, at + list[0].size(), list[1].data(), list[1].size()));
+  return add_half(s, at, list[0].size(), at + list[0].size(), list[1].size());
+}
+
 // lazy log-likelihood of every move of plan p into lnl_dev
 pgpu_status run_scan(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, double *lnl_dev) {
   const size_t nm = p.moves.size();
   if (nm == 0) return PGPU_OK;
+  PGPU_TRY(ensure_half(s, p));
   const int n_blocks = (int)(s->np / s->NP);
   // CTA groups of G pattern blocks; partial sums at most 256 MB
   const size_t budget = size_t(256) << 20;
@@ -1362,8 +1687,8 @@ pgpu_status run_scan(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, double 
   if (s->precision == 32) PGPU_TRY(launch_scan<Fp32>(s, p, d, G, n_groups, n_blocks));
   else if (s->precision == 48) PGPU_TRY(launch_scan<Ff32>(s, p, d, G, n_groups, n_blocks));
   else PGPU_TRY(launch_scan<Fp64>(s, p, d, G, n_groups, n_blocks));
-  spr_reduce_kernel<<<(unsigned)((nm + 255) / 256), 256, 0, s->ctx->stream>>>(s->partials, n_groups, nm,
-                                                                              lnl_dev);
+  spr_reduce_kernel<<<(unsigned)((nm + 31) / 32), dim3(32, RED_Y), 0, s->ctx->stream>>>(s->partials, n_groups, nm,
+                                                                                       lnl_dev);
   return pgpu_after_launch(s->ctx, "spr_reduce_kernel");
 }
 
@@ -1373,7 +1698,7 @@ pgpu_status run_scan(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, double 
 // ---------------------------------------------------------------------------
 pgpu_status ensure_tbr(pgpu_spr *s) {
   if (s->tbr_valid) return PGPU_OK;
-  PGPU_TRY(ensure_pool(s));
+  ensure_pool_plan(s);
   tbr_plan(s->T, s->pp, s->tbr_join, s->tbr_reroot, &s->tbr);
   PGPU_TRY(upload_plan(s, s->tbr.emit, &s->tbr_d));
   if (!s->tbr.keep.empty()) {
@@ -1398,7 +1723,7 @@ pgpu_status launch_emit_rt(pgpu_spr *s, int prune_base, int n_prunes, long long 
   a.prunes = s->tbr_d.prunes;
   a.pi = s->pi;
   a.probs = s->probs;
-  a.wts = s->wf;
+  a.wts = s->w2;
   a.logtab = s->logtab;
   a.partials = nullptr;
   a.flag = s->ctx->d_flag;
@@ -1480,7 +1805,7 @@ pgpu_status launch_tbr_batch(pgpu_spr *s, size_t c0, size_t c1, double *lnl_dev)
   a.xsc = s->tbr_xsc;
   a.tiles = s->tbr_tiles;
   a.cuts = s->tbr_cuts;
-  a.wts = s->wf;
+  a.wts = s->w2;
   a.logtab = s->logtab;
   a.partials = s->partials;
   a.flag = s->ctx->d_flag;
@@ -1496,8 +1821,8 @@ pgpu_status launch_tbr_batch(pgpu_spr *s, size_t c0, size_t c1, double *lnl_dev)
                                          (int)std::max<size_t>(smem, 48 * 1024)));
   tbr_pair_kernel<Pol><<<dim3((unsigned)tiles.size(), (unsigned)n_groups), 256, smem, s->ctx->stream>>>(a);
   PGPU_TRY(pgpu_after_launch(s->ctx, "tbr_pair_kernel"));
-  spr_reduce_kernel<<<(unsigned)((nm + 255) / 256), 256, 0, s->ctx->stream>>>(s->partials, n_groups,
-                                                                              (size_t)nm, lnl_dev + move0);
+  spr_reduce_kernel<<<(unsigned)((nm + 31) / 32), dim3(32, RED_Y), 0, s->ctx->stream>>>(
+      s->partials, n_groups, (size_t)nm, lnl_dev + move0);
   return pgpu_after_launch(s->ctx, "spr_reduce_kernel");
 }
 
@@ -1514,6 +1839,7 @@ __global__ void __launch_bounds__(256) tbr_gather_kernel(const double *grid, con
 // different limits every pair goes into the grid buffer first and the
 // listed moves are gathered from it
 pgpu_status run_tbr_scan(pgpu_spr *s, double *lnl_dev) {
+  PGPU_TRY(ensure_pool(s, true));
   PGPU_TRY(ensure_tbr(s));
   const TbrPlan &tp = s->tbr;
   if (tp.n_moves == 0) return PGPU_OK;
@@ -1558,8 +1884,7 @@ pgpu_status ensure_fitch(pgpu_spr *s) {
   t.n_pat = s->n_pat;
   t.ld = s->ld;
   t.n_codes = s->n_codes;
-  const unsigned gx = (unsigned)((s->W4 + 255) / 256);
-  spr_fitch_tip_kernel<<<dim3(gx, (unsigned)s->n), 256, 0, s->ctx->stream>>>(t);
+  spr_fitch_tip_kernel<<<dim3((unsigned)((s->W4 + 7) / 8), (unsigned)s->n), 256, 0, s->ctx->stream>>>(t);
   PGPU_TRY(pgpu_after_launch(s->ctx, "spr_fitch_tip_kernel"));
   const int n_ops = (int)s->pp.ops.size();
   PGPU_CUDA(s->ctx, cudaMemsetAsync(s->cntF, 0, sizeof(unsigned long long) * (n_ops + 1), s->ctx->stream));
@@ -1571,9 +1896,13 @@ pgpu_status ensure_fitch(pgpu_spr *s) {
   a.W4 = s->W4;
   a.n_ops = n_ops;
   a.n_planes = s->n_planes;
-  spr_fitch_pool_kernel<<<gx, 256, 0, s->ctx->stream>>>(a);
+  spr_fitch_pool_kernel<<<(unsigned)((s->W4 + FPOOL_NT - 1) / FPOOL_NT), FPOOL_NT, 0, s->ctx->stream>>>(a);
   PGPU_TRY(pgpu_after_launch(s->ctx, "spr_fitch_pool_kernel"));
-  spr_fitch_len_kernel<<<1, 32, 0, s->ctx->stream>>>(s->ops, n_ops, s->cntF, s->lenF, s->T.n_dedges());
+  const int nd = s->T.n_dedges();
+  const size_t len_bytes = (size_t)nd * sizeof(unsigned long long);
+  const bool in_shared = len_bytes <= 40 * 1024;   // within 48 KB beside the staged steps
+  spr_fitch_len_kernel<<<1, FLEN_NT, in_shared ? len_bytes : 0, s->ctx->stream>>>(s->ops, n_ops, s->cntF, s->lenF, nd,
+                                                                                 in_shared);
   PGPU_TRY(pgpu_after_launch(s->ctx, "spr_fitch_len_kernel"));
   s->fitch_valid = true;
   return PGPU_OK;
@@ -1615,7 +1944,7 @@ pgpu_status sync_check(pgpu_spr *s, const char *what) {
 }
 
 void invalidate(pgpu_spr *s) {
-  s->pool_valid = s->plan_valid = s->fitch_valid = s->summ_valid = s->tbr_valid = false;
+  s->pp_valid = s->pool_valid = s->half_valid = s->plan_valid = s->fitch_valid = s->summ_valid = s->tbr_valid = false;
 }
 
 }  // namespace
@@ -1686,6 +2015,26 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
   std::copy(codes->table, codes->table + (size_t)nc * 4, hb.begin() + 36);
   SPR_TRY(upload(s, blk, hb.data(), hb.size()));
   SPR_TRY(pgpu_launch_eig(ctx, s->Q, s->pi, 4, 1, s->U, s->lam, s->Ui, s->status));
+  // the code table in the form's layout (store4)
+  std::vector<double> cr((size_t)nc * 4);   // room for the widest form
+  for (int c = 0; c < nc; ++c)
+    for (int i = 0; i < 4; ++i) {
+      const double v = codes->table[(size_t)c * 4 + i];
+      float *f = reinterpret_cast<float *>(cr.data());
+      if (s->precision == 64) {
+        cr[(size_t)c * 4 + i] = v;
+      } else if (s->precision == 32) {
+        f[(size_t)c * 4 + i] = (float)v;
+      } else {
+        float *q = f + (size_t)c * 8 + (i >> 1) * 4 + (i & 1);
+        q[0] = (float)v;
+        q[2] = (float)(v - (double)q[0]);
+      }
+    }
+  double *crd;
+  SPR_TRY(dalloc_t(s, cr.size(), &crd));
+  SPR_TRY(upload(s, crd, cr.data(), cr.size()));
+  s->crows = crd;
   // state-set masks of the codes
   std::vector<uint8_t> cm(nc);
   for (int c = 0; c < nc; ++c) {
@@ -1696,7 +2045,7 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
   }
   SPR_TRY(dalloc_t(s, (size_t)nc, &s->cmask));
   SPR_TRY(upload(s, s->cmask, cm.data(), cm.size()));
-  // weights: FP64 and FP32 copies padded with zeros; integer bit planes for Fitch
+  // weights: FP64 and float-pair copies padded with zeros; integer bit planes for Fitch
   std::vector<double> wh(s->np, 0.0);
   if (weights_dev) {
     if (cudaMemcpy(wh.data(), weights_dev, n_pat * 8, cudaMemcpyDeviceToHost) != cudaSuccess) {
@@ -1712,21 +2061,22 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
     s->wtot += wh[i];
     wmax = std::max<uint64_t>(wmax, (uint64_t)llround(wh[i]));
   }
-  std::vector<float> wfh(wh.begin(), wh.end());
+  std::vector<float2> w2h(s->np);
+  for (size_t i = 0; i < s->np; ++i) w2h[i] = make_float2((float)wh[i], (float)(wh[i] - (double)(float)wh[i]));
   SPR_TRY(dalloc_t(s, s->np, &s->w));
-  SPR_TRY(dalloc_t(s, s->np, &s->wf));
   SPR_TRY(upload(s, s->w, wh.data(), wh.size()));
-  SPR_TRY(upload(s, s->wf, wfh.data(), wfh.size()));
+  SPR_TRY(dalloc_t(s, s->np, &s->w2));
+  SPR_TRY(upload(s, s->w2, w2h.data(), w2h.size()));
   s->n_planes = 1;
   while ((wmax >> s->n_planes) != 0) ++s->n_planes;
-  std::vector<uint32_t> planes((size_t)s->n_planes * s->W4 * 4, 0u);
+  std::vector<uint32_t> planes((size_t)s->n_planes * s->W4, 0u);
   for (size_t i = 0; i < n_pat; ++i) {
     const uint64_t wi = (uint64_t)llround(wh[i]);
     for (int b = 0; b < s->n_planes; ++b)
-      if ((wi >> b) & 1u) planes[(size_t)b * s->W4 * 4 + i / 8] |= 0x8u << (4 * (i % 8));
+      if ((wi >> b) & 1u) planes[(size_t)b * s->W4 + i / 32] |= 1u << (i % 32);
   }
   SPR_TRY(dalloc_t(s, (size_t)s->n_planes * s->W4, &s->planes));
-  SPR_TRY(upload(s, reinterpret_cast<uint32_t *>(s->planes), planes.data(), planes.size()));
+  SPR_TRY(upload(s, s->planes, planes.data(), planes.size()));
   // logarithm table of the pair form
   std::vector<float4> lt(64);
   ff_log_table(lt.data(), [](double c) { return std::log(c); });
@@ -1745,6 +2095,7 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
   SPR_TRY(dalloc_t(s, 2 * (size_t)ne + 2 * (size_t)n_tips, &s->elen));
   SPR_TRY(dalloc_t(s, (size_t)ne, &s->newlen));
   SPR_TRY(dalloc_t(s, (size_t)nd, &s->ops));
+  SPR_TRY(dalloc_t(s, (size_t)nd, &s->half_list));
   SPR_TRY(dalloc_t(s, (size_t)n_tips, &s->tips));
   SPR_TRY(dalloc_t(s, s->np / s->NP, &s->pool_part));
   SPR_TRY(dalloc_t(s, 1, &s->tree_lnl));
@@ -1841,6 +2192,7 @@ pgpu_status pgpu_spr_scan(pgpu_spr *s, double *lnl_dev) {
   if (!s || !lnl_dev) return PGPU_ERR_ARG;
   if (s->T.n == 0) return pgpu_set_err(s->ctx, PGPU_ERR_ARG, "spr: no tree set");
   PGPU_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
+  PGPU_TRY(ensure_pool(s, true));
   PGPU_TRY(ensure_plan(s));
   PGPU_TRY(run_scan(s, s->all, s->all_d, lnl_dev));
   return sync_check(s, "spr_scan");
@@ -1850,6 +2202,7 @@ pgpu_status pgpu_spr_score(pgpu_spr *s, const int64_t *move_idx, size_t k, doubl
   if (!s || (k && (!move_idx || !lnl))) return PGPU_ERR_ARG;
   if (s->T.n == 0) return pgpu_set_err(s->ctx, PGPU_ERR_ARG, "spr: no tree set");
   PGPU_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
+  if (k) PGPU_TRY(ensure_pool(s, k >= (size_t)s->T.n_dedges()));
   PGPU_TRY(ensure_plan(s));
   if (k == 0) return PGPU_OK;
   const size_t nm = s->all.moves.size();
@@ -1909,11 +2262,13 @@ pgpu_status pgpu_spr_features(pgpu_spr *s, float *X_dev) {
     SummaryArgs a;
     a.L = s->L;
     a.probs = s->probs;
-    a.weights = s->w;
+    a.weights = s->w2;
     a.out = s->summ;
     a.np = s->np;
     a.n_pat = s->n_pat;
     a.R = s->R;
+    a.RT = s->RT;
+    a.rt_shift = s->RT == 1 ? 0 : s->RT == 2 ? 1 : s->RT == 4 ? 2 : 3;
     a.inv_w = s->wtot > 0 ? 1.0 / s->wtot : 0.0;
     const unsigned nd = (unsigned)s->T.n_dedges();
     if (s->precision == 32) spr_summary_kernel<Fp32><<<nd, 256, 0, s->ctx->stream>>>(a);
@@ -2098,9 +2453,9 @@ pgpu_status pgpu_spr_optimize(pgpu_spr *s, int passes, double tol, double *lnl_o
     a.tmin = 1e-8;
     a.tmax = 10.0;
     const dim3 g((unsigned)((s->np * s->R + 255) / 256), (unsigned)ne);
-    if (s->precision == 32) bl_sumtab_kernel<Fp32><<<g, 256, 0, s->ctx->stream>>>(a);
-    else if (s->precision == 48) bl_sumtab_kernel<Ff32><<<g, 256, 0, s->ctx->stream>>>(a);
-    else bl_sumtab_kernel<Fp64><<<g, 256, 0, s->ctx->stream>>>(a);
+    if (s->precision == 32) bl_sumtab_pair_kernel<Fp32><<<g, 256, 0, s->ctx->stream>>>(a);
+    else if (s->precision == 48) bl_sumtab_pair_kernel<Ff32><<<g, 256, 0, s->ctx->stream>>>(a);
+    else bl_sumtab_kernel<<<g, 256, 0, s->ctx->stream>>>(a);
     PGPU_TRY(pgpu_after_launch(s->ctx, "bl_sumtab_kernel"));
     bl_newton_kernel<<<(unsigned)ne, 256, 0, s->ctx->stream>>>(a);
     PGPU_TRY(pgpu_after_launch(s->ctx, "bl_newton_kernel"));

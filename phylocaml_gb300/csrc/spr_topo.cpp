@@ -107,15 +107,18 @@ void spr_pool_plan(const SprTopo &T, PoolPlan *out) {
   const int root = T.other(T.inc[0][0], 0);
   std::vector<int32_t> order, pe(2 * n - 2, -1);
   order.reserve(2 * n - 2);
-  order.push_back(root);
-  for (size_t i = 0; i < order.size(); ++i) {
-    const int v = order[i];
+  // depth first: what a step reads was mostly made a few steps before
+  std::vector<int32_t> todo(1, root);
+  while (!todo.empty()) {
+    const int v = todo.back();
+    todo.pop_back();
+    order.push_back(v);
     for (int j = 0; j < T.deg(v); ++j) {
       const int e = T.inc[v][j];
       if (e == pe[v]) continue;
       const int c = T.other(e, v);
       pe[c] = e;
-      order.push_back(c);
+      todo.push_back(c);
     }
   }
   out->ops.clear();

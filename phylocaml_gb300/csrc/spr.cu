@@ -51,7 +51,13 @@ using namespace pgpu_forms;
 
 namespace {
 
-constexpr int SPR_NT = 256;
+// Threads of a pool or scan CTA: the kernels hold 64 to 128 registers a thread,
+// so that small CTAs fill an SM better and wait less for one another (256
+// taxa x 45,675 patterns: pool 2.61 ms against 2.91 with 256 threads; the scan
+// of 128 taxa x 16,852: 72.2 against 74.2).
+constexpr int SPR_NT = 128;
+// What an engine accepts is reckoned in blocks of this many threads.
+constexpr int SPR_LIMIT_NT = 256;
 constexpr int SPR_NW = SPR_NT / 32;
 constexpr int SPR_FEATURES = 64;
 
@@ -61,23 +67,38 @@ __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15);
 // rescaling shared by the pool and scan kernels: exact power of two, agreed
 // by the RT lanes (rate classes) of one pattern; all lanes of the warp call
 // ---------------------------------------------------------------------------
+template <typename Pol>
+__device__ __forceinline__ auto largest(const typename Pol::V *x) {
+  return fmax(fmax(Pol::mag(x[0]), Pol::mag(x[1])), fmax(Pol::mag(x[2]), Pol::mag(x[3])));
+}
+template <typename Pol, int RT, typename T>
+__device__ __forceinline__ void scale_up(typename Pol::V *acc, int &sc, T mx) {
+#pragma unroll
+  for (int o = 1; o < RT; o <<= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (mx < Pol::thresh && mx > 0) {
+    const int ex = frexp_exp(mx);
+    sc += ex;
+    const int k1 = min(-ex, 120), k2 = -ex - k1;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k1);
+    if (k2 > 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k2);
+    }
+  }
+}
 template <typename Pol, int RT>
 __device__ __forceinline__ void rescale(typename Pol::V *acc, int &sc) {
-  auto mx = fmax(fmax(Pol::mag(acc[0]), Pol::mag(acc[1])), fmax(Pol::mag(acc[2]), Pol::mag(acc[3])));
-  if (__any_sync(0xffffffffu, mx < Pol::thresh && mx > 0)) {
-#pragma unroll
-    for (int o = 1; o < RT; o <<= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (mx < Pol::thresh && mx > 0) {
-      const int ex = frexp_exp(mx);
-      sc += ex;
-      const int k1 = min(-ex, 120), k2 = -ex - k1;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k1);
-      if (k2 > 0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] = Pol::scale(acc[e], k2);
-      }
-    }
+  const auto mx = largest<Pol>(acc);
+  if (__any_sync(0xffffffffu, mx < Pol::thresh && mx > 0)) scale_up<Pol, RT>(acc, sc, mx);
+}
+// two vectors, one vote
+template <typename Pol, int RT>
+__device__ __forceinline__ void rescale2(typename Pol::V *x, int &sx, typename Pol::V *y, int &sy) {
+  const auto mx = largest<Pol>(x), my = largest<Pol>(y);
+  if (__any_sync(0xffffffffu, (mx < Pol::thresh && mx > 0) || (my < Pol::thresh && my > 0))) {
+    scale_up<Pol, RT>(x, sx, mx);
+    scale_up<Pol, RT>(y, sy, my);
   }
 }
 
@@ -102,7 +123,7 @@ struct PoolArgs {
 // HBM-bound: two or three vectors written and up to two read per step.  The
 // next step's vectors are read while this step is computed, unless this step
 // makes them (then they pass in registers); depth-first order keeps what a
-// step reads recent.  256 taxa x 45,675 patterns, pair form: 2.88 ms without
+// step reads recent.  256 taxa x 45,675 patterns, pair form: 2.61 ms without
 // H; level by level and with nothing read ahead it was 7.2 ms with H.
 template <typename Pol, int RT, bool HALF>
 __global__ void __launch_bounds__(SPR_NT) spr_pool_kernel(const PoolArgs a) {
@@ -297,7 +318,7 @@ struct ScanArgs {
   double *partials;           // [n_groups][n_moves]
   int *flag;
   size_t np, n_moves;
-  int R, NP, G, n_blocks, depth, max_moves;
+  int R, NP, G, n_blocks, depth;
   // emit mode (TBR): the attach vector of every wanted edge instead of a score
   const void *Dfull;          // [n_edges][R][16]: P(t) of the cut edge (b's side)
   void *xout;                 // [slot][np][R] x 4
@@ -306,10 +327,53 @@ struct ScanArgs {
   int prune_base;             // first prune of the launch
 };
 
+// Shared memory of a scan CTA: the logarithm table, a window of SCAN_WIN moves'
+// values per warp, the two steps' transition blocks per warp and the stack.
+constexpr int SCAN_WIN = 64;
 template <typename Pol>
-__host__ __device__ size_t scan_smem(int depth, int max_moves) {
-  return 1024 + a16((size_t)SPR_NW * max_moves * sizeof(ff)) +
+__host__ __device__ constexpr size_t scan_blocks(int RT) {   // of one step, bytes
+  return 2 * (size_t)RT * 16 * sizeof(typename Pol::Coef);
+}
+template <typename Pol>
+__host__ __device__ size_t scan_smem(int depth, int RT) {
+  return 1024 + (size_t)SPR_NW * SCAN_WIN * sizeof(ff) + 2 * SPR_NW * scan_blocks<Pol>(RT) +
          (size_t)depth * 4 * SPR_NT * sizeof(typename Pol::V) + (size_t)depth * SPR_NT * sizeof(int);
+}
+// What a scan may ask for: room for every move of a prune at once beside the
+// stack, and for the kernel's own memory.
+template <typename Pol>
+size_t scan_limit(int depth, int max_moves, int RT) {
+  const size_t moves = a16((size_t)(SPR_LIMIT_NT / 32) * max_moves * sizeof(ff));
+  return std::max(scan_smem<Pol>(depth, RT),
+                  1024 + moves + (size_t)depth * SPR_LIMIT_NT * (4 * sizeof(typename Pol::V) + sizeof(int)));
+}
+
+// One lane's part of a regraft's site likelihood: sum_e h_e hh_e v_e, v the
+// pruned side's vector with the frequencies and (pair form) the class's
+// probability in it.
+template <typename Pol>
+__device__ __forceinline__ typename Pol::V site_part(const typename Pol::V *h, const typename Pol::V *hh,
+                                                     const typename Pol::V *v, typename Pol::V prob) {
+  using V = typename Pol::V;
+  if constexpr (std::is_same<Pol, Ff32>::value) {
+    // exact products two to an instruction, then exact sums of the terms
+    // (none is negative), the low words left unnormalised until the end
+    ff t[4], u[4];
+    Pol::mul4(h, hh, t);
+    Pol::mul4(t, v, u);
+    const float2 a = make_float2(fmaxf(u[0].h, u[2].h), fmaxf(u[1].h, u[3].h));
+    const float2 b = make_float2(fminf(u[0].h, u[2].h), fminf(u[1].h, u[3].h));
+    const float2 s = __fadd2_rn(a, b);
+    const float2 e = __fadd2_rn(b, neg2(__fadd2_rn(s, neg2(a))));
+    const float2 lo = __fadd2_rn(__fadd2_rn(make_float2(u[0].l, u[1].l), make_float2(u[2].l, u[3].l)), e);
+    const ff w = fast_two_sum(fmaxf(s.x, s.y), fminf(s.x, s.y));
+    return fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(lo.x, lo.y)));
+  } else {
+    V p = Pol::zero();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p = Pol::add(p, Pol::mul(Pol::mul(h[e], hh[e]), v[e]));
+    return Pol::mul(p, prob);
+  }
 }
 
 // EMIT: instead of scoring a regraft, store the walked side's vector at the
@@ -318,50 +382,87 @@ __host__ __device__ size_t scan_smem(int depth, int max_moves) {
 // (a,b): the even one walks a's side and stores X weighted by probs_r pi_i,
 // the odd one walks b's side and stores P(t_ab) Y, carried across the cut,
 // so that a TBR site likelihood is the plain dot product of the two.
+//
+// Bound by issuing pair arithmetic; with 128 registers a thread 16 warps run
+// on an SM, too few to wait for memory, so a step's M vectors (to
+// registers) and transition blocks (to shared memory, classes interleaved) are
+// read one step ahead and its H vectors at its start.  The lanes of a pattern
+// split the two moves of a step: one exchange leaves the even lanes with the
+// first move's sum and the odd ones with the second's, and one logarithm and
+// one sum over the patterns serve both.  The warps' values meet every
+// SCAN_WIN moves.  128 taxa x 16,852 patterns, pair form, 63,000 moves:
+// 72.2 ms against 141.8 with none of this.
 template <typename Pol, int RT, bool EMIT = false>
-__global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
   using V = typename Pol::V;
   using Coef = typename Pol::Coef;
-  constexpr int NT = SPR_NT;
+  constexpr int NT = SPR_NT, U = sizeof(Coef), UNITS = U * RT;   // 16-byte units of a class's block, of an edge's
   extern __shared__ __align__(16) unsigned char smem[];
   const SprPrune pr = a.prunes[a.prune_base + blockIdx.x];
-  float4 *ltab = reinterpret_cast<float4 *>(smem);
-  ff *red = reinterpret_cast<ff *>(smem + 1024);
-  V *stk = reinterpret_cast<V *>(smem + 1024 + a16((size_t)SPR_NW * a.max_moves * sizeof(ff)));
-  int *stk_sc = reinterpret_cast<int *>(stk + (size_t)a.depth * 4 * NT);
   const int c = threadIdx.x, lane = c & 31, warp = c >> 5, pl = c / RT, r = c % RT;
+  float4 *ltab = reinterpret_cast<float4 *>(smem);
+  ff *red = reinterpret_cast<ff *>(smem + 1024);   // [warp][SCAN_WIN]
+  uint4 *dsh = reinterpret_cast<uint4 *>(red + SPR_NW * SCAN_WIN) + (size_t)warp * 4 * UNITS;   // [2][2 edges][UNITS]
+  V *stk = reinterpret_cast<V *>(smem + 1024 + SPR_NW * SCAN_WIN * sizeof(ff) + 2 * SPR_NW * scan_blocks<Pol>(RT));
+  int *stk_sc = reinterpret_cast<int *>(stk + (size_t)a.depth * 4 * NT);
   const bool on = r < a.R;
   const int R = a.R;
   for (int i = c; i < 64; i += NT) ltab[i] = a.logtab[i];
-  for (int i = c; i < SPR_NW * a.max_moves; i += NT) red[i] = ff{0.0f, 0.0f};
   __syncthreads();
-  V piv[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) piv[e] = Pol::from_d(a.pi[e]);
   const V prob = Pol::from_d(on ? a.probs[r] : 0.0);
-  const bool mine1 = r == 0, mine2 = RT == 1 ? true : r == 1;
-  const int lane2 = RT == 1 ? 0 : 1;
-  const Coef *Dh = static_cast<const Coef *>(a.Dhalf);
   const Coef *Dm = static_cast<const Coef *>(a.Dmer) + ((size_t)(a.prune_base + blockIdx.x) * R + (on ? r : 0)) * 16;
+  // blocks of a step's two edges into buffer buf
+  auto blocks = [&](int buf, const SprStep &st) {
+#pragma unroll
+    for (int k = 0; k < (UNITS + 31) / 32; ++k) {
+      const int q = k * 32 + lane, cls = q / U;
+      if (cls < R) {
+        const uint4 *D = static_cast<const uint4 *>(a.Dhalf) + q;
+        uint4 *dst = dsh + (size_t)buf * 2 * UNITS + (q % U) * RT + cls;
+        copy16(dst, D + (size_t)(st.d1 >> 1) * R * U);
+        copy16(dst + UNITS, D + (size_t)(st.d2 >> 1) * R * U);
+      }
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  int base = 0;   // first move of the window
+  auto flush = [&](int to, bool first) {
+    __syncthreads();
+    if (c < to - base) {
+      ff s = red[c];
+      for (int w = 1; w < SPR_NW; ++w) s = ff_add(s, red[w * SCAN_WIN + c]);
+      double *dst = a.partials + (size_t)blockIdx.y * a.n_moves + pr.move_off + base + c;
+      const double v = (double)s.h + (double)s.l;
+      *dst = first ? v : *dst + v;
+    }
+    __syncthreads();
+    base = to;
+  };
   bool ok = true;
 
   for (int g = 0; g < a.G && ok; ++g) {
     const int blk = blockIdx.y * a.G + g;
     if (blk >= a.n_blocks) break;
     const size_t pat = (size_t)blk * a.NP + pl;
-    auto vi = [&](int d) { return ((size_t)d * a.np + pat) * R + r; };
-    auto scv = [&](int d) { return a.sc[(size_t)d * a.np + pat]; };
-    const float2 wp = a.wts[pat];
-    const ff w{wp.x, wp.y};
+    // vector of directed edge d, its scaler: one widening product each (the
+    // strides fit in 32 bits, as three arrays of 6 edges or more fit in memory)
+    const size_t own_vec = pat * R + r;
+    const unsigned vec_step = (unsigned)(a.np * R), sc_step = (unsigned)a.np;
+    auto vi = [&](int d) { return (unsigned long long)(unsigned)d * vec_step + own_vec; };
+    auto scv = [&](int d) { return a.sc[(unsigned long long)(unsigned)d * sc_step + pat]; };
+    const float2 wpat = a.wts[pat];
+    const ff w{wpat.x, wpat.y};
     V vp[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) vp[e] = Pol::zero();
     const int scp = EMIT ? 0 : scv(pr.dp);
     if (on && !EMIT) {
       Pol::load_g(a.M, vi(pr.dp), vp);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) vp[e] = Pol::mul(vp[e], piv[e]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) vp[e] = Pol::zero();
+      for (int e = 0; e < 4; ++e) {
+        vp[e] = Pol::mul(vp[e], Pol::from_d(a.pi[e]));
+        if constexpr (std::is_same<Pol, Ff32>::value) vp[e] = Pol::mul(vp[e], prob);
+      }
     }
     V in[4];
     int in_sc = 0, sp = 0;
@@ -376,31 +477,55 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
       stk_sc[sp * NT + c] = s;
       ++sp;
     };
-    for (int si = 0; si < pr.n_steps && ok; ++si) {
-      const SprStep st = a.steps[pr.step_off + si];
-      if (st.flags & SPR_START) {
-        V ms[4], mg[4];
-        if (on) {
-          V ls[4], lg[4];
-          Pol::load_g(a.L, vi(st.d1), ls);
-          Pol::load_g(a.L, vi(st.d2), lg);
-          Pol::rows(Dm, lg, ms);   // into s, from g's side across the joined edge
-          Pol::rows(Dm, ls, mg);
-        } else {
+    const SprStep *prog = a.steps + pr.step_off;
+    SprStep st = prog[0];
+    {
+      V ms[4], mg[4];
+      if (on) {
+        V ls[4], lg[4];
+        Pol::load_g(a.L, vi(st.d1), ls);
+        Pol::load_g(a.L, vi(st.d2), lg);
+        Pol::rows(Dm, lg, ms);   // into s, from g's side across the joined edge
+        Pol::rows(Dm, ls, mg);
+      } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) ms[e] = mg[e] = Pol::zero();
-        }
-        const int scs = scv(st.d2), scg = scv(st.d1);
-        const bool ds = st.flags & SPR_DOWN1, dg = st.flags & SPR_DOWN2;
-        const bool g_first = ds && dg && (st.flags & SPR_FIRST2);
-        if (ds && dg) push(g_first ? ms : mg, g_first ? scs : scg);
-        const bool take_g = g_first || !ds;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) in[e] = take_g ? mg[e] : ms[e];
-        in_sc = take_g ? scg : scs;
-        have = true;
-        continue;
+        for (int e = 0; e < 4; ++e) ms[e] = mg[e] = Pol::zero();
       }
+      const int scs = scv(st.d2), scg = scv(st.d1);
+      const bool ds = st.flags & SPR_DOWN1, dg = st.flags & SPR_DOWN2;
+      const bool g_first = ds && dg && (st.flags & SPR_FIRST2);
+      if (ds && dg) push(g_first ? ms : mg, g_first ? scs : scg);
+      const bool take_g = g_first || !ds;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) in[e] = take_g ? mg[e] : ms[e];
+      in_sc = take_g ? scg : scs;
+      have = true;
+    }
+    if (!(st.flags & SPR_START)) ok = false;
+    V m1[4], m2[4];
+    int s1 = 0, s2 = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m1[e] = m2[e] = Pol::zero();
+    auto fetch = [&](const SprStep &x) {
+      s1 = scv(x.d1);
+      s2 = scv(x.d2);
+      if (on) {
+        Pol::load_g(a.M, vi(x.d1), m1);
+        Pol::load_g(a.M, vi(x.d2), m2);
+      }
+    };
+    if (pr.n_steps > 1) {
+      st = prog[1];
+      __syncwarp();
+      blocks(1, st);
+      fetch(st);
+    }
+    for (int si = 1; si < pr.n_steps && ok; ++si) {
+      const bool more = si + 1 < pr.n_steps, scored = st.out1 >= 0 || st.out2 >= 0;
+      const SprStep nx = more ? prog[si + 1] : st;
+      V hh1[4], hh2[4];
+      if (!EMIT && on && st.out1 >= 0) Pol::load_g(a.H, vi(st.d1), hh1);
+      if (!EMIT && on && st.out2 >= 0) Pol::load_g(a.H, vi(st.d2), hh2);
       if (!have) {
         if (sp == 0) {
           ok = false;
@@ -411,41 +536,32 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
         for (int e = 0; e < 4; ++e) in[e] = stk[((size_t)sp * 4 + e) * NT + c];
         in_sc = stk_sc[sp * NT + c];
       }
-      const int s1 = scv(st.d1), s2 = scv(st.d2);
       V l1[4], l2[4];
       int sc1 = in_sc + s2, sc2 = in_sc + s1;
-      if (on) {
-        V m1[4], m2[4];
-        Pol::load_g(a.M, vi(st.d1), m1);
-        Pol::load_g(a.M, vi(st.d2), m2);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          l1[e] = Pol::mul(in[e], m2[e]);
-          l2[e] = Pol::mul(in[e], m1[e]);
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) l1[e] = l2[e] = Pol::zero();
-      }
-      rescale<Pol, RT>(l1, sc1);
-      rescale<Pol, RT>(l2, sc2);
-      const int e1 = st.d1 >> 1, e2 = st.d2 >> 1;
-      const Coef *D1 = Dh + ((size_t)e1 * R + (on ? r : 0)) * 16;
-      const Coef *D2 = Dh + ((size_t)e2 * R + (on ? r : 0)) * 16;
+      const int at1 = s1, at2 = s2;
+      Pol::mul4(in, m2, l1);
+      Pol::mul4(in, m1, l2);
+      if (more) fetch(nx);
+      rescale2<Pol, RT>(l1, sc1, l2, sc2);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();   // this step's blocks are here, and all lanes are done with the step before's
+      if (more) blocks((si + 1) & 1, nx);
+      const Coef *D1 = reinterpret_cast<const Coef *>(dsh + (size_t)(si & 1) * 2 * UNITS + (on ? r : 0));
+      const Coef *D2 = reinterpret_cast<const Coef *>(dsh + (size_t)(si & 1) * 2 * UNITS + UNITS + (on ? r : 0));
       V h1[4], h2[4];
-      Pol::rows(D1, l1, h1);
-      Pol::rows(D2, l2, h2);
-      if (EMIT && (st.out1 >= 0 || st.out2 >= 0)) {
+      Pol::rows(D1, l1, h1, RT);
+      Pol::rows(D2, l2, h2, RT);
+      if (EMIT && scored) {
         if (on) {
           const bool side_b = ((a.prune_base + blockIdx.x) & 1) != 0;
-          V hh[4], x[4], y[4];
+          V x[4], y[4];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int out = h == 0 ? st.out1 : st.out2;
             if (out < 0) continue;
-            Pol::load_g(a.H, vi(h == 0 ? st.d1 : st.d2), hh);
+            Pol::load_g(a.H, vi(h == 0 ? st.d1 : st.d2), hh1);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) x[e] = Pol::mul(h == 0 ? h1[e] : h2[e], hh[e]);
+            for (int e = 0; e < 4; ++e) x[e] = Pol::mul(h == 0 ? h1[e] : h2[e], hh1[e]);
             if (side_b) {
               Pol::rows(static_cast<const Coef *>(a.Dfull) + ((size_t)(pr.dp >> 1) * R + r) * 16, x, y);
             } else {
@@ -454,61 +570,54 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
             }
             const size_t slot = (size_t)(out - a.slot_base);
             Pol::store_g(a.xout, (slot * a.np + pat) * R + r, y);
-            if (r == 0) a.xsc[slot * a.np + pat] = h == 0 ? sc1 + s1 : sc2 + s2;
+            if (r == 0) a.xsc[slot * a.np + pat] = h == 0 ? sc1 + at1 : sc2 + at2;
           }
         }
-      } else if (st.out1 >= 0 || st.out2 >= 0) {
+      } else if (scored) {
         V p1 = Pol::zero(), p2 = Pol::zero();
-        if (on) {
-          V hh[4];
-          if (st.out1 >= 0) {
-            Pol::load_g(a.H, vi(st.d1), hh);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) p1 = Pol::add(p1, Pol::mul(Pol::mul(h1[e], hh[e]), vp[e]));
-            p1 = Pol::mul(p1, prob);
-          }
-          if (st.out2 >= 0) {
-            Pol::load_g(a.H, vi(st.d2), hh);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) p2 = Pol::add(p2, Pol::mul(Pol::mul(h2[e], hh[e]), vp[e]));
-            p2 = Pol::mul(p2, prob);
-          }
-        }
-#pragma unroll
-        for (int o = 1; o < RT; o <<= 1) {
-          p1 = Pol::add(p1, Pol::shfl_xor(p1, o));
-          p2 = Pol::add(p2, Pol::shfl_xor(p2, o));
-        }
-        ff v1{0.0f, 0.0f}, v2{0.0f, 0.0f};
-        if (w.h != 0.0f) {
-          if (mine1 && st.out1 >= 0) {
-            if (Pol::positive(p1)) v1 = ff_mul(Pol::site_log(p1, sc1 + s1 + scp, ltab), w);
+        if (on && st.out1 >= 0) p1 = site_part<Pol>(h1, hh1, vp, prob);
+        if (on && st.out2 >= 0) p2 = site_part<Pol>(h2, hh2, vp, prob);
+        const int o1 = st.out1 - pr.move_off, o2 = st.out2 - pr.move_off;
+        const int last = st.out2 >= 0 ? o2 : o1;
+        if (last - base >= SCAN_WIN) flush(st.out1 >= 0 ? o1 : o2, g == 0);
+        ff *own = red + warp * SCAN_WIN - base;
+        auto weighed = [&](V p, int e2, bool wanted) {
+          ff v{0.0f, 0.0f};
+          if (wanted && w.h != 0.0f) {
+            if (Pol::positive(p)) v = ff_mul(Pol::site_log(p, e2, ltab), w);
             else atomicOr(a.flag, PGPU_FLAG_NAN);
           }
-          if (mine2 && st.out2 >= 0) {
-            if (Pol::positive(p2)) v2 = ff_mul(Pol::site_log(p2, sc2 + s2 + scp, ltab), w);
-            else atomicOr(a.flag, PGPU_FLAG_NAN);
-          }
-        }
+          return v;
+        };
+        // sums of pairs, the low words left unnormalised between the patterns
+        auto over_patterns = [&](ff v) {
 #pragma unroll
-        for (int o = RT; o < 32; o <<= 1) {
-          v1 = ff_add(v1, ff_shfl_xor(v1, o));
-          v2 = ff_add(v2, ff_shfl_xor(v2, o));
-        }
-        if (lane == 0 && st.out1 >= 0) {
-          ff &dst = red[warp * a.max_moves + (st.out1 - pr.move_off)];
-          dst = ff_add(dst, v1);
-        }
-        if (lane == lane2 && st.out2 >= 0) {
-          ff &dst = red[warp * a.max_moves + (st.out2 - pr.move_off)];
-          dst = ff_add(dst, v2);
+          for (int o = RT; o < 32; o <<= 1) {
+            const ff x = ff_shfl_xor(v, o), t = two_sum(v.h, x.h);
+            v = {t.h, __fadd_rn(t.l, __fadd_rn(v.l, x.l))};
+          }
+          return v;
+        };
+        if constexpr (RT == 1) {
+          const ff v1 = over_patterns(weighed(p1, sc1 + at1 + scp, st.out1 >= 0));
+          const ff v2 = over_patterns(weighed(p2, sc2 + at2 + scp, st.out2 >= 0));
+          if (lane == 0 && st.out1 >= 0) own[o1] = v1;
+          if (lane == 0 && st.out2 >= 0) own[o2] = v2;
+        } else {
+          const bool odd = r & 1;
+          V p = Pol::add(odd ? p2 : p1, Pol::shfl_xor(odd ? p1 : p2, 1));
+#pragma unroll
+          for (int o = 2; o < RT; o <<= 1) p = Pol::add(p, Pol::shfl_xor(p, o));
+          const bool wanted = odd ? st.out2 >= 0 : st.out1 >= 0;
+          const ff v = over_patterns(weighed(p, (odd ? sc2 + at2 : sc1 + at1) + scp, wanted));
+          if (lane < 2 && wanted) own[odd ? o2 : o1] = v;
         }
       }
       const bool dn1 = st.flags & SPR_DOWN1, dn2 = st.flags & SPR_DOWN2;
       if (dn1 || dn2) {
         V n1[4], n2[4];
-        if (dn1) Pol::rows(D1, h1, n1);   // P(t/2) P(t/2) L = P(t) L
-        if (dn2) Pol::rows(D2, h2, n2);
+        if (dn1) Pol::rows(D1, h1, n1, RT);   // P(t/2) P(t/2) L = P(t) L
+        if (dn2) Pol::rows(D2, h2, n2, RT);
         const bool second_first = dn1 && dn2 && (st.flags & SPR_FIRST2);
         if (dn1 && dn2) push(second_first ? n1 : n2, second_first ? sc1 : sc2);
         const bool take2 = second_first || !dn1;
@@ -519,16 +628,14 @@ __global__ void __launch_bounds__(SPR_NT) spr_scan_kernel(const ScanArgs a) {
       } else {
         have = false;
       }
+      st = nx;
+    }
+    if (!EMIT) {
+      flush(pr.n_moves, g == 0);
+      base = 0;
     }
   }
   if (!ok && c == 0) atomicOr(a.flag, PGPU_FLAG_EIGEN);   // program and stack disagree
-  if (EMIT) return;
-  __syncthreads();
-  for (int j = c; j < pr.n_moves; j += NT) {
-    ff s = red[j];
-    for (int w = 1; w < SPR_NW; ++w) s = ff_add(s, red[w * a.max_moves + j]);
-    a.partials[(size_t)blockIdx.y * a.n_moves + pr.move_off + j] = (double)s.h + (double)s.l;
-  }
 }
 
 // lnl[m] = sum over CTA groups of the partial sums: slice y of a move's groups
@@ -1135,8 +1242,7 @@ __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
 // left as it is: the other eigenvectors' float roundings are larger.
 // 509 edges x 45,675 patterns x 4 classes, pair form: 1.66 ms against 11.4
 // in FP64, which this GPU runs at 1/64 of the FP32 rate.
-__device__ __forceinline__ float2 neg2(float2 v) { return __fmul2_rn(v, make_float2(-1.0f, -1.0f)); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
 __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &e) {
   s = __fadd2_rn(a, b);
   const float2 bb = sub2(s, a);
@@ -1621,15 +1727,15 @@ pgpu_status launch_scan_rt(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, i
   a.G = G;
   a.n_blocks = n_blocks;
   a.depth = std::max(p.max_depth, 1);
-  a.max_moves = std::max(p.max_moves_per_prune, 1);
   a.Dfull = nullptr;
   a.xout = nullptr;
   a.xsc = nullptr;
   a.slot_base = 0;
   a.prune_base = 0;
-  const size_t smem = scan_smem<Pol>(a.depth, a.max_moves);
-  if (smem > s->ctx->smem_optin)
-    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "spr: scan needs %zu bytes of shared memory", smem);
+  const size_t smem = scan_smem<Pol>(a.depth, RT);
+  const size_t need = scan_limit<Pol>(a.depth, std::max(p.max_moves_per_prune, 1), RT);
+  if (need > s->ctx->smem_optin)
+    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "spr: scan needs %zu bytes of shared memory", need);
   PGPU_CUDA(s->ctx, cudaFuncSetAttribute(spr_scan_kernel<Pol, RT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   spr_scan_kernel<Pol, RT><<<dim3((unsigned)p.prunes.size(), (unsigned)n_groups), SPR_NT, smem,
@@ -1676,13 +1782,23 @@ pgpu_status run_scan(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, double 
   const size_t nm = p.moves.size();
   if (nm == 0) return PGPU_OK;
   PGPU_TRY(ensure_half(s, p));
-  const int n_blocks = (int)(s->np / s->NP);
   // CTA groups of G pattern blocks; partial sums at most 256 MB
   const size_t budget = size_t(256) << 20;
-  int G = (int)std::max<size_t>(1, ((size_t)n_blocks * nm * 8 + budget - 1) / budget);
-  G = std::min(G, n_blocks);
-  const int n_groups = (n_blocks + G - 1) / G;
-  if (n_groups > 65535) return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "spr: too many pattern blocks");
+  auto groups = [&](int blocks, int *g) {
+    *g = (int)std::max<size_t>(1, ((size_t)blocks * nm * 8 + budget - 1) / budget);
+    *g = std::min(*g, blocks);
+    return (blocks + *g - 1) / *g;
+  };
+  int G;
+  const int lim_np = SPR_LIMIT_NT / s->RT;
+  if (groups((int)((s->np + lim_np - 1) / lim_np), &G) > 65535)
+    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "spr: too many pattern blocks");
+  const int n_blocks = (int)(s->np / s->NP);
+  int n_groups = groups(n_blocks, &G);
+  if (n_groups > 65535) {   // a grid's second dimension
+    G = (n_blocks + 65534) / 65535;
+    n_groups = (n_blocks + G - 1) / G;
+  }
   PGPU_TRY(grow(s, &s->partials, &s->part_cap, (size_t)n_groups * nm));
   if (s->precision == 32) PGPU_TRY(launch_scan<Fp32>(s, p, d, G, n_groups, n_blocks));
   else if (s->precision == 48) PGPU_TRY(launch_scan<Ff32>(s, p, d, G, n_groups, n_blocks));
@@ -1731,22 +1847,24 @@ pgpu_status launch_emit_rt(pgpu_spr *s, int prune_base, int n_prunes, long long 
   a.n_moves = p.moves.size();
   a.R = s->R;
   a.NP = s->NP;
-  a.G = 1;
   a.n_blocks = (int)(s->np / s->NP);
+  a.G = (a.n_blocks + 65534) / 65535;   // a grid's second dimension
   a.depth = std::max(p.max_depth, 1);
-  a.max_moves = std::max(p.max_moves_per_prune, 1);
   a.Dfull = s->Dfull;
   a.xout = s->tbr_x;
   a.xsc = s->tbr_xsc;
   a.slot_base = slot_base;
   a.prune_base = prune_base;
-  if (a.n_blocks > 65535) return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "tbr: too many pattern blocks");
-  const size_t smem = scan_smem<Pol>(a.depth, a.max_moves);
-  if (smem > s->ctx->smem_optin)
-    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "tbr: walk needs %zu bytes of shared memory", smem);
+  const int lim_np = SPR_LIMIT_NT / s->RT;
+  if ((s->np + lim_np - 1) / lim_np > 65535)
+    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "tbr: too many pattern blocks");
+  const size_t smem = scan_smem<Pol>(a.depth, RT);
+  const size_t need = scan_limit<Pol>(a.depth, std::max(p.max_moves_per_prune, 1), RT);
+  if (need > s->ctx->smem_optin)
+    return pgpu_set_err(s->ctx, PGPU_ERR_LIMIT, "tbr: walk needs %zu bytes of shared memory", need);
   PGPU_CUDA(s->ctx, cudaFuncSetAttribute(spr_scan_kernel<Pol, RT, true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  spr_scan_kernel<Pol, RT, true><<<dim3((unsigned)n_prunes, (unsigned)a.n_blocks), SPR_NT, smem,
+  spr_scan_kernel<Pol, RT, true><<<dim3((unsigned)n_prunes, (unsigned)((a.n_blocks + a.G - 1) / a.G)), SPR_NT, smem,
                                    s->ctx->stream>>>(a);
   return pgpu_after_launch(s->ctx, "spr_scan_kernel (emit)");
 }

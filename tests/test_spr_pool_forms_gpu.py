@@ -99,3 +99,36 @@ def test_fitch_planes(ctx, n, n_pat, fraction):
     for i in range(0, len(mv), max(1, len(mv) // 6)):
         assert lens[i] == SO.fitch_length(SO.apply_move(adj, *mv[i]), n, d["pats"], masks, d["w"])
     e.close()
+
+
+@pytest.mark.parametrize("prec,k,n_pat", [(48, 1, 129), (48, 2, 63), (48, 4, 33), (48, 8, 17), (32, 3, 40), (64, 2, 65)])
+def test_more_moves_than_a_window(ctx, prec, k, n_pat):
+    """Prunes of up to 74 moves, summed over the warps 64 at a time, against the
+    same moves scored a few to a prune and against the oracle."""
+    d = problem(ctx, 40, n_pat, k, 70 + k, 1.0)
+    e = engine(d, ctx, prec)
+    got = e.scan().cpu().numpy()
+    rng = np.random.default_rng(k)
+    some = rng.choice(len(got), 40, replace=False)
+    assert np.allclose(e.score(some), got[some], rtol=1e-12, atol=0)
+    cur = e.get_tree()
+    adj = SO.unroot(cur.left, cur.right, cur.brlen)
+    mv = e.moves()
+    tol = {64: 1e-10, 48: 1e-9}.get(prec)
+    for i in some[:8]:
+        exp = SO.lnl(SO.apply_move(adj, *mv[i]), 40, d["q"], d["pi"], d["rates"], d["probs"], d["pats"],
+                     d["table"], d["w"])
+        assert abs(got[i] - exp) <= (tol * abs(exp) if tol else 2e-6 * d["w"].sum())
+    e.close()
+
+
+def test_groups_of_pattern_blocks(ctx):
+    """Enough moves and patterns that a CTA walks several blocks: the partial
+    sums are added up in place, and agree with the moves scored by themselves."""
+    d = problem(ctx, 120, 80000, 1, 3, 1.0)
+    e = engine(d, ctx, 32)
+    got = e.scan().cpu().numpy()
+    assert len(got) * -(-80000 // 128) * 8 > 256 << 20
+    some = np.random.default_rng(0).choice(len(got), 30, replace=False)
+    assert np.allclose(e.score(some), got[some], rtol=1e-12, atol=0)
+    e.close()

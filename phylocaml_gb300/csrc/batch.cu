@@ -116,11 +116,10 @@ __host__ __device__ inline size_t cm_off(int n, int k, int Kp) {
 // x rounded to the nearest TF32 value (10-bit mantissa, ties away from
 // zero), as bits: the MMA then reads an unbiased operand instead of one
 // whose low bits are dropped.  For a finite x >= 0 adding half a TF32 unit
-// to the bit pattern and clearing the 13 dropped bits rounds it (a carry
-// out of the mantissa raises the exponent), with two integer instructions.
-__device__ __forceinline__ uint32_t tf32_bits(float x) {
-  return (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-}
+// to the bit pattern rounds it (a carry out of the mantissa raises the
+// exponent); the 13 bits below are not part of the operand and are left as
+// they come (clearing them made the codon and protein batch 17.15 ms, not 16.5).
+__device__ __forceinline__ uint32_t tf32_bits(float x) { return __float_as_uint(x) + 0x1000u; }
 
 // W consecutive TMEM columns of this thread's lane (32x32b shape)
 template <int W>
@@ -796,19 +795,26 @@ __global__ void __launch_bounds__(256) batch_finalize_kernel(const double2 *part
 // rate class, P = U diag(exp(lambda r t)) Ui in FP64 (shared memory), then
 //   tip branch      tip rows tab[c][i] = sum_j P[i][j] code_tab[c][j]  (float)
 //   internal branch B block B[n=i][k=j] = P[i][j] in the core-matrix layout
+// Bound by FP64, which this GPU runs at 1/64 of the FP32 rate, so as little
+// of it as gives the same values: U diag(e) is formed once per CTA; U and Ui
+// come from a symmetric eigen system scaled by the frequencies, so that
+// pi_i P_ij = pi_j P_ji and half the entries are summed; a tip row sums the
+// states its code holds.  16 protein (4 classes) and 16 codon models, 254
+// branches each: 1.26 ms against 5.04.
 struct SetupArgs {
   const BVar *vars;
   const int *members;             // variants of this group
   const double *U, *lam, *Ui;     // group eigen systems [g][S][S], [g][S], [g][S][S]
   const int *status;              // [g]
-  const double *brlen, *rates, *ctab;
+  const double *brlen, *rates, *ctab, *pis;
   float *bmat, *tiptab;
   int *flag;
   int S;
 };
 
 __global__ void __launch_bounds__(256) batch_setup_kernel(const SetupArgs a) {
-  extern __shared__ __align__(16) double P[];   // [S][S] then e[S]
+  extern __shared__ __align__(16) double P[];   // [S][S], then U diag(e) [S][S], Ui [S][S], e[S], pi[S], 1/pi[S]
+  __shared__ unsigned long long holds[256];     // states of each code
   const int S = a.S, SS = S * S;
   const int vi = a.members[blockIdx.z];
   const BVar &v = a.vars[vi];
@@ -821,31 +827,61 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(const SetupArgs a) {
     return;
   }
   const double *U = a.U + (size_t)g * SS, *Ui = a.Ui + (size_t)g * SS, *lam = a.lam + (size_t)g * S;
-  double *e = P + SS;
+  double *W = P + SS, *V = W + SS, *e = V + SS, *pi = e + S, *rpi = pi + S;
   const double t = a.brlen[v.brlen_off + c], rate = a.rates[v.rates_off + r];
   const bool ident = !(t * rate >= 1e-10);   // effective time: a rate-0 class gets I exactly
-  for (int k = tid; k < S; k += nt) e[k] = exp(lam[k] * rate * t);
-  __syncthreads();
-  for (int o = tid; o < SS; o += nt) {
-    const int i = o / S, j = o % S;
-    double x = 0.0;
-    if (ident) {
-      x = i == j ? 1.0 : 0.0;
-    } else {
-      for (int k = 0; k < S; ++k) x = fma(U[i * S + k] * e[k], Ui[k * S + j], x);
+  const double *ct = a.ctab + v.ctab_off;
+  for (int k = tid; k < S; k += nt) {
+    e[k] = exp(lam[k] * rate * t);
+    pi[k] = a.pis[v.pi_off + k];
+    rpi[k] = 1.0 / pi[k];
+  }
+  if (c < v.n_tips)
+    for (int code = tid >> 5; code < v.n_codes; code += nt >> 5) {
+      const int lane = tid & 31;
+      unsigned m[2];
+      for (int h = 0; h < 2; ++h) {
+        const int j = 32 * h + lane;
+        m[h] = __ballot_sync(0xffffffffu, j < S && __double_as_longlong(ct[code * S + j]) != 0);
+      }
+      if (lane == 0) holds[code] = m[0] | (unsigned long long)m[1] << 32;
     }
-    P[o] = fmax(x, 0.0);   // transition probabilities: clamp eigen-product noise below 0
+  __syncthreads();
+  if (ident) {
+    for (int o = tid; o < SS; o += nt) P[o] = o / S == o % S ? 1.0 : 0.0;
+  } else {
+    for (int o = tid; o < SS; o += nt) {
+      W[o] = U[o] * e[o % S];
+      V[o] = Ui[o];
+    }
+    __syncthreads();
+    // the entries on and above the diagonal: rows a and S - 1 - a together
+    // are S + 1 of them
+    for (int o = tid; o < S * (S + 1) / 2; o += nt) {
+      const int q = o / (S + 1), m = o % (S + 1);
+      const int i = m < S - q ? q : S - 1 - q, j = m < S - q ? q + m : m - 1;
+      double x = 0.0;
+      for (int k = 0; k < S; ++k) x = fma(W[i * S + k], V[k * S + j], x);
+      x = fmax(x, 0.0);   // transition probabilities: clamp eigen-product noise below 0
+      P[i * S + j] = x;
+      if (i != j) P[j * S + i] = fmax(x * (pi[i] * rpi[j]), 0.0);
+    }
   }
   __syncthreads();
   if (c < v.n_tips) {
     float *out = a.tiptab + v.tip_off + ((size_t)c * v.R + r) * v.NCp * v.SpT;
-    const double *ct = a.ctab + v.ctab_off;
     for (int o = tid; o < v.NCp * v.SpT; o += nt) {
       const int code = o / v.SpT, i = o % v.SpT;
-      double y = 0.0;
-      if (i < S && code < v.n_codes)
-        for (int j = 0; j < S; ++j) y = fma(P[i * S + j], ct[code * S + j], y);
-      out[o] = (float)y;
+      float y = 0.0f;
+      if (i < S && code < v.n_codes) {
+        double x = 0.0;
+        for (unsigned long long m = holds[code]; m; m &= m - 1) {
+          const int j = __ffsll((long long)m) - 1;
+          x = fma(P[i * S + j], ct[code * S + j], x);
+        }
+        y = (float)x;
+      }
+      out[o] = y;
     }
   } else {
     unsigned char *out = reinterpret_cast<unsigned char *>(
@@ -1269,6 +1305,7 @@ pgpu_status pgpu_batch_run(pgpu_ctx *ctx, pgpu_batch *b, double *lnl_dev, double
     a.brlen = b->brlen;
     a.rates = b->rates;
     a.ctab = b->ctab;
+    a.pis = b->pis;
     a.bmat = b->bmat;
     a.tiptab = b->tiptab;
     a.flag = ctx->d_flag;
@@ -1278,7 +1315,7 @@ pgpu_status pgpu_batch_run(pgpu_ctx *ctx, pgpu_batch *b, double *lnl_dev, double
       max_tips = std::max(max_tips, b->hvars[vi].n_tips);
       max_R = std::max(max_R, b->hvars[vi].R);
     }
-    const size_t smem = sizeof(double) * ((size_t)S * S + S);
+    const size_t smem = sizeof(double) * (3 * (size_t)S * S + 3 * S);
     PGPU_CUDA(ctx, cudaFuncSetAttribute(batch_setup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)std::max<size_t>(smem, 1024)));
     batch_setup_kernel<<<dim3(2 * max_tips - 2, max_R, (unsigned)b->group_members[g].size()), 256, smem,

@@ -269,8 +269,8 @@ struct Share {
 // 2*RP*NP + (s*RP + q)*KP.
 template <int KP, int RP, int PT>
 __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, const int4 op, int lane,
-                                         int slot, uint64_t *empty, float (*xch)[BT_M], int &escale,
-                                         bool &ok, ff &Lp) {
+                                         int slot, uint64_t *empty, uint64_t *mma_bar, uint32_t mma_par,
+                                         float (*xch)[BT_M], int &escale, bool &ok, ff &Lp) {
   using SH = Share<KP, RP, PT>;
   constexpr int B = SH::B, e0 = SH::e0, rate = SH::rate;
   constexpr int BA = B > 0 ? B : 1;
@@ -281,33 +281,51 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
   for (int e = 0; e < BA; ++e) acc[e] = 1.0f;
   // states S .. KP-1 need no masks: the tip rows and the B blocks are zero
   // there, so every vector's padding is a product of zeros
+  const bool tips[2] = {op.y < in.n_tips, op.z < in.n_tips};
+  // the tip rows first, while the MMAs of the other child run
+  if constexpr (B > 0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (!ok || !tips[h]) continue;
+      int code = in.sl[h * 128 + in.m];
+      if (code >= in.n_codes) {
+        if (in.active && PT == 0) atomicOr(p.flag, PGPU_FLAG_BADCODE);
+        code = 0;
+      }
+      const float *row = reinterpret_cast<const float *>(in.sl + 256 + (size_t)(h * RP + rate) * in.BB) +
+                         code * SPT + e0;
+#pragma unroll
+      for (int e = 0; e < B; ++e) acc[e] *= row[e];
+    }
+  }
+  {
+    const bool got = __all_sync(0xffffffffu, ok && mbar_wait_bounded_for(mma_bar, mma_par, p.flag));
+    if (ok && !got) atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
+    ok = got;
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if constexpr (B > 0) {
     // TMEM loads of W columns: the widest of 16, 8, 4 that divides both the
     // first column and the width of the share
     constexpr int W = (e0 % 16 == 0 && B % 16 == 0) ? 16 : (e0 % 8 == 0 && B % 8 == 0) ? 8 : 4;
+    auto product = [&](int h, float *d) {   // child h's D columns
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (!ok) break;
-      const int ch = h == 0 ? op.y : op.z;
-      if (ch < in.n_tips) {
-        int code = in.sl[h * 128 + in.m];
-        if (code >= in.n_codes) {
-          if (in.active && PT == 0) atomicOr(p.flag, PGPU_FLAG_BADCODE);
-          code = 0;
-        }
-        const float *row = reinterpret_cast<const float *>(in.sl + 256 + (size_t)(h * RP + rate) * in.BB) +
-                           code * SPT + e0;
+      for (int c = 0; c < B; c += W)
+        tmem_ld<W>(in.tmem + in.lane_base + (uint32_t)((h * RP + rate) * NP + e0 + c), &d[c]);
+    };
+    float d[B];
+    if (ok && !tips[0] && !tips[1]) {
+      float d2[B];
+      product(0, d);
+      product(1, d2);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int e = 0; e < B; ++e) acc[e] *= row[e];
-      } else {
-        float d[B];
+      for (int e = 0; e < B; ++e) acc[e] = d[e] * d2[e];
+    } else if (ok && !(tips[0] && tips[1])) {
+      product(tips[0] ? 1 : 0, d);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < B; c += W)
-          tmem_ld<W>(in.tmem + in.lane_base + (uint32_t)((h * RP + rate) * NP + e0 + c), &d[c]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int e = 0; e < B; ++e) acc[e] *= d[e];
-      }
+      for (int e = 0; e < B; ++e) acc[e] *= d[e];
     }
   }
   __syncwarp();
@@ -438,24 +456,24 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
       const uint32_t par = (uint32_t)((seq / BT_ST) & 1);
       in.sl = sh.smem + (size_t)slot * p.slot_bytes;
       bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
-      got = got && mbar_wait_bounded_for(&sh.mma_bar[my_rate], (uint32_t)(seq & 1), p.flag);
       got = __all_sync(0xffffffffu, got);
       if (!got) {
         ok = false;
         atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int4 op = sh.slot_op[slot];
+      uint64_t *const mma_bar = &sh.mma_bar[my_rate];
+      const uint32_t mma_par = (uint32_t)(seq & 1);
       in.last = i == n_ops - 1;
       // the max exchange is double-buffered by step parity: a group's next
       // write cannot meet a read of the previous step's values
       float(*xch)[BT_M] = sh.xch + (seq & 1) * BT_PARTS;
       // pt is warp-uniform
       switch (pt) {
-        case 0: epi_step<KP, RP, 0>(p, in, op, lane, slot, sh.empty, xch, escale, ok, Lp); break;
-        case 1: epi_step<KP, RP, 1>(p, in, op, lane, slot, sh.empty, xch, escale, ok, Lp); break;
-        case 2: epi_step<KP, RP, 2>(p, in, op, lane, slot, sh.empty, xch, escale, ok, Lp); break;
-        default: epi_step<KP, RP, 3>(p, in, op, lane, slot, sh.empty, xch, escale, ok, Lp); break;
+        case 0: epi_step<KP, RP, 0>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
+        case 1: epi_step<KP, RP, 1>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
+        case 2: epi_step<KP, RP, 2>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
+        default: epi_step<KP, RP, 3>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -550,7 +568,8 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
   constexpr uint32_t LBO = 128, SBO = (uint32_t)(KP / 4) * 128;
   constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NP >> 3) << 17) |
                              ((uint32_t)(BT_M >> 4) << 24);
-  const int n_ops = vg.n_ops, R = vg.R, n_tips = vg.n_tips, BB = blk_bytes(vg);
+  const int n_ops = vg.n_ops, R = vg.R, n_tips = vg.n_tips, BB16 = blk_bytes(vg) / 16;
+  const uint64_t desc0 = smem_desc(sh.smem + 256, LBO, SBO);
   auto commit = [&](uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      su32(bar))
@@ -566,7 +585,7 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
         return;
       }
       const int4 op = sh.slot_op[slot];
-      const unsigned char *sl = sh.smem + (size_t)slot * p.slot_bytes;
+      const uint64_t slot_desc = desc0 + (uint32_t)slot * (uint32_t)(p.slot_bytes / 16);
       const bool any = op.y >= n_tips || op.z >= n_tips;
 #pragma unroll
       for (int q = 0; q < RP; ++q) {
@@ -591,10 +610,11 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
           const int sa = (op.w >> (8 * h)) & 0xff;
           const uint32_t d_col = (uint32_t)((h * RP + q) * NP);
           const uint32_t a_col = (uint32_t)(2 * RP * NP + (sa * RP + q) * KP);
-          const unsigned char *blk = sl + 256 + (size_t)(h * RP + q) * BB;
+          // the start address (16-byte units) is the descriptor's low field
+          const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + q) * BB16);
 #pragma unroll
           for (int ks = 0; ks < KP / 8; ++ks) {
-            const uint64_t bd = smem_desc(blk + (size_t)ks * 2 * LBO, LBO, SBO);
+            const uint64_t bd = bd0 + (uint32_t)(ks * 2 * LBO / 16);
             const uint32_t accf = ks > 0 ? 1u : 0u;
             asm volatile(
                 "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"

@@ -25,7 +25,7 @@
 //                  bulk-copies the B blocks of internal children, the
 //                  tip-table blocks and tip-code rows of tip children into a
 //                  shared ring slot, and publishes the step itself;
-//     warp 9       MMA issue (one thread);
+//     warps 9, 10  MMA issue, one per rate class of the pass;
 //     warps 0-7    epilogue: two warps per TMEM lane group of 32 patterns,
 //                  each owning a share of the row (half the states, or a
 //                  whole rate class when two share a pass); a thread reads
@@ -61,8 +61,8 @@ constexpr int BT_ST = 4;           // ring slots (power of two)
 constexpr int BT_EPI_WARPS = 8;    // epilogue warps, two per TMEM lane group
 constexpr int BT_PARTS = BT_EPI_WARPS / 4;   // shares of a row (one per warp of a lane group)
 constexpr int BT_EPI = 32 * BT_EPI_WARPS;
-constexpr int BT_THREADS = BT_EPI + 64;   // + the producer warp and the MMA warp
-constexpr int BT_PRODUCER = BT_EPI_WARPS, BT_MMA = BT_EPI_WARPS + 1;   // their warp indices
+constexpr int BT_THREADS = BT_EPI + 96;   // + the producer warp and the two MMA warps
+constexpr int BT_PRODUCER = BT_EPI_WARPS, BT_MMA = BT_EPI_WARPS + 1;   // the first of each
 constexpr int BT_TMEM_COLS = 512;
 
 struct BVar {
@@ -94,6 +94,11 @@ struct BVar {
 
 __device__ __forceinline__ uint32_t su32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// mbarrier arrival of `n` threads by one
+__device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared.b64 _, [%0], %1;" ::"r"(su32(bar)), "r"(n) : "memory");
 }
 
 // K-major, no-swizzle shared-memory descriptor: 8-row x 16-byte core
@@ -407,8 +412,8 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
 // Shared state of the epilogue warps.
 struct EpiShared {
   uint64_t *full, *empty;
-  uint64_t *mma_bar;         // [2]: per rate class of the pass (both complete once per step)
-  uint64_t *stored;          // [2]: the epilogue warps of the first and second half of the shares
+  uint64_t *mma_bar;         // [2]: for the first and second half of the shares; both complete once per step
+  uint64_t *stored;          // [2]: for the two MMA warps; likewise
   const int4 *slot_op;       // each ring slot's postorder step, written by the producer
   unsigned char *smem;
   float (*xch)[BT_M];        // [2][BT_PARTS]: per step parity and share, lane: max entry
@@ -432,6 +437,7 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
   const int m = 32 * lg + lane;   // pattern within the tile
   constexpr int PPR = BT_PARTS / RP;
   const int my_rate = pt / PPR;
+  const int half = pt / (BT_PARTS / 2);   // whose barriers the warp keeps step with
   // the share that combines its rate class's root likelihood
   const bool lead = pt % PPR == 0;
   // the variant's fields, once per item
@@ -462,7 +468,7 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
         atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
       }
       const int4 op = sh.slot_op[slot];
-      uint64_t *const mma_bar = &sh.mma_bar[my_rate];
+      uint64_t *const mma_bar = &sh.mma_bar[half];
       const uint32_t mma_par = (uint32_t)(seq & 1);
       in.last = i == n_ops - 1;
       // the max exchange is double-buffered by step parity: a group's next
@@ -479,7 +485,14 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       // this warp's vectors of the step are in TMEM and its D columns read
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.stored[pt / (BT_PARTS / 2)]);
+      if (lane == 0) {
+        if (RP == 2) {
+          mbar_arrive_n(&sh.stored[half], 2);
+        } else {
+          mbar_arrive(&sh.stored[0]);
+          mbar_arrive(&sh.stored[1]);
+        }
+      }
       if (!ok) break;
     }
     // one verdict for every epilogue warp before the barriers below
@@ -553,102 +566,93 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
   asm volatile("bar.sync 1, %0;" ::"n"(BT_EPI) : "memory");
 }
 
-// The MMA warp's side of one work item: per step, once the slot is loaded,
-// one thread issues the step's tcgen05.mma for the internal children, rate
-// class by rate class.  A class's MMAs wait until its epilogue warps have
-// stored the previous step's vectors (and read its D columns), and are
-// committed to that class's mma_bar; the last commit also goes to the
-// slot's empty barrier.  With one rate class per pass the MMAs wait for
-// both halves of the epilogue and are committed to both mma_bar barriers,
-// so each barrier completes once per step either way.
+// An MMA warp's side of one work item: per step, once the slot is loaded, the
+// step's tcgen05.mma for the internal children of rate class q.  They wait
+// until the epilogue warps that write and read the class's columns have
+// stored the previous step's vectors, and are committed to the class's
+// mma_bar and the slot's empty barrier.  With one rate class per pass warp 0
+// issues and commits for both, and warp 1 keeps step with the barriers.  The
+// warp stays converged: the descriptors are uniform and the elected thread,
+// always the same, issues under a predicate (one thread issuing for both
+// classes took 1,200 cycles of a step's 1,650).
 template <int KP, int RP>
-__device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg,
-                                         long long &seq, bool &ok) {
+__device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
+                                         const int lane, long long &seq, bool &ok) {
   constexpr int NP = (KP + 15) / 16 * 16;
   constexpr uint32_t LBO = 128, SBO = (uint32_t)(KP / 4) * 128;
   constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NP >> 3) << 17) |
                              ((uint32_t)(BT_M >> 4) << 24);
   const int n_ops = vg.n_ops, R = vg.R, n_tips = vg.n_tips, BB16 = blk_bytes(vg) / 16;
+  const bool issues = RP == 2 || q == 0;
+  const int rq = RP == 2 ? q : 0;   // the class it issues for
   const uint64_t desc0 = smem_desc(sh.smem + 256, LBO, SBO);
   auto commit = [&](uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     su32(bar))
-                 : "memory");
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(su32(bar))
+        : "memory");
   };
   for (int r0 = 0; r0 < R && ok; r0 += RP) {
     for (int i = 0; i < n_ops; ++i, ++seq) {
       const int slot = (int)(seq & (BT_ST - 1));
       const uint32_t par = (uint32_t)((seq / BT_ST) & 1);
-      if (!mbar_wait_bounded_for(&sh.full[slot], par, p.flag)) {
+      bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
+      // the epilogue warps of this class are done with the previous step
+      if (seq > 0) got = got && mbar_wait_bounded_for(&sh.stored[q], (uint32_t)((seq - 1) & 1), p.flag);
+      if (!__all_sync(0xffffffffu, got)) {
         ok = false;
         atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
         return;
       }
       const int4 op = sh.slot_op[slot];
-      const uint64_t slot_desc = desc0 + (uint32_t)slot * (uint32_t)(p.slot_bytes / 16);
       const bool any = op.y >= n_tips || op.z >= n_tips;
-#pragma unroll
-      for (int q = 0; q < RP; ++q) {
-        // this class's epilogue warps are done with the previous step (with
-        // one class per pass, all of them)
-        bool got = true;
-        if (seq > 0) {
-          const uint32_t prev = (uint32_t)((seq - 1) & 1);
-          got = mbar_wait_bounded_for(&sh.stored[q], prev, p.flag);
-          if (RP == 1) got = got && mbar_wait_bounded_for(&sh.stored[1], prev, p.flag);
-        }
-        if (!got) {
-          ok = false;
-          atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
-          return;
-        }
+      if (issues && any) {
+        const uint64_t slot_desc = desc0 + (uint32_t)slot * (uint32_t)(p.slot_bytes / 16);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int ch = h == 0 ? op.y : op.z;
           if (ch < n_tips) continue;
           const int sa = (op.w >> (8 * h)) & 0xff;
-          const uint32_t d_col = (uint32_t)((h * RP + q) * NP);
-          const uint32_t a_col = (uint32_t)(2 * RP * NP + (sa * RP + q) * KP);
+          const uint32_t d_col = (uint32_t)((h * RP + rq) * NP);
+          const uint32_t a_col = (uint32_t)(2 * RP * NP + (sa * RP + rq) * KP);
           // the start address (16-byte units) is the descriptor's low field
-          const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + q) * BB16);
+          const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + rq) * BB16);
 #pragma unroll
           for (int ks = 0; ks < KP / 8; ++ks) {
             const uint64_t bd = bd0 + (uint32_t)(ks * 2 * LBO / 16);
-            const uint32_t accf = ks > 0 ? 1u : 0u;
             asm volatile(
-                "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, q;\n\t}" ::"r"(sh.tmem + d_col),
-                "r"(sh.tmem + a_col + (uint32_t)(ks * 8)), "l"(bd), "r"(IDESC), "r"(accf)
+                "{\n\t.reg .pred e, q;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, q;\n\t}" ::"r"(sh.tmem + d_col),
+                "r"(sh.tmem + a_col + (uint32_t)(ks * 8)), "l"(bd), "r"(IDESC), "r"(ks > 0 ? 1u : 0u)
                 : "memory");
           }
         }
-        if (any)
-          commit(&sh.mma_bar[q]);
-        else
-          mbar_arrive(&sh.mma_bar[q]);
-      }
-      if (any) {
+        commit(&sh.mma_bar[q]);
         if (RP == 1) commit(&sh.mma_bar[1]);
         commit(&sh.empty[slot]);
-      } else {
-        if (RP == 1) mbar_arrive(&sh.mma_bar[1]);
+      } else if (lane == 0) {
+        if (issues) {
+          mbar_arrive(&sh.mma_bar[q]);
+          if (RP == 1) mbar_arrive(&sh.mma_bar[1]);
+        }
         mbar_arrive(&sh.empty[slot]);
       }
+      __syncwarp();
     }
   }
 }
 
 template <int KP>
-__device__ __forceinline__ void mma_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg,
-                                            long long &seq, bool &ok) {
+__device__ __forceinline__ void mma_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
+                                            const int lane, long long &seq, bool &ok) {
   if constexpr (KP <= 32) {
     if (vg.RP == 2) {
-      mma_item<KP, 2>(p, sh, vg, seq, ok);
+      mma_item<KP, 2>(p, sh, vg, q, lane, seq, ok);
       return;
     }
   }
-  mma_item<KP, 1>(p, sh, vg, seq, ok);
+  mma_item<KP, 1>(p, sh, vg, q, lane, seq, ok);
 }
 
 template <int KP>
@@ -683,11 +687,11 @@ __global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs
   if (tid == 0) {
     for (int s = 0; s < BT_ST; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1 + BT_EPI_WARPS);   // the MMA commit + the epilogue warps
+      mbar_init(&empty[s], 2 + BT_EPI_WARPS);   // the MMA warps + the epilogue warps
     }
     for (int q = 0; q < 2; ++q) {
       mbar_init(&mma_bar[q], 1);
-      mbar_init(&stored[q], BT_EPI_WARPS / 2);   // half the epilogue warps, after a step's TMEM stores
+      mbar_init(&stored[q], BT_EPI_WARPS);   // after a step's TMEM stores
     }
     fence_mbarrier_init();
   }
@@ -750,28 +754,27 @@ __global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs
       for (long long s = seq - BT_ST; s < seq; ++s)
         if (s >= 0) (void)mbar_wait_bounded_for(&full[s & (BT_ST - 1)], (uint32_t)((s / BT_ST) & 1), p.flag);
     }
-  } else if (warp == BT_MMA) {
+  } else if (warp >= BT_MMA) {
     // ------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      long long seq = 0;
-      bool ok = true;
-      for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
-        const int2 wk = __ldg(p.work + w);
-        const BVar &v = p.vars[wk.x];
-        switch (v.Kp) {
-          case 8: mma_item_rp<8>(p, sh, v, seq, ok); break;
-          case 16: mma_item_rp<16>(p, sh, v, seq, ok); break;
-          case 24: mma_item_rp<24>(p, sh, v, seq, ok); break;
-          case 32: mma_item_rp<32>(p, sh, v, seq, ok); break;
-          case 40: mma_item_rp<40>(p, sh, v, seq, ok); break;
-          case 48: mma_item_rp<48>(p, sh, v, seq, ok); break;
-          case 56: mma_item_rp<56>(p, sh, v, seq, ok); break;
-          default: mma_item_rp<64>(p, sh, v, seq, ok); break;
-        }
+    const int q = warp - BT_MMA;
+    long long seq = 0;
+    bool ok = true;
+    for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
+      const int2 wk = __ldg(p.work + w);
+      const BVar &v = p.vars[wk.x];
+      switch (v.Kp) {
+        case 8: mma_item_rp<8>(p, sh, v, q, lane, seq, ok); break;
+        case 16: mma_item_rp<16>(p, sh, v, q, lane, seq, ok); break;
+        case 24: mma_item_rp<24>(p, sh, v, q, lane, seq, ok); break;
+        case 32: mma_item_rp<32>(p, sh, v, q, lane, seq, ok); break;
+        case 40: mma_item_rp<40>(p, sh, v, q, lane, seq, ok); break;
+        case 48: mma_item_rp<48>(p, sh, v, q, lane, seq, ok); break;
+        case 56: mma_item_rp<56>(p, sh, v, q, lane, seq, ok); break;
+        default: mma_item_rp<64>(p, sh, v, q, lane, seq, ok); break;
       }
-      // the last MMAs finish before TMEM is released
-      if (seq > 0) (void)mbar_wait_bounded_for(&mma_bar[1], (uint32_t)((seq - 1) & 1), p.flag);
     }
+    // the last MMAs finish before TMEM is released
+    if (seq > 0) (void)mbar_wait_bounded_for(&mma_bar[q], (uint32_t)((seq - 1) & 1), p.flag);
   } else {
     // ------------------------------------------------------------ epilogue
     // warp w: TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31, share w / 4 of the

@@ -12,10 +12,11 @@
 //                  B[n=i][k=j] = P(t r)[i][j] in the tcgen05 K-major
 //                  core-matrix layout, and per tip branch the FP64-formed tip
 //                  rows tab[c][i] = sum_j P[i][j] code_tab[c][j];
-//   batch_tc_kernel  persistent, one CTA per SM, over work items
+//   batch_tc_kernel  persistent, two CTAs per SM, over work items
 //                  (variant, tile of 128 patterns).  A tile's conditional
 //                  likelihood vectors live in tensor memory (TMEM lane =
-//                  pattern, columns = states) and are the A operand of
+//                  pattern, columns = states; the few that a CTA's half of
+//                  TMEM has no room for, in global memory) and are the A operand of
 //                  tcgen05.mma.kind::tf32 for internal children; D (FP32) is
 //                  accumulated in TMEM.  Tip children need no MMA: their rows
 //                  come from the staged tip table.  Rate classes are separate
@@ -32,6 +33,13 @@
 //                  its D columns (tcgen05.ld) or tip rows, forms the product,
 //                  rescales, writes the parent's vector back into TMEM
 //                  (tcgen05.st).
+//   A step is a chain of latencies (MMAs about 1,100 cycles from one epilogue's
+//   stores to the next one's loads, epilogue 700) that left an SM with one
+//   codon chain or two protein chains two thirds idle.  Two CTAs per SM, each
+//   with half of TMEM, run twice the chains; a tree that needs more stack than
+//   its half spills a vector for the length of a subtree (13 of 127 steps on
+//   codon Yule trees of 128 taxa, 3 or 4 on protein ones).  32 models, 128
+//   taxa, 5,000 to 100,000 patterns: 9.8 ms against 15.9 with one CTA.
 //   The MMA (tcgen05.commit -> mma_bar) and the epilogue (an mbarrier,
 //   `stored`, after its TMEM stores) alternate per step, so a step's MMA
 //   never reads a vector before it is written and no mbarrier phase can be
@@ -57,18 +65,43 @@ using namespace pgpu_forms;
 namespace {
 
 constexpr int BT_M = 128;          // patterns per tile (TMEM lanes)
-constexpr int BT_ST = 4;           // ring slots (power of two)
+constexpr int BT_ST = 4;           // ring slots at most
 constexpr int BT_EPI_WARPS = 8;    // epilogue warps, two per TMEM lane group
 constexpr int BT_PARTS = BT_EPI_WARPS / 4;   // shares of a row (one per warp of a lane group)
 constexpr int BT_EPI = 32 * BT_EPI_WARPS;
 constexpr int BT_THREADS = BT_EPI + 96;   // + the producer warp and the two MMA warps
 constexpr int BT_PRODUCER = BT_EPI_WARPS, BT_MMA = BT_EPI_WARPS + 1;   // the first of each
-constexpr int BT_TMEM_COLS = 512;
+constexpr int BT_TMEM_COLS = 256;  // of a CTA: two share an SM
+constexpr int BT_LIMIT_COLS = 512; // what a tree's depth is held against
+
+// TMEM columns of a rate class's chain: SL stack slots of KP, then D of NP.
+// D of the second of two internal children goes to the free slot above them;
+// where it is wider than a slot its padding falls on columns that are free or
+// that the first child's MMAs, issued after it, write.
+template <int KP, int RP>
+struct Cols {
+  static constexpr int NP = (KP + 15) / 16 * 16;
+  static constexpr int CH = BT_TMEM_COLS / RP;
+  static constexpr int SL = (CH - NP) / KP < 15 ? (CH - NP) / KP : 15;
+  static constexpr int D = SL * KP;
+};
+int stack_slots(int Kp, int Np, int RP) { return std::min((BT_TMEM_COLS / RP - Np) / Kp, 15); }
+
+// a ring position and the parity of its barriers' current phase
+struct Ring {
+  int slot = 0;
+  uint32_t par = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++slot == n) {
+      slot = 0;
+      par ^= 1u;
+    }
+  }
+};
 
 struct BVar {
   int n_tips, n_ops, S, R, n_codes;
   int Kp, Np, SpT, NCp;            // padded K (A columns), N (D columns), odd tip-row stride, padded code rows
-  int n_slots;                     // TMEM stack slots available
   int RP;                          // rate classes per pass (1 or 2): their MMAs share a step
   int n_tiles;
   long long n_pat;
@@ -89,8 +122,13 @@ struct BVar {
   float probsf[4];                 // probs rounded to float (the root's join)
 };
 
-// op.x = internal index k, op.y = first child, op.z = second child,
-// op.w = slot_a | slot_b << 8 | slot_out << 16 (TMEM stack positions)
+// op.x = internal index k, op.y = first child, op.z = second child, op.w =
+// four-bit fields: the stack slots of child a, child b and the result, the
+// spill place + 1 that takes the result instead (0: none), the spill place + 1
+// to bring back after the step, the slot it goes to, and the slot that takes D
+// of child b when both children are internal
+__host__ __device__ inline int op_field(int w, int k) { return (w >> (4 * k)) & 15; }
+enum { OP_SA, OP_SB, OP_SO, OP_SPILL, OP_BACK, OP_BACK_SLOT, OP_DB };
 
 __device__ __forceinline__ uint32_t su32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -162,32 +200,28 @@ __device__ __forceinline__ void tmem_ld<16>(uint32_t ta, float *v) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// W consecutive TMEM columns of this thread's lane, each value rounded to
-// the nearest TF32 value (32x32b shape)
+// W consecutive TMEM columns of this thread's lane (32x32b shape)
 template <int W>
-__device__ __forceinline__ void tmem_st(uint32_t ta, const float *v);
+__device__ __forceinline__ void tmem_st(uint32_t ta, const uint32_t *v);
 template <>
-__device__ __forceinline__ void tmem_st<4>(uint32_t ta, const float *v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(ta), "r"(tf32_bits(v[0])),
-               "r"(tf32_bits(v[1])), "r"(tf32_bits(v[2])), "r"(tf32_bits(v[3]))
+__device__ __forceinline__ void tmem_st<4>(uint32_t ta, const uint32_t *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(ta), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3])
                : "memory");
 }
 template <>
-__device__ __forceinline__ void tmem_st<8>(uint32_t ta, const float *v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(ta),
-               "r"(tf32_bits(v[0])), "r"(tf32_bits(v[1])), "r"(tf32_bits(v[2])), "r"(tf32_bits(v[3])),
-               "r"(tf32_bits(v[4])), "r"(tf32_bits(v[5])), "r"(tf32_bits(v[6])), "r"(tf32_bits(v[7]))
+__device__ __forceinline__ void tmem_st<8>(uint32_t ta, const uint32_t *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(ta), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
 template <>
-__device__ __forceinline__ void tmem_st<16>(uint32_t ta, const float *v) {
+__device__ __forceinline__ void tmem_st<16>(uint32_t ta, const uint32_t *v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
           ta),
-      "r"(tf32_bits(v[0])), "r"(tf32_bits(v[1])), "r"(tf32_bits(v[2])), "r"(tf32_bits(v[3])), "r"(tf32_bits(v[4])),
-      "r"(tf32_bits(v[5])), "r"(tf32_bits(v[6])), "r"(tf32_bits(v[7])), "r"(tf32_bits(v[8])), "r"(tf32_bits(v[9])),
-      "r"(tf32_bits(v[10])), "r"(tf32_bits(v[11])), "r"(tf32_bits(v[12])), "r"(tf32_bits(v[13])),
-      "r"(tf32_bits(v[14])), "r"(tf32_bits(v[15]))
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
 
@@ -223,7 +257,11 @@ struct BatchArgs {
   double2 *partials;              // [n_work]
   int *flag;
   int slot_bytes;                 // ring slot size
+  int n_st;                       // ring slots
+  uint32_t *spill;                // [grid][n_spill][BT_SPILL_WORDS]
+  int n_spill;
 };
+constexpr int BT_SPILL_WORDS = 64 * BT_M;   // the classes of a pass together have at most 64 states
 
 // ring slot layout: [0,128) codes of child a, [128,256) codes of child b,
 // then block a and block b (each the larger of a B block and a tip block)
@@ -245,6 +283,7 @@ struct EpiIn {
   int lg;                    // TMEM lane group (its warps of one rate class share a named barrier)
   bool active, last;
   const float2 *pi2;         // the variant's stationary frequencies as float pairs
+  uint32_t *spill;           // this CTA's spill places, at this thread's lane
 };
 
 // The share of a row that epilogue warp w owns (PT = w / 4; the warps of a
@@ -267,11 +306,9 @@ struct Share {
 // One postorder step for this warp's share of the row: the product of the
 // two children (tip rows from the slot, or the MMA results from TMEM),
 // rescaled by a power of two agreed with the other shares of the same rate
-// class, written into the node's TMEM stack slot.  KP, RP and the share are
-// template parameters so that every state index and TMEM column is a
-// compile-time constant and the vectors stay in registers.  TMEM columns: D
-// of child h, rate q at (h*RP + q)*NP; stack slot s, rate q at
-// 2*RP*NP + (s*RP + q)*KP.
+// class, written into the node's TMEM stack slot (or to its spill place).
+// KP, RP and the share are template parameters so that every state index and
+// TMEM column is a compile-time constant and the vectors stay in registers.
 template <int KP, int RP, int PT>
 __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, const int4 op, int lane,
                                          int slot, uint64_t *empty, uint64_t *mma_bar, uint32_t mma_par,
@@ -279,8 +316,9 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
   using SH = Share<KP, RP, PT>;
   constexpr int B = SH::B, e0 = SH::e0, rate = SH::rate;
   constexpr int BA = B > 0 ? B : 1;
-  constexpr int NP = (KP + 15) / 16 * 16;
+  using C = Cols<KP, RP>;
   constexpr int SPT = KP | 1;
+  const uint32_t chain = in.tmem + in.lane_base + (uint32_t)(rate * C::CH + e0);   // slot 0, this share's columns
   float acc[BA];
 #pragma unroll
   for (int e = 0; e < BA; ++e) acc[e] = 1.0f;
@@ -313,24 +351,32 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
     // TMEM loads of W columns: the widest of 16, 8, 4 that divides both the
     // first column and the width of the share
     constexpr int W = (e0 % 16 == 0 && B % 16 == 0) ? 16 : (e0 % 8 == 0 && B % 8 == 0) ? 8 : 4;
-    auto product = [&](int h, float *d) {   // child h's D columns
+    auto load = [&](uint32_t col, int c0, int c1, float *d) {
 #pragma unroll
-      for (int c = 0; c < B; c += W)
-        tmem_ld<W>(in.tmem + in.lane_base + (uint32_t)((h * RP + rate) * NP + e0 + c), &d[c]);
+      for (int c = c0; c < c1; c += W) tmem_ld<W>(chain + col + (uint32_t)c, &d[c - c0]);
     };
-    float d[B];
-    if (ok && !tips[0] && !tips[1]) {
-      float d2[B];
-      product(0, d);
-      product(1, d2);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // 16 columns or so at a time: two CTAs of these warps share the registers
+    constexpr int CW = B <= 24 ? B : 16;
+    static_assert(CW % W == 0 && B % W == 0, "a load's columns stay within its part of the row");
+    auto times = [&](uint32_t col) {
 #pragma unroll
-      for (int e = 0; e < B; ++e) acc[e] = d[e] * d2[e];
-    } else if (ok && !(tips[0] && tips[1])) {
-      product(tips[0] ? 1 : 0, d);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      for (int c0 = 0; c0 < B; c0 += CW) {
+        constexpr int c_all = CW;
+        float d[c_all];
+        const int c1 = c0 + CW < B ? c0 + CW : B;
+        load(col, c0, c1, d);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int e = 0; e < B; ++e) acc[e] *= d[e];
+        for (int e = c0; e < c1; ++e) acc[e] *= d[e - c0];
+      }
+    };
+    if (ok && !(tips[0] && tips[1])) {
+      if (!tips[0] && !tips[1]) {
+        load(C::D, 0, B, acc);
+        times((uint32_t)(op_field(op.w, OP_DB) * KP));
+      } else {
+        times(C::D);
+      }
     }
   }
   __syncwarp();
@@ -380,12 +426,33 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
     for (int e = 0; e < BA; ++e) acc[e] = acc[e] * f1 * f2;
   }
   if constexpr (B > 0) {
-    // into the TMEM stack slot: columns e0 .. e0 + B - 1 of rate class rate
-    const int so = (op.w >> 16) & 0xff;
-    const uint32_t col = in.tmem + in.lane_base + (uint32_t)(2 * RP * NP + (so * RP + rate) * KP + e0);
     constexpr int WS = (e0 % 16 == 0 && B % 16 == 0) ? 16 : (e0 % 8 == 0 && B % 8 == 0) ? 8 : 4;
+    uint32_t *place = in.spill + (size_t)(rate * KP + e0) * BT_M;   // [state][lane] of spill place 0
+    if (const int sp = op_field(op.w, OP_SPILL)) {
+      uint32_t *to = place + (size_t)(sp - 1) * BT_SPILL_WORDS;
 #pragma unroll
-    for (int c0 = 0; c0 < B; c0 += WS) tmem_st<WS>(col + (uint32_t)c0, &acc[c0]);
+      for (int e = 0; e < B; ++e) to[e * BT_M] = tf32_bits(acc[e]);
+    } else {
+      const uint32_t col = chain + (uint32_t)(op_field(op.w, OP_SO) * KP);
+#pragma unroll
+      for (int c0 = 0; c0 < B; c0 += WS) {
+        uint32_t v[WS];
+#pragma unroll
+        for (int e = 0; e < WS; ++e) v[e] = tf32_bits(acc[c0 + e]);
+        tmem_st<WS>(col + (uint32_t)c0, v);
+      }
+    }
+    if (const int sp = op_field(op.w, OP_BACK)) {   // each thread its own values
+      const uint32_t *from = place + (size_t)(sp - 1) * BT_SPILL_WORDS;
+      const uint32_t col = chain + (uint32_t)(op_field(op.w, OP_BACK_SLOT) * KP);
+#pragma unroll
+      for (int c0 = 0; c0 < B; c0 += WS) {
+        uint32_t v[WS];
+#pragma unroll
+        for (int e = 0; e < WS; ++e) v[e] = __ldcg(from + (c0 + e) * BT_M);
+        tmem_st<WS>(col + (uint32_t)c0, v);
+      }
+    }
     if (in.last) {
       // sum_e pi_e x_e as a float pair: pi as (hi, lo), every product exact
       // with its cross term, the high parts added by an ordered Fast2Sum
@@ -431,7 +498,7 @@ struct EpiShared {
 // the per-pass barriers below are reached by every warp alike.
 template <int KP, int RP>
 __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int2 wk,
-                                         int tid, long long &seq, bool &ok) {
+                                         int tid, long long &seq, Ring &ring, bool &ok) {
   const int warp = tid >> 5, lane = tid & 31;
   const int lg = warp & 3, pt = warp >> 2;
   const int m = 32 * lg + lane;   // pattern within the tile
@@ -454,12 +521,13 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
   const long long pat = (long long)wk.y * BT_M + m;
   in.active = pat < vg.n_pat;
   in.pi2 = p.pis2 + vg.pi_off;
+  in.spill = p.spill + (size_t)blockIdx.x * p.n_spill * BT_SPILL_WORDS + m;
   ff Lp{0.0f, 0.0f};
   for (int r0 = 0; r0 < R && ok; r0 += RP) {
     int escale = 0;
-    for (int i = 0; i < n_ops; ++i, ++seq) {
-      const int slot = (int)(seq & (BT_ST - 1));
-      const uint32_t par = (uint32_t)((seq / BT_ST) & 1);
+    for (int i = 0; i < n_ops; ++i, ++seq, ring.next(p.n_st)) {
+      const int slot = ring.slot;
+      const uint32_t par = ring.par;
       in.sl = sh.smem + (size_t)slot * p.slot_bytes;
       bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
       got = __all_sync(0xffffffffu, got);
@@ -577,8 +645,9 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
 // classes took 1,200 cycles of a step's 1,650).
 template <int KP, int RP>
 __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
-                                         const int lane, long long &seq, bool &ok) {
-  constexpr int NP = (KP + 15) / 16 * 16;
+                                         const int lane, long long &seq, Ring &ring, bool &ok) {
+  using C = Cols<KP, RP>;
+  constexpr int NP = C::NP;
   constexpr uint32_t LBO = 128, SBO = (uint32_t)(KP / 4) * 128;
   constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NP >> 3) << 17) |
                              ((uint32_t)(BT_M >> 4) << 24);
@@ -593,9 +662,9 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
         : "memory");
   };
   for (int r0 = 0; r0 < R && ok; r0 += RP) {
-    for (int i = 0; i < n_ops; ++i, ++seq) {
-      const int slot = (int)(seq & (BT_ST - 1));
-      const uint32_t par = (uint32_t)((seq / BT_ST) & 1);
+    for (int i = 0; i < n_ops; ++i, ++seq, ring.next(p.n_st)) {
+      const int slot = ring.slot;
+      const uint32_t par = ring.par;
       bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
       // the epilogue warps of this class are done with the previous step
       if (seq > 0) got = got && mbar_wait_bounded_for(&sh.stored[q], (uint32_t)((seq - 1) & 1), p.flag);
@@ -609,13 +678,13 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
       if (issues && any) {
         const uint64_t slot_desc = desc0 + (uint32_t)slot * (uint32_t)(p.slot_bytes / 16);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const bool both = op.y >= n_tips && op.z >= n_tips;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 1; h >= 0; --h) {
           const int ch = h == 0 ? op.y : op.z;
           if (ch < n_tips) continue;
-          const int sa = (op.w >> (8 * h)) & 0xff;
-          const uint32_t d_col = (uint32_t)((h * RP + rq) * NP);
-          const uint32_t a_col = (uint32_t)(2 * RP * NP + (sa * RP + rq) * KP);
+          const uint32_t a_col = (uint32_t)(rq * C::CH + op_field(op.w, h == 0 ? OP_SA : OP_SB) * KP);
+          const uint32_t d_col = (uint32_t)(rq * C::CH + (both && h == 1 ? op_field(op.w, OP_DB) * KP : C::D));
           // the start address (16-byte units) is the descriptor's low field
           const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + rq) * BB16);
 #pragma unroll
@@ -645,29 +714,29 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
 
 template <int KP>
 __device__ __forceinline__ void mma_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
-                                            const int lane, long long &seq, bool &ok) {
+                                            const int lane, long long &seq, Ring &ring, bool &ok) {
   if constexpr (KP <= 32) {
     if (vg.RP == 2) {
-      mma_item<KP, 2>(p, sh, vg, q, lane, seq, ok);
+      mma_item<KP, 2>(p, sh, vg, q, lane, seq, ring, ok);
       return;
     }
   }
-  mma_item<KP, 1>(p, sh, vg, q, lane, seq, ok);
+  mma_item<KP, 1>(p, sh, vg, q, lane, seq, ring, ok);
 }
 
 template <int KP>
 __device__ __forceinline__ void epi_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg,
-                                            const int2 wk, int tid, long long &seq, bool &ok) {
+                                            const int2 wk, int tid, long long &seq, Ring &ring, bool &ok) {
   if constexpr (KP <= 32) {
     if (vg.RP == 2) {
-      epi_item<KP, 2>(p, sh, vg, wk, tid, seq, ok);
+      epi_item<KP, 2>(p, sh, vg, wk, tid, seq, ring, ok);
       return;
     }
   }
-  epi_item<KP, 1>(p, sh, vg, wk, tid, seq, ok);
+  epi_item<KP, 1>(p, sh, vg, wk, tid, seq, ring, ok);
 }
 
-__global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs p) {
+__global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t full[BT_ST], empty[BT_ST], mma_bar[2], stored[2];
   __shared__ int4 slot_op[BT_ST];
@@ -705,6 +774,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs
     // ------------------------------------------------------------ producer
     if (lane == 0) {
       long long seq = 0;
+      Ring ring;
       bool ok = true;
       for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
         const int2 wk = __ldg(p.work + w);
@@ -717,11 +787,10 @@ __global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs
         const uint8_t *codes = v.codes;
         const long long bstride = (long long)v.Np * v.Kp, tstride = (long long)v.NCp * v.SpT;
         for (int r0 = 0; r0 < R && ok; r0 += RP) {
-          for (int i = 0; i < n_ops; ++i, ++seq) {
-            const int slot = (int)(seq & (BT_ST - 1));
-            const long long round = seq / BT_ST;
+          for (int i = 0; i < n_ops; ++i, ++seq, ring.next(p.n_st)) {
+            const int slot = ring.slot;
             const int4 op = __ldg(p.ops + ops_off + i);
-            if (round > 0 && !mbar_wait_bounded_for(&empty[slot], (uint32_t)((round - 1) & 1), p.flag)) {
+            if (seq >= p.n_st && !mbar_wait_bounded_for(&empty[slot], ring.par ^ 1u, p.flag)) {
               ok = false;
               break;
             }
@@ -751,48 +820,51 @@ __global__ void __launch_bounds__(BT_THREADS, 1) batch_tc_kernel(const BatchArgs
           }
         }
       }
-      for (long long s = seq - BT_ST; s < seq; ++s)
-        if (s >= 0) (void)mbar_wait_bounded_for(&full[s & (BT_ST - 1)], (uint32_t)((s / BT_ST) & 1), p.flag);
+      // its last copies have arrived before it returns
+      for (int s = 0; s < p.n_st; ++s)
+        if (seq > s) (void)mbar_wait_bounded_for(&full[s], s < ring.slot ? ring.par : ring.par ^ 1u, p.flag);
     }
-  } else if (warp >= BT_MMA) {
+  } else if (warp == BT_MMA || warp == BT_MMA + 1) {
     // ------------------------------------------------------------ MMA issue
     const int q = warp - BT_MMA;
     long long seq = 0;
+    Ring ring;
     bool ok = true;
     for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
       const int2 wk = __ldg(p.work + w);
       const BVar &v = p.vars[wk.x];
       switch (v.Kp) {
-        case 8: mma_item_rp<8>(p, sh, v, q, lane, seq, ok); break;
-        case 16: mma_item_rp<16>(p, sh, v, q, lane, seq, ok); break;
-        case 24: mma_item_rp<24>(p, sh, v, q, lane, seq, ok); break;
-        case 32: mma_item_rp<32>(p, sh, v, q, lane, seq, ok); break;
-        case 40: mma_item_rp<40>(p, sh, v, q, lane, seq, ok); break;
-        case 48: mma_item_rp<48>(p, sh, v, q, lane, seq, ok); break;
-        case 56: mma_item_rp<56>(p, sh, v, q, lane, seq, ok); break;
-        default: mma_item_rp<64>(p, sh, v, q, lane, seq, ok); break;
+        case 8: mma_item_rp<8>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 16: mma_item_rp<16>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 24: mma_item_rp<24>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 32: mma_item_rp<32>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 40: mma_item_rp<40>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 48: mma_item_rp<48>(p, sh, v, q, lane, seq, ring, ok); break;
+        case 56: mma_item_rp<56>(p, sh, v, q, lane, seq, ring, ok); break;
+        default: mma_item_rp<64>(p, sh, v, q, lane, seq, ring, ok); break;
       }
     }
     // the last MMAs finish before TMEM is released
     if (seq > 0) (void)mbar_wait_bounded_for(&mma_bar[q], (uint32_t)((seq - 1) & 1), p.flag);
-  } else {
+  } else if (warp < BT_EPI_WARPS) {
     // ------------------------------------------------------------ epilogue
     // warp w: TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31, share w / 4 of the
     // row.
     long long seq = 0;
+    Ring ring;
     bool ok = true;
     for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
       const int2 wk = __ldg(p.work + w);
       const BVar &v = p.vars[wk.x];
       switch (v.Kp) {
-        case 8: epi_item_rp<8>(p, sh, v, wk, tid, seq, ok); break;
-        case 16: epi_item_rp<16>(p, sh, v, wk, tid, seq, ok); break;
-        case 24: epi_item_rp<24>(p, sh, v, wk, tid, seq, ok); break;
-        case 32: epi_item_rp<32>(p, sh, v, wk, tid, seq, ok); break;
-        case 40: epi_item_rp<40>(p, sh, v, wk, tid, seq, ok); break;
-        case 48: epi_item_rp<48>(p, sh, v, wk, tid, seq, ok); break;
-        case 56: epi_item_rp<56>(p, sh, v, wk, tid, seq, ok); break;
-        default: epi_item_rp<64>(p, sh, v, wk, tid, seq, ok); break;
+        case 8: epi_item_rp<8>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 16: epi_item_rp<16>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 24: epi_item_rp<24>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 32: epi_item_rp<32>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 40: epi_item_rp<40>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 48: epi_item_rp<48>(p, sh, v, wk, tid, seq, ring, ok); break;
+        case 56: epi_item_rp<56>(p, sh, v, wk, tid, seq, ring, ok); break;
+        default: epi_item_rp<64>(p, sh, v, wk, tid, seq, ring, ok); break;
       }
     }
   }
@@ -1031,6 +1103,62 @@ __global__ void __launch_bounds__(F64_NP) batch_fp64_kernel(const F64Args a) {
 // host side
 // ---------------------------------------------------------------------------
 
+namespace {
+
+// shared memory: what each of two CTAs on an SM may ask for beside the static
+// part, and that part
+constexpr size_t BT_SMEM_STATIC = 10 * 1024;
+constexpr size_t BT_SMEM_PAIR = (228 * 1024) / 2 - 1024 - BT_SMEM_STATIC;
+
+// Stack slots of a postorder schedule over `slots` slots, appended to ops;
+// returns the spill places used.  A step whose children are both internal
+// needs them in two slots and a third free; `need` is what a subtree takes
+// above its own base.  The first child's vector keeps its slot while the
+// second child's subtree is walked if that fits, else it is spilled and
+// brought back by the step that ends that subtree.
+int place_ops(const TreeSchedule &sch, int n, int slots, std::vector<int4> *ops) {
+  const size_t first = ops->size(), m = sch.ops.size();
+  std::vector<int> need(m), base(m, 0), place(m, 0), at(2 * n, -1);
+  for (size_t i = 0; i < m; ++i) {
+    const SchedOp &o = sch.ops[i];
+    at[n + o.k] = (int)i;
+    const int a = o.a >= n ? need[at[o.a]] : 0, b = o.b >= n ? need[at[o.b]] : 0;
+    need[i] = a && b ? std::min(std::max(std::max(a, 1 + b), 3), slots) : std::max(std::max(a, b), 1);
+    ops->push_back(make_int4(o.k, o.a, o.b, 0));
+  }
+  int used = 0;
+  for (size_t i = m; i-- > 0;) {
+    const SchedOp &o = sch.ops[i];
+    const int x = base[i], ia = o.a >= n ? at[o.a] : -1, ib = o.b >= n ? at[o.b] : -1;
+    int sa = x, sb = x, db = 0;
+    if (ia >= 0) {
+      base[ia] = x;
+      place[ia] = place[i];
+    }
+    if (ib >= 0) {
+      base[ib] = x;
+      place[ib] = place[i];
+    }
+    if (ia >= 0 && ib >= 0) {
+      db = x + 2;
+      if (x + 1 + need[ib] <= slots) {
+        base[ib] = sb = x + 1;
+      } else {
+        const int sp = place[i];
+        used = std::max(used, sp + 1);
+        place[ib] = sp + 1;
+        sa = x + 1;
+        (*ops)[first + ia].w |= (sp + 1) << (4 * OP_SPILL);
+        (*ops)[first + ib].w |= (sp + 1) << (4 * OP_BACK) | sa << (4 * OP_BACK_SLOT);
+      }
+    }
+    (*ops)[first + i].w |= sa << (4 * OP_SA) | sb << (4 * OP_SB) | x << (4 * OP_SO) | db << (4 * OP_DB);
+  }
+  return used;
+}
+
+}  // namespace
+
 struct pgpu_batch {
   int n_var = 0;
   int max_depth = 0;
@@ -1052,7 +1180,9 @@ struct pgpu_batch {
   int *n_tiles = nullptr;
   double2 *partials = nullptr;
   std::vector<long long> gQ, gL, gM;            // group bases (doubles, doubles, ints)
-  int slot_bytes = 0;
+  int slot_bytes = 0, n_st = BT_ST, grid = 1, n_spill = 0;
+  size_t lim_smem = 0;                          // what a run may ask for
+  uint32_t *spill = nullptr;
 };
 
 namespace {
@@ -1069,7 +1199,7 @@ pgpu_status upload(pgpu_ctx *ctx, T **dst, const std::vector<T> &src) {
 void free_batch(pgpu_batch *b) {
   void *ptrs[] = {b->vars, b->work,   b->ops, b->bmat,   b->tiptab,  b->pis,      b->brlen,
                   b->rates, b->ctab,  b->Q,   b->U,      b->Ui,      b->lam,      b->status,
-                  b->members, b->tile_base, b->n_tiles, b->partials, b->pis2, b->logtab};
+                  b->members, b->tile_base, b->n_tiles, b->partials, b->pis2, b->logtab, b->spill};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   delete b;
@@ -1101,7 +1231,7 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
   std::vector<long long> tile_base;
   std::vector<int> ntiles, members;
   long long bm_off = 0, tt_off = 0, pat_off = 0;
-  size_t max_blk = 0;
+  size_t max_blk = 0, lim_blk = 0;
   auto fail = [&](pgpu_status st, const char *msg, int v) {
     free_batch(b);
     return pgpu_set_err(ctx, st, "batch: variant %d: %s", v, msg);
@@ -1135,7 +1265,6 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     v.Np = (S + 15) / 16 * 16;
     v.SpT = v.Kp | 1;                     // odd row stride (distinct codes, distinct banks), entries S.. zero
     v.NCp = (x.codes.n_codes + 3) / 4 * 4; // rows padded so a block is a multiple of 16 bytes
-    v.n_slots = (BT_TMEM_COLS - 2 * v.Np) / v.Kp;
     v.n_tiles = (int)nt;
     v.n_pat = (long long)x.n_pat;
     v.ld = (long long)x.ld_pat;
@@ -1153,22 +1282,19 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
       v.probs[r] = r < R ? m.probs[r] : 0.0;
       v.probsf[r] = (float)v.probs[r];
     }
-    if (sch.max_depth > v.n_slots) return fail(PGPU_ERR_LIMIT, "tree too deep for the TMEM stack", vi);
-    // two rate classes per pass when their D columns and stacks fit in TMEM
-    v.RP = 1;
-    if (rate_pairs && R % 2 == 0 && v.Kp <= 32 &&
-        (BT_TMEM_COLS - 4 * v.Np) / (2 * v.Kp) >= sch.max_depth)
-      v.RP = 2;
+    if (sch.max_depth > (BT_LIMIT_COLS - 2 * v.Np) / v.Kp)
+      return fail(PGPU_ERR_LIMIT, "tree too deep for the TMEM stack", vi);
+    const size_t blk = (std::max<size_t>((size_t)v.Np * v.Kp * 4, (size_t)v.NCp * v.SpT * 4) + 127) & ~size_t(127);
+    // two rate classes per pass: their chains overlap, and two ring slots of
+    // both still let two CTAs share an SM
+    const bool pairs = rate_pairs && R % 2 == 0 && v.Kp <= 32;
+    v.RP = pairs && 2 * (256 + 4 * blk) <= BT_SMEM_PAIR ? 2 : 1;
+    // what the engine accepts is reckoned with one CTA per SM and its stack
+    const bool lim_pairs = pairs && (BT_LIMIT_COLS - 4 * v.Np) / (2 * v.Kp) >= sch.max_depth;
+    lim_blk = std::max(lim_blk, (lim_pairs ? 2 : 1) * blk);
+    max_blk = std::max(max_blk, v.RP * blk);
     b->max_depth = std::max(b->max_depth, sch.max_depth);
-    // TMEM stack positions from the stack simulation
-    int sp = 0;
-    for (const SchedOp &o : sch.ops) {
-      int sa = 0, sb = 0;
-      if (o.b >= n) sb = --sp;
-      if (o.a >= n) sa = --sp;
-      const int so = sp++;
-      ops.push_back(make_int4(o.k, o.a, o.b, sa | (sb << 8) | (so << 16)));
-    }
+    b->n_spill = std::max(b->n_spill, place_ops(sch, n, stack_slots(v.Kp, v.Np, v.RP), &ops));
     v.tile0 = (long long)work.size();
     for (long long t = 0; t < nt; ++t) work.push_back(make_int2(vi, (int)t));
     tile_base.push_back((long long)work.size() - nt);
@@ -1182,8 +1308,6 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     bm_off = (bm_off + 3) / 4 * 4;
     tt_off = (tt_off + 3) / 4 * 4;
     pat_off += v.n_pat;
-    const size_t blk = std::max<size_t>((size_t)v.Np * v.Kp * 4, (size_t)v.NCp * v.SpT * 4);
-    max_blk = std::max(max_blk, (size_t)v.RP * ((blk + 127) & ~size_t(127)));
     // eigen group by state count
     int g = -1;
     for (size_t k = 0; k < b->group_S.size(); ++k)
@@ -1215,12 +1339,18 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     q_acc += (long long)b->group_members[g].size() * S * S;
     l_acc += (long long)b->group_members[g].size() * S;
   }
+  b->slot_bytes = (int)(256 + 2 * max_blk);
+  b->lim_smem = std::max<size_t>(BT_ST * (256 + 2 * lim_blk), 120 * 1024);
+  // two CTAs per SM where two ring slots or more fit in half of its memory
+  const int per_sm = 2 * (size_t)b->slot_bytes <= BT_SMEM_PAIR ? 2 : 1;
+  b->n_st = (int)std::min<size_t>(BT_ST, (per_sm == 2 ? BT_SMEM_PAIR : ctx->smem_optin - BT_SMEM_STATIC) / b->slot_bytes);
+  b->grid = std::max(per_sm * ctx->num_sms, 1);
   if (order == PGPU_BATCH_ORDER_COST && !work.empty()) {
     // Largest items first, dealt back and forth over the persistent CTAs
     // (CTA c runs items c, c + G, c + 2G, ...), so every CTA's total is close
     // to the mean.  An item's cost is its postorder steps times the state
     // columns each step handles.
-    const long long G = std::min<long long>(ctx->num_sms, (long long)work.size());
+    const long long G = std::min<long long>(b->grid, (long long)work.size());
     std::vector<double> cost(work.size());
     for (size_t i = 0; i < work.size(); ++i) {
       const BVar &v = b->hvars[work[i].x];
@@ -1246,7 +1376,6 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
   }
   b->n_work = (long long)work.size();
   b->total_pat = pat_off;
-  b->slot_bytes = (int)(256 + 2 * max_blk);
   pgpu_status st = PGPU_OK;
   if (st == PGPU_OK) st = upload(ctx, &b->vars, b->hvars);
   if (st == PGPU_OK) st = upload(ctx, &b->work, work);
@@ -1275,6 +1404,7 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     PGPU_CUDA(ctx, cudaMalloc(p, std::max<size_t>(bytes, 16)));
     return PGPU_OK;
   };
+  if (st == PGPU_OK) st = alloc((void **)&b->spill, (size_t)b->grid * b->n_spill * BT_SPILL_WORDS * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->bmat, (size_t)bm_off * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->tiptab, (size_t)tt_off * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->U, (size_t)q_acc * 8);
@@ -1359,14 +1489,18 @@ pgpu_status pgpu_batch_run(pgpu_ctx *ctx, pgpu_batch *b, double *lnl_dev, double
   a.partials = b->partials;
   a.flag = ctx->d_flag;
   a.slot_bytes = b->slot_bytes;
-  // at least 120 KB, so that one CTA (which holds all 512 TMEM columns)
-  // occupies each SM
-  const size_t smem = std::max<size_t>((size_t)BT_ST * b->slot_bytes, 120 * 1024);
-  if (smem > ctx->smem_optin)
-    return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "batch: %zu bytes of shared memory needed", smem);
+  a.n_st = b->n_st;
+  a.spill = b->spill;
+  a.n_spill = b->n_spill;
+  if (b->lim_smem > ctx->smem_optin)
+    return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "batch: %zu bytes of shared memory needed", b->lim_smem);
+  // at least 72 KB, so that no third CTA waits on an SM for TMEM columns
+  const size_t smem = std::max<size_t>((size_t)b->n_st * b->slot_bytes, 72 * 1024);
   PGPU_CUDA(ctx, cudaFuncSetAttribute(batch_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)std::max<size_t>(smem, 48 * 1024)));
-  const long long grid = std::min<long long>(ctx->num_sms, b->n_work);
+  PGPU_CUDA(ctx, cudaFuncSetAttribute(batch_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      cudaSharedmemCarveoutMaxShared));
+  const long long grid = std::min<long long>(b->grid, b->n_work);
   batch_tc_kernel<<<(unsigned)std::max<long long>(grid, 1), BT_THREADS, smem, ctx->stream>>>(a);
   PGPU_TRY(pgpu_after_launch(ctx, "batch_tc_kernel"));
   batch_finalize_kernel<<<b->n_var, 256, 0, ctx->stream>>>(b->partials, b->tile_base,

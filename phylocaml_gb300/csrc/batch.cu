@@ -26,7 +26,7 @@
 //                  bulk-copies the B blocks of internal children, the
 //                  tip-table blocks and tip-code rows of tip children into a
 //                  shared ring slot, and publishes the step itself;
-//     warps 9, 10  MMA issue, one per rate class of the pass;
+//     warps 9, 10  MMA issue, one per rate class of the pass (9 alone with one);
 //     warps 0-7    epilogue: two warps per TMEM lane group of 32 patterns,
 //                  each owning a share of the row (half the states, or a
 //                  whole rate class when two share a pass); a thread reads
@@ -39,7 +39,7 @@
 //   with half of TMEM, run twice the chains; a tree that needs more stack than
 //   its half spills a vector for the length of a subtree (13 of 127 steps on
 //   codon Yule trees of 128 taxa, 3 or 4 on protein ones).  32 models, 128
-//   taxa, 5,000 to 100,000 patterns: 9.8 ms against 15.9 with one CTA.
+//   taxa, 5,000 to 100,000 patterns: 10.2 ms against 15.9 with one CTA.
 //   The MMA (tcgen05.commit -> mma_bar) and the epilogue (an mbarrier,
 //   `stored`, after its TMEM stores) alternate per step, so a step's MMA
 //   never reads a vector before it is written and no mbarrier phase can be
@@ -48,8 +48,11 @@
 //   epilogue warps: the MMAs of one class's next step run while the other
 //   class's epilogue runs, and no warp waits for another to agree on a
 //   rescaling exponent.
-//   Every wait is bounded.  Each work item runs a step loop compiled for its
-//   padded state count and rate classes per pass.
+//   Every wait is bounded.  A barrier's parity tells neighbouring phases apart
+//   only, so every warp that waits on one waits for each of its phases in turn.
+//   Work items of one padded state count and number of rate classes per pass
+//   are one launch of a kernel compiled for them; the launches are chained and
+//   overlap at their ends.
 //   batch_fp64_kernel  the FP64 comparison form on a sample of patterns.
 #include <algorithm>
 #include <cmath>
@@ -69,7 +72,7 @@ constexpr int BT_ST = 4;           // ring slots at most
 constexpr int BT_EPI_WARPS = 8;    // epilogue warps, two per TMEM lane group
 constexpr int BT_PARTS = BT_EPI_WARPS / 4;   // shares of a row (one per warp of a lane group)
 constexpr int BT_EPI = 32 * BT_EPI_WARPS;
-constexpr int BT_THREADS = BT_EPI + 96;   // + the producer warp and the two MMA warps
+constexpr int bt_threads(int RP) { return BT_EPI + 32 + 32 * RP; }   // + the producer warp and an MMA warp per class
 constexpr int BT_PRODUCER = BT_EPI_WARPS, BT_MMA = BT_EPI_WARPS + 1;   // the first of each
 constexpr int BT_TMEM_COLS = 256;  // of a CTA: two share an SM
 constexpr int BT_LIMIT_COLS = 512; // what a tree's depth is held against
@@ -87,15 +90,17 @@ struct Cols {
 };
 int stack_slots(int Kp, int Np, int RP) { return std::min((BT_TMEM_COLS / RP - Np) / Kp, 15); }
 
-// a ring position and the parity of its barriers' current phase
+// A ring position, the parity of its barriers' current phase, and that of the
+// barriers with a phase per step.
 struct Ring {
   int slot = 0;
-  uint32_t par = 0;
+  uint32_t par = 0, par_step = 0;
   __device__ __forceinline__ void next(int n) {
     if (++slot == n) {
       slot = 0;
       par ^= 1u;
     }
+    par_step ^= 1u;
   }
 };
 
@@ -132,11 +137,6 @@ enum { OP_SA, OP_SB, OP_SO, OP_SPILL, OP_BACK, OP_BACK_SLOT, OP_DB };
 
 __device__ __forceinline__ uint32_t su32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// mbarrier arrival of `n` threads by one
-__device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
-  asm volatile("mbarrier.arrive.shared.b64 _, [%0], %1;" ::"r"(su32(bar)), "r"(n) : "memory");
 }
 
 // K-major, no-swizzle shared-memory descriptor: 8-row x 16-byte core
@@ -265,7 +265,7 @@ constexpr int BT_SPILL_WORDS = 64 * BT_M;   // the classes of a pass together ha
 
 // ring slot layout: [0,128) codes of child a, [128,256) codes of child b,
 // then block a and block b (each the larger of a B block and a tip block)
-__device__ __forceinline__ int blk_bytes(const BVar &v) {
+__host__ __device__ inline int blk_bytes(const BVar &v) {
   const int b = v.Np * v.Kp * 4, t = v.NCp * v.SpT * 4;
   return ((b > t ? b : t) + 127) & ~127;
 }
@@ -275,70 +275,76 @@ __device__ __forceinline__ int blk_bytes(const BVar &v) {
 // count are template parameters of the step; these are the rest, read from
 // the variant once per work item.
 struct EpiIn {
-  const unsigned char *sl;   // the step's ring slot
+  uint32_t sl;               // the step's ring slot (shared-window address)
   int BB;                    // bytes of one child block in the slot
-  int n_tips, n_codes, S;
-  uint32_t tmem, lane_base;
-  int m;                     // pattern within the tile (TMEM lane)
-  int lg;                    // TMEM lane group (its warps of one rate class share a named barrier)
-  bool active, last;
-  const float2 *pi2;         // the variant's stationary frequencies as float pairs
-  uint32_t *spill;           // this CTA's spill places, at this thread's lane
+  int n_tips, n_codes;
+  uint32_t chain;            // TMEM: stack slot 0 of this warp's class, at its lanes and share
+  int m, n_live;             // pattern within the tile (TMEM lane), patterns of the tile
+  bool last;
 };
 
-// The share of a row that epilogue warp w owns (PT = w / 4; the warps of a
-// TMEM lane group own the BT_PARTS shares).  A rate class of the pass has
-// PPR = BT_PARTS / RP shares: share PT is rate class PT / PPR and the
-// (PT % PPR)-th range of WD states, WD = Kp / PPR rounded up to a multiple
-// of 4, so the last range of a small Kp may be short or empty.  Every range
-// starts on a multiple of 4 columns and is a multiple of 4 wide.  With two
-// shares per lane group and two rate classes per pass, a warp owns a whole
-// rate class's row and needs no exchange with another warp.
-template <int KP, int RP, int PT>
+__device__ __forceinline__ float lds_f32(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ int lds_u8(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+  return (int)v;
+}
+
+// The share of a row that epilogue warp w owns (pt = w / 4): with one rate
+// class per pass half of the states, with two the whole row of class pt, so
+// that it needs no exchange with another warp.  Both are B columns wide; which
+// of the two is a run-time offset, so that the warps run the same instructions
+// from cache (a copy of every step for each took 16.0 ms where one took 12.0).
+template <int KP, int RP>
 struct Share {
+  static_assert(BT_PARTS == 2, "two warps per lane group");
   static constexpr int PPR = BT_PARTS / RP;
-  static constexpr int WD = ((KP / PPR) + 3) & ~3;
-  static constexpr int rate = PT / PPR;
-  static constexpr int e0 = (PT % PPR) * WD;
-  static constexpr int B = KP - e0 <= 0 ? 0 : (KP - e0 < WD ? KP - e0 : WD);
+  static constexpr int B = KP / PPR;
 };
+
+// a code outside the table counts as code 0, reported for lanes of patterns
+__device__ __noinline__ int bad_code(int *flag, bool report) {
+  if (report) atomicOr(flag, PGPU_FLAG_BADCODE);
+  return 0;
+}
 
 // One postorder step for this warp's share of the row: the product of the
 // two children (tip rows from the slot, or the MMA results from TMEM),
 // rescaled by a power of two agreed with the other shares of the same rate
 // class, written into the node's TMEM stack slot (or to its spill place).
-// KP, RP and the share are template parameters so that every state index and
-// TMEM column is a compile-time constant and the vectors stay in registers.
-template <int KP, int RP, int PT>
-__device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, const int4 op, int lane,
+// KP and RP are template parameters so that every index into the vectors is a
+// compile-time constant and they stay in registers.
+template <int KP, int RP>
+__device__ __forceinline__ void epi_step(const BatchArgs &p, const BVar &vg, const EpiIn &in, const int4 op, int lane,
+                                         int pt,
                                          int slot, uint64_t *empty, uint64_t *mma_bar, uint32_t mma_par,
                                          float (*xch)[BT_M], int &escale, bool &ok, ff &Lp) {
-  using SH = Share<KP, RP, PT>;
-  constexpr int B = SH::B, e0 = SH::e0, rate = SH::rate;
-  constexpr int BA = B > 0 ? B : 1;
+  using SH = Share<KP, RP>;
+  constexpr int B = SH::B, PPR = SH::PPR;
+  const int rate = RP == 2 ? pt : 0, e0 = RP == 2 ? 0 : pt * B;
   using C = Cols<KP, RP>;
   constexpr int SPT = KP | 1;
-  const uint32_t chain = in.tmem + in.lane_base + (uint32_t)(rate * C::CH + e0);   // slot 0, this share's columns
-  float acc[BA];
+  const uint32_t chain = in.chain;
+  float acc[B];
 #pragma unroll
-  for (int e = 0; e < BA; ++e) acc[e] = 1.0f;
+  for (int e = 0; e < B; ++e) acc[e] = 1.0f;
   // states S .. KP-1 need no masks: the tip rows and the B blocks are zero
   // there, so every vector's padding is a product of zeros
   const bool tips[2] = {op.y < in.n_tips, op.z < in.n_tips};
   // the tip rows first, while the MMAs of the other child run
-  if constexpr (B > 0) {
+  {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (!ok || !tips[h]) continue;
-      int code = in.sl[h * 128 + in.m];
-      if (code >= in.n_codes) {
-        if (in.active && PT == 0) atomicOr(p.flag, PGPU_FLAG_BADCODE);
-        code = 0;
-      }
-      const float *row = reinterpret_cast<const float *>(in.sl + 256 + (size_t)(h * RP + rate) * in.BB) +
-                         code * SPT + e0;
+      int code = lds_u8(in.sl + (uint32_t)(h * 128 + in.m));
+      if (code >= in.n_codes) code = bad_code(p.flag, in.m < in.n_live && pt == 0);
+      const uint32_t row = in.sl + 256 + (uint32_t)((h * RP + rate) * in.BB + (code * SPT + e0) * 4);
 #pragma unroll
-      for (int e = 0; e < B; ++e) acc[e] *= row[e];
+      for (int e = 0; e < B; ++e) acc[e] *= lds_f32(row + 4 * e);
     }
   }
   {
@@ -347,10 +353,10 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
     ok = got;
   }
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if constexpr (B > 0) {
+  {
     // TMEM loads of W columns: the widest of 16, 8, 4 that divides both the
     // first column and the width of the share
-    constexpr int W = (e0 % 16 == 0 && B % 16 == 0) ? 16 : (e0 % 8 == 0 && B % 8 == 0) ? 8 : 4;
+    constexpr int W = B % 16 == 0 ? 16 : B % 8 == 0 ? 8 : 4;
     auto load = [&](uint32_t col, int c0, int c1, float *d) {
 #pragma unroll
       for (int c = c0; c < c1; c += W) tmem_ld<W>(chain + col + (uint32_t)c, &d[c - c0]);
@@ -383,21 +389,20 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
   if (lane == 0) mbar_arrive(&empty[slot]);
   // rescale by an exact power of two per rate class; the shares agree
   float mx = 0.0f;
-  if constexpr (B > 0) {
-    // pairwise maxima: a short dependency chain
-    float t[B];
+  {
+    // three-way maxima in four chains
+    float t[4] = {acc[0], acc[1], acc[2], acc[3]};
 #pragma unroll
-    for (int e = 0; e < B; ++e) t[e] = acc[e];
+    for (int e = 4; e + 7 < B; e += 8)
 #pragma unroll
-    for (int w = 1; w < B; w *= 2)
+      for (int k = 0; k < 4; ++k) t[k] = fmaxf(fmaxf(t[k], acc[e + 2 * k]), acc[e + 2 * k + 1]);
 #pragma unroll
-      for (int e = 0; e + w < B; e += 2 * w) t[e] = fmaxf(t[e], t[e + w]);
-    mx = t[0];
+    for (int e = 4 + (B - 4) / 8 * 8; e < B; ++e) t[e & 3] = fmaxf(t[e & 3], acc[e]);
+    mx = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
   }
-  constexpr int PPR = SH::PPR;
   float m2 = mx;
   if constexpr (PPR > 1) {
-    xch[PT][in.m] = mx;
+    xch[pt][in.m] = mx;
     // the exchange joins only the warps of this TMEM lane group that share
     // the rate class (named barrier 2 + lg + 4 rate); it also makes the
     // timeout verdict uniform over them, so they leave the step loop
@@ -407,11 +412,10 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
         "{\n\t.reg .pred a, b;\n\tsetp.ne.u32 a, %1, 0;\n\t"
         "bar.red.and.pred b, %2, %3, a;\n\tselp.u32 %0, 1, 0, b;\n\t}"
         : "=r"(all_ok)
-        : "r"((uint32_t)ok), "r"(2 + in.lg + 4 * rate), "n"(PPR * 32)
+        : "r"((uint32_t)ok), "r"(2 + (in.m >> 5) + 4 * rate), "n"(PPR * 32)
         : "memory");
     ok = all_ok != 0;
-#pragma unroll
-    for (int pp = rate * PPR; pp < rate * PPR + PPR; ++pp) m2 = fmaxf(m2, xch[pp][in.m]);
+    m2 = fmaxf(m2, xch[pt ^ 1][in.m]);
   } else {
     // this warp holds the whole row of its rate class
     ok = __all_sync(0xffffffffu, ok);
@@ -423,13 +427,16 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
     const int k1 = min(-ex, 120), k2 = -ex - k1;
     const float f1 = __int_as_float((127 + k1) << 23), f2 = __int_as_float((127 + k2) << 23);
 #pragma unroll
-    for (int e = 0; e < BA; ++e) acc[e] = acc[e] * f1 * f2;
+    for (int e = 0; e < B; ++e) acc[e] = acc[e] * f1 * f2;
   }
-  if constexpr (B > 0) {
-    constexpr int WS = (e0 % 16 == 0 && B % 16 == 0) ? 16 : (e0 % 8 == 0 && B % 8 == 0) ? 8 : 4;
-    uint32_t *place = in.spill + (size_t)(rate * KP + e0) * BT_M;   // [state][lane] of spill place 0
+  {
+    constexpr int WS = B % 16 == 0 ? 16 : B % 8 == 0 ? 8 : 4;
+    // spill place 0, [state][lane], at this thread's
+    auto place = [&]() {
+      return p.spill + (size_t)blockIdx.x * p.n_spill * BT_SPILL_WORDS + (size_t)(rate * KP + e0) * BT_M + in.m;
+    };
     if (const int sp = op_field(op.w, OP_SPILL)) {
-      uint32_t *to = place + (size_t)(sp - 1) * BT_SPILL_WORDS;
+      uint32_t *to = place() + (size_t)(sp - 1) * BT_SPILL_WORDS;
 #pragma unroll
       for (int e = 0; e < B; ++e) to[e * BT_M] = tf32_bits(acc[e]);
     } else {
@@ -443,7 +450,7 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
       }
     }
     if (const int sp = op_field(op.w, OP_BACK)) {   // each thread its own values
-      const uint32_t *from = place + (size_t)(sp - 1) * BT_SPILL_WORDS;
+      const uint32_t *from = place() + (size_t)(sp - 1) * BT_SPILL_WORDS;
       const uint32_t col = chain + (uint32_t)(op_field(op.w, OP_BACK_SLOT) * KP);
 #pragma unroll
       for (int c0 = 0; c0 < B; c0 += WS) {
@@ -458,10 +465,12 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
       // with its cross term, the high parts added by an ordered Fast2Sum
       // (the terms are non-negative), all low parts in one float
       float hs = 0.0f, lo = 0.0f;
+      const int S = vg.S;
+      const float2 *pi2 = p.pis2 + vg.pi_off + e0;
 #pragma unroll
       for (int e = 0; e < B; ++e)
-        if (e0 + e < in.S) {
-          const float2 pv = in.pi2[e0 + e];
+        if (e0 + e < S) {
+          const float2 pv = pi2[e];
           const float q = __fmul_rn(pv.x, acc[e]);
           float err = __fmaf_rn(pv.x, acc[e], -q);
           err = __fmaf_rn(pv.y, acc[e], err);
@@ -471,16 +480,14 @@ __device__ __forceinline__ void epi_step(const BatchArgs &p, const EpiIn &in, co
         }
       Lp = fast_two_sum(hs, lo);
     }
-  } else {
-    if (in.last) Lp = ff{0.0f, 0.0f};
   }
 }
 
 // Shared state of the epilogue warps.
 struct EpiShared {
   uint64_t *full, *empty;
-  uint64_t *mma_bar;         // [2]: for the first and second half of the shares; both complete once per step
-  uint64_t *stored;          // [2]: for the two MMA warps; likewise
+  uint64_t *mma_bar;         // [RP]: per rate class of the pass; a phase per step
+  uint64_t *stored;          // [RP]: the class's epilogue warps, likewise
   const int4 *slot_op;       // each ring slot's postorder step, written by the producer
   unsigned char *smem;
   float (*xch)[BT_M];        // [2][BT_PARTS]: per step parity and share, lane: max entry
@@ -498,13 +505,12 @@ struct EpiShared {
 // the per-pass barriers below are reached by every warp alike.
 template <int KP, int RP>
 __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int2 wk,
-                                         int tid, long long &seq, Ring &ring, bool &ok) {
+                                         int tid, Ring &ring, bool &ok) {
   const int warp = tid >> 5, lane = tid & 31;
   const int lg = warp & 3, pt = warp >> 2;
   const int m = 32 * lg + lane;   // pattern within the tile
   constexpr int PPR = BT_PARTS / RP;
   const int my_rate = pt / PPR;
-  const int half = pt / (BT_PARTS / 2);   // whose barriers the warp keeps step with
   // the share that combines its rate class's root likelihood
   const bool lead = pt % PPR == 0;
   // the variant's fields, once per item
@@ -513,22 +519,18 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
   in.BB = blk_bytes(vg);
   in.n_tips = vg.n_tips;
   in.n_codes = vg.n_codes;
-  in.S = vg.S;
-  in.tmem = sh.tmem;
-  in.lane_base = (uint32_t)(32 * lg) << 16;
+  in.chain = sh.tmem + ((uint32_t)(32 * lg) << 16) +
+             (uint32_t)(RP == 2 ? pt * Cols<KP, RP>::CH : pt * Share<KP, RP>::B);
   in.m = m;
-  in.lg = lg;
-  const long long pat = (long long)wk.y * BT_M + m;
-  in.active = pat < vg.n_pat;
-  in.pi2 = p.pis2 + vg.pi_off;
-  in.spill = p.spill + (size_t)blockIdx.x * p.n_spill * BT_SPILL_WORDS + m;
+  in.n_live = (int)min((long long)BT_M, vg.n_pat - (long long)wk.y * BT_M);
+  const uint32_t smem0 = su32(sh.smem);
   ff Lp{0.0f, 0.0f};
   for (int r0 = 0; r0 < R && ok; r0 += RP) {
     int escale = 0;
-    for (int i = 0; i < n_ops; ++i, ++seq, ring.next(p.n_st)) {
+    for (int i = 0; i < n_ops; ++i, ring.next(p.n_st)) {
       const int slot = ring.slot;
       const uint32_t par = ring.par;
-      in.sl = sh.smem + (size_t)slot * p.slot_bytes;
+      in.sl = smem0 + (uint32_t)(slot * p.slot_bytes);
       bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
       got = __all_sync(0xffffffffu, got);
       if (!got) {
@@ -536,31 +538,18 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
         atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
       }
       const int4 op = sh.slot_op[slot];
-      uint64_t *const mma_bar = &sh.mma_bar[half];
-      const uint32_t mma_par = (uint32_t)(seq & 1);
+      uint64_t *const mma_bar = &sh.mma_bar[my_rate];
+      const uint32_t mma_par = ring.par_step;
       in.last = i == n_ops - 1;
       // the max exchange is double-buffered by step parity: a group's next
       // write cannot meet a read of the previous step's values
-      float(*xch)[BT_M] = sh.xch + (seq & 1) * BT_PARTS;
-      // pt is warp-uniform
-      switch (pt) {
-        case 0: epi_step<KP, RP, 0>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
-        case 1: epi_step<KP, RP, 1>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
-        case 2: epi_step<KP, RP, 2>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
-        default: epi_step<KP, RP, 3>(p, in, op, lane, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp); break;
-      }
+      float(*xch)[BT_M] = sh.xch + ring.par_step * BT_PARTS;
+      epi_step<KP, RP>(p, vg, in, op, lane, pt, slot, sh.empty, mma_bar, mma_par, xch, escale, ok, Lp);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       // this warp's vectors of the step are in TMEM and its D columns read
       __syncwarp();
-      if (lane == 0) {
-        if (RP == 2) {
-          mbar_arrive_n(&sh.stored[half], 2);
-        } else {
-          mbar_arrive(&sh.stored[0]);
-          mbar_arrive(&sh.stored[1]);
-        }
-      }
+      if (lane == 0) mbar_arrive(&sh.stored[my_rate]);
       if (!ok) break;
     }
     // one verdict for every epilogue warp before the barriers below
@@ -592,7 +581,8 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
   // class's logarithm as a float pair plus the float logarithm of a sum in
   // [probs_min, 1]
   ff s{0.0f, 0.0f};
-  if (ok && in.active && pt == 0) {
+  const long long pat = (long long)wk.y * BT_M + m;
+  if (ok && pat < vg.n_pat && pt == 0) {
     ff mx = sh.lnr[0][m];
     for (int r = 1; r < R; ++r)
       if (sh.lnr[r][m].h > mx.h) mx = sh.lnr[r][m];
@@ -638,22 +628,19 @@ __device__ __forceinline__ void epi_item(const BatchArgs &p, const EpiShared &sh
 // step's tcgen05.mma for the internal children of rate class q.  They wait
 // until the epilogue warps that write and read the class's columns have
 // stored the previous step's vectors, and are committed to the class's
-// mma_bar and the slot's empty barrier.  With one rate class per pass warp 0
-// issues and commits for both, and warp 1 keeps step with the barriers.  The
+// mma_bar and the slot's empty barrier.  The
 // warp stays converged: the descriptors are uniform and the elected thread,
 // always the same, issues under a predicate (one thread issuing for both
 // classes took 1,200 cycles of a step's 1,650).
 template <int KP, int RP>
 __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
-                                         const int lane, long long &seq, Ring &ring, bool &ok) {
+                                         const int lane, bool &first, Ring &ring, bool &ok) {
   using C = Cols<KP, RP>;
   constexpr int NP = C::NP;
   constexpr uint32_t LBO = 128, SBO = (uint32_t)(KP / 4) * 128;
   constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NP >> 3) << 17) |
                              ((uint32_t)(BT_M >> 4) << 24);
   const int n_ops = vg.n_ops, R = vg.R, n_tips = vg.n_tips, BB16 = blk_bytes(vg) / 16;
-  const bool issues = RP == 2 || q == 0;
-  const int rq = RP == 2 ? q : 0;   // the class it issues for
   const uint64_t desc0 = smem_desc(sh.smem + 256, LBO, SBO);
   auto commit = [&](uint64_t *bar) {
     asm volatile(
@@ -662,12 +649,13 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
         : "memory");
   };
   for (int r0 = 0; r0 < R && ok; r0 += RP) {
-    for (int i = 0; i < n_ops; ++i, ++seq, ring.next(p.n_st)) {
+    for (int i = 0; i < n_ops; ++i, ring.next(p.n_st)) {
       const int slot = ring.slot;
       const uint32_t par = ring.par;
       bool got = mbar_wait_bounded_for(&sh.full[slot], par, p.flag);
       // the epilogue warps of this class are done with the previous step
-      if (seq > 0) got = got && mbar_wait_bounded_for(&sh.stored[q], (uint32_t)((seq - 1) & 1), p.flag);
+      if (!first) got = got && mbar_wait_bounded_for(&sh.stored[q], ring.par_step ^ 1u, p.flag);
+      first = false;
       if (!__all_sync(0xffffffffu, got)) {
         ok = false;
         atomicOr(p.flag, PGPU_FLAG_TIMEOUT);
@@ -675,7 +663,7 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
       }
       const int4 op = sh.slot_op[slot];
       const bool any = op.y >= n_tips || op.z >= n_tips;
-      if (issues && any) {
+      if (any) {
         const uint64_t slot_desc = desc0 + (uint32_t)slot * (uint32_t)(p.slot_bytes / 16);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const bool both = op.y >= n_tips && op.z >= n_tips;
@@ -683,10 +671,10 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
         for (int h = 1; h >= 0; --h) {
           const int ch = h == 0 ? op.y : op.z;
           if (ch < n_tips) continue;
-          const uint32_t a_col = (uint32_t)(rq * C::CH + op_field(op.w, h == 0 ? OP_SA : OP_SB) * KP);
-          const uint32_t d_col = (uint32_t)(rq * C::CH + (both && h == 1 ? op_field(op.w, OP_DB) * KP : C::D));
+          const uint32_t a_col = (uint32_t)(q * C::CH + op_field(op.w, h == 0 ? OP_SA : OP_SB) * KP);
+          const uint32_t d_col = (uint32_t)(q * C::CH + (both && h == 1 ? op_field(op.w, OP_DB) * KP : C::D));
           // the start address (16-byte units) is the descriptor's low field
-          const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + rq) * BB16);
+          const uint64_t bd0 = slot_desc + (uint32_t)((h * RP + q) * BB16);
 #pragma unroll
           for (int ks = 0; ks < KP / 8; ++ks) {
             const uint64_t bd = bd0 + (uint32_t)(ks * 2 * LBO / 16);
@@ -698,13 +686,9 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
           }
         }
         commit(&sh.mma_bar[q]);
-        if (RP == 1) commit(&sh.mma_bar[1]);
         commit(&sh.empty[slot]);
       } else if (lane == 0) {
-        if (issues) {
-          mbar_arrive(&sh.mma_bar[q]);
-          if (RP == 1) mbar_arrive(&sh.mma_bar[1]);
-        }
+        mbar_arrive(&sh.mma_bar[q]);
         mbar_arrive(&sh.empty[slot]);
       }
       __syncwarp();
@@ -712,33 +696,14 @@ __device__ __forceinline__ void mma_item(const BatchArgs &p, const EpiShared &sh
   }
 }
 
-template <int KP>
-__device__ __forceinline__ void mma_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg, const int q,
-                                            const int lane, long long &seq, Ring &ring, bool &ok) {
-  if constexpr (KP <= 32) {
-    if (vg.RP == 2) {
-      mma_item<KP, 2>(p, sh, vg, q, lane, seq, ring, ok);
-      return;
-    }
-  }
-  mma_item<KP, 1>(p, sh, vg, q, lane, seq, ring, ok);
-}
-
-template <int KP>
-__device__ __forceinline__ void epi_item_rp(const BatchArgs &p, const EpiShared &sh, const BVar &vg,
-                                            const int2 wk, int tid, long long &seq, Ring &ring, bool &ok) {
-  if constexpr (KP <= 32) {
-    if (vg.RP == 2) {
-      epi_item<KP, 2>(p, sh, vg, wk, tid, seq, ring, ok);
-      return;
-    }
-  }
-  epi_item<KP, 1>(p, sh, vg, wk, tid, seq, ring, ok);
-}
-
-__global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs p) {
+// One padded state count and number of rate classes per pass: a kernel of its
+// own for each holds its instructions in cache and its vectors in registers
+// (one kernel with a case for each took
+// 11.3 ms on 16 protein and 16 codon models, two of these 10.2).
+template <int KP, int RP>
+__global__ void __launch_bounds__(bt_threads(RP), 2) batch_tc_kernel(const BatchArgs p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ uint64_t full[BT_ST], empty[BT_ST], mma_bar[2], stored[2];
+  __shared__ uint64_t full[BT_ST], empty[BT_ST], mma_bar[RP], stored[RP];
   __shared__ int4 slot_op[BT_ST];
   __shared__ uint32_t tmem_base;
   __shared__ float xch[2 * BT_PARTS][BT_M];   // per step parity and share, lane: max entry
@@ -747,6 +712,8 @@ __global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs
   __shared__ double2 red[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  // the next kernel of the chain may take SMs as they come free
+  asm volatile("griddepcontrol.launch_dependents;");
   if (warp == BT_EPI_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      su32(&tmem_base)),
@@ -756,11 +723,11 @@ __global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs
   if (tid == 0) {
     for (int s = 0; s < BT_ST; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 2 + BT_EPI_WARPS);   // the MMA warps + the epilogue warps
+      mbar_init(&empty[s], RP + BT_EPI_WARPS);   // the MMA warps + the epilogue warps
     }
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < RP; ++q) {
       mbar_init(&mma_bar[q], 1);
-      mbar_init(&stored[q], BT_EPI_WARPS);   // after a step's TMEM stores
+      mbar_init(&stored[q], BT_EPI_WARPS / RP);   // after a step's TMEM stores
     }
     fence_mbarrier_init();
   }
@@ -782,7 +749,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs
         const int BB = blk_bytes(v);
         const uint32_t bmat_bytes = (uint32_t)(v.Np * v.Kp * 4);
         const uint32_t tip_bytes = (uint32_t)(v.NCp * v.SpT * 4);
-        const int RP = v.RP, R = v.R, n_ops = v.n_ops, n_tips = v.n_tips;
+        const int R = v.R, n_ops = v.n_ops, n_tips = v.n_tips;
         const long long ops_off = v.ops_off, ld = v.ld, tip_off = v.tip_off, bmat_off = v.bmat_off;
         const uint8_t *codes = v.codes;
         const long long bstride = (long long)v.Np * v.Kp, tstride = (long long)v.NCp * v.SpT;
@@ -824,48 +791,24 @@ __global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs
       for (int s = 0; s < p.n_st; ++s)
         if (seq > s) (void)mbar_wait_bounded_for(&full[s], s < ring.slot ? ring.par : ring.par ^ 1u, p.flag);
     }
-  } else if (warp == BT_MMA || warp == BT_MMA + 1) {
+  } else if (warp >= BT_MMA) {
     // ------------------------------------------------------------ MMA issue
     const int q = warp - BT_MMA;
-    long long seq = 0;
     Ring ring;
-    bool ok = true;
-    for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
-      const int2 wk = __ldg(p.work + w);
-      const BVar &v = p.vars[wk.x];
-      switch (v.Kp) {
-        case 8: mma_item_rp<8>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 16: mma_item_rp<16>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 24: mma_item_rp<24>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 32: mma_item_rp<32>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 40: mma_item_rp<40>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 48: mma_item_rp<48>(p, sh, v, q, lane, seq, ring, ok); break;
-        case 56: mma_item_rp<56>(p, sh, v, q, lane, seq, ring, ok); break;
-        default: mma_item_rp<64>(p, sh, v, q, lane, seq, ring, ok); break;
-      }
-    }
+    bool ok = true, first = true;
+    for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x)
+      mma_item<KP, RP>(p, sh, p.vars[__ldg(p.work + w).x], q, lane, first, ring, ok);
     // the last MMAs finish before TMEM is released
-    if (seq > 0) (void)mbar_wait_bounded_for(&mma_bar[q], (uint32_t)((seq - 1) & 1), p.flag);
-  } else if (warp < BT_EPI_WARPS) {
+    if (!first) (void)mbar_wait_bounded_for(&mma_bar[q], ring.par_step ^ 1u, p.flag);
+  } else {
     // ------------------------------------------------------------ epilogue
     // warp w: TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31, share w / 4 of the
     // row.
-    long long seq = 0;
     Ring ring;
     bool ok = true;
     for (long long w = blockIdx.x; w < p.n_work && ok; w += gridDim.x) {
       const int2 wk = __ldg(p.work + w);
-      const BVar &v = p.vars[wk.x];
-      switch (v.Kp) {
-        case 8: epi_item_rp<8>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 16: epi_item_rp<16>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 24: epi_item_rp<24>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 32: epi_item_rp<32>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 40: epi_item_rp<40>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 48: epi_item_rp<48>(p, sh, v, wk, tid, seq, ring, ok); break;
-        case 56: epi_item_rp<56>(p, sh, v, wk, tid, seq, ring, ok); break;
-        default: epi_item_rp<64>(p, sh, v, wk, tid, seq, ring, ok); break;
-      }
+      epi_item<KP, RP>(p, sh, p.vars[wk.x], wk, tid, ring, ok);
     }
   }
 
@@ -874,6 +817,8 @@ __global__ void __launch_bounds__(BT_THREADS, 2) batch_tc_kernel(const BatchArgs
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == BT_EPI_WARPS)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BT_TMEM_COLS));
+  // done only when the kernels before it in the chain are
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Per variant: sum its tiles' (sum, compensation) pairs in tile order.
@@ -1159,6 +1104,11 @@ int place_ops(const TreeSchedule &sch, int n, int slots, std::vector<int4> *ops)
 
 }  // namespace
 
+struct BatchLaunch {
+  int Kp, RP, slot_bytes, n_st, grid;
+  long long n_work, work0;
+};
+
 struct pgpu_batch {
   int n_var = 0;
   int max_depth = 0;
@@ -1180,7 +1130,8 @@ struct pgpu_batch {
   int *n_tiles = nullptr;
   double2 *partials = nullptr;
   std::vector<long long> gQ, gL, gM;            // group bases (doubles, doubles, ints)
-  int slot_bytes = 0, n_st = BT_ST, grid = 1, n_spill = 0;
+  std::vector<BatchLaunch> launches;
+  int n_spill = 0;
   size_t lim_smem = 0;                          // what a run may ask for
   uint32_t *spill = nullptr;
 };
@@ -1194,6 +1145,57 @@ pgpu_status upload(pgpu_ctx *ctx, T **dst, const std::vector<T> &src) {
   if (!src.empty())
     PGPU_CUDA(ctx, cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
   return PGPU_OK;
+}
+
+// words of spill places: the launches overlap at their ends, so each has its own
+size_t launch_spill(const pgpu_batch *b) {
+  size_t ctas = 0;
+  for (const BatchLaunch &l : b->launches) ctas += l.grid;
+  return ctas * b->n_spill * BT_SPILL_WORDS;
+}
+
+template <int KP, int RP>
+pgpu_status launch_tc(pgpu_ctx *ctx, const BatchArgs &a, const BatchLaunch &l, bool chained) {
+  auto kernel = batch_tc_kernel<KP, RP>;
+  // at least 72 KB, so that no third CTA waits on an SM for TMEM columns
+  const size_t smem = std::max<size_t>((size_t)l.n_st * l.slot_bytes, 72 * 1024);
+  PGPU_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // without it the driver may leave room for one CTA only
+  PGPU_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      cudaSharedmemCarveoutMaxShared));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)l.grid);
+  cfg.blockDim = dim3(bt_threads(RP));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = chained ? 1 : 0;
+  PGPU_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, a));
+  return pgpu_after_launch(ctx, "batch_tc_kernel");
+}
+
+pgpu_status launch_tc(pgpu_ctx *ctx, const BatchArgs &a, const BatchLaunch &l, bool chained) {
+  if (l.RP == 2) {
+    switch (l.Kp) {
+      case 8: return launch_tc<8, 2>(ctx, a, l, chained);
+      case 16: return launch_tc<16, 2>(ctx, a, l, chained);
+      case 24: return launch_tc<24, 2>(ctx, a, l, chained);
+      default: return launch_tc<32, 2>(ctx, a, l, chained);
+    }
+  }
+  switch (l.Kp) {
+    case 8: return launch_tc<8, 1>(ctx, a, l, chained);
+    case 16: return launch_tc<16, 1>(ctx, a, l, chained);
+    case 24: return launch_tc<24, 1>(ctx, a, l, chained);
+    case 32: return launch_tc<32, 1>(ctx, a, l, chained);
+    case 40: return launch_tc<40, 1>(ctx, a, l, chained);
+    case 48: return launch_tc<48, 1>(ctx, a, l, chained);
+    case 56: return launch_tc<56, 1>(ctx, a, l, chained);
+    default: return launch_tc<64, 1>(ctx, a, l, chained);
+  }
 }
 
 void free_batch(pgpu_batch *b) {
@@ -1231,7 +1233,7 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
   std::vector<long long> tile_base;
   std::vector<int> ntiles, members;
   long long bm_off = 0, tt_off = 0, pat_off = 0;
-  size_t max_blk = 0, lim_blk = 0;
+  size_t lim_blk = 0;
   auto fail = [&](pgpu_status st, const char *msg, int v) {
     free_batch(b);
     return pgpu_set_err(ctx, st, "batch: variant %d: %s", v, msg);
@@ -1292,7 +1294,6 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     // what the engine accepts is reckoned with one CTA per SM and its stack
     const bool lim_pairs = pairs && (BT_LIMIT_COLS - 4 * v.Np) / (2 * v.Kp) >= sch.max_depth;
     lim_blk = std::max(lim_blk, (lim_pairs ? 2 : 1) * blk);
-    max_blk = std::max(max_blk, v.RP * blk);
     b->max_depth = std::max(b->max_depth, sch.max_depth);
     b->n_spill = std::max(b->n_spill, place_ops(sch, n, stack_slots(v.Kp, v.Np, v.RP), &ops));
     v.tile0 = (long long)work.size();
@@ -1339,41 +1340,63 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     q_acc += (long long)b->group_members[g].size() * S * S;
     l_acc += (long long)b->group_members[g].size() * S;
   }
-  b->slot_bytes = (int)(256 + 2 * max_blk);
   b->lim_smem = std::max<size_t>(BT_ST * (256 + 2 * lim_blk), 120 * 1024);
-  // two CTAs per SM where two ring slots or more fit in half of its memory
-  const int per_sm = 2 * (size_t)b->slot_bytes <= BT_SMEM_PAIR ? 2 : 1;
-  b->n_st = (int)std::min<size_t>(BT_ST, (per_sm == 2 ? BT_SMEM_PAIR : ctx->smem_optin - BT_SMEM_STATIC) / b->slot_bytes);
-  b->grid = std::max(per_sm * ctx->num_sms, 1);
-  if (order == PGPU_BATCH_ORDER_COST && !work.empty()) {
-    // Largest items first, dealt back and forth over the persistent CTAs
-    // (CTA c runs items c, c + G, c + 2G, ...), so every CTA's total is close
-    // to the mean.  An item's cost is its postorder steps times the state
-    // columns each step handles.
-    const long long G = std::min<long long>(b->grid, (long long)work.size());
-    std::vector<double> cost(work.size());
-    for (size_t i = 0; i < work.size(); ++i) {
-      const BVar &v = b->hvars[work[i].x];
-      cost[i] = (double)(v.R / v.RP) * v.n_ops * (v.RP * v.Kp + 16.0);
-    }
-    std::vector<size_t> idx(work.size());
-    for (size_t i = 0; i < idx.size(); ++i) idx[i] = i;
-    std::stable_sort(idx.begin(), idx.end(), [&](size_t a, size_t c) { return cost[a] > cost[c]; });
-    std::vector<std::vector<int2>> per(G);
-    for (size_t r = 0; r < idx.size(); ++r) {
-      const long long round = (long long)r / G, pos = (long long)r % G;
-      per[round % 2 == 0 ? pos : G - 1 - pos].push_back(work[idx[r]]);
-    }
-    // CTA c's k-th item goes to position k G + c; the last, partial round
-    // is packed to the front of its row
-    std::vector<int2> compact;
-    compact.reserve(work.size());
-    const size_t rounds = (work.size() + G - 1) / G;
-    for (size_t k = 0; k < rounds; ++k)
-      for (long long c = 0; c < G; ++c)
-        if (k < per[c].size()) compact.push_back(per[c][k]);
-    work.swap(compact);
+  // A launch per padded state count and rate classes per pass, those with the
+  // longest items first; its ring takes what its variants need, two CTAs per SM
+  // where two slots or more fit in half of the shared memory.
+  std::vector<BatchLaunch> launches;
+  for (const BVar &v : b->hvars) {
+    const int slot_bytes = 256 + 2 * v.RP * blk_bytes(v);
+    auto it = std::find_if(launches.begin(), launches.end(),
+                           [&](const BatchLaunch &l) { return l.Kp == v.Kp && l.RP == v.RP; });
+    if (it == launches.end()) it = launches.insert(it, BatchLaunch{v.Kp, v.RP, 0, BT_ST, 1, 0, 0});
+    it->slot_bytes = std::max(it->slot_bytes, slot_bytes);
   }
+  std::stable_sort(launches.begin(), launches.end(), [](const BatchLaunch &x, const BatchLaunch &y) {
+    return x.RP * x.Kp > y.RP * y.Kp;
+  });
+  std::vector<int2> all;
+  all.swap(work);
+  work.reserve(all.size());
+  for (BatchLaunch &l : launches) {
+    l.work0 = (long long)work.size();
+    const int per_sm = 2 * (size_t)l.slot_bytes <= BT_SMEM_PAIR ? 2 : 1;
+    l.n_st = (int)std::min<size_t>(BT_ST, (per_sm == 2 ? BT_SMEM_PAIR : ctx->smem_optin - BT_SMEM_STATIC) / l.slot_bytes);
+    std::vector<int2> mine;
+    for (const int2 &w : all) {
+      const BVar &v = b->hvars[w.x];
+      if (v.Kp == l.Kp && v.RP == l.RP) mine.push_back(w);
+    }
+    l.n_work = (long long)mine.size();
+    l.grid = (int)std::min<long long>(std::max(per_sm * ctx->num_sms, 1), std::max<long long>(l.n_work, 1));
+    if (order == PGPU_BATCH_ORDER_COST && !mine.empty()) {
+      // Largest items first, dealt back and forth over the persistent CTAs
+      // (CTA c runs items c, c + G, c + 2G, ...), so every CTA's total is close
+      // to the mean.  An item's cost is its postorder steps times its passes.
+      const long long G = l.grid;
+      std::vector<size_t> idx(mine.size());
+      for (size_t i = 0; i < idx.size(); ++i) idx[i] = i;
+      auto cost = [&](size_t i) {
+        const BVar &v = b->hvars[mine[i].x];
+        return (long long)(v.R / v.RP) * v.n_ops;
+      };
+      std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return cost(x) > cost(y); });
+      std::vector<std::vector<int2>> per(G);
+      for (size_t r = 0; r < idx.size(); ++r) {
+        const long long round = (long long)r / G, pos = (long long)r % G;
+        per[round % 2 == 0 ? pos : G - 1 - pos].push_back(mine[idx[r]]);
+      }
+      // CTA c's k-th item goes to position k G + c; the last, partial round
+      // is packed to the front of its row
+      mine.clear();
+      const size_t rounds = (idx.size() + G - 1) / G;
+      for (size_t k = 0; k < rounds; ++k)
+        for (long long c = 0; c < G; ++c)
+          if (k < per[c].size()) mine.push_back(per[c][k]);
+    }
+    work.insert(work.end(), mine.begin(), mine.end());
+  }
+  b->launches = launches;
   b->n_work = (long long)work.size();
   b->total_pat = pat_off;
   pgpu_status st = PGPU_OK;
@@ -1404,7 +1427,7 @@ pgpu_status pgpu_batch_create_opts(pgpu_ctx *ctx, const pgpu_variant *vs, int n_
     PGPU_CUDA(ctx, cudaMalloc(p, std::max<size_t>(bytes, 16)));
     return PGPU_OK;
   };
-  if (st == PGPU_OK) st = alloc((void **)&b->spill, (size_t)b->grid * b->n_spill * BT_SPILL_WORDS * 4);
+  if (st == PGPU_OK) st = alloc((void **)&b->spill, launch_spill(b) * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->bmat, (size_t)bm_off * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->tiptab, (size_t)tt_off * 4);
   if (st == PGPU_OK) st = alloc((void **)&b->U, (size_t)q_acc * 8);
@@ -1477,8 +1500,6 @@ pgpu_status pgpu_batch_run(pgpu_ctx *ctx, pgpu_batch *b, double *lnl_dev, double
   }
   BatchArgs a;
   a.vars = b->vars;
-  a.work = b->work;
-  a.n_work = b->n_work;
   a.ops = b->ops;
   a.bmat = b->bmat;
   a.tiptab = b->tiptab;
@@ -1488,21 +1509,22 @@ pgpu_status pgpu_batch_run(pgpu_ctx *ctx, pgpu_batch *b, double *lnl_dev, double
   a.site_lnl = site_lnl_dev;
   a.partials = b->partials;
   a.flag = ctx->d_flag;
-  a.slot_bytes = b->slot_bytes;
-  a.n_st = b->n_st;
-  a.spill = b->spill;
   a.n_spill = b->n_spill;
   if (b->lim_smem > ctx->smem_optin)
     return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "batch: %zu bytes of shared memory needed", b->lim_smem);
-  // at least 72 KB, so that no third CTA waits on an SM for TMEM columns
-  const size_t smem = std::max<size_t>((size_t)b->n_st * b->slot_bytes, 72 * 1024);
-  PGPU_CUDA(ctx, cudaFuncSetAttribute(batch_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)std::max<size_t>(smem, 48 * 1024)));
-  PGPU_CUDA(ctx, cudaFuncSetAttribute(batch_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      cudaSharedmemCarveoutMaxShared));
-  const long long grid = std::min<long long>(b->grid, b->n_work);
-  batch_tc_kernel<<<(unsigned)std::max<long long>(grid, 1), BT_THREADS, smem, ctx->stream>>>(a);
-  PGPU_TRY(pgpu_after_launch(ctx, "batch_tc_kernel"));
+  // independent of one another: each after the first starts on the SMs that the
+  // one before leaves
+  uint32_t *spill = b->spill;
+  for (size_t k = 0; k < b->launches.size(); ++k) {
+    const BatchLaunch &l = b->launches[k];
+    a.work = b->work + l.work0;
+    a.n_work = l.n_work;
+    a.slot_bytes = l.slot_bytes;
+    a.n_st = l.n_st;
+    a.spill = spill;
+    spill += (size_t)l.grid * b->n_spill * BT_SPILL_WORDS;
+    PGPU_TRY(launch_tc(ctx, a, l, k > 0));
+  }
   batch_finalize_kernel<<<b->n_var, 256, 0, ctx->stream>>>(b->partials, b->tile_base,
                                                                         b->n_tiles, b->n_var, lnl_dev);
   return pgpu_after_launch(ctx, "batch_finalize_kernel");

@@ -29,8 +29,8 @@
 // float pairs per warp, per CTA in warp order, then per move over the CTA
 // groups in FP64 (spr_reduce_kernel), which fixes the summation order.
 //
-// The Fitch part (spr_fitch_*_kernel) runs the same programs on packed
-// 4-bit state sets: the parsimony length of every neighbour, exactly.
+// The Fitch part (spr_fitch_*_kernel) runs the same programs on state sets
+// (32 patterns to a word, a word per state): the parsimony length of every neighbour, exactly.
 //
 // TBR moves that reroot both sides of a cut edge (a,b): the scan program of
 // the prune carrying b's side away walks a's side, and in emit mode stores
@@ -106,6 +106,28 @@ __device__ __forceinline__ void copy16(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
+
+// A sum of floats and of products of floats to about 70 bits: three words, each
+// the rounding errors of the one before.
+struct Sum3 {
+  float a = 0.0f, b = 0.0f, c = 0.0f;
+  __device__ __forceinline__ void add_low(float x) {
+    const ff t = two_sum(b, x);
+    b = t.h;
+    c = __fadd_rn(c, t.l);
+  }
+  __device__ __forceinline__ void add(float x) {
+    const ff t = two_sum(a, x);
+    a = t.h;
+    add_low(t.l);
+  }
+  __device__ __forceinline__ void add_product(float x, float y) {
+    const float p = __fmul_rn(x, y);
+    add(p);
+    add_low(__fmaf_rn(x, y, -p));
+  }
+  __device__ __forceinline__ double value() const { return (double)a + ((double)b + (double)c); }
+};
 
 struct PoolArgs {
   void *L, *M, *H;
@@ -313,9 +335,10 @@ struct ScanArgs {
   const SprStep *steps;
   const SprPrune *prunes;
   const double *pi, *probs;
+  const float2 *pairs;        // pi [4] and probs [8] as float pairs
   const float2 *wts;          // [np] float pairs, zero beyond n_pat
   const float4 *logtab;       // 64 entries
-  double *partials;           // [n_groups][n_moves]
+  float2 *partials;           // [n_groups][n_moves] float pairs
   int *flag;
   size_t np, n_moves;
   int R, NP, G, n_blocks, depth;
@@ -391,7 +414,7 @@ __device__ __forceinline__ typename Pol::V site_part(const typename Pol::V *h, c
 // first move's sum and the odd ones with the second's, and one logarithm and
 // one sum over the patterns serve both.  The warps' values meet every
 // SCAN_WIN moves.  128 taxa x 16,852 patterns, pair form, 63,000 moves:
-// 72.2 ms against 141.8 with none of this.
+// 71.8 ms against 141.8 with none of this.
 template <typename Pol, int RT, bool EMIT = false>
 __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
   using V = typename Pol::V;
@@ -409,7 +432,17 @@ __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
   const int R = a.R;
   for (int i = c; i < 64; i += NT) ltab[i] = a.logtab[i];
   __syncthreads();
-  const V prob = Pol::from_d(on ? a.probs[r] : 0.0);
+  // the pair form takes these ready: converting them from FP64 in every thread
+  // cost 0.4 ms of the 63,000 moves' 72.2
+  auto constant = [&](int k, const double *d) {
+    if constexpr (std::is_same<Pol, Ff32>::value) {
+      const float2 v = __ldg(a.pairs + k);
+      return ff{v.x, v.y};
+    } else {
+      return Pol::from_d(*d);
+    }
+  };
+  const V prob = on ? constant(4 + r, a.probs + r) : Pol::zero();
   const Coef *Dm = static_cast<const Coef *>(a.Dmer) + ((size_t)(a.prune_base + blockIdx.x) * R + (on ? r : 0)) * 16;
   // blocks of a step's two edges into buffer buf
   auto blocks = [&](int buf, const SprStep &st) {
@@ -431,9 +464,9 @@ __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
     if (c < to - base) {
       ff s = red[c];
       for (int w = 1; w < SPR_NW; ++w) s = ff_add(s, red[w * SCAN_WIN + c]);
-      double *dst = a.partials + (size_t)blockIdx.y * a.n_moves + pr.move_off + base + c;
-      const double v = (double)s.h + (double)s.l;
-      *dst = first ? v : *dst + v;
+      float2 *dst = a.partials + (size_t)blockIdx.y * a.n_moves + pr.move_off + base + c;
+      if (!first) s = ff_add(ff{dst->x, dst->y}, s);
+      *dst = make_float2(s.h, s.l);
     }
     __syncthreads();
     base = to;
@@ -460,7 +493,7 @@ __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
       Pol::load_g(a.M, vi(pr.dp), vp);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        vp[e] = Pol::mul(vp[e], Pol::from_d(a.pi[e]));
+        vp[e] = Pol::mul(vp[e], constant(e, a.pi + e));
         if constexpr (std::is_same<Pol, Ff32>::value) vp[e] = Pol::mul(vp[e], prob);
       }
     }
@@ -640,33 +673,34 @@ __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
 
 // lnl[m] = sum over CTA groups of the partial sums: slice y of a move's groups
 // by thread (move, y), the slices in order.  A chain over all the groups kept
-// a few moves of 714 groups waiting 210 us; 56 us in 32 slices.
+// a few moves of 714 groups waiting 210 us; 56 us in 32 slices.  Sums in three
+// floats: in FP64 the 33 million partials of 63,000 moves took 0.48 ms, 0.055
+// now.
 constexpr int RED_Y = 32;
-__global__ void __launch_bounds__(32 * RED_Y) spr_reduce_kernel(const double *partials, int n_groups, size_t n_moves,
+__global__ void __launch_bounds__(32 * RED_Y) spr_reduce_kernel(const float2 *partials, int n_groups, size_t n_moves,
                                                                 double *lnl) {
-  __shared__ double2 part[RED_Y][33];
+  __shared__ float part[3][RED_Y][33];
   const int x = threadIdx.x, y = threadIdx.y;
   const size_t m = (size_t)blockIdx.x * 32 + x;
   const int per = (n_groups + RED_Y - 1) / RED_Y, g0 = y * per, g1 = min(g0 + per, n_groups);
-  double s = 0.0, c = 0.0;
+  Sum3 s;
   if (m < n_moves)
     for (int g = g0; g < g1; ++g) {
-      double t, e;
-      two_sum(s, partials[(size_t)g * n_moves + m], t, e);
-      s = t;
-      c += e;
+      const float2 v = partials[(size_t)g * n_moves + m];
+      s.add(v.x);
+      s.add_low(v.y);
     }
-  part[y][x] = make_double2(s, c);
+  part[0][y][x] = s.a;
+  part[1][y][x] = s.b;
+  part[2][y][x] = s.c;
   __syncthreads();
   if (y != 0 || m >= n_moves) return;
   for (int k = 1; k < RED_Y; ++k) {
-    const double2 v = part[k][x];
-    double t, e;
-    two_sum(s, v.x, t, e);
-    s = t;
-    c += e + v.y;
+    s.add(part[0][k][x]);
+    s.add_low(part[1][k][x]);
+    s.c = __fadd_rn(s.c, part[2][k][x]);
   }
-  lnl[m] = s + c;
+  lnl[m] = s.value();
 }
 
 // ---------------------------------------------------------------------------
@@ -695,7 +729,7 @@ struct PairArgs {
   const TbrCutDev *cuts;
   const float2 *wts;        // [np] float pairs, zero beyond n_pat
   const float4 *logtab;
-  double *partials;         // [n_groups][n_moves]
+  float2 *partials;         // [n_groups][n_moves] float pairs
   int *flag;
   size_t np;
   long long n_moves;
@@ -800,7 +834,7 @@ __global__ void __launch_bounds__(256) tbr_pair_kernel(const PairArgs a) {
   }
   if (mine)
     a.partials[(size_t)blockIdx.y * a.n_moves + cut.move_off + (long long)j * cut.nB + k] =
-        (double)sum.h + (double)sum.l;
+        make_float2(sum.h, sum.l);
 }
 
 // ---------------------------------------------------------------------------
@@ -1335,28 +1369,6 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
   reinterpret_cast<float4 *>(a.S)[(size_t)e * a.np * a.R + i] = make_float4(s[0], s[1], s[2], s[3]);
 }
 
-// A sum of floats and of products of floats to about 70 bits: three words, each
-// the rounding errors of the one before.
-struct Sum3 {
-  float a = 0.0f, b = 0.0f, c = 0.0f;
-  __device__ __forceinline__ void add_low(float x) {
-    const ff t = two_sum(b, x);
-    b = t.h;
-    c = __fadd_rn(c, t.l);
-  }
-  __device__ __forceinline__ void add(float x) {
-    const ff t = two_sum(a, x);
-    a = t.h;
-    add_low(t.l);
-  }
-  __device__ __forceinline__ void add_product(float x, float y) {
-    const float p = __fmul_rn(x, y);
-    add(p);
-    add_low(__fmaf_rn(x, y, -p));
-  }
-  __device__ __forceinline__ double value() const { return (double)a + ((double)b + (double)c); }
-};
-
 // One CTA per edge: Newton iterations on t with the derivatives of
 // sum_s w_s log f_s(t) summed over all patterns.  An iteration reads the
 // edge's S once and should take no longer than that; FP64 runs at 1/64 of the
@@ -1480,7 +1492,8 @@ struct pgpu_spr {
   int *status = nullptr;
   uint8_t *cmask = nullptr;
   double *w = nullptr;
-  float2 *w2 = nullptr;   // weights as float pairs
+  float2 *w2 = nullptr;      // weights as float pairs
+  float2 *pairs = nullptr;   // pi [4] and probs [8] as float pairs
   float4 *logtab = nullptr;
   // pool
   void *L = nullptr, *M = nullptr, *H = nullptr;
@@ -1496,7 +1509,7 @@ struct pgpu_spr {
   unsigned long long *cntF = nullptr, *lenF = nullptr, *ins = nullptr, *join = nullptr;
   float *summ = nullptr;
   // scratch
-  double *partials = nullptr;
+  float2 *partials = nullptr;
   size_t part_cap = 0;
   float *S = nullptr;
   // host state
@@ -1753,6 +1766,7 @@ pgpu_status launch_scan_rt(pgpu_spr *s, const SprPlan &p, const SprPlanDev &d, i
   a.prunes = d.prunes;
   a.pi = s->pi;
   a.probs = s->probs;
+  a.pairs = s->pairs;
   a.wts = s->w2;
   a.logtab = s->logtab;
   a.partials = s->partials;
@@ -1876,6 +1890,7 @@ pgpu_status launch_emit_rt(pgpu_spr *s, int prune_base, int n_prunes, long long 
   a.prunes = s->tbr_d.prunes;
   a.pi = s->pi;
   a.probs = s->probs;
+  a.pairs = s->pairs;
   a.wts = s->w2;
   a.logtab = s->logtab;
   a.partials = nullptr;
@@ -2170,6 +2185,13 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
   std::copy(codes->table, codes->table + (size_t)nc * 4, hb.begin() + 36);
   SPR_TRY(upload(s, blk, hb.data(), hb.size()));
   SPR_TRY(pgpu_launch_eig(ctx, s->Q, s->pi, 4, 1, s->U, s->lam, s->Ui, s->status));
+  std::vector<float2> ph(12, make_float2(0.0f, 0.0f));
+  for (int i = 0; i < 4 + R; ++i) {
+    const double v = i < 4 ? m->pi[i] : m->probs[i - 4];
+    ph[i] = make_float2((float)v, (float)(v - (double)(float)v));
+  }
+  SPR_TRY(dalloc_t(s, ph.size(), &s->pairs));
+  SPR_TRY(upload(s, s->pairs, ph.data(), ph.size()));
   // the code table in the form's layout (store4)
   std::vector<double> cr((size_t)nc * 4);   // room for the widest form
   for (int c = 0; c < nc; ++c)

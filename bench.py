@@ -501,11 +501,11 @@ PRUNE_TAXA, PRUNE_SITES, PRUNE_BL = 512, 500_000, 0.05
 PRUNE_GATE = 1e-3
 FORMS = {32: "fp32", 48: "fp32x2", 64: "fp64"}
 # FP32 thread instructions of each form, counted from csrc/forms.cuh: per row
-# of a P x child product (internal children only; tip children are table
-# rows; the pair form computes two rows per packed float2 instruction, 44 per
-# row pair), and per node and rate class for the product of the two children
-# and the rescale test
-FP32_INSTR_PER_ROW = {32: 5, 48: 22}
+# of a P x child product (internal children of the reduced tree only; its
+# leaves, subtrees of up to three tips, are table rows; the pair form computes
+# two rows per packed float2 instruction, 40 per row pair), and per node and
+# rate class for the product of the two children and the rescale test
+FP32_INSTR_PER_ROW = {32: 5, 48: 20}
 FP32_INSTR_PER_NODE = {32: 4 + 6, 48: 4 * 4 + 6}
 
 
@@ -633,9 +633,15 @@ def bench_prune(args, rank, world, local):
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
     lane_peak = n_sm * 128 * sm_mhz * 1e6 / 1e12            # Tinst/s at the sampled clock
     flop_peak = 2.0 * lane_peak                              # FP32 FMA: 2 flop per lane-cycle
-    internal_children = int(np.sum(tr.left >= tr.n_tips) + np.sum(tr.right >= tr.n_tips))
+    # steps of the reduced tree: nodes above more than three tips (the codes'
+    # 4096 combinations are tabulated below them at this many patterns)
+    tips = np.ones(tr.n_tips + tr.n_internal, np.int64)
+    for i in range(tr.n_internal):
+        tips[tr.n_tips + i] = tips[tr.left[i]] + tips[tr.right[i]]
+    walked = tips[tr.n_tips:] > 3
+    internal_children = int(np.sum(tips[tr.left[walked]] > 3) + np.sum(tips[tr.right[walked]] > 3))
     instr = R * n_pat * (internal_children * 4 * FP32_INSTR_PER_ROW[head_prec] +
-                         tr.n_internal * FP32_INSTR_PER_NODE[head_prec])
+                         int(walked.sum()) * FP32_INSTR_PER_NODE[head_prec])
     # the algorithm's own flops per pattern: every internal node, every rate
     # class, two S x S matrix-vector products and S products, whatever the
     # arithmetic form spends on them
@@ -700,7 +706,7 @@ def bench_clv(args, rank, world, local):
     """Likelihood_c node by node on the pruning workload (512 taxa x 446k
     patterns, GTR+Gamma4, float vectors): median_2 folded over the postorder
     as Node.Make1D drives it, every node's vectors materialised in HBM.  The
-    dominant kernel, clv_median_kernel, is HBM-bound: per launch it reads two
+    dominant kernel, clv_median4_kernel, is HBM-bound: per launch it reads two
     children (n_pat x R x S floats and an int exponent each) and the weights
     and writes the parent."""
     import torch
@@ -762,7 +768,7 @@ def bench_clv(args, rank, world, local):
                      "algorithmic_bytes": alg_bytes,
                      "bytes_formula": "3 x n_pat x (R*S*4 + 4) + 8 x n_pat (two children read, "
                                       "parent written, weights)",
-                     "kernel": "clv_median_kernel<float,4>", "per_launch_ms": per_launch_ms,
+                     "kernel": "clv_median4_kernel<float,2>", "per_launch_ms": per_launch_ms,
                      "traffic": None,
                      "traffic_note": "the capturable case (32 taxa, profiles/clv_median_kernel_191k.md) "
                                      "fits in L2, so its DRAM bytes do not scale to this launch"},

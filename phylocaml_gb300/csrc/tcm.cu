@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(TC_THREADS) tcm_tree_kernel(const TcmArgs a) {
 // code as short as a single state.  The row stride is an odd multiple of 16
 // bytes, so the rows of 8 lanes' 16-byte loads fall in distinct banks.
 // Bound by instruction issue (the per-state minima and sums), not by memory.
-// 128 taxa x 20,003 sites of 20 states, metric rule: 65 us a call against
+// 128 taxa x 20,003 sites of 20 states, metric rule: 59 us a call against
 // 1,252 us with one thread per word searching the candidates one by one.
 struct TcmWideArgs {
   const uint32_t *tips;      // [n_tips][ld] lanes of LB bits

@@ -167,7 +167,7 @@ struct NetView {   // device pointers of one network
 };
 
 // ---- ranking: 128 rows per CTA through every layer ------------------------
-// 257,048 rows: 0.25 ms; the three-launch form, which wrote each hidden
+// 257,048 rows: 0.30 ms; the three-launch form, which wrote each hidden
 // layer to memory and read it back, took 1.8 ms.
 __global__ void __launch_bounds__(MLP_NT, 2) mlp_forward_kernel(const NetView net, const float *X, size_t n,
                                                                 float *y, int *flag) {

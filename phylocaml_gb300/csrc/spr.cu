@@ -1273,9 +1273,11 @@ __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
 // (TwoSum) in pairs, two eigenvectors to a packed float2 instruction.  S is
 // the float that FP64 gives: where the pairs' error leaves two candidates
 // (Ziv's rounding test, error at most 2^-45 of the terms' sizes) the value is
-// formed again in FP64.  A value below 2^-28 of the terms it came from is
-// left as it is: the other eigenvectors' float roundings are larger.
-// 509 edges x 45,675 patterns x 4 classes, pair form: 1.66 ms against 11.4
+// formed again in FP64: the Newton steps' float exponentials turn a last bit
+// here into 3e-7 of a length.  Below 2^-60 of the terms, less than FP64's own
+// rounding of them, it is left as it is (sums that cancel to nothing: 2.47 ms
+// with those formed again as well).
+// 509 edges x 45,675 patterns x 4 classes, pair form: 1.73 ms against 11.4
 // in FP64, which this GPU runs at 1/64 of the FP32 rate.
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
 __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &e) {
@@ -1358,8 +1360,8 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
     const float2 up = __fadd2_rn(v, __fadd2_rn(rest, d)), down = __fadd2_rn(v, sub2(rest, d));
     s[2 * kp] = v.x;
     s[2 * kp + 1] = v.y;
-    if (!(up.x == down.x) && !(fabsf(v.x) < 0x1p-28f * all.x)) unsure |= 1 << (2 * kp);
-    if (!(up.y == down.y) && !(fabsf(v.y) < 0x1p-28f * all.y)) unsure |= 2 << (2 * kp);
+    if (!(up.x == down.x) && !(fabsf(v.x) < 0x1p-60f * all.x)) unsure |= 1 << (2 * kp);
+    if (!(up.y == down.y) && !(fabsf(v.y) < 0x1p-60f * all.y)) unsure |= 2 << (2 * kp);
   }
   if (unsure) {
 #pragma unroll

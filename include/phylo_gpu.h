@@ -445,7 +445,10 @@ pgpu_status pgpu_lk_create(pgpu_ctx *ctx, const pgpu_model *model, const pgpu_ti
                            size_t n_pat, const double *weights, int precision, pgpu_lk **out);
 void pgpu_lk_destroy(pgpu_lk *lk);
 /* A leaf: codes is a host array [n_pat] of rows of the tip-code table.
- * Its branch length is 0 until set. */
+ * Its branch length is 0 until set.  A code outside the table counts as code
+ * 0, and the next call on the context that synchronises (pgpu_synchronize, a
+ * cost, a host call) fails with PGPU_ERR_ARG, once; with four states not for
+ * a leaf that was overwritten or destroyed before then and that nothing read. */
 pgpu_status pgpu_clv_leaf(pgpu_lk *lk, pgpu_clv *reuse, const uint8_t *codes, pgpu_clv **out);
 /* Length of the branch above the node (>= 0); builds that branch's P
  * matrices in FP64 on the GPU.  A node must have one before it is used as

@@ -72,7 +72,6 @@ struct pgpu_lk {
   void *tabv = nullptr;
   bool leaf_codes = false;
   int resident[3] = {};      // CTAs of clv_median4_kernel per SM, by neighbour count (0: not asked yet)
-  std::vector<pgpu_clv *> unchecked;   // leaves whose codes no kernel has read yet
 };
 
 struct pgpu_clv {
@@ -93,7 +92,9 @@ struct pgpu_clv {
   bool has_P = false;
   bool leaf = false;
   bool expanded = false;     // a leaf whose vector is in x
-  int unchecked = -1;        // index in the model's list
+  // a leaf with codes outside the table that nothing has read or reported yet:
+  // the context's count of reports when it was made, else -1
+  long long bad = -1;
 };
 
 namespace {
@@ -347,7 +348,6 @@ struct Med4Args {
   int R, RL, rl_shift, n_codes, int_w;   // RL = 1 << rl_shift
   const int32_t *wint;
   long long *acc, *acc_next;
-  int *flag;
 };
 
 template <typename V, int NCH>
@@ -388,7 +388,6 @@ __global__ void __launch_bounds__(CLV_THREADS, sizeof(V) == 4 ? 4 : 2) clv_media
   if (a.int_w && blockIdx.x == 0 && tid == 0) *a.acc_next = 0;
   double s = 0.0, c = 0.0;
   long long iacc = 0;
-  uint32_t bad = 0;
   // what one item reads; the next item's is on its way while one is computed
   struct Item {
     V x[NCH][4];
@@ -438,7 +437,6 @@ __global__ void __launch_bounds__(CLV_THREADS, sizeof(V) == 4 ? 4 : 2) clv_media
             for (int j = 0; j < 4; ++j) t[i] = fma(Pr[j], cur.x[k][j], t[i]);
           }
         } else {
-          bad |= cur.code[k] >= (uint32_t)a.n_codes;
           Row4<V>::load_shared(
               rows + leaf * n_rows + (min(cur.code[k], (uint32_t)a.n_codes - 1u) * R + r) * 4, t);
           ++leaf;
@@ -475,18 +473,14 @@ __global__ void __launch_bounds__(CLV_THREADS, sizeof(V) == 4 ? 4 : 2) clv_media
     cur = next;
     g += stride;
   }
-  if (bad) atomicOr(a.flag, PGPU_FLAG_BADCODE);
   if (a.int_w) cta_add_i64<CLV_THREADS>(iacc, a.acc);
   else cta_partial_and_finish<CLV_THREADS>(s, c, a.part, a.counter, a.cost, NEG_LN2);
 }
 
-// codes at or above n_codes raise the error word
-__global__ void __launch_bounds__(CLV_THREADS) clv_codes_kernel(const uint8_t *codes, size_t n, int n_codes,
-                                                                int *flag) {
-  bool bad = false;
+// codes at or above n_codes become 0, as clv_leaf_kernel reads them
+__global__ void __launch_bounds__(CLV_THREADS) clv_codes_kernel(uint8_t *codes, size_t n, int n_codes) {
   for (size_t i = (size_t)blockIdx.x * CLV_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * CLV_THREADS)
-    bad |= codes[i] >= n_codes;
-  if (bad) atomicOr(flag, PGPU_FLAG_BADCODE);
+    if (codes[i] >= n_codes) codes[i] = 0;
 }
 
 // root_cost: -sum_p w_p log(sum_r probs_r sum_i pi_i x[p][r][i]); the
@@ -580,28 +574,30 @@ pgpu_status clv_malloc(pgpu_ctx *ctx, size_t bytes, char **out) {
   return PGPU_OK;
 }
 
-// no kernel needs to read t's codes to find a bad one any more
-void clv_checked(pgpu_clv *t) {
-  if (t->unchecked < 0) return;
-  auto &u = t->lk->unchecked;
-  u[t->unchecked] = u.back();
-  u[t->unchecked]->unchecked = t->unchecked;
-  u.pop_back();
-  t->unchecked = -1;
+// A leaf's codes are looked at while they are copied; ctx->bad_leaves makes the
+// next call that checks the error word report those outside the table.  A bad
+// leaf that is overwritten or destroyed before such a call is not reported,
+// unless something has read it.
+void bad_leaf_read(pgpu_clv *t) { t->bad = -1; }
+void bad_leaf_gone(pgpu_clv *t) {
+  if (t->bad >= 0 && t->bad == t->lk->ctx->bad_reports) --t->lk->ctx->bad_leaves;
+  t->bad = -1;
 }
 
-// reads the codes of every leaf that nothing has read yet, so that a bad
-// code is reported by the calls that synchronise
-pgpu_status check_leaves(pgpu_lk *lk) {
-  pgpu_ctx *ctx = lk->ctx;
-  while (!lk->unchecked.empty()) {
-    pgpu_clv *t = lk->unchecked.back();
-    const unsigned grid = (unsigned)std::min<size_t>((lk->n_pat + CLV_THREADS - 1) / CLV_THREADS, 1024);
-    clv_codes_kernel<<<grid, CLV_THREADS, 0, ctx->stream>>>(t->codes, lk->n_pat, lk->n_codes, ctx->d_flag);
-    PGPU_TRY(pgpu_after_launch(ctx, "clv_codes_kernel"));
-    clv_checked(t);
+// Four maxima over the quarters of the codes: one is a chain of dependent
+// operations (3.9 us per 100,000 codes on the host's cores, 1.1 with four;
+// copying them takes 1.1).
+bool codes_outside(const uint8_t *codes, size_t n, int n_codes) {
+  uint8_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+  const size_t q = n / 4;
+  for (size_t i = 0; i < q; ++i) {
+    m0 = std::max(m0, codes[i]);
+    m1 = std::max(m1, codes[q + i]);
+    m2 = std::max(m2, codes[2 * q + i]);
+    m3 = std::max(m3, codes[3 * q + i]);
   }
-  return PGPU_OK;
+  for (size_t i = 4 * q; i < n; ++i) m0 = std::max(m0, codes[i]);
+  return std::max(std::max(m0, m1), std::max(m2, m3)) >= n_codes;
 }
 
 // a handle for lk (or `reuse`, its memory taken over), without its vector
@@ -615,7 +611,7 @@ pgpu_status clv_alloc(pgpu_lk *lk, pgpu_clv *reuse, pgpu_clv **out) {
     reuse->leaf = false;
     reuse->expanded = false;
     reuse->brlen = 0.0;
-    clv_checked(reuse);
+    bad_leaf_gone(reuse);
     return PGPU_OK;
   }
   const size_t pb = lk->S == 4 ? 0 : al256((size_t)lk->R * lk->S * lk->S * vbytes(lk));
@@ -654,7 +650,7 @@ pgpu_status clv_vector(pgpu_clv *t) {
 
 void clv_free(pgpu_clv *t) {
   pgpu_ctx *ctx = t->lk->ctx;
-  clv_checked(t);
+  bad_leaf_gone(t);
   if (t->vec) cudaFreeAsync(t->vec, ctx->stream);
   cudaFreeAsync(t->mem, ctx->stream);
   t->lk->live--;
@@ -677,7 +673,7 @@ pgpu_status clv_expand(pgpu_clv *t, const uint8_t *codes) {
                                                                    ctx->d_flag);
   PGPU_TRY(pgpu_after_launch(ctx, "clv_leaf_kernel"));
   t->expanded = true;
-  clv_checked(t);
+  bad_leaf_read(t);
   return PGPU_OK;
 }
 
@@ -714,7 +710,6 @@ pgpu_status launch_median4(pgpu_lk *lk, pgpu_clv *t, pgpu_clv *const *ch) {
   a.wint = lk->wint;
   a.acc = reinterpret_cast<long long *>(t->scal + t->slot);
   a.acc_next = reinterpret_cast<long long *>(t->scal + (t->slot ^ 1));
-  a.flag = ctx->d_flag;
   const size_t smem = sizeof(V) * (size_t)lk->R * (NCH * 16 + (size_t)n_leaf * lk->n_codes * 4);
   if (lk->resident[NCH - 1] == 0 || smem > 48 * 1024)
     PGPU_CUDA(ctx, cudaFuncSetAttribute(clv_median4_kernel<V, NCH>,
@@ -776,7 +771,7 @@ pgpu_status median(pgpu_lk *lk, pgpu_clv *reuse, const pgpu_clv *const *nbr, int
   if (lk->int_w) t->slot ^= 1;
   if (lk->S == 4) {
     for (int k = 0; k < n_ch; ++k)
-      if (ch[k]->leaf) clv_checked(ch[k]);   // the kernel checks the codes it reads
+      bad_leaf_read(ch[k]);
     if (lk->precision == 32)
       st = n_ch == 1 ? launch_median4<float, 1>(lk, t, ch)
                      : n_ch == 2 ? launch_median4<float, 2>(lk, t, ch) : launch_median4<float, 3>(lk, t, ch);
@@ -981,19 +976,32 @@ pgpu_status pgpu_clv_leaf(pgpu_lk *lk, pgpu_clv *reuse, const uint8_t *codes, pg
   PGPU_TRY(clv_alloc(lk, reuse, &t));
   const cudaStream_t s = ctx->stream;
   if (lk->leaf_codes) {
-    // the codes themselves are the leaf; its first reader checks them
-    // Up to 1 MB they go through the pinned staging blocks: a copy straight
-    // from pageable memory holds the caller up (20 us against 9 at 100 KB).
+    // The codes themselves are the leaf.  Up to 1 MB they go through the pinned
+    // staging blocks: a copy straight from pageable memory holds the caller up
+    // (20 us against 9 at 100 KB).
+    bool bad = false;
     if (lk->n_pat <= (size_t)1 << 20) {
       void *h;
       PGPU_TRY(pgpu_stage(ctx, lk->n_pat, &h, nullptr));
-      std::memcpy(h, codes, lk->n_pat);
+      uint8_t *to = static_cast<uint8_t *>(h);
+      constexpr size_t block = 16 * 1024;   // looked at while it is in the first-level cache
+      for (size_t i = 0; i < lk->n_pat; i += block) {
+        const size_t k = std::min(block, lk->n_pat - i);
+        std::memcpy(to + i, codes + i, k);
+        bad |= codes_outside(codes + i, k, lk->n_codes);
+      }
       PGPU_TRY(pgpu_stage_copy(ctx, t->codes, lk->n_pat));
     } else {
       PGPU_CUDA(ctx, cudaMemcpyAsync(t->codes, codes, lk->n_pat, cudaMemcpyHostToDevice, s));
+      bad = codes_outside(codes, lk->n_pat, lk->n_codes);
     }
-    t->unchecked = (int)lk->unchecked.size();
-    lk->unchecked.push_back(t);
+    if (bad) {
+      const unsigned grid = (unsigned)std::min<size_t>((lk->n_pat + CLV_THREADS - 1) / CLV_THREADS, 1024);
+      clv_codes_kernel<<<grid, CLV_THREADS, 0, s>>>(t->codes, lk->n_pat, lk->n_codes);
+      PGPU_TRY(pgpu_after_launch(ctx, "clv_codes_kernel"));
+      t->bad = ctx->bad_reports;
+      ++ctx->bad_leaves;
+    }
   } else {
     // the codes are copied into the context's tip buffer; later calls on the
     // stream are ordered after this leaf's kernel
@@ -1071,7 +1079,6 @@ pgpu_status pgpu_clv_cost(pgpu_clv *t, double *cost) {
   if (!t || !cost) return PGPU_ERR_ARG;
   pgpu_ctx *ctx = t->lk->ctx;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
-  PGPU_TRY(check_leaves(t->lk));
   double *h = reinterpret_cast<double *>(ctx->h_pinned);
   PGPU_CUDA(ctx, cudaMemcpyAsync(h, cost_at(t), sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PGPU_TRY(pgpu_check_flag(ctx, "likelihood"));
@@ -1087,7 +1094,6 @@ pgpu_status pgpu_clv_costs(pgpu_lk *lk, const pgpu_clv *const *nodes, size_t n, 
     if (!nodes[i] || nodes[i]->lk != lk)
       return lk_err(lk, PGPU_ERR_ARG, "likelihood: a node is null or belongs to another model");
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
-  PGPU_TRY(check_leaves(lk));
   void *h, *d, *dout;
   PGPU_TRY(pgpu_stage(ctx, n * sizeof(double *), &h, &d));
   const double **src = static_cast<const double **>(h);
@@ -1108,7 +1114,6 @@ pgpu_status pgpu_clv_root_cost(pgpu_clv *t, double *cost, double *site_lnl) {
   pgpu_ctx *ctx = lk->ctx;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
   if (t->leaf && !t->expanded) PGPU_TRY(clv_expand(t, t->codes));
-  PGPU_TRY(check_leaves(lk));
   void *dsl = nullptr;
   if (site_lnl) PGPU_TRY(pgpu_buf(ctx, BUF_SITECOST, lk->n_pat * 8, &dsl));
   const unsigned grid = (unsigned)lk->n_cta;

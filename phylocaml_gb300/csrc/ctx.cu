@@ -49,7 +49,12 @@ pgpu_status pgpu_check_flag(pgpu_ctx *ctx, const char *what) {
   int *h = reinterpret_cast<int *>(static_cast<char *>(ctx->h_pinned) + PGPU_PINNED_FLAG);
   PGPU_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const int flag = *h;
+  int flag = *h;
+  if (ctx->bad_leaves) {
+    flag |= PGPU_FLAG_BADCODE;
+    ctx->bad_leaves = 0;
+    ++ctx->bad_reports;
+  }
   if (flag) {
     PGPU_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     if (flag & PGPU_FLAG_TIMEOUT)

@@ -102,6 +102,9 @@ struct pgpu_ctx {
   void *buf[BUF_COUNT] = {};
   size_t cap[BUF_COUNT] = {};
   int *d_flag = nullptr;       // device error word written by bounded waits
+  // likelihood leaves with codes outside their table that are still to be
+  // reported beside the error word, and how often such leaves have been
+  long long bad_leaves = 0, bad_reports = 0;
   void *h_pinned = nullptr;    // small pinned staging area for scalars
   // the last tree scheduled, kept on the device (BUF_OPS, BUF_TIPSEQ) so
   // repeated calls on one tree upload nothing

@@ -105,6 +105,14 @@ pgpu_status pgpu_copy_stream(pgpu_ctx *ctx) {
   return PGPU_OK;
 }
 
+pgpu_status pgpu_not_capturing(pgpu_ctx *ctx, const char *what) {
+  cudaStreamCaptureStatus st;
+  PGPU_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &st));
+  if (st != cudaStreamCaptureStatusNone)
+    return pgpu_set_err(ctx, PGPU_ERR_CUDA, "%s while the stream is captured: make the same call once before", what);
+  return PGPU_OK;
+}
+
 // Pinned staging for small per-call parameters, so that no call waits for the
 // stream: PGPU_STAGES blocks take turns, and a block is refilled once the
 // copy issued from it that many uses earlier is done.

@@ -1280,6 +1280,7 @@ pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitS
                    std::memcmp(ctx->split_right.data(), tree->right, n_int * 4) == 0;
   const SplitSchedule &sp = ctx->split;
   if (!hit) {
+    PGPU_TRY(pgpu_not_capturing(ctx, "a tree that is new to the context"));
     ctx->split_valid = false;
     PGPU_TRY(build_split(ctx, tree, &ctx->split));
     const size_t bytes =
@@ -1484,14 +1485,14 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
 }  // namespace
 
 // The cost-matrix postorder (csrc/tcm.cu) on the segmented schedule: 4-bit
-// codes, the packed pair table already on the device.  flush_period > 0
+// codes, the packed pair table in host memory.  flush_period > 0
 // (every cost small enough) selects the re-packed table with one add per
 // site.  *launched is false when the tree's stacks and the lane-replicated
 // table do not fit one CTA's shared memory; the caller then uses its
 // single-walk kernel.
 pgpu_status pgpu_tcm_tree_split(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
                                 size_t ld, const uint32_t *weights, size_t n_sites,
-                                const uint32_t *table_dev, int flush_period, uint32_t *node_sets,
+                                const uint32_t *table, int flush_period, uint32_t *node_sets,
                                 uint32_t *site_cost, unsigned long long *total, bool *launched,
                                 const HostRows *io) {
   *launched = false;
@@ -1503,6 +1504,8 @@ pgpu_status pgpu_tcm_tree_split(pgpu_ctx *ctx, const pgpu_tree *tree, const uint
   PGPU_TRY(pgpu_split_device(ctx, tree, &spp, &a.ops, &a.seg, &a.top, &a.wseg, &a.tip_seq));
   const SplitSchedule &sp = *spp;
   if (split_smem<TcmOp<false>>(sp.rows, false) > ctx->smem_optin) return PGPU_OK;
+  PGPU_TRY(pgpu_tcm_table(ctx, table, &a.table));
+  PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
   a.tips = tips;
   a.weights = weights;
   a.node_sets = node_sets;
@@ -1518,7 +1521,6 @@ pgpu_status pgpu_tcm_tree_split(pgpu_ctx *ctx, const pgpu_tree *tree, const uint
   a.tile_base = 0;
   a.count16 = 0;
   a.tcm_period = flush_period;
-  a.table = table_dev;
   a.flag = ctx->d_flag;
   const size_t tiles = (n_words + 127) / 128;
   PGPU_TRY(split_chunks(ctx, a, tiles, io, [&](size_t t0, size_t t1) -> pgpu_status {

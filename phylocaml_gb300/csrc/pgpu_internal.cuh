@@ -184,6 +184,11 @@ pgpu_status pgpu_after_launch(pgpu_ctx *ctx, const char *what);
 // Waits for the context's stream, then reads and clears the device error
 // word: a host call queues its result copies and ends with this.
 pgpu_status pgpu_check_flag(pgpu_ctx *ctx, const char *what);
+// Fails while the context's stream is captured.  What a context keeps for a
+// tree goes to the device once, when the tree is new: recorded into a graph,
+// that copy would not run now (and later calls would find the tree kept but
+// not there), and on replay would take whatever its staging block then holds.
+pgpu_status pgpu_not_capturing(pgpu_ctx *ctx, const char *what);
 // Pinned host block and its device twin for `bytes` of small parameters;
 // fill *host, then pgpu_stage_commit copies it on the context's stream.
 // PGPU_STAGES blocks take turns, so the host only waits for the copy issued
@@ -214,12 +219,14 @@ pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitS
                               const int4 **ops, const int4 **seg, const int4 **top, const int4 **wseg,
                               const int32_t **tips);
 
+// The packed pair table of a cost-matrix call, staged to the device (tcm.cu).
+pgpu_status pgpu_tcm_table(pgpu_ctx *ctx, const uint32_t *table, const uint32_t **dev);
 // The cost-matrix postorder on the Fitch kernel's segmented schedule
-// (fitch.cu); *launched is false when the tree does not fit its shared
-// memory.
+// (fitch.cu); table: 256 words in host memory; *launched is false when the
+// tree does not fit its shared memory.
 pgpu_status pgpu_tcm_tree_split(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
                                 size_t ld, const uint32_t *weights, size_t n_sites,
-                                const uint32_t *table_dev, int flush_period, uint32_t *node_sets,
+                                const uint32_t *table, int flush_period, uint32_t *node_sets,
                                 uint32_t *site_cost, unsigned long long *total, bool *launched,
                                 const HostRows *io = nullptr);
 

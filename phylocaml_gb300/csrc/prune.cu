@@ -768,6 +768,7 @@ pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes,
     return PGPU_OK;
   }
   TreeSchedule sch;
+  PGPU_TRY(pgpu_not_capturing(ctx, "a tree or a form that is new to the context"));
   PGPU_TRY(pgpu_check_tree(ctx, tree));
   pl.valid = false;
   pl.asked = level;

@@ -114,6 +114,7 @@ pgpu_status pgpu_schedule_device(pgpu_ctx *ctx, const pgpu_tree *tree, const Tre
                     std::memcmp(ctx->sched_right.data(), tree->right, n_int * 4) == 0;
   void *dops, *dseq;
   if (!same) {
+    PGPU_TRY(pgpu_not_capturing(ctx, "a tree that is new to the context"));
     ctx->sched_valid = false;
     PGPU_TRY(pgpu_build_schedule(ctx, tree, &ctx->sched));
     PGPU_TRY(pgpu_buf(ctx, BUF_OPS, ctx->sched.ops.size() * sizeof(SchedOp), &dops));

@@ -25,6 +25,15 @@
 
 #include "pgpu_internal.cuh"
 
+// The packed pair table (256 words) of a call, staged to the device.
+pgpu_status pgpu_tcm_table(pgpu_ctx *ctx, const uint32_t *table, const uint32_t **dev) {
+  void *h, *d;
+  PGPU_TRY(pgpu_stage(ctx, 256 * sizeof(uint32_t), &h, &d));
+  std::memcpy(h, table, 256 * sizeof(uint32_t));
+  *dev = static_cast<const uint32_t *>(d);
+  return pgpu_stage_commit(ctx, 256 * sizeof(uint32_t));
+}
+
 namespace {
 
 constexpr int TC_THREADS = 256;
@@ -460,13 +469,11 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
     return pgpu_set_err(ctx, PGPU_ERR_OVERFLOW,
                         "tcm_tree: a site's cost can reach %llu x %d, above 2^32 - 1",
                         (unsigned long long)emax, tree->n_tips - 1);
-  if (n_words == 0) PGPU_TRY(pgpu_check_tree(ctx, tree));
-  void *h, *d;
-  PGPU_TRY(pgpu_stage(ctx, 256 * sizeof(uint32_t), &h, &d));
-  std::memcpy(h, table, 256 * sizeof(uint32_t));
-  PGPU_TRY(pgpu_stage_commit(ctx, 256 * sizeof(uint32_t)));
-  PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
-  if (n_words == 0) return PGPU_OK;
+  if (n_words == 0) {
+    PGPU_TRY(pgpu_check_tree(ctx, tree));
+    PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
+    return PGPU_OK;
+  }
   // the segmented schedule: subtrees walked by four warps per 128-word slice.
   // It sums costs in the low 28 bits of a register under the codes' top 4,
   // flushing every p steps so that a site's sum, at most p * emax, stays
@@ -475,21 +482,21 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
   const int period = per >= 16 ? (int)std::min<uint64_t>(per, 1u << 30) : 0;
   bool launched = false;
   PGPU_TRY(pgpu_tcm_tree_split(ctx, tree, tips, ld, weights, n_sites,
-                               static_cast<const uint32_t *>(d), period, node_sets, site_cost, total,
-                               &launched, io));
+                               table, period, node_sets, site_cost, total, &launched, io));
   if (launched) return PGPU_OK;
   const TreeSchedule *sch;
   const int4 *d_ops;
   const int32_t *d_seq;
   PGPU_TRY(pgpu_schedule_device(ctx, tree, &sch, &d_ops, &d_seq));
   const size_t n = (size_t)tree->n_tips;
+  TcmArgs a;
+  PGPU_TRY(pgpu_tcm_table(ctx, table, &a.table));
+  PGPU_CUDA(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
   if (io)
     PGPU_CUDA(ctx, cudaMemcpy2DAsync(const_cast<uint32_t *>(tips), ld * 4, io->tips, n_words * 4, n_words * 4,
                                      n, cudaMemcpyHostToDevice, ctx->stream));
-  TcmArgs a;
   a.tips = tips;
   a.weights = weights;
-  a.table = static_cast<const uint32_t *>(d);
   a.ops = d_ops;
   a.node_sets = node_sets;
   a.site_cost = site_cost;

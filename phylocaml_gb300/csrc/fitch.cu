@@ -1274,6 +1274,7 @@ pgpu_status build_split(pgpu_ctx *ctx, const pgpu_tree *tree, SplitSchedule *out
 pgpu_status pgpu_split_device(pgpu_ctx *ctx, const pgpu_tree *tree, const SplitSchedule **out,
                               const int4 **ops, const int4 **seg, const int4 **top, const int4 **wseg,
                               const int32_t **tips) {
+  if (!tree->left || !tree->right) return pgpu_set_err(ctx, PGPU_ERR_ARG, "tree: null child arrays");
   const int32_t n_int = tree->n_tips - 1;
   const bool hit = ctx->split_valid && (int32_t)ctx->split_left.size() == n_int &&
                    std::memcmp(ctx->split_left.data(), tree->left, n_int * 4) == 0 &&

@@ -75,6 +75,12 @@ const char *pgpu_last_error(const pgpu_ctx *ctx);
  * (handle 0) therefore cannot be selected -- pass an explicit stream. */
 pgpu_status pgpu_set_stream(pgpu_ctx *ctx, void *cuda_stream);
 pgpu_status pgpu_synchronize(pgpu_ctx *ctx);
+/* Largest scratch buffer (bytes) that the context may ask for from now on; 0,
+ * the default: what the device has left.  A call that needs a larger one
+ * treats it as a failed allocation: pruning goes on with smaller tables and
+ * in pieces, others return PGPU_ERR_OOM.  For programs that keep the
+ * device's memory to themselves. */
+pgpu_status pgpu_set_scratch_limit(pgpu_ctx *ctx, size_t bytes);
 /* The cudaStream_t the context's work runs on (its own stream unless
  * pgpu_set_stream chose another), for callers that order their own work
  * against it with events. */

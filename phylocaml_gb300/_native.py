@@ -91,6 +91,7 @@ SIGNATURES: dict[str, tuple] = {
     "pgpu_last_error": (C.c_char_p, [_P]),
     "pgpu_set_stream": (_I, [_P, _P]),
     "pgpu_synchronize": (_I, [_P]),
+    "pgpu_set_scratch_limit": (_I, [_P, _SZ]),
     "pgpu_kernel_launches": (C.c_uint64, [_P]),
     "pgpu_get_stream": (_P, [_P]),
     "pgpu_version": (_I, []),

@@ -18,16 +18,23 @@ pgpu_status pgpu_set_err(pgpu_ctx *ctx, pgpu_status st, const char *fmt, ...) {
   return st;
 }
 
+pgpu_status pgpu_buf_release(pgpu_ctx *ctx, int slot) {
+  if (!ctx->buf[slot]) return PGPU_OK;
+  // the contents may still be in use by queued work
+  PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  PGPU_CUDA(ctx, cudaFree(ctx->buf[slot]));
+  ctx->buf[slot] = nullptr;
+  ctx->cap[slot] = 0;
+  return PGPU_OK;
+}
+
 pgpu_status pgpu_buf(pgpu_ctx *ctx, int slot, size_t bytes, void **out) {
   if (bytes == 0) bytes = 16;
+  if (ctx->scratch_limit && bytes > ctx->scratch_limit)
+    return pgpu_set_err(ctx, PGPU_ERR_OOM, "a scratch buffer of %zu bytes is above the limit of %zu", bytes,
+                        ctx->scratch_limit);
   if (ctx->cap[slot] < bytes) {
-    if (ctx->buf[slot]) {
-      // the previous contents may still be in use by queued work
-      PGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      PGPU_CUDA(ctx, cudaFree(ctx->buf[slot]));
-      ctx->buf[slot] = nullptr;
-      ctx->cap[slot] = 0;
-    }
+    PGPU_TRY(pgpu_buf_release(ctx, slot));
     size_t want = (bytes + 255) & ~size_t(255);
     PGPU_CUDA(ctx, cudaMalloc(&ctx->buf[slot], want));
     ctx->cap[slot] = want;
@@ -244,6 +251,12 @@ pgpu_status pgpu_synchronize(pgpu_ctx *ctx) {
   if (!ctx) return PGPU_ERR_ARG;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
   return pgpu_check_flag(ctx, "synchronize");
+}
+
+pgpu_status pgpu_set_scratch_limit(pgpu_ctx *ctx, size_t bytes) {
+  if (!ctx) return PGPU_ERR_ARG;
+  ctx->scratch_limit = bytes;
+  return PGPU_OK;
 }
 
 uint64_t pgpu_kernel_launches(const pgpu_ctx *ctx) { return ctx ? ctx->launches : 0; }

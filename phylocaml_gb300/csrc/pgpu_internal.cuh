@@ -101,6 +101,7 @@ struct pgpu_ctx {
   uint64_t launches = 0;
   void *buf[BUF_COUNT] = {};
   size_t cap[BUF_COUNT] = {};
+  size_t scratch_limit = 0;    // bytes a buffer may take (0: what the device has)
   int *d_flag = nullptr;       // device error word written by bounded waits
   // likelihood leaves with codes outside their table that are still to be
   // reported beside the error word, and how often such leaves have been
@@ -179,6 +180,8 @@ pgpu_status pgpu_set_err(pgpu_ctx *ctx, pgpu_status st, const char *fmt, ...);
 
 // Grow-only device buffer owned by the context.
 pgpu_status pgpu_buf(pgpu_ctx *ctx, int slot, size_t bytes, void **out);
+// Gives a slot's memory back.
+pgpu_status pgpu_buf_release(pgpu_ctx *ctx, int slot);
 // Launch bookkeeping: checks the launch error and counts it.
 pgpu_status pgpu_after_launch(pgpu_ctx *ctx, const char *what);
 // Waits for the context's stream, then reads and clears the device error

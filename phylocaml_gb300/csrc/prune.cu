@@ -752,18 +752,21 @@ Ptr *rebase(void *base, Ptr *off) {
 // k - 1 nodes for every pattern, so it is worth it while the table is the
 // smaller side: at most half the patterns (16 codes: from 8,192 patterns on
 // three tips, from 512 on two).  call_bytes is what one row takes over all
-// models; the tables of a call stay below 1 GB.
+// models; the tables of a call stay below 1 GB.  most: the highest level to
+// try, lowered when the device has no room for the tables (the plan made then
+// serves this tree's later calls too).
 pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes, size_t n_pat,
-                       size_t row_bytes, size_t call_bytes, const PrunePlan **out) {
+                       size_t row_bytes, size_t call_bytes, int most, const PrunePlan **out) {
   const int32_t n = tree->n_tips, n_int = n - 1;
   const size_t NC = (size_t)n_codes;
-  int level = 2 * NC * NC * NC <= n_pat && NC * NC * NC <= 65536 ? 3 : 2 * NC * NC <= n_pat ? 2 : 1;
+  const int asked = 2 * NC * NC * NC <= n_pat && NC * NC * NC <= 65536 ? 3 : 2 * NC * NC <= n_pat ? 2 : 1;
+  int level = std::min(asked, most);
   PrunePlan &pl = ctx->prune_plan;
   const bool same_tree = pl.valid && (int32_t)pl.left.size() == n_int &&
                          std::memcmp(pl.left.data(), tree->left, n_int * 4) == 0 &&
                          std::memcmp(pl.right.data(), tree->right, n_int * 4) == 0;
-  if (same_tree && pl.R == R && pl.n_codes == n_codes && pl.row_bytes == row_bytes && pl.asked == level &&
-      pl.made_rows * call_bytes <= (size_t)1 << 30) {
+  if (same_tree && pl.R == R && pl.n_codes == n_codes && pl.row_bytes == row_bytes && pl.asked == asked &&
+      pl.level <= level && pl.made_rows * call_bytes <= (size_t)1 << 30) {
     *out = &pl;
     return PGPU_OK;
   }
@@ -771,7 +774,7 @@ pgpu_status prune_plan(pgpu_ctx *ctx, const pgpu_tree *tree, int R, int n_codes,
   PGPU_TRY(pgpu_not_capturing(ctx, "a tree or a form that is new to the context"));
   PGPU_TRY(pgpu_check_tree(ctx, tree));
   pl.valid = false;
-  pl.asked = level;
+  pl.asked = asked;
   pl.R = R;
   pl.n_codes = n_codes;
   pl.row_bytes = row_bytes;
@@ -906,8 +909,45 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
     if (!(tree->brlen[i] >= 0.0) || !std::isfinite(tree->brlen[i]))
       return pgpu_set_err(ctx, PGPU_ERR_ARG, "prune: branch length %d is negative or not finite", i);
   const size_t row_bytes = precision == 32 ? 16 : 32;
+  const int RT = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : 8;
+  const size_t tile = PR_THREADS / RT, n_tiles = (n_pat + tile - 1) / tile;
+  const size_t SS = (size_t)S * S;
+  const size_t coef = precision == 32 ? 4 : 8;   // float, double, or float pair
+  const size_t p_bytes = align16((size_t)n_br * RT * SS * coef);
+  const size_t tip_rows = (size_t)n * R * codes->n_codes;
+  const size_t clear = align16((size_t)V * 2 * sizeof(int));
+
+  // Device scratch: P matrices, per-CTA partial sums, leaf rows (every tip's,
+  // then the collapsed leaves'), CTA counters and exponent flags (cleared by
+  // the setup kernel) and the rows' exponents, and the leaf indexes, of all
+  // patterns or in pieces of at most 1 GB.  Where the device has no room,
+  // smaller pieces, then less collapsed: what a call cannot do without is what
+  // the walk over every node takes, and indexes of one tile.
   const PrunePlan *pp;
-  PGPU_TRY(prune_plan(ctx, tree, R, codes->n_codes, n_pat, row_bytes, row_bytes * V, &pp));
+  void *dP, *dpart, *drows, *dexp, *dix = nullptr;
+  size_t cols = 0, rows_bytes = 0;
+  PGPU_TRY(pgpu_buf(ctx, BUF_I, (size_t)V * p_bytes, &dP));
+  PGPU_TRY(pgpu_buf(ctx, BUF_G, std::max<size_t>(n_tiles, 1) * V * sizeof(double2), &dpart));
+  for (int most = 3;; most = pp->level - 1) {
+    PGPU_TRY(prune_plan(ctx, tree, R, codes->n_codes, n_pat, row_bytes, row_bytes * V, most, &pp));
+    rows_bytes = align16((tip_rows + pp->made_rows) * row_bytes);
+    pgpu_status st = pgpu_buf(ctx, BUF_J, (size_t)V * rows_bytes, &drows);
+    if (st == PGPU_OK) st = pgpu_buf(ctx, BUF_E, clear + (size_t)V * pp->made_rows * sizeof(int), &dexp);
+    const size_t n_leaf = pp->leaves.size();   // the padding included
+    size_t piece = std::min(n_tiles, std::max<size_t>(((size_t)1 << 29) / n_leaf / tile, 1));
+    for (; st == PGPU_OK && n_tiles > 0; piece = (piece + 1) / 2) {
+      cols = piece * tile;
+      st = pgpu_buf(ctx, BUF_D, n_leaf * cols * sizeof(uint16_t), &dix);
+      if (st != PGPU_ERR_OOM || piece == 1) break;
+      st = PGPU_OK;
+    }
+    if (st == PGPU_OK) break;
+    if (st != PGPU_ERR_OOM || pp->level == 1) return st;
+    PGPU_TRY(pgpu_buf_release(ctx, BUF_J));   // the larger tables' room
+    PGPU_TRY(pgpu_buf_release(ctx, BUF_E));
+  }
+  const size_t made_rows = pp->made_rows;
+  const int n_leaf = (int)pp->leaves.size();
 
   // stage every model's Q, pi, rates, probs, then the code table and the
   // branch lengths
@@ -933,23 +973,6 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
                          rebase(h, lay.lam) + (size_t)v * 4, rebase(h, lay.Ui) + (size_t)v * 16);
   PGPU_TRY(pgpu_stage_commit(ctx, lay.bytes));
 
-  // device scratch: eigen systems, P matrices, leaf rows (every tip's, then
-  // the collapsed leaves'), their exponents, and per-CTA partial sums
-  const int RT = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : 8;
-  const size_t n_tiles = (n_pat + (PR_THREADS / RT) - 1) / (PR_THREADS / RT);
-  const size_t SS = (size_t)S * S;
-  const size_t coef = precision == 32 ? 4 : 8;   // float, double, or float pair
-  const size_t p_bytes = align16((size_t)n_br * RT * SS * coef);
-  const size_t tip_rows = (size_t)n * R * codes->n_codes, made_rows = pp->made_rows;
-  const size_t rows_bytes = align16((tip_rows + made_rows) * row_bytes);
-  const int n_leaf = (int)pp->leaves.size();   // the padding included
-  void *dP, *dpart, *drows, *dexp;
-  PGPU_TRY(pgpu_buf(ctx, BUF_I, (size_t)V * p_bytes, &dP));
-  PGPU_TRY(pgpu_buf(ctx, BUF_G, std::max<size_t>(n_tiles, 1) * V * sizeof(double2), &dpart));
-  PGPU_TRY(pgpu_buf(ctx, BUF_J, (size_t)V * rows_bytes, &drows));
-  // CTA counters and exponent flags (cleared by the setup kernel), then exponents
-  const size_t clear = align16((size_t)V * 2 * sizeof(int));
-  PGPU_TRY(pgpu_buf(ctx, BUF_E, clear + (size_t)V * made_rows * sizeof(int), &dexp));
   const double *dU = rebase(d, lay.U), *dUi = rebase(d, lay.Ui), *dlam = rebase(d, lay.lam);
   const int *dst = rebase(d, lay.status);
   if (!host_eig) {
@@ -1022,9 +1045,6 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   t.n_made = (int)pp->made.size();
   t.status = dst;
   t.blocks = (codes->n_codes * codes->n_codes + 255) / 256;
-  // leaf indexes: of all patterns, or in pieces of at most 1 GB
-  const size_t tile = PR_THREADS / RT;
-  const size_t cols = std::min(n_tiles, std::max<size_t>(((size_t)1 << 29) / n_leaf / tile, 1)) * tile;
   IndexArgs x{};
   x.tip_codes = tips;
   x.leaves = pp->d_leaves;
@@ -1033,8 +1053,6 @@ pgpu_status prune_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *mo
   x.n_pat = n_pat;
   x.n_codes = codes->n_codes;
   x.flag = ctx->d_flag;
-  void *dix;
-  PGPU_TRY(pgpu_buf(ctx, BUF_D, (size_t)n_leaf * cols * sizeof(uint16_t), &dix));
   x.index = static_cast<uint16_t *>(dix);
   if (precision == 32) return launch_prune<Fp32>(ctx, a, RT, V, pl, htp != nullptr, t, x, cols);
   if (precision == 48) return launch_prune<Ff32>(ctx, a, RT, V, pl, htp != nullptr, t, x, cols);

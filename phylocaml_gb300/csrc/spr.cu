@@ -1272,13 +1272,24 @@ __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
 // product is a sum of four signed terms, exact products and exact sums
 // (TwoSum) in pairs, two eigenvectors to a packed float2 instruction.  S is
 // the float that FP64 gives: where the pairs' error leaves two candidates
-// (Ziv's rounding test, error at most 2^-45 of the terms' sizes) the value is
-// formed again in FP64: the Newton steps' float exponentials turn a last bit
-// here into 3e-7 of a length.  Below 2^-60 of the terms, less than FP64's own
-// rounding of them, it is left as it is (sums that cancel to nothing: 2.47 ms
-// with those formed again as well).
-// 509 edges x 45,675 patterns x 4 classes, pair form: 1.73 ms against 11.4
+// (Ziv's rounding test with EIGEN_ERR) the value is formed again in FP64: the
+// Newton steps' float exponentials turn a last bit here into 3e-7 of a length.
+// Below 2^-60 of the terms, less than FP64's own rounding of them, it is left
+// as it is (sums that cancel to nothing: 2.47 ms with those formed again as
+// well).
+//
+// The error of a sum, with u = 2^-24 and T the sum of the terms' sizes: each
+// product leaves out its low parts' product and the coefficient's own rest
+// (u^2 each) and rounds its low word twice (2 u^2 and 3 u^2): 7 u^2 T in all.
+// An addition's low word is its TwoSum rest, at most u T, plus the product's,
+// 3 u of its term: forming the three rounds 6 u^2 T, gathering them 15 u^2 T
+// (they grow by u T a term).  28 u^2 T.  The product of two such sums A, B
+// adds three roundings of its low word, 3 u^2 (T_A |B| + |A| T_B), and the test
+// itself and FP64's own error under 2 u^2.  33 u^2 in all; 14 u^2 T is the
+// largest error of a sum that a search has found.
+// 509 edges x 45,675 patterns x 4 classes, pair form: 1.74 ms against 11.4
 // in FP64, which this GPU runs at 1/64 of the FP32 rate.
+constexpr float EIGEN_ERR = 0x1p-42f;   // 64 u^2
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
 __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &e) {
   s = __fadd2_rn(a, b);
@@ -1354,7 +1365,7 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
     er = __ffma2_rn(al, bh, er);
     const float2 v = __fadd2_rn(p, er), rest = sub2(er, sub2(v, p));
     const float2 all = __fmul2_rn(am, bm);
-    const float2 d = __fmul2_rn(make_float2(0x1p-45f, 0x1p-45f),
+    const float2 d = __fmul2_rn(make_float2(EIGEN_ERR, EIGEN_ERR),
                                 make_float2(fmaf(fabsf(ah.x), bm.x, fabsf(bh.x) * am.x),
                                             fmaf(fabsf(ah.y), bm.y, fabsf(bh.y) * am.y)));
     const float2 up = __fadd2_rn(v, __fadd2_rn(rest, d)), down = __fadd2_rn(v, sub2(rest, d));

@@ -1243,6 +1243,7 @@ struct BlArgs {
   const void *L;
   const double *U, *Ui, *lam, *pi, *rates, *probs;
   const float2 *w2;         // [np] weights as float pairs
+  const float *w3;          // [np] what the pairs leave of the weights, or null: nothing
   float *S;                 // [n_edges][np][R][4]: eigen-basis products
   const double *len_in;
   double *len_out;
@@ -1400,6 +1401,7 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
 // FP32 rate, so the exponentials are formed once per CTA and the sums of an
 // iteration kept in three floats, closer than FP64.  509 edges x 45,675
 // patterns x 4 classes: 2.0 ms against 2.71 with both in FP64 in every thread.
+// A weight is taken with all the bits of its FP64 value.
 __global__ void __launch_bounds__(256) bl_newton_kernel(const BlArgs a) {
   __shared__ double red[2][8];
   __shared__ double t_sh;
@@ -1435,7 +1437,7 @@ __global__ void __launch_bounds__(256) bl_newton_kernel(const BlArgs a) {
         }
       }
       if (f > 0.0f) {
-        // w d1 and w (f2 / f - d1^2), w as a pair
+        // w d1 and w (f2 / f - d1^2), w in two floats, or three: all of its bits
         const float d1 = f1 / f, d2 = f2 / f, q = __fmul_rn(d1, d1), qe = __fmaf_rn(d1, d1, -q);
         const float2 w = a.w2[pat];
         gs.add_product(w.x, d1);
@@ -1446,6 +1448,12 @@ __global__ void __launch_bounds__(256) bl_newton_kernel(const BlArgs a) {
           gs.add_product(w.y, d1);
           hs.add_product(w.y, d2);
           hs.add_product(w.y, -q);
+          hs.add_low(__fmul_rn(w.y, -qe));
+          if (a.w3) {
+            const float v = a.w3[pat];
+            gs.add_low(__fmul_rn(v, d1));
+            hs.add_low(__fmul_rn(v, __fadd_rn(d2, -q)));
+          }
         }
       }
     }
@@ -1518,6 +1526,7 @@ struct pgpu_spr {
   uint8_t *cmask = nullptr;
   double *w = nullptr;
   float2 *w2 = nullptr;      // weights as float pairs
+  float *w3 = nullptr;       // what the pairs leave of them (null: nothing)
   float2 *pairs = nullptr;   // pi [4] and probs [8] as float pairs
   float4 *logtab = nullptr;
   // pool
@@ -2269,6 +2278,16 @@ pgpu_status pgpu_spr_create(pgpu_ctx *ctx, const pgpu_model *m, const pgpu_tip_c
   SPR_TRY(upload(s, s->w, wh.data(), wh.size()));
   SPR_TRY(dalloc_t(s, s->np, &s->w2));
   SPR_TRY(upload(s, s->w2, w2h.data(), w2h.size()));
+  std::vector<float> w3h(s->np);
+  bool rest = false;
+  for (size_t i = 0; i < s->np; ++i) {
+    w3h[i] = (float)(wh[i] - (double)w2h[i].x - (double)w2h[i].y);
+    rest |= w3h[i] != 0.0f;
+  }
+  if (rest) {
+    SPR_TRY(dalloc_t(s, s->np, &s->w3));
+    SPR_TRY(upload(s, s->w3, w3h.data(), w3h.size()));
+  }
   s->n_planes = 1;
   while ((wmax >> s->n_planes) != 0) ++s->n_planes;
   std::vector<uint32_t> planes((size_t)s->n_planes * s->W4, 0u);
@@ -2643,6 +2662,7 @@ pgpu_status pgpu_spr_optimize(pgpu_spr *s, int passes, double tol, double *lnl_o
     a.rates = s->rates;
     a.probs = s->probs;
     a.w2 = s->w2;
+    a.w3 = s->w3;
     a.S = s->S;
     a.len_in = s->elen;
     a.len_out = s->newlen;

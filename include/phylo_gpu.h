@@ -265,8 +265,8 @@ pgpu_status pgpu_tcm_tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32
  * e.g. Alphabet.aminoacids' 22 states, lib/alphabet.ml:328-343).  A table
  * over every pair of codes no longer fits, so each node forms its medians
  * from the TCM itself with the same rule (mode as for pgpu_tcm_tables;
- * symmetric != 0 orders each pair's codes first, as the reference's table
- * for a symmetric TCM is filled for i <= j and mirrored).  Sites are codes
+ * the rules give a pair of codes the same median in either order, so
+ * symmetric, which for a table orders them, changes nothing).  Sites are codes
  * of lane_bits (8, 16 or 32) bits, one site per lane as for pgpu_fitch_tree,
  * n_states <= lane_bits; tcm is the row-major n_states x n_states cost of
  * atomic state i to j, each in [0, 2^25].  node_sets, site_cost and total as
@@ -375,17 +375,20 @@ pgpu_status pgpu_compose_sym(pgpu_ctx *ctx, const double *U, const double *D, in
  *              floats, every sum and product error-free, about 48
  *              significant bits, on the FP32 units;
  *              64: the FP64 form.  P matrices are always built in FP64 on
- *              the GPU; the log-likelihood is always summed in FP64 with
+ *              the GPU (the eigen systems of up to 24 models on the host);
+ *              the log-likelihood is always summed in FP64 with
  *              compensation.
  *   lnl        out: sum_s weights[s] * site_lnl[s]
  *   site_lnl   [n_pat] out (or NULL)
  * tree->brlen is required.  This entry point takes S = 4 (DNA); 20- and
- * 61-state models go through the batched tensor-core path.  The tip codes
- * are copied in column chunks on a second stream of the context, so the
- * copy overlaps the scoring (pinned host memory lets the copies run
+ * 61-state models go through the batched tensor-core path.  Codes and
+ * weights of up to 128 KB go over in one pinned block.  Above that the tip
+ * codes are copied in column chunks on a second stream of the context, so
+ * the copy overlaps the scoring (pinned host memory lets the copies run
  * asynchronously): the first chunk is one wave of the scoring kernel's
- * CTAs, each next a fixed factor larger.  The call returns once lnl is
- * written. */
+ * CTAs, each next a fixed factor larger.  Subtrees of two or three tips are
+ * tabulated where that is less work than the patterns; where the device has
+ * no room for the tables, fewer are.  The call returns once lnl is written. */
 pgpu_status pgpu_prune_lnl(pgpu_ctx *ctx, const pgpu_tree *tree, const pgpu_model *model,
                            const pgpu_tip_codes *codes, const uint8_t *tip_codes,
                            const double *weights, size_t n_pat, int precision, double *lnl,
@@ -457,8 +460,8 @@ void pgpu_lk_destroy(pgpu_lk *lk);
  * a leaf that was overwritten or destroyed before then and that nothing read. */
 pgpu_status pgpu_clv_leaf(pgpu_lk *lk, pgpu_clv *reuse, const uint8_t *codes, pgpu_clv **out);
 /* Length of the branch above the node (>= 0); builds that branch's P
- * matrices in FP64 on the GPU.  A node must have one before it is used as
- * a neighbour. */
+ * matrices in FP64, on the host for four states, else on the GPU.  A node
+ * must have one before it is used as a neighbour. */
 pgpu_status pgpu_clv_set_brlen(pgpu_clv *t, double brlen);
 pgpu_status pgpu_clv_get_brlen(const pgpu_clv *t, double *brlen);
 /* median_1: P(t_a) a.  median_2: (P(t_a) a) * (P(t_b) b).  median_3: the

@@ -316,38 +316,34 @@ __global__ void __launch_bounds__(256) stationary_kernel(const double *Q, int S,
 // FP64 and, if P32 is given, an FP32 copy.  t == -1 (compose only) gives Q;
 // t < 1e-10 gives I.
 struct ComposeArgs {
-  const double *U, *lam, *Ui;   // model 0; model m at m*S*S, m*S, m*S*S
+  const double *U, *lam, *Ui;
   const double *t;              // [n_br]
-  const double *rates;          // [R] or null (rate 1); model m at m*R
+  const double *rates;          // [R] or null (rate 1)
   double *P;                    // [n_br][R][S][S] or null
   float *P32;                   // [n_br][R][S][S] or null
   int S, R;
   int n_br;
   int allow_q;                  // t == -1 returns Q (the reference's compose)
-  const int *status;            // eigendecomposition status or null; model m at m
+  const int *status;            // eigendecomposition status or null
   int *flag;
   int p32_mode;                 // P32Mode
-  size_t model_bytes;           // byte stride of P and P32 between models
 };
 
 __global__ void __launch_bounds__(256) compose_kernel(const ComposeArgs p) {
   extern __shared__ __align__(16) double sm[];
   const int S = p.S, R = p.R, SS = S * S;
   double *U = sm, *Ui = U + SS, *e = Ui + SS;   // e: [R][S]
-  const int b = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
-  const int *status = p.status ? p.status + m : nullptr;
-  if (status && *status) {
-    if (b == 0 && tid == 0) atomicOr(p.flag, pgpu_model_flag(*status));
+  const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  if (p.status && *p.status) {
+    if (b == 0 && tid == 0) atomicOr(p.flag, pgpu_model_flag(*p.status));
     return;
   }
-  const double *gU = p.U + (size_t)m * SS, *gUi = p.Ui + (size_t)m * SS;
-  const double *lam = p.lam + (size_t)m * S;
-  const double *rates = p.rates ? p.rates + (size_t)m * R : nullptr;
-  double *P = p.P ? (double *)((char *)p.P + m * p.model_bytes) : nullptr;
-  float *P32 = p.P32 ? (float *)((char *)p.P32 + m * p.model_bytes) : nullptr;
+  const double *lam = p.lam, *rates = p.rates;
+  double *P = p.P;
+  float *P32 = p.P32;
   for (int i = tid; i < SS; i += nt) {
-    U[i] = gU[i];
-    Ui[i] = gUi[i];
+    U[i] = p.U[i];
+    Ui[i] = p.Ui[i];
   }
   const double t = p.t[b];
   const bool q_mode = p.allow_q && t == -1.0;
@@ -388,31 +384,29 @@ __global__ void __launch_bounds__(256) compose_kernel(const ComposeArgs p) {
 
 // Tip rows: tab[t][r][c][i] = sum_j P(t, r)[i][j] * code_tab[c][j] for every
 // tip t (the branch above it), rate r and tip code c, formed in FP64 from the
-// eigen system and stored as float, float pair (hi, lo) or double.  A tip
+// eigen system and stored as float, float pair or double.  A tip
 // child then costs the pruning kernel one table read instead of a
 // matrix-vector product.
 struct TipTabArgs {
-  const double *U, *lam, *Ui;   // model 0; model m at m*S*S, m*S, m*S*S
+  const double *U, *lam, *Ui;
   const double *t;          // [n_tips] branch lengths above the tips
-  const double *rates;      // [R]; model m at m*R
+  const double *rates;      // [R]
   const double *code_tab;   // [n_codes][S]
   void *out;
-  int S, R, n_codes, form;  // form: 0 float, 1 float pair, 2 double, 3 float pairs element pairs first (S = 4)
-  const int *status;        // model m at m
-  size_t model_bytes;       // byte stride of out between models
+  int S, R, n_codes, form;  // form: 0 float, 2 double, 3 float pairs, element pairs first (S = 4)
+  const int *status;
 };
 
-// One CTA per tip, rate (blockIdx.y) and model (blockIdx.z).
+// One CTA per tip and rate (blockIdx.y).
 __global__ void __launch_bounds__(128) tip_table_kernel(const TipTabArgs p) {
   extern __shared__ __align__(16) double sm[];
   const int S = p.S, SS = S * S;
   double *P = sm;   // [S][S]
-  const int tip = blockIdx.x, r = blockIdx.y, m = blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
-  if (p.status && p.status[m]) return;
-  const double *U = p.U + (size_t)m * SS, *Ui = p.Ui + (size_t)m * SS;
-  const double *lam = p.lam + (size_t)m * S;
-  char *out = static_cast<char *>(p.out) + m * p.model_bytes;
-  const double tt = p.t[tip], rate = p.rates ? p.rates[(size_t)m * p.R + r] : 1.0;
+  const int tip = blockIdx.x, r = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  if (p.status && *p.status) return;
+  const double *U = p.U, *Ui = p.Ui, *lam = p.lam;
+  char *out = static_cast<char *>(p.out);
+  const double tt = p.t[tip], rate = p.rates ? p.rates[r] : 1.0;
   const bool ident = !(tt * rate >= 1e-10);   // effective time, as in compose_kernel
   for (int o = tid; o < SS; o += nt) {
     const int i = o / S, j = o % S;
@@ -439,10 +433,6 @@ __global__ void __launch_bounds__(128) tip_table_kernel(const TipTabArgs p) {
       q[2] = (float)(v - (double)hi);
     } else if (p.form == 0) {
       reinterpret_cast<float *>(out)[at] = (float)v;
-    } else if (p.form == 1) {
-      const float hi = (float)v;
-      reinterpret_cast<float *>(out)[2 * at] = hi;
-      reinterpret_cast<float *>(out)[2 * at + 1] = (float)(v - (double)hi);
     } else {
       reinterpret_cast<double *>(out)[at] = v;
     }
@@ -558,42 +548,34 @@ pgpu_status pgpu_launch_eig(pgpu_ctx *ctx, const double *Q_dev, const double *pi
 pgpu_status pgpu_launch_compose(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
                                 const double *Ui_dev, int S, const double *t_dev, int n_br,
                                 const double *rates_dev, int R, double *P_dev, float *P32_dev,
-                                bool allow_q, const int *status_dev, int p32_mode, int n_models,
-                                size_t model_bytes) {
-  if (n_br <= 0 || n_models <= 0) return PGPU_OK;
+                                bool allow_q, const int *status_dev, int p32_mode) {
+  if (n_br <= 0) return PGPU_OK;
   if (p32_mode == P32_PAIRS_ROWS4 && S != 4)
     return pgpu_set_err(ctx, PGPU_ERR_ARG, "compose: the row-pair layout is for 4 states (got %d)", S);
-  if (n_models > 65535)
-    return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "compose: %d models in one launch; at most 65535",
-                        n_models);
   ComposeArgs a{U_dev, lam_dev, Ui_dev, t_dev,       rates_dev,  P_dev,       P32_dev,
                 S,     R,       n_br,   allow_q ? 1 : 0, status_dev, ctx->d_flag,
-                p32_mode, model_bytes};
+                p32_mode};
   const size_t smem = sizeof(double) * (2 * (size_t)S * S + (size_t)R * S);
   PGPU_CUDA(ctx, cudaFuncSetAttribute(compose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)std::max<size_t>(smem, 1024)));
   const int threads = R * S * S <= 64 ? 64 : (R * S * S <= 128 ? 128 : 256);
-  compose_kernel<<<dim3(n_br, n_models), threads, smem, ctx->stream>>>(a);
+  compose_kernel<<<n_br, threads, smem, ctx->stream>>>(a);
   return pgpu_after_launch(ctx, "compose_kernel");
 }
 
 pgpu_status pgpu_launch_tip_table(pgpu_ctx *ctx, const double *U_dev, const double *lam_dev,
                                   const double *Ui_dev, int S, const double *t_dev, int n_tips,
                                   const double *rates_dev, int R, const double *code_tab_dev,
-                                  int n_codes, void *out_dev, int form, const int *status_dev,
-                                  int n_models, size_t model_bytes) {
-  if (n_tips <= 0 || n_models <= 0) return PGPU_OK;
+                                  int n_codes, void *out_dev, int form, const int *status_dev) {
+  if (n_tips <= 0) return PGPU_OK;
   if (form == 3 && S != 4)
     return pgpu_set_err(ctx, PGPU_ERR_ARG, "tip table: the element-pair layout is for 4 states (got %d)", S);
-  if (n_models > 65535)
-    return pgpu_set_err(ctx, PGPU_ERR_LIMIT, "tip table: %d models in one launch; at most 65535",
-                        n_models);
   TipTabArgs a{U_dev, lam_dev, Ui_dev, t_dev, rates_dev, code_tab_dev, out_dev, S, R, n_codes, form,
-               status_dev, model_bytes};
+               status_dev};
   const size_t smem = sizeof(double) * (size_t)S * S;
   PGPU_CUDA(ctx, cudaFuncSetAttribute(tip_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)std::max<size_t>(smem, 1024)));
-  tip_table_kernel<<<dim3(n_tips, R, n_models), 128, smem, ctx->stream>>>(a);
+  tip_table_kernel<<<dim3(n_tips, R), 128, smem, ctx->stream>>>(a);
   return pgpu_after_launch(ctx, "tip_table_kernel");
 }
 

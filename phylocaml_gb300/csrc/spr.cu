@@ -27,7 +27,7 @@
 // message on a stack in shared memory, so the stack holds at most
 // log2(n) + 1 entries.  Site log-likelihoods are weighted and summed as
 // float pairs per warp, per CTA in warp order, then per move over the CTA
-// groups in FP64 (spr_reduce_kernel), which fixes the summation order.
+// groups in three floats (spr_reduce_kernel), which fixes the summation order.
 //
 // The Fitch part (spr_fitch_*_kernel) runs the same programs on state sets
 // (32 patterns to a word, a word per state): the parsimony length of every neighbour, exactly.

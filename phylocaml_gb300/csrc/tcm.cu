@@ -524,7 +524,7 @@ pgpu_status tree_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
 
 pgpu_status tree_wide_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips, size_t ld,
                           const uint32_t *weights, size_t n_sites, int lb, const int32_t *tcm,
-                          int S, int mode, int symmetric, uint32_t *node_sets, uint32_t *site_cost,
+                          int S, int mode, uint32_t *node_sets, uint32_t *site_cost,
                           unsigned long long *total) {
   if (!tree || tree->n_tips < 2)
     return pgpu_set_err(ctx, PGPU_ERR_ARG, "tcm_tree_wide: need at least 2 tips");
@@ -640,18 +640,18 @@ pgpu_status pgpu_tcm_median(const int32_t *tcm, int n_states, int mode, int symm
 pgpu_status pgpu_tcm_tree_wide_dev(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips_dev,
                                    size_t ld_words, const uint32_t *weights_dev, size_t n_sites,
                                    int lane_bits, const int32_t *tcm, int n_states, int mode,
-                                   int symmetric, uint32_t *node_sets_dev, uint32_t *site_cost_dev,
+                                   int /*symmetric*/, uint32_t *node_sets_dev, uint32_t *site_cost_dev,
                                    uint64_t *total_dev) {
   if (!ctx) return PGPU_ERR_ARG;
   PGPU_CUDA(ctx, cudaSetDevice(ctx->device));
   return tree_wide_dev(ctx, tree, tips_dev, ld_words, weights_dev, n_sites, lane_bits, tcm, n_states,
-                       mode, symmetric, node_sets_dev, site_cost_dev,
+                       mode, node_sets_dev, site_cost_dev,
                        reinterpret_cast<unsigned long long *>(total_dev));
 }
 
 pgpu_status pgpu_tcm_tree_wide(pgpu_ctx *ctx, const pgpu_tree *tree, const uint32_t *tips,
                                const uint32_t *weights, size_t n_sites, int lane_bits,
-                               const int32_t *tcm, int n_states, int mode, int symmetric,
+                               const int32_t *tcm, int n_states, int mode, int /*symmetric*/,
                                uint32_t *node_sets, uint32_t *site_cost, uint64_t *total) {
   if (!ctx) return PGPU_ERR_ARG;
   if (!tree || !tips || !node_sets || !total || !tcm)
@@ -677,7 +677,7 @@ pgpu_status pgpu_tcm_tree_wide(pgpu_ctx *ctx, const pgpu_tree *tree, const uint3
     if (weights) PGPU_CUDA(ctx, cudaMemcpyAsync(dw, weights, n_sites * 4, cudaMemcpyHostToDevice, s));
   }
   PGPU_TRY(tree_wide_dev(ctx, tree, (const uint32_t *)dt, ld, (const uint32_t *)dw, n_sites,
-                         lane_bits, tcm, n_states, mode, symmetric, (uint32_t *)dn, (uint32_t *)dsc,
+                         lane_bits, tcm, n_states, mode, (uint32_t *)dn, (uint32_t *)dsc,
                          (unsigned long long *)dtot));
   if (n_words) {
     PGPU_CUDA(ctx, cudaMemcpy2DAsync(node_sets, n_words * 4, dn, ld * 4, n_words * 4, n_int,

@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(CLV_THREADS) clv_median_kernel(const MedArgs a
 
 // The same for four states.  The next item's reads in flight while one is
 // computed, P and the leaves' rows by code in shared memory.
-// 100,003 patterns, 4 classes, float: 6.3 us a median over a 128-taxon tree (18
-// at 446,427) against 14.4 us with vectors for leaves, P read per item and one
+// 100,003 patterns, 4 classes, float: 6.1 us a median over a 128-taxon tree (18
+// at 446,427; 23 with internal neighbours only, more of them than L2 holds) against 14.4 us with vectors for leaves, P read per item and one
 // item in flight; P in registers spills at 4 CTAs per SM (8.0 us), and at 2
 // or 3 CTAs too few reads are in flight (8.3, 7.4).
 template <typename V, int NCH>

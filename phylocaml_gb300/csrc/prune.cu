@@ -282,11 +282,11 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
 // the pair form): a warp's gather touches 8 lines.  With a warp per class it
 // touched up to 32, and the line lookups bounded the kernel.
 //
-// Bound by the float-pair arithmetic of the rows and products (FMA pipe).
 // 512 taxa x 446,427 patterns, 4 rate classes, pair form: 3.83 ms with
 // the collapsed subtrees (about half the steps), 7.12 ms walking every node
-// with the tip rows staged per step by the producer; issue slots 57 %, FMA
-// pipe 50 %.
+// with the tip rows staged per step by the producer.  Issue slots 57 % busy,
+// FMA pipe 50 %; the first stall is the wait for gathered leaf rows (2.8 of
+// 10 an instruction), then the pair arithmetic's own chains.
 template <typename Pol, int RT>
 __global__ void __launch_bounds__(32 + PR_THREADS, PruneTune<Pol>::min_ctas)
     prune_tree_kernel(const PruneArgs p) {

@@ -54,7 +54,7 @@ namespace {
 // Threads of a pool or scan CTA: the kernels hold 64 to 128 registers a thread,
 // so that small CTAs fill an SM better and wait less for one another (256
 // taxa x 45,675 patterns: pool 2.61 ms against 2.91 with 256 threads; the scan
-// of 128 taxa x 16,852: 72.2 against 74.2).
+// of 128 taxa x 16,852: 72.2 against 74.2 when it was chosen).
 constexpr int SPR_NT = 128;
 // What an engine accepts is reckoned in blocks of this many threads.
 constexpr int SPR_LIMIT_NT = 256;
@@ -414,7 +414,7 @@ __device__ __forceinline__ typename Pol::V site_part(const typename Pol::V *h, c
 // first move's sum and the odd ones with the second's, and one logarithm and
 // one sum over the patterns serve both.  The warps' values meet every
 // SCAN_WIN moves.  128 taxa x 16,852 patterns, pair form, 63,000 moves:
-// 71.8 ms against 141.8 with none of this.
+// 72.3 ms against 141.8 with none of this.
 template <typename Pol, int RT, bool EMIT = false>
 __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
   using V = typename Pol::V;
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(SPR_NT, 4) spr_scan_kernel(const ScanArgs a) {
   for (int i = c; i < 64; i += NT) ltab[i] = a.logtab[i];
   __syncthreads();
   // the pair form takes these ready: converting them from FP64 in every thread
-  // cost 0.4 ms of the 63,000 moves' 72.2
+  // cost 0.4 ms of the 63,000 moves' 72
   auto constant = [&](int k, const double *d) {
     if constexpr (std::is_same<Pol, Ff32>::value) {
       const float2 v = __ldg(a.pairs + k);

@@ -1264,13 +1264,20 @@ struct BlArgs {
 // S[e][pat][r][k] = (sum_i pi_i L[a|b]_i U_ik) (sum_j Ui_kj L[b|a]_j), so that
 // the site likelihood across edge e is sum_r probs_r sum_k S_k exp(lam_k rate_r t)
 template <typename Pol>
-__device__ __forceinline__ float eigen_product(const BlArgs &a, const typename Pol::V *x, const typename Pol::V *y,
-                                               int k) {
+__device__ __forceinline__ void eigen_values(const BlArgs &a, const typename Pol::V *x, const typename Pol::V *y,
+                                             double *xd, double *yd) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    xd[j] = a.pi[j] * Pol::to_d(x[j]);
+    yd[j] = Pol::to_d(y[j]);
+  }
+}
+__device__ __forceinline__ float eigen_product(const BlArgs &a, const double *x, const double *y, int k) {
   double A = 0.0, B = 0.0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    A += a.pi[j] * Pol::to_d(x[j]) * a.U[j * 4 + k];
-    B += a.Ui[k * 4 + j] * Pol::to_d(y[j]);
+    A = fma(x[j], a.U[j * 4 + k], A);
+    B = fma(a.Ui[k * 4 + j], y[j], B);
   }
   return (float)(A * B);
 }
@@ -1284,9 +1291,11 @@ __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
   V x[4], y[4];
   Pol::load_g(a.L, (size_t)(2 * e) * a.np * a.R + i, x);
   Pol::load_g(a.L, (size_t)(2 * e + 1) * a.np * a.R + i, y);
+  double xd[4], yd[4];
+  eigen_values<Pol>(a, x, y, xd, yd);
   float s[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) s[k] = eigen_product<Pol>(a, x, y, k);
+  for (int k = 0; k < 4; ++k) s[k] = eigen_product(a, xd, yd, k);
   reinterpret_cast<float4 *>(a.S)[(size_t)e * a.np * a.R + i] = make_float4(s[0], s[1], s[2], s[3]);
 }
 
@@ -1295,10 +1304,11 @@ __global__ void __launch_bounds__(256) bl_sumtab_kernel(const BlArgs a) {
 // (TwoSum) in pairs, two eigenvectors to a packed float2 instruction.  S is
 // the float that FP64 gives: where the pairs' error leaves two candidates
 // (Ziv's rounding test with EIGEN_ERR) the value is formed again in FP64: the
-// Newton steps' float exponentials turn a last bit here into 3e-7 of a length.
-// Below 2^-60 of the terms, less than FP64's own rounding of them, it is left
-// as it is (sums that cancel to nothing: 2.47 ms with those formed again as
-// well).
+// Newton steps' float exponentials turn a last bit here into 3e-7 of a length,
+// and where a whole edge is flat the rounding of sums that cancel is all there
+// is to step on.  Nearly all such sums are a missing tip's (1, 1, 1, 1), for
+// which FP64's own are formed once per CTA (2.25 ms with each of them formed
+// again).
 //
 // The error of a sum, with u = 2^-24 and T the sum of the terms' sizes: each
 // product leaves out its low parts' product and the coefficient's own rest
@@ -1347,14 +1357,29 @@ __device__ __forceinline__ void eigen_pair(const float4 (*c)[2], int kp, const f
   two_sum2(s, lo, sum, err);
 }
 
+__device__ __forceinline__ void take_sum(float4 q, float2 &sum, float2 &err, float2 &mag) {
+  sum = make_float2(q.x, q.y);
+  err = make_float2(q.z, q.w);
+  mag = make_float2(fabsf(q.x), fabsf(q.y));
+}
+
 template <typename Pol>
 __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
   using V = typename Pol::V;
   __shared__ float4 cA[4][2], cB[4][2];   // [j][eigenvector pair]
+  __shared__ float4 ones[2][2];           // FP64's sums of a missing tip's vector, as pairs: [side][eigenvector pair]
   if (threadIdx.x < 32) {
     const int side = threadIdx.x >> 4, j = (threadIdx.x >> 2) & 3, k = threadIdx.x & 3;
     const double v = side == 0 ? a.pi[j] * a.U[j * 4 + k] : a.Ui[k * 4 + j];
     float *dst = reinterpret_cast<float *>(side == 0 ? &cA[j][k >> 1] : &cB[j][k >> 1]) + (k & 1);
+    const float h = (float)v;
+    dst[0] = h;
+    dst[2] = (float)(v - (double)h);
+  } else if (threadIdx.x < 40) {
+    const int side = (threadIdx.x >> 2) & 1, k = threadIdx.x & 3;
+    double v = 0.0;   // as eigen_product sums the vector 1, 1, 1, 1
+    for (int j = 0; j < 4; ++j) v = side == 0 ? fma(a.pi[j], a.U[j * 4 + k], v) : fma(a.Ui[k * 4 + j], 1.0, v);
+    float *dst = reinterpret_cast<float *>(&ones[side][k >> 1]) + (k & 1);
     const float h = (float)v;
     dst[0] = h;
     dst[2] = (float)(v - (double)h);
@@ -1374,6 +1399,12 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
     x[j] = fast_two_sum(x[j].h, x[j].l);
     y[j] = fast_two_sum(y[j].h, y[j].l);
   }
+  bool x_ones = true, y_ones = true;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    x_ones = x_ones && x[j].h == 1.0f && x[j].l == 0.0f;
+    y_ones = y_ones && y[j].h == 1.0f && y[j].l == 0.0f;
+  }
   float s[4];
   int unsure = 0;
 #pragma unroll
@@ -1381,25 +1412,28 @@ __global__ void __launch_bounds__(256) bl_sumtab_pair_kernel(const BlArgs a) {
     float2 ah, al, am, bh, bl, bm;
     eigen_pair(cA, kp, x, ah, al, am);
     eigen_pair(cB, kp, y, bh, bl, bm);
+    if (x_ones) take_sum(ones[0][kp], ah, al, am);
+    if (y_ones) take_sum(ones[1][kp], bh, bl, bm);
     const float2 p = __fmul2_rn(ah, bh);
     float2 er = __ffma2_rn(ah, bh, neg2(p));
     er = __ffma2_rn(ah, bl, er);
     er = __ffma2_rn(al, bh, er);
     const float2 v = __fadd2_rn(p, er), rest = sub2(er, sub2(v, p));
-    const float2 all = __fmul2_rn(am, bm);
     const float2 d = __fmul2_rn(make_float2(EIGEN_ERR, EIGEN_ERR),
                                 make_float2(fmaf(fabsf(ah.x), bm.x, fabsf(bh.x) * am.x),
                                             fmaf(fabsf(ah.y), bm.y, fabsf(bh.y) * am.y)));
     const float2 up = __fadd2_rn(v, __fadd2_rn(rest, d)), down = __fadd2_rn(v, sub2(rest, d));
     s[2 * kp] = v.x;
     s[2 * kp + 1] = v.y;
-    if (!(up.x == down.x) && !(fabsf(v.x) < 0x1p-60f * all.x)) unsure |= 1 << (2 * kp);
-    if (!(up.y == down.y) && !(fabsf(v.y) < 0x1p-60f * all.y)) unsure |= 2 << (2 * kp);
+    if (!(up.x == down.x)) unsure |= 1 << (2 * kp);
+    if (!(up.y == down.y)) unsure |= 2 << (2 * kp);
   }
   if (unsure) {
+    double xd[4], yd[4];
+    eigen_values<Pol>(a, xv, yv, xd, yd);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (unsure >> k & 1) s[k] = eigen_product<Pol>(a, xv, yv, k);
+      if (unsure >> k & 1) s[k] = eigen_product(a, xd, yd, k);
   }
   reinterpret_cast<float4 *>(a.S)[(size_t)e * a.np * a.R + i] = make_float4(s[0], s[1], s[2], s[3]);
 }
